@@ -644,13 +644,19 @@ __global__ void embedding_bwd_kernel(const long* __restrict__ sorted_tok, const 
 
 // --------------------------------------------------------------------------- AdamW
 // Multi-tensor: one launch updates up to ADAM_MAX tensors (a whole layer). dtype codes: 0 bf16, 1 fp32.
+// Bound by memory: 22 bytes an element with bf16 weights and gradients and fp32 state (14 with bf16 state), each read
+// and written once.  A thread takes 8 neighbouring elements, all of whose 16-byte loads are issued before the first
+// use; the types are template arguments, chosen once per block (a block lies in one tensor).
+// 218 M bf16 weights and gradients: fp32 state 931 us (5.2 TB/s) with one element a load, 691 us (6.9 TB/s) so; bf16
+// state 741 us (4.1 TB/s) before, 441 us (6.9 TB/s) now.
 constexpr int ADAM_MAX = 24;
 struct AdamTensor {
   void* p; const void* g; void* m; void* v;
   long n;
   long block_start;  // first block of this tensor in the flattened grid
   float lr, wd;
-  int p_dt, g_dt, s_dt, pad;
+  int p_dt, g_dt, s_dt;
+  int vec;           // all four pointers on 16 bytes: whole groups of 8 elements go as vectors
 };
 struct AdamArgs {
   AdamTensor t[ADAM_MAX];
@@ -668,6 +674,61 @@ __device__ __forceinline__ void st_any(void* p, long i, int dt, float v) {
   else reinterpret_cast<bf16*>(p)[i] = __float2bfloat16(v);
 }
 
+// Eight elements as they lie in memory: one 16-byte word of bf16, two of fp32.
+template <bool F32> struct Raw8 { uint4 w[F32 ? 2 : 1]; };
+template <bool F32>
+__device__ __forceinline__ Raw8<F32> ld_raw8(const void* p, long i) {
+  Raw8<F32> r;
+  const uint4* q = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(p) + i * (F32 ? 4 : 2));
+#pragma unroll
+  for (int k = 0; k < (F32 ? 2 : 1); ++k) r.w[k] = __ldcs(q + k);
+  return r;
+}
+template <bool F32>
+__device__ __forceinline__ void unpack_raw8(const Raw8<F32>& r, float (&f)[8]) {
+  if constexpr (F32) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      f[4 * k] = __uint_as_float(r.w[k].x); f[4 * k + 1] = __uint_as_float(r.w[k].y);
+      f[4 * k + 2] = __uint_as_float(r.w[k].z); f[4 * k + 3] = __uint_as_float(r.w[k].w);
+    }
+  } else {
+    unpack8(r.w[0], f);
+  }
+}
+template <bool F32>
+__device__ __forceinline__ void st_raw8(void* p, long i, const float (&f)[8]) {
+  uint4* q = reinterpret_cast<uint4*>(reinterpret_cast<char*>(p) + i * (F32 ? 4 : 2));
+  if constexpr (F32) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      __stcs(q + k, make_uint4(__float_as_uint(f[4 * k]), __float_as_uint(f[4 * k + 1]),
+                               __float_as_uint(f[4 * k + 2]), __float_as_uint(f[4 * k + 3])));
+  } else {
+    __stcs(q, pack8(f));
+  }
+}
+
+__device__ __forceinline__ void adamw_one(const AdamArgs& a, float lr, float wd, float g, float& p, float& m, float& v) {
+  g *= a.grad_scale;
+  p -= lr * wd * p;
+  m = a.beta1 * m + (1.f - a.beta1) * g;
+  v = a.beta2 * v + (1.f - a.beta2) * g * g;
+  p -= lr * (m / a.bc1) / (sqrtf(v / a.bc2) + a.eps);
+}
+
+template <bool PF, bool GF, bool SF>
+__device__ __forceinline__ void adamw_vec8(const AdamArgs& a, const AdamTensor& t, long i) {
+  const Raw8<PF> rp = ld_raw8<PF>(t.p, i);
+  const Raw8<GF> rg = ld_raw8<GF>(t.g, i);
+  const Raw8<SF> rm = ld_raw8<SF>(t.m, i), rv = ld_raw8<SF>(t.v, i);
+  float p[8], g[8], m[8], v[8];
+  unpack_raw8<PF>(rp, p); unpack_raw8<GF>(rg, g); unpack_raw8<SF>(rm, m); unpack_raw8<SF>(rv, v);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) adamw_one(a, t.lr, t.wd, g[j], p[j], m[j], v[j]);
+  st_raw8<PF>(t.p, i, p); st_raw8<SF>(t.m, i, m); st_raw8<SF>(t.v, i, v);
+}
+
 __global__ void __launch_bounds__(ADAM_THREADS) adamw_kernel(const __grid_constant__ AdamArgs a) {
   int ti = 0;
 #pragma unroll 1
@@ -675,21 +736,27 @@ __global__ void __launch_bounds__(ADAM_THREADS) adamw_kernel(const __grid_consta
     if ((long)blockIdx.x >= a.t[i].block_start) ti = i;
   const AdamTensor& t = a.t[ti];
   const long base = ((long)blockIdx.x - t.block_start) * ADAM_PER_BLOCK;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const long i = base + threadIdx.x + (long)j * ADAM_THREADS;
-    if (i < t.n) {
-      float p = ld_any(t.p, i, t.p_dt);
-      const float g = ld_any(t.g, i, t.g_dt) * a.grad_scale;
-      float m = ld_any(t.m, i, t.s_dt), v = ld_any(t.v, i, t.s_dt);
-      p -= t.lr * t.wd * p;
-      m = a.beta1 * m + (1.f - a.beta1) * g;
-      v = a.beta2 * v + (1.f - a.beta2) * g * g;
-      p -= t.lr * (m / a.bc1) / (sqrtf(v / a.bc2) + a.eps);
-      st_any(t.p, i, t.p_dt, p);
-      st_any(t.m, i, t.s_dt, m);
-      st_any(t.v, i, t.s_dt, v);
+  const long i0 = base + (long)threadIdx.x * 8;
+  if (t.vec && i0 + 8 <= t.n) {
+    switch (t.p_dt * 4 + t.g_dt * 2 + t.s_dt) {
+      case 0: adamw_vec8<false, false, false>(a, t, i0); break;
+      case 1: adamw_vec8<false, false, true>(a, t, i0); break;
+      case 2: adamw_vec8<false, true, false>(a, t, i0); break;
+      case 3: adamw_vec8<false, true, true>(a, t, i0); break;
+      case 4: adamw_vec8<true, false, false>(a, t, i0); break;
+      case 5: adamw_vec8<true, false, true>(a, t, i0); break;
+      case 6: adamw_vec8<true, true, false>(a, t, i0); break;
+      default: adamw_vec8<true, true, true>(a, t, i0); break;
     }
+    return;
+  }
+#pragma unroll 1
+  for (long i = i0; i < i0 + 8 && i < t.n; ++i) {       // the last, incomplete group; tensors off the 16-byte grid
+    float p = ld_any(t.p, i, t.p_dt), m = ld_any(t.m, i, t.s_dt), v = ld_any(t.v, i, t.s_dt);
+    adamw_one(a, t.lr, t.wd, ld_any(t.g, i, t.g_dt), p, m, v);
+    st_any(t.p, i, t.p_dt, p);
+    st_any(t.m, i, t.s_dt, m);
+    st_any(t.v, i, t.s_dt, v);
   }
 }
 
@@ -984,7 +1051,8 @@ int ftb_adamw_multi(int count, void** p, const void** g, void** m, void** v, con
     a.t[i].p = p[i]; a.t[i].g = g[i]; a.t[i].m = m[i]; a.t[i].v = v[i];
     a.t[i].n = n[i]; a.t[i].block_start = blocks;
     a.t[i].lr = lr[i]; a.t[i].wd = wd[i];
-    a.t[i].p_dt = p_dt[i]; a.t[i].g_dt = g_dt[i]; a.t[i].s_dt = s_dt[i]; a.t[i].pad = 0;
+    a.t[i].p_dt = p_dt[i]; a.t[i].g_dt = g_dt[i]; a.t[i].s_dt = s_dt[i];
+    a.t[i].vec = (((uintptr_t)p[i] | (uintptr_t)g[i] | (uintptr_t)m[i] | (uintptr_t)v[i]) & 15) == 0;
     blocks += (n[i] + ADAM_PER_BLOCK - 1) / ADAM_PER_BLOCK;
   }
   a.count = count; a.beta1 = beta1; a.beta2 = beta2; a.eps = eps; a.bc1 = bc1; a.bc2 = bc2; a.grad_scale = grad_scale;

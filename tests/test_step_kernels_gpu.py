@@ -1,0 +1,42 @@
+"""Kernels of the optimizer step against the plain PyTorch reference, at the sizes where the vector paths end."""
+
+import itertools
+
+import pytest
+import torch
+
+from flextrain_b200 import ops
+from flextrain_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+BF16, F32 = torch.bfloat16, torch.float32
+
+
+@pytest.mark.parametrize("pdt,gdt,sdt", list(itertools.product((BF16, F32), repeat=3)))
+@pytest.mark.parametrize("shift", [0, 1, 8])
+def test_adamw_types_tails_and_alignment(pdt, gdt, sdt, shift):
+    """Every type combination, lengths around a group of 8 and around a block of 2048, and tensors that start off the
+    16-byte grid (``shift`` elements into their buffer): update and state as in the fp32 reference.  The momentum has
+    the gradient's sign, so nothing cancels but the weight against its update: the fp32 values before the last rounding
+    differ by some ten roundings of 2^-24, of the weight and of the update, and by 1 - 0.95 in fp32 (2^-22 off); a bf16
+    result may then round to the neighbouring value.
+    """
+    torch.manual_seed(0)
+    sizes = (1, 7, 8, 9, 2040, 2047, 2048, 2049, 5003)
+    mk = lambda n, dt, f: f(torch.randn(n + shift, device=DEV)).to(dt)[shift:]
+    same = lambda t: t
+    P, G = [mk(n, pdt, same) for n in sizes], [mk(n, gdt, same) for n in sizes]
+    M = [(mk(n, F32, torch.abs) * g.float().sign()).to(sdt) for n, g in zip(sizes, G)]
+    M = [torch.cat([m.new_zeros(shift), m])[shift:] for m in M]
+    V = [mk(n, sdt, torch.square) for n in sizes]
+    before = [p.clone() for p in P]
+    want = [[t.clone() for t in ts] for ts in (P, M, V)]
+    kw = dict(beta1=0.9, beta2=0.95, eps=1e-8, step=3, grad_scale=0.5)
+    ops.adamw_multi(P, G, M, V, lrs=[1e-2] * len(sizes), wds=[0.1] * len(sizes), **kw)
+    for p, g, m, v in zip(want[0], G, want[1], want[2]):
+        ref.adamw_step(p, g, m, v, lr=1e-2, weight_decay=0.1, **kw)
+    for got, new, old, dt in ((P, want[0], before, pdt), (M, want[1], want[1], sdt), (V, want[2], want[2], sdt)):
+        for a, b, o in zip(got, new, old):
+            room = 2.0 ** -20 * (b.float().abs() + o.float().abs()) + (2.0 ** -7 * b.float().abs() if dt == BF16 else 0)
+            assert torch.all((a.float() - b.float()).abs() <= room)
