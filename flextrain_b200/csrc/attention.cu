@@ -13,11 +13,9 @@
 //
 // Backward, one CTA per (128-key tile, KV head): loops over the query heads of the group and over the query
 // tiles that see these keys; five MMAs per pair (S, dP, dV += Pᵀ·dO, dK += dSᵀ·Q, dQ += dS·K); dK / dV accumulate
-// in TMEM across the loop (deterministic).  dQ goes into an fp32 workspace with vector reductions (red.v4.f32) issued
-// straight from the registers that hold the tile.  In deterministic mode the CTAs that add to the same (query tile,
-// head) take turns in DEscending key-tile order through a counter (the CTA of key tile j adds once the j_hi - j tiles
-// above it have added; those reach the query tile earlier in their own loops, so the wait is normally already
-// satisfied), which fixes the summation order and makes dQ bit-reproducible.
+// in TMEM across the loop (deterministic).  dQ goes into an fp32 workspace as tiled reduce-adds.  In deterministic mode
+// the CTAs that add to the same (query tile, head) take turns in a fixed order of key tiles through a counter, which fixes
+// the summation order and makes dQ bit-reproducible; the wait is normally already satisfied (see BWD_* for the orders).
 #include "ptx.cuh"
 
 namespace ftb {
@@ -46,19 +44,39 @@ __device__ __forceinline__ float tanh_fast(float x) {
   return y;
 }
 
-__device__ __forceinline__ bool find_tile(const int* cu_q, int num_seqs, int tile, int& seq, int& q0) {
+// Sequence and first row of the `tile`-th tile when every sequence is cut into tiles of `unit` rows.  A whole warp looks
+// at 32 sequences at a time (one load and a prefix sum): walking hundreds of short sequences one by one, each step waiting
+// for its load, took longer than the tile itself.  Called by full warps; every lane gets the same answer.
+__device__ __forceinline__ bool find_tile(const int* cu, int num_seqs, int tile, int unit, int& seq, int& row0) {
+  const int lane = threadIdx.x & 31;
   int acc = 0;
-  for (int s = 0; s < num_seqs; ++s) {
-    const int len = cu_q[s + 1] - cu_q[s];
-    const int nt = (len + TQ - 1) / TQ;
-    if (tile < acc + nt) {
-      seq = s;
-      q0 = (tile - acc) * TQ;
+  for (int s0 = 0; s0 < num_seqs; s0 += 32) {
+    const int s = s0 + lane;
+    const int nt = s < num_seqs ? (cu[s + 1] - cu[s] + unit - 1) / unit : 0;
+    int upto = nt;                                   // tiles of this group's sequences up to and including the lane's
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const unsigned past = __ballot_sync(0xffffffffu, tile < acc + upto);
+    if (past != 0) {
+      const int src = __ffs(past) - 1;
+      seq = s0 + src;
+      row0 = (tile - acc - __shfl_sync(0xffffffffu, upto - nt, src)) * unit;
       return true;
     }
-    acc += nt;
+    acc += __shfl_sync(0xffffffffu, upto, 31);
   }
   return false;
+}
+// Tiles of the first `count` sequences (same warp-wide form).
+__device__ __forceinline__ int tiles_before(const int* cu, int count, int unit) {
+  int n = 0;
+  for (int s = threadIdx.x & 31; s < count; s += 32) n += (cu[s + 1] - cu[s] + unit - 1) / unit;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+  return n;
 }
 
 // Byte offset of element (row, col) inside a K-major 128B-swizzled tile made of 64-column blocks of `rows` rows.
@@ -100,7 +118,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   const int head = blockIdx.y;
   const int kvh = head / (p.H / p.KV);
   int seq = 0, q0 = 0;
-  const bool live = find_tile(p.cu_q, p.num_seqs, blockIdx.x, seq, q0);
+  const bool live = find_tile(p.cu_q, p.num_seqs, blockIdx.x, TQ, seq, q0);
   if (!live) return;   // uniform for the CTA: nothing allocated yet
   const int qs = p.cu_q[seq], len_q = p.cu_q[seq + 1] - qs;
   const int ks = p.cu_k[seq], len_k = p.cu_k[seq + 1] - ks;
@@ -353,21 +371,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 constexpr int FA2_THREADS = 320;
 constexpr float FA2_RESCALE_LOG2 = 8.0f;
 
-__device__ __forceinline__ bool find_tile2(const int* cu_q, int num_seqs, int tile, int& seq, int& q0) {
-  int acc = 0;
-  for (int s = 0; s < num_seqs; ++s) {
-    const int len = cu_q[s + 1] - cu_q[s];
-    const int nt = (len + 2 * TQ - 1) / (2 * TQ);
-    if (tile < acc + nt) {
-      seq = s;
-      q0 = (tile - acc) * 2 * TQ;
-      return true;
-    }
-    acc += nt;
-  }
-  return false;
-}
-
 template <int HD, bool CAP>
 __global__ void __launch_bounds__(FA2_THREADS, 1)
 fa_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -398,7 +401,7 @@ fa_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   int seq = 0, q0 = 0;
   // Blocks are handed out in increasing blockIdx; walking the tiles backwards puts the late query blocks of a sequence
   // (the ones with the most K / V tiles under a causal mask) first and leaves the short ones for the tail of the grid.
-  if (!find_tile2(p.cu_q, p.num_seqs, static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x), seq, q0))
+  if (!find_tile(p.cu_q, p.num_seqs, static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x), 2 * TQ, seq, q0))
     return;                                                            // uniform for the CTA: nothing allocated yet
   const int qs = p.cu_q[seq], len_q = p.cu_q[seq + 1] - qs;
   const int ks = p.cu_k[seq], len_k = p.cu_k[seq + 1] - ks;
@@ -790,6 +793,22 @@ static int g_dq_bulk = 1;     // ftb_attn_set_dq_bulk(0): per-thread vector redu
 // =====================================================================================================
 namespace ftb {
 
+// Orders of the backward's work.  A CTA that adds to a query tile in a fixed order may only wait for CTAs that were handed
+// out before it (one that waited for a later CTA could fill the GPU with waiters and starve it), and should come to the
+// tile after them by itself.
+//   FIRST_FIRST  key tiles ascending (the causal ones with the most query tiles first, so the short ones fill the end of
+//                the grid), head by head, query tiles ascending.  For dQ added in any order.
+//   LAST_FIRST   key tiles descending, head by head, query tiles ascending: every key tile starts at its own diagonal and
+//                so comes to a query tile one step after the key tile above it.  But the longest CTAs come last.
+//   IN_STEP      key tiles ascending, query tiles descending with the heads of the group inside: all key tiles of a
+//                sequence walk the same (query tile, head) list in step, the short ones leave it early.  The longest CTAs
+//                come first; the price is a wait per key tile at the start and additions that meet at the same addresses.
+// 32 / 8 heads of 128, LAST_FIRST against IN_STEP: 16 x 1024 tokens 646 / 722 us, 4 x 4096 2157 / 2169, 2 x 8192 4569 /
+// 3974, 1 x 16384 9699 / 7760; 16 / 8 heads: 2 x 8192 2016 / 2048, 1 x 16384 4294 / 3971; 16 / 16 heads: 1 x 16384 3986 /
+// 4257, 1 x 32768 16249 / 16626; head dim 64, 32 / 8 heads: 2 x 8192 3050 / 3370, 1 x 16384 7190 / 6794.  So IN_STEP where
+// the longest CTA walks more than 128 pairs (256 at head dim 64, whose pairs are shorter) and heads share keys.
+constexpr int BWD_FIRST_FIRST = 0, BWD_LAST_FIRST = 1, BWD_IN_STEP = 2;
+
 struct BwdParams {
   const int* cu_q;
   const int* cu_k;
@@ -797,6 +816,7 @@ struct BwdParams {
   int H, KV;
   float* dq_acc;            // (Tq, H, HD) fp32, zero-initialised by the caller
   int* dq_sem;              // deterministic mode: one counter per (query tile, head), zeroed by the caller; else NULL
+  int order;                // BWD_*: the order of the key tiles over the grid and of the query tiles in a CTA
   int dq_bulk;              // 1: dQ tiles leave through shared memory as tiled reduce-adds; 0: per-thread vector reductions
   __nv_bfloat16* dk;        // (Tk, KV, HD) contiguous
   __nv_bfloat16* dv;
@@ -809,69 +829,119 @@ struct BwdParams {
   int window;
 };
 
-// delta[h, t] = sum_d dO[t, h, d] * O[t, h, d]; one warp per (t, h).
+// delta[h, t] = sum_d dO[t, h, d] * O[t, h, d]; hd / 8 lanes per (t, h), each with one 16-byte load of either tensor.
+// Bound by memory; 16384 x 32 heads of 128: 110 us (2.4 TB/s) with a warp per row and 4-byte loads, 54 us (5.0 TB/s)
+// so.
+template <int HD>
 __global__ void fa_delta_kernel(const __nv_bfloat16* __restrict__ dout, long do_stride, const __nv_bfloat16* __restrict__ out,
-                                long o_stride, float* __restrict__ delta, int T, int H, int hd) {
-  const long w = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (w >= (long)T * H) return;
-  const int t = (int)(w / H), h = (int)(w % H), lane = threadIdx.x & 31;
-  const __nv_bfloat16* a = dout + (size_t)t * do_stride + (size_t)h * hd;
-  const __nv_bfloat16* b = out + (size_t)t * o_stride + (size_t)h * hd;
+                                long o_stride, float* __restrict__ delta, int T, int H) {
+  constexpr int LANES = HD / 8;
+  const long w = ((long)blockIdx.x * blockDim.x + threadIdx.x) / LANES;
+  const int part = threadIdx.x % LANES;
+  if (w >= (long)T * H) return;                     // whole groups of LANES lanes leave together
+  const int t = (int)(w / H), h = (int)(w % H);
+  const uint4 a = __ldg(reinterpret_cast<const uint4*>(dout + (size_t)t * do_stride + (size_t)h * HD) + part);
+  const uint4 b = __ldg(reinterpret_cast<const uint4*>(out + (size_t)t * o_stride + (size_t)h * HD) + part);
+  const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
+  const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&b);
   float s = 0.f;
-  for (int i = lane * 2; i < hd; i += 64) {
-    const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(a + i));
-    const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(b + i));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 x = __bfloat1622float2(a2[i]), y = __bfloat1622float2(b2[i]);
     s += x.x * y.x + x.y * y.y;
   }
+  const unsigned mask = ((1u << LANES) - 1u) << ((threadIdx.x & 31) / LANES * LANES);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) delta[(size_t)h * T + t] = s;
+  for (int o = LANES / 2; o > 0; o >>= 1) s += __shfl_xor_sync(mask, s, o);
+  if (part == 0) delta[(size_t)h * T + t] = s;
 }
 
-// Backward thread layout: warp 0 TMA, warp 1 MMA, warps 2-9 softmax / drain.  Warps w and w + 4 share a tensor-memory
-// lane quadrant (rows) and split the columns of every tile between them, so two warps per scheduler work on the
-// P / dS tile instead of one.
-constexpr int FAB_THREADS = 320;
+// Backward thread layout: warp 0 TMA, warp 1 MMA, warps 2-9 softmax, warps 10-13 dQ drain.
+//
+// Scores are formed transposed (Sᵀ = K·Qᵀ, dPᵀ = V·dOᵀ; one key row per thread), so that Pᵀ goes back into tensor memory
+// as packed bf16 over the score columns it came from and is the A operand of dV += Pᵀ·dO without touching shared memory.
+// dSᵀ is one shared tile that feeds dK += dSᵀ·Q (K-major) and dQ = dS·K (M-major).  The MMAs are issued one query tile
+// ahead:
+//     ... dQ(j) dK(j) | dP(j+1) dV(j+1) S(j+2) | dQ(j+1) dK(j+1) ...
+// P(j+1) is computed under dQ(j), dK(j) and dP(j+1); dS(j+1) under dV(j+1) and S(j+2); the dQ tile is drained by warps of
+// its own under dK(j) and what follows.  At head dim 128 the tensor memory is full (S, dP, dV, dK) and dQ(j) takes dP(j)'s
+// columns, which the softmax warps have read by then; dP(j+1) waits until they are drained.
+// Two softmax warps share a tensor-memory lane quadrant (rows) and split the 128 query columns.
+// Bound by shared-memory bandwidth: a tile pair takes 2560 cycles of tensor core at hd 128, but the four products with
+// both operands in shared memory, the dQ staging and the tile loads move some 4300 cycles' worth of it.
+// Causal, 32 / 8 heads of 128, dQ in any order: 16 x 1024 tokens 771 us with one chain S, dP -> softmax -> dV, dK, dQ ->
+// drain per tile pair, 580 us so; 1 x 16384 9160 us (600 TFLOP/s) before, 6420 us (856) so.  With dQ in a fixed order 926 ->
+// 646 us and 12300 -> 7640 us.
+constexpr int FAB_THREADS = 448;
+constexpr int FAB_SOFTMAX_WARPS = 8;
+
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// One answer for the whole warp: its lanes go on together or leave their loops together.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int where) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, where));
+}
+
+template <int HD>
+struct BwdSmem {
+  static constexpr int T_BYTES = 128 * HD * 2;       // one Q / dO / K / V tile
+  static constexpr int DS_BYTES = 128 * 128 * 2;
+  static constexpr int STAGE_BYTES = 32 * 32 * 4;    // 32 rows x 32 fp32 columns of dQ; two per drain warp
+  static constexpr int USED = 5 * T_BYTES + DS_BYTES + 8 * STAGE_BYTES + 2 * 2 * 128 * 4 + 256;
+  static constexpr int SIZE = USED + 1024 < 232448 ? USED + 1024 : 232448;      // the 227 KB a CTA may have
+};
 
 template <int HD, bool CAP>
 __global__ void __launch_bounds__(FAB_THREADS, 1)
 fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
               const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
               const __grid_constant__ CUtensorMap tmDQ, const BwdParams p) {
+  using L = BwdSmem<HD>;
   constexpr int KB = HD / 64;
-  constexpr int T_BYTES = 128 * HD * 2;       // one Q / dO / K / V tile
-  constexpr int P_BYTES = 128 * 128 * 2;
+  constexpr int T_BYTES = L::T_BYTES;
+  constexpr bool DQ_OVER_DP = HD == 128;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sK = smem;
   uint8_t* sV = sK + T_BYTES;
-  uint8_t* sQ = sV + T_BYTES;
-  uint8_t* sDO = sQ + T_BYTES;
-  uint8_t* sP = sDO + T_BYTES;
-  uint8_t* sDS = sP + P_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sDS + P_BYTES);
+  uint8_t* sQ = sV + T_BYTES;                 // 2 stages
+  uint8_t* sDO = sQ + 2 * T_BYTES;
+  uint8_t* sDS = sDO + T_BYTES;
+  uint8_t* sStg = sDS + L::DS_BYTES;          // dQ staging, two blocks for each drain warp
+  float* sStat = reinterpret_cast<float*>(sStg + 8 * L::STAGE_BYTES);     // [stage][lse2 | delta][128]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + 2 * 2 * 128);
   uint64_t* kv_full = bars;
-  uint64_t* qdo_full = bars + 1;
-  uint64_t* qdo_empty = bars + 2;
-  uint64_t* sdp_full = bars + 3;
-  uint64_t* pds_full = bars + 4;
-  uint64_t* dq_full = bars + 5;
-  uint64_t* dq_empty = bars + 6;
-  uint64_t* stage_bar = bars + 7;
-  uint64_t* drain_bar = bars + 9;          // (bars + 8 holds the tensor-memory slot and the abort flag)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  uint64_t* q_full = bars + 1;                // 2
+  uint64_t* q_empty = bars + 3;               // 2
+  uint64_t* do_full = bars + 5;
+  uint64_t* do_empty = bars + 6;
+  uint64_t* stat_full = bars + 7;             // 2
+  uint64_t* s_full = bars + 9;
+  uint64_t* p_full = bars + 10;
+  uint64_t* dp_full = bars + 11;
+  uint64_t* ds_full = bars + 12;
+  uint64_t* dq_full = bars + 13;
+  uint64_t* dq_empty = bars + 14;
+  uint64_t* acc_full = bars + 15;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  if (smem + L::USED > smem_raw + L::SIZE) {  // the base of the block's shared memory is aligned in practice
+    set_error(5, 241);
+    return;
+  }
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kvh = blockIdx.y;
+  const int kvh = blockIdx.x;
   const int rep = p.H / p.KV;
   int seq = 0, k0 = 0;
-  // Blocks are handed out in increasing blockIdx.  Unordered dQ: ascending key tiles, so the causal key tiles with the
-  // most query tiles start first.  Ordered dQ: DEscending key tiles, so every CTA only ever waits for CTAs that were
-  // handed out before it (a CTA that waited for a later one could fill the GPU with waiters and starve it).
-  const int tile_x = p.dq_sem != nullptr ? static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)
-                                         : static_cast<int>(blockIdx.x);
-  if (!find_tile(p.cu_k, p.num_seqs, tile_x, seq, k0)) return;
+  // Blocks are handed out in increasing blockIdx: all heads of a key tile, then the next key tile; see BWD_*.
+  if (!find_tile(p.cu_k, p.num_seqs,
+                 static_cast<int>(p.order == BWD_LAST_FIRST ? gridDim.y - 1 - blockIdx.y : blockIdx.y), TK, seq, k0))
+    return;
   const int qs = p.cu_q[seq], len_q = p.cu_q[seq + 1] - qs;
   const int ks = p.cu_k[seq], len_k = p.cu_k[seq + 1] - ks;
   const int off = len_k - len_q;
@@ -881,16 +951,23 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   i_lo = (i_lo / 128) * 128;
   const int n_qt = i_hi > i_lo ? (i_hi - i_lo + 127) / 128 : 0;
   const int n_iter = n_qt * rep;
-  int qtile_base = 0;                                   // index of this sequence's first query tile (semaphores)
-  if (p.dq_sem != nullptr)
-    for (int s2 = 0; s2 < seq; ++s2) qtile_base += (p.cu_q[s2 + 1] - p.cu_q[s2] + 127) / 128;
-  const int n_kt = (len_k + 127) / 128;
+  const bool in_step = p.order == BWD_IN_STEP;
+  const int qt_first = in_step ? i_lo + (n_qt - 1) * 128 : i_lo;
+  auto next_tile = [&](int& h, int& qt) {
+    if (in_step) {
+      if (++h == (kvh + 1) * rep) { h = kvh * rep; qt -= 128; }
+    } else {
+      qt += 128;
+      if (qt == i_lo + n_qt * 128) { qt = i_lo; ++h; }
+    }
+  };
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    mbar_init(kv_full, 1); mbar_init(qdo_full, 1); mbar_init(qdo_empty, 1); mbar_init(sdp_full, 1);
-    mbar_init(pds_full, 8); mbar_init(dq_full, 1); mbar_init(dq_empty, 8); mbar_init(stage_bar, 8);
-    mbar_init(drain_bar, 1);
+    mbar_init(kv_full, 1); mbar_init(do_full, 1); mbar_init(do_empty, 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); mbar_init(&stat_full[i], 1); }
+    mbar_init(s_full, 1); mbar_init(p_full, FAB_SOFTMAX_WARPS); mbar_init(dp_full, 1);
+    mbar_init(ds_full, FAB_SOFTMAX_WARPS); mbar_init(dq_full, 1); mbar_init(dq_empty, 4); mbar_init(acc_full, 1);
     fence_barrier_init();
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmDO); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
   }
@@ -903,9 +980,10 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tm_S = tmem_base, tm_dP = tmem_base + 128, tm_dV = tmem_base + 256, tm_dK = tmem_base + 256 + HD;
-  const uint32_t tm_dQ = tm_S;   // dQ reuses the S columns once the softmax warps have consumed S
+  const uint32_t tm_dQ = DQ_OVER_DP ? tm_dP : tmem_base + 256 + 2 * HD;
 
   if (warp == 0) {
+    // ------------------------------------------------------------------------- loads
     if (lane == 0 && n_iter > 0) {
       mbar_expect_tx(kv_full, 2 * T_BYTES);
 #pragma unroll
@@ -913,263 +991,232 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         tma_load_3d(sK + kb * (128 * 128), &tmK, kv_full, kb * 64, kvh, ks + k0);
         tma_load_3d(sV + kb * (128 * 128), &tmV, kv_full, kb * 64, kvh, ks + k0);
       }
-      for (int it = 0; it < n_iter; ++it) {
-        const int h = kvh * rep + it / n_qt;
-        const int qt = i_lo + (it % n_qt) * 128;
-        if (!mbar_wait(qdo_empty, (it & 1) ^ 1, abort_flag, 210)) break;
-        mbar_expect_tx(qdo_full, 2 * T_BYTES);
+    }
+    int h = kvh * rep, qt = qt_first;
+    for (int it = 0; it < n_iter; ++it) {
+      const int st = it & 1;
+      // the stage's last tenant has been through its dK product, so its row statistics have been read as well
+      if (!mbar_wait_warp(&q_empty[st], ((it >> 1) & 1) ^ 1, abort_flag, 210)) break;
+      if (lane == 0) {
+        mbar_expect_tx(&q_full[st], T_BYTES);
 #pragma unroll
-        for (int kb = 0; kb < KB; ++kb) {
-          tma_load_3d(sQ + kb * (128 * 128), &tmQ, qdo_full, kb * 64, h, qs + qt);
-          tma_load_3d(sDO + kb * (128 * 128), &tmDO, qdo_full, kb * 64, h, qs + qt);
-        }
+        for (int kb = 0; kb < KB; ++kb)
+          tma_load_3d(sQ + st * T_BYTES + kb * (128 * 128), &tmQ, &q_full[st], kb * 64, h, qs + qt);
       }
+      float* stat = sStat + st * 256;
+      const size_t base = static_cast<size_t>(h) * p.total_q + qs + qt;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int q = e * 32 + lane;
+        const bool vq = qt + q < len_q;
+        const float l = vq ? p.lse[base + q] : -INFINITY;
+        stat[q] = l == -INFINITY ? INFINITY : l * 1.4426950408889634f;     // past the end, or sees no key: P = 0
+        stat[128 + q] = vq ? p.delta[base + q] : 0.f;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&stat_full[st]);
+      if (!mbar_wait_warp(do_empty, (it & 1) ^ 1, abort_flag, 211)) break;
+      if (lane == 0) {
+        mbar_expect_tx(do_full, T_BYTES);
+#pragma unroll
+        for (int kb = 0; kb < KB; ++kb)
+          tma_load_3d(sDO + kb * (128 * 128), &tmDO, do_full, kb * 64, h, qs + qt);
+      }
+      next_tile(h, qt);
     }
   } else if (warp == 1) {
+    // --------------------------------------------------------------------------- MMA issuer
     if (lane == 0 && n_iter > 0) {
-      constexpr uint32_t id_s = make_idesc_bf16(128, 128, 0, 0);       // S, dP: both operands K-major
-      constexpr uint32_t id_t = make_idesc_bf16(128, HD, 1, 1);        // dV, dK: transposed A, MN-major B
-      constexpr uint32_t id_q = make_idesc_bf16(128, HD, 0, 1);        // dQ: K-major A, MN-major B
-      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ = smem_u32(sQ), aDO = smem_u32(sDO);
-      const uint32_t aP = smem_u32(sP), aDS = smem_u32(sDS);
-      bool ok = mbar_wait(kv_full, 0, abort_flag, 220);
-      for (int it = 0; it < n_iter && ok; ++it) {
-        const uint32_t ph = it & 1;
-        if (!(ok = mbar_wait(qdo_full, ph, abort_flag, 221))) break;
-        if (!(ok = mbar_wait(dq_empty, ph ^ 1, abort_flag, 222))) break;
-        tc_fence_after();
+      constexpr uint32_t id_s = make_idesc_bf16(128, 128, 0, 0);       // Sᵀ, dPᵀ: both operands K-major
+      constexpr uint32_t id_v = make_idesc_bf16(128, HD, 0, 1);        // dV (A in tensor memory), dK: MN-major B
+      constexpr uint32_t id_q = make_idesc_bf16(128, HD, 1, 1);        // dQ: transposed A, MN-major B
+      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ0 = smem_u32(sQ), aDO = smem_u32(sDO), aDS = smem_u32(sDS);
+      auto issue_s = [&](int j) {
+        const uint32_t aQ = aQ0 + (j & 1) * T_BYTES;
 #pragma unroll
         for (int kb = 0; kb < KB; ++kb)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {
             const uint32_t o = kb * (128 * 128) + kk * 32;
-            umma_f16(tm_S, make_smem_desc(aQ + o, 16, 1024), make_smem_desc(aK + o, 16, 1024), id_s, (kb | kk) != 0);
+            umma_f16(tm_S, make_smem_desc(aK + o, 16, 1024), make_smem_desc(aQ + o, 16, 1024), id_s, (kb | kk) != 0);
           }
+        umma_commit(s_full);
+      };
+      auto issue_dp = [&]() {
 #pragma unroll
         for (int kb = 0; kb < KB; ++kb)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {
             const uint32_t o = kb * (128 * 128) + kk * 32;
-            umma_f16(tm_dP, make_smem_desc(aDO + o, 16, 1024), make_smem_desc(aV + o, 16, 1024), id_s, (kb | kk) != 0);
+            umma_f16(tm_dP, make_smem_desc(aV + o, 16, 1024), make_smem_desc(aDO + o, 16, 1024), id_s, (kb | kk) != 0);
           }
-        umma_commit(sdp_full);
-        if (!(ok = mbar_wait(pds_full, ph, abort_flag, 223))) break;
-        tc_fence_after();
+        umma_commit(dp_full);
+      };
+      auto issue_dv = [&](int j) {          // Pᵀ: 16 queries in 8 columns; the second half starts at column 64
 #pragma unroll
-        for (int s = 0; s < 8; ++s) {      // reduction over the 128 query rows, 16 per step
-          const uint32_t o = s * (16 * 128);
-          umma_f16(tm_dV, make_smem_desc(aP + o, 128 * 128, 1024), make_smem_desc(aDO + o, 128 * 128, 1024), id_t,
-                   (it | s) != 0);
-          umma_f16(tm_dK, make_smem_desc(aDS + o, 128 * 128, 1024), make_smem_desc(aQ + o, 128 * 128, 1024), id_t,
-                   (it | s) != 0);
-        }
+        for (int s = 0; s < 8; ++s)
+          umma_f16_ts(tm_dV, tm_S + (s >> 2) * 64 + (s & 3) * 8, make_smem_desc(aDO + s * (16 * 128), 128 * 128, 1024),
+                      id_v, (j | s) != 0);
+        umma_commit(do_empty);
+      };
+      bool ok = mbar_wait(kv_full, 0, abort_flag, 220) && mbar_wait(&q_full[0], 0, abort_flag, 221);
+      if (ok) { tc_fence_after(); issue_s(0); }
+      for (int j = -1; j < n_iter && ok; ++j) {
+        if (j >= 0) {
+          if (!(ok = mbar_wait(ds_full, j & 1, abort_flag, 222))) break;
+          if (!DQ_OVER_DP && j > 0 && !(ok = mbar_wait(dq_empty, (j - 1) & 1, abort_flag, 223))) break;
+          tc_fence_after();
+          const uint32_t aQ = aQ0 + (j & 1) * T_BYTES;
 #pragma unroll
-        for (int s = 0; s < 8; ++s) {      // reduction over the 128 keys
-          const uint64_t ad = make_smem_desc(aDS + (s >> 2) * (128 * 128) + (s & 3) * 32, 16, 1024);
-          const uint64_t bd = make_smem_desc(aK + s * (16 * 128), 128 * 128, 1024);
-          umma_f16(tm_dQ, ad, bd, id_q, s != 0);
+          for (int s = 0; s < 8; ++s)        // reduction over the 128 keys, 16 per step
+            umma_f16(tm_dQ, make_smem_desc(aDS + s * (16 * 128), 128 * 128, 1024),
+                     make_smem_desc(aK + s * (16 * 128), 128 * 128, 1024), id_q, s != 0);
+          umma_commit(dq_full);
+#pragma unroll
+          for (int s = 0; s < 8; ++s)        // reduction over the 128 queries
+            umma_f16(tm_dK, make_smem_desc(aDS + (s >> 2) * (128 * 128) + (s & 3) * 32, 16, 1024),
+                     make_smem_desc(aQ + s * (16 * 128), 128 * 128, 1024), id_v, (j | s) != 0);
+          umma_commit(&q_empty[j & 1]);
         }
-        umma_commit(dq_full);
-        umma_commit(qdo_empty);
+        if (j + 1 < n_iter) {
+          if (!(ok = mbar_wait(do_full, (j + 1) & 1, abort_flag, 224))) break;
+          if (DQ_OVER_DP && j >= 0 && !(ok = mbar_wait(dq_empty, j & 1, abort_flag, 225))) break;
+          tc_fence_after();
+          issue_dp();
+          if (!(ok = mbar_wait(p_full, (j + 1) & 1, abort_flag, 226))) break;
+          tc_fence_after();
+          issue_dv(j + 1);
+        }
+        if (j + 2 < n_iter) {
+          if (!(ok = mbar_wait(&q_full[(j + 2) & 1], ((j + 2) >> 1) & 1, abort_flag, 227))) break;
+          tc_fence_after();
+          issue_s(j + 2);
+        }
       }
+      if (ok) umma_commit(acc_full);
     }
-  } else {
+  } else if (warp < 2 + FAB_SOFTMAX_WARPS) {
+    // ------------------------------------------------------------------------- softmax: P and dS
     const int quad = warp & 3;
-    const int half = (warp - 2) >> 2;               // which half of the columns this warp owns
-    const int r = quad * 32 + lane;
+    const int half = (warp - 2) >> 2;               // which half of the query columns this warp owns
+    const int r = quad * 32 + lane;                 // key row inside the tile
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
     const float c = p.scale * 1.4426950408889634f;
-    constexpr bool capped = CAP;   // soft-cap is a template parameter: the plain path carries no extra work
     const float cap2 = p.softcap * 1.4426950408889634f;
-    const float soc = capped ? p.scale / p.softcap : 0.f;
+    const float soc = CAP ? p.scale / p.softcap : 0.f;
+    const int win = min(p.window, 1 << 29);
     bool ok = true;
+    int h = kvh * rep, qt = qt_first;
     for (int it = 0; it < n_iter && ok; ++it) {
       const uint32_t ph = it & 1;
-      const int h = kvh * rep + it / n_qt;
-      const int qt = i_lo + (it % n_qt) * 128;
-      const int i = qt + r;
-      const bool vq = i < len_q;
-      const size_t grow = static_cast<size_t>(qs + (vq ? i : 0));
-      const float lse2 = vq ? p.lse[static_cast<size_t>(h) * p.total_q + grow] * 1.4426950408889634f : INFINITY;
-      const float dl = vq ? p.delta[static_cast<size_t>(h) * p.total_q + grow] : 0.f;
-      const int qi = i + off;
+      const float4* lse4 = reinterpret_cast<const float4*>(sStat + ph * 256 + half * 64);
+      const float4* dl4 = lse4 + 32;
       // a tile needs masking only if it touches the end of the queries / keys, the causal diagonal or the window edge
       const bool edge = (qt + 128 > len_q) || (k0 + 128 > len_k) ||
                         (p.causal && (k0 + 127 > qt + off || (p.window > 0 && k0 <= qt + 127 + off - p.window)));
-      if (!(ok = mbar_wait(sdp_full, ph, abort_flag, 230))) break;
+      if (!(ok = mbar_wait_warp(&stat_full[ph], (it >> 1) & 1, abort_flag, 230))) break;
+      if (!(ok = mbar_wait_warp(s_full, ph, abort_flag, 231))) break;
       tc_fence_after();
-#pragma unroll 1
-      for (int cb = half * 64; cb < half * 64 + 64; cb += 32) {
-        uint32_t vs[32], vd[32];
-        tmem_ld_32x32(tm_S + lane_base + cb, vs);
-        tmem_ld_32x32(tm_dP + lane_base + cb, vd);
-        tmem_ld_wait();
-        float pr[32], ds[32];
-        if (edge || capped) {
+      uint32_t sv[2][32];                           // scores, then P (with soft-cap: the raw scores)
+      tmem_ld_32x32(tm_S + lane_base + half * 64, sv[0]);
+      tmem_ld_32x32(tm_S + lane_base + half * 64 + 32, sv[1]);
+      tmem_ld_wait();
+      if (edge) {
+        // query columns this key row is seen by: [lo, hi)
+        const int kj = k0 + r;
+        const int first = p.causal ? kj - off - qt : 0;
+        const int lo = (kj < len_k ? first : 1 << 30) - half * 64;
+        const int hi = min(len_q - qt, (p.causal && win > 0) ? first + win : 128) - half * 64;
 #pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const int kj = k0 + cb + e;
-            bool keep = vq && kj < len_k;
-            if (p.causal) keep = keep && (kj <= qi) && (p.window <= 0 || kj > qi - p.window);
-            const float raw = __uint_as_float(vs[e]);
-            const float th = capped ? tanh_fast(raw * soc) : 0.f;
-            const float pe = keep ? exp2f((capped ? cap2 * th : raw * c) - lse2) : 0.f;
-            pr[e] = pe;
-            // d(cap * tanh(scale * s / cap)) / ds = scale * (1 - tanh^2)
-            ds[e] = pe * (__uint_as_float(vd[e]) - dl) * p.scale * (1.f - th * th);
-          }
-        } else {
+        for (int q2 = 0; q2 < 2; ++q2)
 #pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const float pe = exp2f(__uint_as_float(vs[e]) * c - lse2);
-            pr[e] = pe;
-            ds[e] = pe * (__uint_as_float(vd[e]) - dl) * p.scale;
-          }
-        }
+          for (int e = 0; e < 32; ++e)
+            if (q2 * 32 + e < lo || q2 * 32 + e >= hi) sv[q2][e] = 0xff800000u;        // -inf: exponential 0
+      }
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          uint4 a, b;
-          __nv_bfloat162* a2 = reinterpret_cast<__nv_bfloat162*>(&a);
-          __nv_bfloat162* b2 = reinterpret_cast<__nv_bfloat162*>(&b);
+      for (int q2 = 0; q2 < 2; ++q2) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          const float4 l4 = lse4[q2 * 8 + g];
+          const float ls[4] = {l4.x, l4.y, l4.z, l4.w};
+          float pe[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            a2[e] = __floats2bfloat162_rn(pr[g * 8 + 2 * e], pr[g * 8 + 2 * e + 1]);
-            b2[e] = __floats2bfloat162_rn(ds[g * 8 + 2 * e], ds[g * 8 + 2 * e + 1]);
+            const float s = __uint_as_float(sv[q2][g * 4 + e]);
+            if constexpr (CAP) {
+              pe[e] = s == -INFINITY ? 0.f : ex2_approx(cap2 * tanh_fast(s * soc) - ls[e]);
+            } else {
+              pe[e] = ex2_approx(s * c - ls[e]);
+              sv[q2][g * 4 + e] = __float_as_uint(pe[e]);
+            }
           }
-          const uint32_t o = sw128_offset(r, cb + g * 8, 128);
-          *reinterpret_cast<uint4*>(sP + o) = a;
-          *reinterpret_cast<uint4*>(sDS + o) = b;
+          const __nv_bfloat162 a = __floats2bfloat162_rn(pe[0], pe[1]), b = __floats2bfloat162_rn(pe[2], pe[3]);
+          pk[g * 2] = *reinterpret_cast<const uint32_t*>(&a);
+          pk[g * 2 + 1] = *reinterpret_cast<const uint32_t*>(&b);
+        }
+        // over the columns that this warp itself has read
+        tmem_st_32x16(tm_S + lane_base + half * 64 + q2 * 16, pk);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+      if (!(ok = mbar_wait_warp(dp_full, ph, abort_flag, 232))) break;
+      tc_fence_after();
+#pragma unroll
+      for (int q2 = 0; q2 < 2; ++q2) {
+        uint32_t vd[32];
+        tmem_ld_32x32(tm_dP + lane_base + half * 64 + q2 * 32, vd);
+        tmem_ld_wait();
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          const float4 da = dl4[q2 * 8 + g * 2], db = dl4[q2 * 8 + g * 2 + 1];
+          const float dl[8] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w};
+          float ds[8];
+          if constexpr (CAP) {
+            const float4 la = lse4[q2 * 8 + g * 2], lb = lse4[q2 * 8 + g * 2 + 1];
+            const float ls[8] = {la.x, la.y, la.z, la.w, lb.x, lb.y, lb.z, lb.w};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float s = __uint_as_float(sv[q2][g * 8 + e]);
+              const float th = tanh_fast(s * soc);
+              const float pe = s == -INFINITY ? 0.f : ex2_approx(cap2 * th - ls[e]);
+              // d(cap * tanh(scale * s / cap)) / ds = scale * (1 - tanh^2); the scale follows on dQ and dK
+              ds[e] = pe * (__uint_as_float(vd[g * 8 + e]) - dl[e]) * (1.f - th * th);
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              ds[e] = __uint_as_float(sv[q2][g * 8 + e]) * (__uint_as_float(vd[g * 8 + e]) - dl[e]);
+          }
+          uint4 b;
+          __nv_bfloat162* b2 = reinterpret_cast<__nv_bfloat162*>(&b);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) b2[e] = __floats2bfloat162_rn(ds[2 * e], ds[2 * e + 1]);
+          *reinterpret_cast<uint4*>(sDS + sw128_offset(r, half * 64 + q2 * 32 + g * 8, 128)) = b;
         }
       }
       tc_fence_before();
       fence_proxy_async();
       __syncwarp();
-      if (lane == 0) mbar_arrive(pds_full);
-      if (!(ok = mbar_wait(dq_full, ph, abort_flag, 231))) break;
-      tc_fence_after();
-      constexpr int HC = HD / 2;
-      if (p.dq_bulk) {
-        // dQ tile: tensor memory -> registers -> fp32 staging in shared memory (the P / dS buffers, free now that the
-        // MMAs of this query tile are done; one 16 KB block of 128 rows x 32 columns per 32 columns, 128-byte
-        // swizzle) -> four (two at hd 64) tiled reduce-adds into the fp32 workspace.  L2 then sees whole 128-byte
-        // lines per reduction instead of one 16-byte piece per row and thread, which is what bounded this kernel.
-        // Rows past the end of the sequence hold exact zeros (their P and dS were masked), so adding them is harmless.
-        uint8_t* stg = sP;
-#pragma unroll 1
-        for (int cb = half * HC; cb < half * HC + HC; cb += 32) {
-          uint32_t v[32];
-          tmem_ld_32x32(tm_dQ + lane_base + cb, v);
-          tmem_ld_wait();
-          uint8_t* rowp = stg + (cb >> 5) * (128 * 128) + r * 128;
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<uint4*>(rowp + ((j ^ (r & 7)) << 4)) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-        }
-        tc_fence_before();
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(dq_empty);                  // TMEM columns are free: the next S / dP may be issued now
-          mbar_arrive(stage_bar);                 // this warp's rows are staged
-        }
-        if (warp == 2 && lane == 0) {
-          bool go = mbar_wait(stage_bar, ph, abort_flag, 232);
-          int* sem = nullptr;
-          if (go && p.dq_sem != nullptr) {
-            // deterministic order: wait until the key tiles above this one have added their share of this query tile
-            // (word 0 of the array is the give-up flag, the counters follow it)
-            sem = p.dq_sem + 1 + (static_cast<size_t>(qtile_base + qt / 128)) * p.H + h;
-            const int j_hi = p.causal ? min(n_kt - 1, (qt + 127 + off) / 128) : n_kt - 1;
-            const int expected = j_hi - k0 / 128;
-            uint32_t spins = 0;
-            volatile int* gave_up = p.dq_sem;
-            while (expected > 0 && !*gave_up && ld_acquire_gpu_s32(sem) < expected) {
-              if (++spins > (1u << 21) || *abort_flag) { *gave_up = 1; set_error(4, 240); break; }
-              __nanosleep(32);
-            }
-          }
-          if (go) {
-#pragma unroll
-            for (int q4 = 0; q4 < HD / 32; ++q4)
-              tma_reduce_add_2d(&tmDQ, stg + q4 * (128 * 128), h * HD + q4 * 32, qs + qt);
-            bulk_commit();
-            if (sem != nullptr) {
-              bulk_wait_all();                    // the additions have been performed: the next key tile may add
-              red_release_gpu_add_s32(sem, 1);
-            } else {
-              bulk_wait_read_all();               // the staging buffers have been read: P / dS may be rewritten
-            }
-          }
-          mbar_arrive(drain_bar);
-        }
-        if (!(ok = mbar_wait(drain_bar, ph, abort_flag, 233))) break;
-        continue;
-      }
-      // dQ tile: tensor memory -> registers -> vector reductions into the fp32 workspace, one row per thread (eight
-      // 16-byte red.v4 per 32 columns).  Each warp drains its own half of the columns of its 32 rows.
-      int* sem = nullptr;
-      if (p.dq_sem != nullptr) {
-        // deterministic order: wait until the key tiles above this one have added their share of this query tile
-        // (word 0 of the array is the give-up flag, the counters follow it)
-        sem = p.dq_sem + 1 + (static_cast<size_t>(qtile_base + qt / 128)) * p.H + h;
-        const int j_hi = p.causal ? min(n_kt - 1, (qt + 127 + off) / 128) : n_kt - 1;
-        const int expected = j_hi - k0 / 128;
-        if (lane == 0 && expected > 0) {
-          uint32_t spins = 0;
-          volatile int* gave_up = p.dq_sem;
-          while (!*gave_up && ld_acquire_gpu_s32(sem) < expected) {
-            // give up: the order is lost, not data.  The flag makes every later wait of this launch return at once,
-            // so one lost turn costs one time limit (about a second), not one per tile.
-            if (++spins > (1u << 21) || *abort_flag) { *gave_up = 1; set_error(4, 240); break; }
-            __nanosleep(32);
-          }
-        }
-        __syncwarp();
-      }
-      float* dq_row = p.dq_acc + ((static_cast<size_t>(qs + (vq ? i : 0))) * p.H + h) * HD;
-#pragma unroll 1
-      for (int cb = half * HC; cb < half * HC + HC; cb += 32) {
-        uint32_t v[32];
-        tmem_ld_32x32(tm_dQ + lane_base + cb, v);
-        tmem_ld_wait();
-        if (vq) {
-#pragma unroll
-          for (int e = 0; e < 32; e += 4)
-            red_add_v4_f32(dq_row + cb + e, __uint_as_float(v[e]), __uint_as_float(v[e + 1]), __uint_as_float(v[e + 2]),
-                           __uint_as_float(v[e + 3]));
-        }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(dq_empty);       // TMEM columns are free: the next S / dP may be issued now
-      if (sem != nullptr) {
-        // all eight warps' reductions must be visible before the next key tile in the order may add
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(stage_bar);
-        if (!(ok = mbar_wait(stage_bar, ph, abort_flag, 232))) break;
-        if (warp == 2 && lane == 0) red_release_gpu_add_s32(sem, 1);
-      }
+      if (lane == 0) mbar_arrive(ds_full);
+      next_tile(h, qt);
     }
-    if (p.dq_bulk && warp == 2 && lane == 0) bulk_wait_all();   // none of this thread's reduce-adds outlives the kernel
     // dK / dV of this key tile (thread = key row)
     constexpr int HC2 = HD / 2;
-    if (r < kr) {
-      const size_t row = static_cast<size_t>(ks + k0 + r);
-      __nv_bfloat16* dk_row = p.dk + (row * p.KV + kvh) * HD;
-      __nv_bfloat16* dv_row = p.dv + (row * p.KV + kvh) * HD;
-      if (n_iter == 0 || !ok) {
+    if (n_iter > 0 && ok) ok = mbar_wait_warp(acc_full, 0, abort_flag, 233);
+    const size_t row = static_cast<size_t>(ks + k0 + min(r, kr - 1));
+    __nv_bfloat16* dk_row = p.dk + (row * p.KV + kvh) * HD;
+    __nv_bfloat16* dv_row = p.dv + (row * p.KV + kvh) * HD;
+    if (n_iter == 0 || !ok) {
+      if (r < kr)
         for (int cidx = half * HC2; cidx < half * HC2 + HC2; cidx += 8) {
           *reinterpret_cast<uint4*>(dk_row + cidx) = make_uint4(0, 0, 0, 0);
           *reinterpret_cast<uint4*>(dv_row + cidx) = make_uint4(0, 0, 0, 0);
         }
-      }
-    }
-    if (n_iter > 0 && ok) {
+    } else {
       tc_fence_after();
-      const size_t row = static_cast<size_t>(ks + k0 + min(r, kr - 1));
-      __nv_bfloat16* dk_row = p.dk + (row * p.KV + kvh) * HD;
-      __nv_bfloat16* dv_row = p.dv + (row * p.KV + kvh) * HD;
 #pragma unroll 1
       for (int cb = half * HC2; cb < half * HC2 + HC2; cb += 32) {
         uint32_t a[32], b[32];
@@ -1185,7 +1232,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               x2[e] = __floats2bfloat162_rn(__uint_as_float(a[g * 8 + 2 * e]), __uint_as_float(a[g * 8 + 2 * e + 1]));
-              y2[e] = __floats2bfloat162_rn(__uint_as_float(b[g * 8 + 2 * e]), __uint_as_float(b[g * 8 + 2 * e + 1]));
+              y2[e] = __floats2bfloat162_rn(__uint_as_float(b[g * 8 + 2 * e]) * p.scale,
+                                            __uint_as_float(b[g * 8 + 2 * e + 1]) * p.scale);
             }
             *reinterpret_cast<uint4*>(dv_row + cb + g * 8) = x;
             *reinterpret_cast<uint4*>(dk_row + cb + g * 8) = y;
@@ -1193,6 +1241,129 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         }
       }
     }
+  } else {
+    // ------------------------------------------------------------------------- dQ drain, 32 query rows a warp
+    // Tensor memory -> registers -> fp32 staging in shared memory (blocks of 32 rows x 32 columns, 128-byte swizzle) ->
+    // tiled reduce-adds into the fp32 workspace: L2 sees whole 128-byte lines per reduction.  Each warp is on its own.
+    // Rows past the end of the sequence hold exact zeros (their P and dS were masked), so adding them is harmless.
+    const int quad = warp & 3;
+    const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
+    uint8_t* stg = sStg + quad * 2 * L::STAGE_BYTES;
+    // index of this sequence's first query tile (semaphores)
+    const int qtile_base = p.dq_sem != nullptr ? tiles_before(p.cu_q, seq, 128) : 0;
+    auto stage = [&](int slot, const uint32_t (&v)[32]) {
+      uint8_t* rowp = stg + slot * L::STAGE_BYTES + lane * 128;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        *reinterpret_cast<uint4*>(rowp + ((j ^ (lane & 7)) << 4)) =
+            make_uint4(__float_as_uint(__uint_as_float(v[4 * j]) * p.scale),
+                       __float_as_uint(__uint_as_float(v[4 * j + 1]) * p.scale),
+                       __float_as_uint(__uint_as_float(v[4 * j + 2]) * p.scale),
+                       __float_as_uint(__uint_as_float(v[4 * j + 3]) * p.scale));
+    };
+    auto add_row = [&](float* dst, const uint32_t (&v)[32]) {
+#pragma unroll
+      for (int e = 0; e < 32; e += 4)
+        red_add_v4_f32(dst + e, __uint_as_float(v[e]) * p.scale, __uint_as_float(v[e + 1]) * p.scale,
+                       __uint_as_float(v[e + 2]) * p.scale, __uint_as_float(v[e + 3]) * p.scale);
+    };
+    int h = kvh * rep, qt = qt_first;
+    for (int it = 0; it < n_iter; ++it) {
+      if (!mbar_wait_warp(dq_full, it & 1, abort_flag, 235)) break;
+      tc_fence_after();
+      const bool live = qt + quad * 32 < len_q;
+      // the two halves of the tile's columns go through the same registers; the second is read before the first leaves
+      uint32_t v0[32], v1[32];
+      auto load_half = [&](int col) {
+        tmem_ld_32x32(tm_dQ + lane_base + col, v0);
+        tmem_ld_32x32(tm_dQ + lane_base + col + 32, v1);
+        tmem_ld_wait();
+      };
+      auto release = [&]() {                            // the columns may be written again
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(dq_empty);
+      };
+      int* sem = nullptr;
+      if (p.dq_sem != nullptr && live)
+        // deterministic order, for each 32 rows of a query tile (word 0 of the array is the give-up flag)
+        sem = p.dq_sem + 1 + ((static_cast<size_t>(qtile_base + qt / 128)) * p.H + h) * 4 + quad;
+      auto wait_turn = [&]() {
+        // wait until the key tiles before this one in the order have added their share of these rows.  Giving up loses the order, not
+        // data; the flag makes every later wait of this launch return at once, so one lost turn costs one time limit
+        // (about a second), not one per tile.
+        int expected;
+        if (in_step) {
+          expected = k0 / 128 - (p.causal && p.window > 0 ? max(0, qt + off - p.window + 1) / 128 : 0);
+        } else {
+          const int n_kt = (len_k + 127) / 128;
+          expected = (p.causal ? min(n_kt - 1, (qt + 127 + off) / 128) : n_kt - 1) - k0 / 128;
+        }
+        uint32_t spins = 0;
+        volatile int* gave_up = p.dq_sem;
+        while (expected > 0 && !*gave_up && ld_acquire_gpu_s32(sem) < expected) {
+          if (++spins > (1u << 21) || *abort_flag) { *gave_up = 1; set_error(4, 240); break; }
+          __nanosleep(32);
+        }
+      };
+      if (!live) {
+        release();
+      } else if (p.dq_bulk) {
+        if (lane == 0) bulk_wait_read_all();            // the staging blocks have left
+        __syncwarp();
+        load_half(0);
+        stage(0, v0);
+        stage(1, v1);
+        if constexpr (HD == 128) load_half(64);
+        release();
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) {
+          if (sem != nullptr) wait_turn();
+          tma_reduce_add_2d(&tmDQ, stg, h * HD, qs + qt + quad * 32);
+          tma_reduce_add_2d(&tmDQ, stg + L::STAGE_BYTES, h * HD + 32, qs + qt + quad * 32);
+          bulk_commit();
+        }
+        if constexpr (HD == 128) {
+          if (lane == 0) bulk_wait_read_all();
+          __syncwarp();
+          stage(0, v0);
+          stage(1, v1);
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+            tma_reduce_add_2d(&tmDQ, stg, h * HD + 64, qs + qt + quad * 32);
+            tma_reduce_add_2d(&tmDQ, stg + L::STAGE_BYTES, h * HD + 96, qs + qt + quad * 32);
+            bulk_commit();
+          }
+        }
+        if (lane == 0 && sem != nullptr) {
+          bulk_wait_all();                              // the additions have been performed: the next key tile may add
+          red_release_gpu_add_s32(sem, 1);
+        }
+      } else {                                          // 16-byte reductions, one row per thread
+        const int i = qt + quad * 32 + lane;
+        float* dst = p.dq_acc + (static_cast<size_t>(qs + min(i, len_q - 1)) * p.H + h) * HD;
+        if (lane == 0 && sem != nullptr) wait_turn();
+        __syncwarp();
+#pragma unroll 1
+        for (int col = 0; col < HD; col += 64) {
+          load_half(col);
+          if (col + 64 == HD) release();
+          if (i < len_q) {
+            add_row(dst + col, v0);
+            add_row(dst + col + 32, v1);
+          }
+        }
+        if (sem != nullptr) {
+          __threadfence();
+          __syncwarp();
+          if (lane == 0) red_release_gpu_add_s32(sem, 1);
+        }
+      }
+      next_tile(h, qt);
+    }
+    if (p.dq_bulk && lane == 0) bulk_wait_all();        // none of this thread's reduce-adds outlives the kernel
   }
   tc_fence_before();
   __syncthreads();
@@ -1205,7 +1376,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 template <int HD, bool CAP>
 static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap& tk, const CUtensorMap& tv,
                       const CUtensorMap& tdq, const BwdParams& p, int tiles, cudaStream_t s) {
-  constexpr int SMEM = 4 * 128 * HD * 2 + 2 * 128 * 128 * 2 + 256 + 1024;
+  constexpr int SMEM = BwdSmem<HD>::SIZE;
   auto kern = fa_bwd_kernel<HD, CAP>;
   static bool configured = false;
   if (!configured) {
@@ -1213,7 +1384,7 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tdo, const CUten
     if (e != cudaSuccess) return -300 - static_cast<int>(e);
     configured = true;
   }
-  dim3 grid(tiles, p.KV);
+  dim3 grid(p.KV, tiles);
   kern<<<grid, FAB_THREADS, SMEM, s>>>(tq, tdo, tk, tv, tdq, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -400 - static_cast<int>(e);
@@ -1226,22 +1397,22 @@ extern "C" {
 // dout / q / out (Tq, H, hd), k / v (Tk, KV, hd) bf16 with token strides; lse (H, Tq) from the forward.
 // Workspaces supplied by the caller: delta (H, Tq) fp32, dq_acc (Tq, H, hd) fp32 ZEROED.
 // Outputs: dq (bf16, converted from dq_acc), dk, dv (Tk, KV, hd) bf16 contiguous, every row written.
-// dq_sem: NULL, or 1 + (sum over sequences of ceil(len_q / 128)) x H int32 words, ZEROED (word 0 is the kernel's
-//   give-up flag, the rest one counter per (query tile, head)): makes the dQ summation order
+// dq_sem: NULL, or 1 + (sum over sequences of ceil(len_q / 128)) x H x 4 int32 words, ZEROED (word 0 is the kernel's
+//   give-up flag, the rest one counter per (query tile, head, 32 rows)): makes the dQ summation order
 // fixed (bit-reproducible gradients) at the price of ordering the CTAs that share a query tile.
+// max_k: the longest sequence's keys (it chooses the order of the work only).
 int ftb_attn_bwd(const void* dout, const void* q, const void* k, const void* v, const void* out, const float* lse,
                  float* delta, float* dq_acc, int* dq_sem, void* dq, void* dk, void* dv, const int* cu_q, const int* cu_k,
                  int num_seqs, int total_q, int total_k, int H, int KV, int hd, long q_stride, long k_stride,
                  long v_stride, long do_stride, long o_stride, float scale, float softcap, int causal, int window,
-                 int max_tiles, cudaStream_t stream) {
+                 int max_tiles, int max_k, cudaStream_t stream) {
   if (total_q <= 0 || num_seqs <= 0) return 0;
   if ((hd != 64 && hd != 128) || H % KV) return -2;
-  if ((q_stride & 7) || (k_stride & 7) || (v_stride & 7) || (do_stride & 7)) return -2;
+  if ((q_stride & 7) || (k_stride & 7) || (v_stride & 7) || (do_stride & 7) || (o_stride & 7)) return -2;
   {
-    const long warps = (long)total_q * H;
-    fa_delta_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, stream>>>((const __nv_bfloat16*)dout, do_stride,
-                                                                     (const __nv_bfloat16*)out, o_stride, delta,
-                                                                     total_q, H, hd);
+    const long threads = (long)total_q * H * (hd / 8);
+    (hd == 128 ? fa_delta_kernel<128> : fa_delta_kernel<64>)<<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(
+        (const __nv_bfloat16*)dout, do_stride, (const __nv_bfloat16*)out, o_stride, delta, total_q, H);
   }
   CUtensorMap tq, tdo, tk, tv;
   int rc = make_tmap_3d(&tq, q, hd, H, total_q, q_stride, 128);
@@ -1252,14 +1423,14 @@ int ftb_attn_bwd(const void* dout, const void* q, const void* k, const void* v, 
   if (rc) return rc;
   rc = make_tmap_3d(&tv, v, hd, KV, total_k, v_stride, 128);
   if (rc) return rc;
-  // fp32 workspace as a 2-D tensor (total_q rows of H * hd columns): boxes of 128 rows x 32 columns for the reduce-adds
+  // fp32 workspace as a 2-D tensor (total_q rows of H * hd columns): boxes of 32 rows x 32 columns for the reduce-adds
   CUtensorMap tdq;
   {
     EncodeTiledFn enc = get_encode();
     if (enc == nullptr) return -100;
     cuuint64_t gdim[2] = {(cuuint64_t)H * hd, (cuuint64_t)total_q};
     cuuint64_t gstr[1] = {(cuuint64_t)H * hd * 4};
-    cuuint32_t box[2] = {32, 128};
+    cuuint32_t box[2] = {32, 32};
     cuuint32_t es[2] = {1, 1};
     CUresult r = enc(&tdq, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, dq_acc, gdim, gstr, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1268,6 +1439,9 @@ int ftb_attn_bwd(const void* dout, const void* q, const void* k, const void* v, 
   BwdParams p;
   p.cu_q = cu_q; p.cu_k = cu_k; p.num_seqs = num_seqs; p.H = H; p.KV = KV; p.dq_bulk = g_dq_bulk;
   p.dq_acc = dq_acc; p.dq_sem = dq_sem; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv; p.lse = lse; p.delta = delta;
+  const long pairs = (long)(H / KV) * ((max_k + 127) / 128);
+  p.order = dq_sem == nullptr ? BWD_FIRST_FIRST
+            : (H > KV && pairs > (hd == 128 ? 128 : 256)) ? BWD_IN_STEP : BWD_LAST_FIRST;
   p.total_q = total_q; p.scale = scale; p.softcap = softcap; p.causal = causal; p.window = window;
   if (softcap > 0.f)
     rc = (hd == 128) ? launch_bwd<128, true>(tq, tdo, tk, tv, tdq, p, max_tiles, stream)

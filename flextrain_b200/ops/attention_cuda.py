@@ -66,13 +66,13 @@ def bwd(dout, q, k, v, out, lse, cu_q, cu_k, max_q, max_k, *, scale, causal=True
     cu_q = cu_q.to(torch.int32)
     cu_k = cu_k.to(torch.int32)
     det = deterministic_default() if deterministic is None else bool(deterministic)
-    sem = torch.zeros(1 + (Tq // 128 + nseq) * H, dtype=torch.int32, device=q.device) if det else None
+    sem = torch.zeros(1 + (Tq // 128 + nseq) * H * 4, dtype=torch.int32, device=q.device) if det else None
     rc = lib.ftb_attn_bwd(_ptr(dout), _ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(lse), _ptr(delta), _ptr(dq_acc),
                           _ptr(sem), _ptr(dq), _ptr(dk), _ptr(dv), _ptr(cu_q), _ptr(cu_k), c_int(nseq), c_int(Tq), c_int(Tk),
                           c_int(H), c_int(KV), c_int(hd), c_long(q.stride(0)), c_long(k.stride(0)),
                           c_long(v.stride(0)), c_long(dout.stride(0)), c_long(out.stride(0)), c_float(scale),
                           c_float(float(softcap or 0.0)), c_int(1 if causal else 0), c_int(int(window or 0)),
-                          c_int(Tk // 128 + nseq), _stream())
+                          c_int(Tk // 128 + nseq), c_int(int(max_k)), _stream())
     _check(rc, "ftb_attn_bwd")
     dq.copy_(dq_acc)
     return dq, dk, dv

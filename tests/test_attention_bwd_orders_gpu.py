@@ -1,0 +1,58 @@
+"""Attention backward at the sizes where its order of work and its pipeline change: one tile pair, few pairs (the software
+pipeline's start and end), many short sequences (the warp-wide tile search crosses 32), and both fixed orders of dQ."""
+
+import pytest
+import torch
+
+from flextrain_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+CASES = {                                       # lens_q, lens_k, H, KV, window, softcap
+    "one_pair": ([128], [128], 1, 1, 0, 0.0),
+    "one_token": ([1, 2], [1, 2], 2, 1, 0, 0.0),
+    "two_pairs": ([129], [129], 1, 1, 0, 0.0),
+    "rep_three": ([257, 5], [257, 5], 3, 1, 0, 0.0),
+    "more_than_32_sequences": ([3 + 5 * i for i in range(70)], [3 + 5 * i for i in range(70)], 4, 2, 0, 0.0),
+    "prior": ([130, 64], [700, 300], 4, 2, 0, 0.0),
+    "more_queries_than_keys": ([300], [100], 2, 1, 0, 0.0),
+    "in_step": ([2300], [2300], 8, 1, 0, 0.0),
+    "in_step_prior": ([500, 77], [2333, 99], 8, 1, 0, 0.0),
+    "in_step_window": ([2300, 300], [2300, 300], 8, 1, 200, 0.0),
+    "in_step_softcap": ([2300], [2300], 8, 1, 0, 20.0),
+    "in_step_window_prior": ([600], [2500], 16, 2, 129, 0.0),
+}
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("name", list(CASES))
+def test_attention_bwd(hd, name):
+    """dQ, dK, dV against the fp32 reference: P and dS are rounded to bf16 (2^-9 relative each) before products whose
+    terms add up at random, and the results once more, so the relative error of a whole tensor stays below 2^-6.  The fixed
+    order repeats bit for bit and agrees with the free one to fp32 rounding before the result is rounded to bf16."""
+    from flextrain_b200.ops import attention_cuda as fa
+    from flextrain_b200.ops import cuda as kk
+    lens_q, lens_k, H, KV, window, softcap = CASES[name]
+    if hd == 64 and name.startswith("in_step"):
+        H, KV = 2 * H, KV                       # the order changes at 256 pairs there
+    torch.manual_seed(1)
+    cu = lambda n: torch.tensor([0] + list(torch.tensor(n).cumsum(0)), dtype=torch.int32, device=DEV)
+    cu_q, cu_k = cu(lens_q), cu(lens_k)
+    mk = lambda n, h: torch.randn(n, h, hd, device=DEV).to(torch.bfloat16)
+    q, do, k, v = mk(sum(lens_q), H), mk(sum(lens_q), H), mk(sum(lens_k), KV), mk(sum(lens_k), KV)
+    kw = dict(scale=hd ** -0.5, window=window, softcap=softcap)
+    o, lse = fa.fwd(q, k, v, cu_q, cu_k, max(lens_q), max(lens_k), **kw)
+    blind = max(lens_q[0] - lens_k[0], 0)       # queries that see no key: the reference is given the others alone
+    cu_w = (cu_q - blind).clamp_min(0)
+    ow, lw = ref.attention_fwd(q[blind:], k, v, cu_w, cu_k, **kw)
+    want = list(ref.attention_bwd(do[blind:], q[blind:], k, v, ow, lw, cu_w, cu_k, **kw))
+    want[0] = torch.cat([want[0].new_zeros(blind, H, hd), want[0]])
+    got = [fa.bwd(do, q, k, v, o, lse, cu_q, cu_k, max(lens_q), max(lens_k), deterministic=d, **kw)
+           for d in (True, True, False)]
+    assert kk.device_error_words().get("attention", 0) == 0
+    for first, again, free, w in zip(*got, want):
+        assert torch.equal(first, again)
+        for g in (first, free):
+            assert torch.isfinite(g).all()
+            assert float((g.float() - w.float()).norm()) <= 2.0 ** -6 * float(w.float().norm()) + 1e-6
