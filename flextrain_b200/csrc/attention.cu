@@ -469,14 +469,16 @@ fa_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       constexpr uint32_t idesc_pv = make_idesc_bf16(TQ, HD, 0, 1);
       bool ok = mbar_wait(q_full, 0, abort_flag, 150);
       // S_t(j) = Q_t · K_jᵀ into the tile's score columns (they are free: the tile's P·V of j-1 was issued before)
+      const uint64_t dQ = make_smem_desc(smem_u32(sQ), 16, 1024), dK = make_smem_desc(smem_u32(sK), 16, 1024);
+      const uint64_t dV = make_smem_desc(smem_u32(sV), TK * 128, 1024);
       auto issue_s = [&](int t, int j) {
-        const uint32_t aQ = smem_u32(sQ + t * Q_BYTES), aK = smem_u32(sK + (j & 1) * KV_BYTES);
+        const uint64_t dq = dQ + t * (Q_BYTES >> 4), dk = dK + (j & 1) * (KV_BYTES >> 4);
 #pragma unroll
         for (int kb = 0; kb < KB; ++kb)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            umma_f16(tmem_base + t * TK, make_smem_desc(aQ + kb * (TQ * 128) + kk * 32, 16, 1024),
-                     make_smem_desc(aK + kb * (TK * 128) + kk * 32, 16, 1024), idesc_s, (kb | kk) != 0);
+            umma_f16(tmem_base + t * TK, dq + (kb * (TQ * 128) + kk * 32 >> 4), dk + (kb * (TK * 128) + kk * 32 >> 4), idesc_s,
+                     (kb | kk) != 0);
         umma_commit(&s_full[t]);
       };
       if (ok) ok = mbar_wait(&k_full[0], 0, abort_flag, 151);
@@ -498,11 +500,11 @@ fa_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           if (!ok || j >= nt) continue;
           if (!(ok = mbar_wait(&p_full[t], j & 1, abort_flag, 154 + t))) break;
           tc_fence_after();
-          const uint32_t aV = smem_u32(sV + st * KV_BYTES);
+          const uint64_t dv = dV + st * (KV_BYTES >> 4);
 #pragma unroll
           for (int s2 = 0; s2 < TK / 16; ++s2)       // P (tensor memory, 8 columns per 16 keys) times V
-            umma_f16_ts(tmem_base + 256 + t * HD, tmem_base + t * TK + s2 * 8,
-                        make_smem_desc(aV + s2 * (16 * 128), TK * 128, 1024), idesc_pv, (j | s2) != 0);
+            umma_f16_ts(tmem_base + 256 + t * HD, tmem_base + t * TK + s2 * 8, dv + s2 * (16 * 128 >> 4), idesc_pv,
+                        s2 == 0 ? j != 0 : 1);
           umma_commit(&o_full[t]);
           if (j + 1 < nt) issue_s(t, j + 1);
         }
@@ -803,10 +805,11 @@ namespace ftb {
 //   IN_STEP      key tiles ascending, query tiles descending with the heads of the group inside: all key tiles of a
 //                sequence walk the same (query tile, head) list in step, the short ones leave it early.  The longest CTAs
 //                come first; the price is a wait per key tile at the start and additions that meet at the same addresses.
-// 32 / 8 heads of 128, LAST_FIRST against IN_STEP: 16 x 1024 tokens 646 / 722 us, 4 x 4096 2157 / 2169, 2 x 8192 4569 /
-// 3974, 1 x 16384 9699 / 7760; 16 / 8 heads: 2 x 8192 2016 / 2048, 1 x 16384 4294 / 3971; 16 / 16 heads: 1 x 16384 3986 /
-// 4257, 1 x 32768 16249 / 16626; head dim 64, 32 / 8 heads: 2 x 8192 3050 / 3370, 1 x 16384 7190 / 6794.  So IN_STEP where
-// the longest CTA walks more than 128 pairs (256 at head dim 64, whose pairs are shorter) and heads share keys.
+// With a fixed order, LAST_FIRST against IN_STEP, us: head dim 128, 32 / 8 heads: 16 x 1024 tokens 614 / 635, 4 x 4096
+// 2033 / 2056, 2 x 8192 4253 / 3824, 1 x 16384 9406 / 8411; 16 / 16 heads: 4 x 4096 1061 / 1165, 2 x 8192 1930 / 1892,
+// 1 x 16384 4183 / 3702; 16 / 8 heads: 2 x 8192 1943 / 2043, 1 x 16384 4146 / 3860.  Head dim 64, 32 / 8 heads: 8 x 2048
+// 808 / 774, 1 x 16384 5826 / 5054.  So IN_STEP where the longest sequence has more than 4096 keys (1024 at head dim 64,
+// whose tile pairs are shorter).
 constexpr int BWD_FIRST_FIRST = 0, BWD_LAST_FIRST = 1, BWD_IN_STEP = 2;
 
 struct BwdParams {
@@ -856,22 +859,26 @@ __global__ void fa_delta_kernel(const __nv_bfloat16* __restrict__ dout, long do_
   if (part == 0) delta[(size_t)h * T + t] = s;
 }
 
-// Backward thread layout: warp 0 TMA, warp 1 MMA, warps 2-9 softmax, warps 10-13 dQ drain.
+// Backward thread layout: warps 0-7 softmax, warps 8-11 dQ drain, warp 12 loads, warp 13 MMA.
 //
 // Scores are formed transposed (Sᵀ = K·Qᵀ, dPᵀ = V·dOᵀ; one key row per thread), so that Pᵀ goes back into tensor memory
 // as packed bf16 over the score columns it came from and is the A operand of dV += Pᵀ·dO without touching shared memory.
 // dSᵀ is one shared tile that feeds dK += dSᵀ·Q (K-major) and dQ = dS·K (M-major).  The MMAs are issued one query tile
 // ahead:
-//     ... dQ(j) dK(j) | dP(j+1) dV(j+1) S(j+2) | dQ(j+1) dK(j+1) ...
-// P(j+1) is computed under dQ(j), dK(j) and dP(j+1); dS(j+1) under dV(j+1) and S(j+2); the dQ tile is drained by warps of
-// its own under dK(j) and what follows.  At head dim 128 the tensor memory is full (S, dP, dV, dK) and dQ(j) takes dP(j)'s
-// columns, which the softmax warps have read by then; dP(j+1) waits until they are drained.
+//     ... dQ(j) S(j+1) dK(j) | dP(j+1) dV(j+1) | dQ(j+1) S(j+2) dK(j+1) ...
+// P(j+1) is computed under dK(j) and dP(j+1); dS(j+1) under dV(j+1); the dQ tile is emptied by warps of its own under
+// S(j+1) and dK(j), and leaves under what follows; Q(j+2) takes the place of Q(j) and has dP, dV and dQ of j+1 to arrive.
+// At head dim 128 the tensor memory is full (S, dP, dV, dK) and dQ(j) takes dP(j)'s columns, which the softmax warps have
+// read by then; dP(j+1) waits until they are empty.
 // Two softmax warps share a tensor-memory lane quadrant (rows) and split the 128 query columns.
-// Bound by shared-memory bandwidth: a tile pair takes 2560 cycles of tensor core at hd 128, but the four products with
-// both operands in shared memory, the dQ staging and the tile loads move some 4300 cycles' worth of it.
+//
+// In the transposed scores a query's lse and delta belong to a column, the same for all 32 lanes: read from shared memory
+// they cost a pass of its pipe per warp and column, 1500 cycles a tile pair, half of them in the chain.  Instead the tensor
+// core subtracts them: one more step of 16 in the reduction, whose A rows are (1, 1, 1, 0 ...) and whose B rows hold
+// -lse / scale (or -delta) as the sum of three bf16 (24 bits, as exact as the fp32 value).
 // Causal, 32 / 8 heads of 128, dQ in any order: 16 x 1024 tokens 771 us with one chain S, dP -> softmax -> dV, dK, dQ ->
-// drain per tile pair, 580 us so; 1 x 16384 9160 us (600 TFLOP/s) before, 6420 us (856) so.  With dQ in a fixed order 926 ->
-// 646 us and 12300 -> 7640 us.
+// drain per tile pair, 506 us so; 1 x 16384 9160 us (600 TFLOP/s) before, 5510 us (997) so.  With dQ in a fixed order 926 ->
+// 613 us and 12300 -> 6990 us.
 constexpr int FAB_THREADS = 448;
 constexpr int FAB_SOFTMAX_WARPS = 8;
 
@@ -880,18 +887,43 @@ __device__ __forceinline__ float ex2_approx(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-
 // One answer for the whole warp: its lanes go on together or leave their loops together.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int where) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, where));
+}
+
+// A 128 x 16 bf16 operand (K-major, 32-byte swizzle): row r is 32 bytes, its two 16-byte halves swapped in every other
+// group of four rows; eight rows (256 bytes) repeat.
+constexpr int AUG_BYTES = 128 * 32;
+__device__ __forceinline__ uint64_t make_aug_desc(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
+  d |= static_cast<uint64_t>(1) << 16;            // LBO: not used, one atom wide
+  d |= static_cast<uint64_t>(256 >> 4) << 32;     // SBO: eight rows
+  d |= static_cast<uint64_t>(1) << 46;            // descriptor version (Blackwell)
+  d |= static_cast<uint64_t>(6) << 61;            // SWIZZLE_32B
+  return d;
+}
+__device__ __forceinline__ void write_aug_row(uint8_t* tile, int row, float v) {
+  const __nv_bfloat16 hi = __float2bfloat16(v);
+  float rest = v - __bfloat162float(hi);
+  if (!isfinite(v)) rest = 0.f;                   // an infinite or undefined value stands alone
+  const __nv_bfloat16 mid = __float2bfloat16(rest);
+  const __nv_bfloat16 lo = __float2bfloat16(rest - __bfloat162float(mid));
+  const __nv_bfloat162 a = __halves2bfloat162(hi, mid), b = __halves2bfloat162(lo, __float2bfloat16(0.f));
+  const int swap = (row >> 2) & 1;
+  *reinterpret_cast<uint4*>(tile + row * 32 + swap * 16) =
+      make_uint4(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b), 0u, 0u);
+  *reinterpret_cast<uint4*>(tile + row * 32 + (swap ^ 1) * 16) = make_uint4(0u, 0u, 0u, 0u);
 }
 
 template <int HD>
 struct BwdSmem {
   static constexpr int T_BYTES = 128 * HD * 2;       // one Q / dO / K / V tile
   static constexpr int DS_BYTES = 128 * 128 * 2;
-  static constexpr int STAGE_BYTES = 32 * 32 * 4;    // 32 rows x 32 fp32 columns of dQ; two per drain warp
-  static constexpr int USED = 5 * T_BYTES + DS_BYTES + 8 * STAGE_BYTES + 2 * 2 * 128 * 4 + 256;
+  static constexpr int STAGE_BYTES = 32 * 32 * 4;    // 32 rows x 32 fp32 columns of dQ; STAGES of them per drain warp
+  static constexpr int STAGES = HD == 128 ? 1 : 2;
+  static constexpr int USED = 5 * T_BYTES + DS_BYTES + 4 * STAGES * STAGE_BYTES + 3 * AUG_BYTES + 256;
   static constexpr int SIZE = USED + 1024 < 232448 ? USED + 1024 : 232448;      // the 227 KB a CTA may have
 };
 
@@ -911,15 +943,18 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   uint8_t* sQ = sV + T_BYTES;                 // 2 stages
   uint8_t* sDO = sQ + 2 * T_BYTES;
   uint8_t* sDS = sDO + T_BYTES;
-  uint8_t* sStg = sDS + L::DS_BYTES;          // dQ staging, two blocks for each drain warp
-  float* sStat = reinterpret_cast<float*>(sStg + 8 * L::STAGE_BYTES);     // [stage][lse2 | delta][128]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + 2 * 2 * 128);
+  uint8_t* sStg = sDS + L::DS_BYTES;          // dQ staging
+  uint8_t* sOnes = sStg + 4 * L::STAGES * L::STAGE_BYTES;
+  uint8_t* sLse = sOnes + AUG_BYTES;                        // -lse / scale of the query tile
+  uint8_t* sDelta = sLse + AUG_BYTES;                       // -delta
+  float* sStat = reinterpret_cast<float*>(sLse);            // with soft-cap instead: [stage][128] lse in log2 units
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sDelta + AUG_BYTES);
   uint64_t* kv_full = bars;
   uint64_t* q_full = bars + 1;                // 2
   uint64_t* q_empty = bars + 3;               // 2
   uint64_t* do_full = bars + 5;
   uint64_t* do_empty = bars + 6;
-  uint64_t* stat_full = bars + 7;             // 2
+  uint64_t* lse_full = bars + 7;              // 2
   uint64_t* s_full = bars + 9;
   uint64_t* p_full = bars + 10;
   uint64_t* dp_full = bars + 11;
@@ -927,7 +962,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   uint64_t* dq_full = bars + 13;
   uint64_t* dq_empty = bars + 14;
   uint64_t* acc_full = bars + 15;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint64_t* delta_full = bars + 16;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   if (smem + L::USED > smem_raw + L::SIZE) {  // the base of the block's shared memory is aligned in practice
     set_error(5, 241);
@@ -965,15 +1001,22 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     mbar_init(kv_full, 1); mbar_init(do_full, 1); mbar_init(do_empty, 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); mbar_init(&stat_full[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); mbar_init(&lse_full[i], 1); }
+    mbar_init(delta_full, 1);
     mbar_init(s_full, 1); mbar_init(p_full, FAB_SOFTMAX_WARPS); mbar_init(dp_full, 1);
     mbar_init(ds_full, FAB_SOFTMAX_WARPS); mbar_init(dq_full, 1); mbar_init(dq_empty, 4); mbar_init(acc_full, 1);
     fence_barrier_init();
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmDO); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
   }
-  if (warp == 1) {
+  if (warp == 13) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
+  }
+  if (threadIdx.x < 128) {                    // the constant A rows (1, 1, 1, 0 ...)
+    const int swap = (threadIdx.x >> 2) & 1;
+    *reinterpret_cast<uint4*>(sOnes + threadIdx.x * 32 + swap * 16) = make_uint4(0x3f803f80u, 0x00003f80u, 0u, 0u);
+    *reinterpret_cast<uint4*>(sOnes + threadIdx.x * 32 + (swap ^ 1) * 16) = make_uint4(0u, 0u, 0u, 0u);
+    fence_proxy_async();
   }
   tc_fence_before();
   __syncthreads();
@@ -982,7 +1025,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   const uint32_t tm_S = tmem_base, tm_dP = tmem_base + 128, tm_dV = tmem_base + 256, tm_dK = tmem_base + 256 + HD;
   const uint32_t tm_dQ = DQ_OVER_DP ? tm_dP : tmem_base + 256 + 2 * HD;
 
-  if (warp == 0) {
+  if (warp == 12) {
     // ------------------------------------------------------------------------- loads
     if (lane == 0 && n_iter > 0) {
       mbar_expect_tx(kv_full, 2 * T_BYTES);
@@ -992,10 +1035,19 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         tma_load_3d(sV + kb * (128 * 128), &tmV, kv_full, kb * 64, kvh, ks + k0);
       }
     }
+    const float inv_scale = 1.f / p.scale;
     int h = kvh * rep, qt = qt_first;
     for (int it = 0; it < n_iter; ++it) {
       const int st = it & 1;
-      // the stage's last tenant has been through its dK product, so its row statistics have been read as well
+      float l[4], dl[4];
+      const size_t base = static_cast<size_t>(h) * p.total_q + qs + qt;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const bool vq = qt + e * 32 + lane < len_q;
+        l[e] = vq ? p.lse[base + e * 32 + lane] : -INFINITY;
+        dl[e] = vq ? p.delta[base + e * 32 + lane] : 0.f;
+      }
+      // the stage's last tenant has been through its dK product
       if (!mbar_wait_warp(&q_empty[st], ((it >> 1) & 1) ^ 1, abort_flag, 210)) break;
       if (lane == 0) {
         mbar_expect_tx(&q_full[st], T_BYTES);
@@ -1003,18 +1055,19 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         for (int kb = 0; kb < KB; ++kb)
           tma_load_3d(sQ + st * T_BYTES + kb * (128 * 128), &tmQ, &q_full[st], kb * 64, h, qs + qt);
       }
-      float* stat = sStat + st * 256;
-      const size_t base = static_cast<size_t>(h) * p.total_q + qs + qt;
+      if constexpr (CAP) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int q = e * 32 + lane;
-        const bool vq = qt + q < len_q;
-        const float l = vq ? p.lse[base + q] : -INFINITY;
-        stat[q] = l == -INFINITY ? INFINITY : l * 1.4426950408889634f;     // past the end, or sees no key: P = 0
-        stat[128 + q] = vq ? p.delta[base + q] : 0.f;
+        for (int e = 0; e < 4; ++e)            // a query past the end, or one that sees no key: P = 0
+          sStat[st * 128 + e * 32 + lane] = l[e] == -INFINITY ? INFINITY : l[e] * 1.4426950408889634f;
+      } else {
+        if (it > 0 && !mbar_wait_warp(s_full, (it - 1) & 1, abort_flag, 212)) break;     // S of the last tile has read it
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          write_aug_row(sLse, e * 32 + lane, l[e] == -INFINITY ? copysignf(1e30f, -p.scale) : -l[e] * inv_scale);
+        fence_proxy_async();
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&stat_full[st]);
+      if (lane == 0) mbar_arrive(&lse_full[st]);
       if (!mbar_wait_warp(do_empty, (it & 1) ^ 1, abort_flag, 211)) break;
       if (lane == 0) {
         mbar_expect_tx(do_full, T_BYTES);
@@ -1022,24 +1075,39 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         for (int kb = 0; kb < KB; ++kb)
           tma_load_3d(sDO + kb * (128 * 128), &tmDO, do_full, kb * 64, h, qs + qt);
       }
+      // (dV of the last tile is done, so its dP, which has read these rows, is too)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) write_aug_row(sDelta, e * 32 + lane, -dl[e]);
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(delta_full);
       next_tile(h, qt);
     }
-  } else if (warp == 1) {
+  } else if (warp == 13) {
     // --------------------------------------------------------------------------- MMA issuer
     if (lane == 0 && n_iter > 0) {
       constexpr uint32_t id_s = make_idesc_bf16(128, 128, 0, 0);       // Sᵀ, dPᵀ: both operands K-major
       constexpr uint32_t id_v = make_idesc_bf16(128, HD, 0, 1);        // dV (A in tensor memory), dK: MN-major B
       constexpr uint32_t id_q = make_idesc_bf16(128, HD, 1, 1);        // dQ: transposed A, MN-major B
-      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ0 = smem_u32(sQ), aDO = smem_u32(sDO), aDS = smem_u32(sDS);
+      // Operand descriptors of whole tiles, K-major (_k) and MN-major (_m); a step adds its byte offset / 16.  Built once: with
+      // a descriptor put together for every MMA this thread needed some 100 cycles for each, and the tensor core 64.
+      const uint64_t dK_k = make_smem_desc(smem_u32(sK), 16, 1024), dK_m = make_smem_desc(smem_u32(sK), 128 * 128, 1024);
+      const uint64_t dV_k = make_smem_desc(smem_u32(sV), 16, 1024);
+      const uint64_t dQ_k = make_smem_desc(smem_u32(sQ), 16, 1024), dQ_m = make_smem_desc(smem_u32(sQ), 128 * 128, 1024);
+      const uint64_t dDO_k = make_smem_desc(smem_u32(sDO), 16, 1024), dDO_m = make_smem_desc(smem_u32(sDO), 128 * 128, 1024);
+      const uint64_t dDS_k = make_smem_desc(smem_u32(sDS), 16, 1024), dDS_m = make_smem_desc(smem_u32(sDS), 128 * 128, 1024);
+      const uint64_t dOnes = make_aug_desc(smem_u32(sOnes)), dLse = make_aug_desc(smem_u32(sLse));
+      const uint64_t dDelta = make_aug_desc(smem_u32(sDelta));
       auto issue_s = [&](int j) {
-        const uint32_t aQ = aQ0 + (j & 1) * T_BYTES;
+        const uint64_t dq = dQ_k + (j & 1) * (T_BYTES >> 4);
 #pragma unroll
         for (int kb = 0; kb < KB; ++kb)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {
-            const uint32_t o = kb * (128 * 128) + kk * 32;
-            umma_f16(tm_S, make_smem_desc(aK + o, 16, 1024), make_smem_desc(aQ + o, 16, 1024), id_s, (kb | kk) != 0);
+            const uint32_t o = (kb * (128 * 128) + kk * 32) >> 4;
+            umma_f16(tm_S, dK_k + o, dq + o, id_s, (kb | kk) != 0);
           }
+        if constexpr (!CAP) umma_f16(tm_S, dOnes, dLse, id_s, 1);
         umma_commit(s_full);
       };
       auto issue_dp = [&]() {
@@ -1047,58 +1115,63 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         for (int kb = 0; kb < KB; ++kb)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {
-            const uint32_t o = kb * (128 * 128) + kk * 32;
-            umma_f16(tm_dP, make_smem_desc(aV + o, 16, 1024), make_smem_desc(aDO + o, 16, 1024), id_s, (kb | kk) != 0);
+            const uint32_t o = (kb * (128 * 128) + kk * 32) >> 4;
+            umma_f16(tm_dP, dV_k + o, dDO_k + o, id_s, (kb | kk) != 0);
           }
+        umma_f16(tm_dP, dOnes, dDelta, id_s, 1);
         umma_commit(dp_full);
       };
       auto issue_dv = [&](int j) {          // Pᵀ: 16 queries in 8 columns; the second half starts at column 64
 #pragma unroll
         for (int s = 0; s < 8; ++s)
-          umma_f16_ts(tm_dV, tm_S + (s >> 2) * 64 + (s & 3) * 8, make_smem_desc(aDO + s * (16 * 128), 128 * 128, 1024),
-                      id_v, (j | s) != 0);
+          umma_f16_ts(tm_dV, tm_S + (s >> 2) * 64 + (s & 3) * 8, dDO_m + s * (16 * 128 >> 4), id_v, s == 0 ? j != 0 : 1);
         umma_commit(do_empty);
       };
-      bool ok = mbar_wait(kv_full, 0, abort_flag, 220) && mbar_wait(&q_full[0], 0, abort_flag, 221);
+      bool ok = mbar_wait(kv_full, 0, abort_flag, 220) && mbar_wait(&q_full[0], 0, abort_flag, 221) &&
+                (CAP || mbar_wait(&lse_full[0], 0, abort_flag, 221));
       if (ok) { tc_fence_after(); issue_s(0); }
       for (int j = -1; j < n_iter && ok; ++j) {
+        const bool more = j + 1 < n_iter;
         if (j >= 0) {
           if (!(ok = mbar_wait(ds_full, j & 1, abort_flag, 222))) break;
           if (!DQ_OVER_DP && j > 0 && !(ok = mbar_wait(dq_empty, (j - 1) & 1, abort_flag, 223))) break;
           tc_fence_after();
-          const uint32_t aQ = aQ0 + (j & 1) * T_BYTES;
 #pragma unroll
           for (int s = 0; s < 8; ++s)        // reduction over the 128 keys, 16 per step
-            umma_f16(tm_dQ, make_smem_desc(aDS + s * (16 * 128), 128 * 128, 1024),
-                     make_smem_desc(aK + s * (16 * 128), 128 * 128, 1024), id_q, s != 0);
+            umma_f16(tm_dQ, dDS_m + s * (16 * 128 >> 4), dK_m + s * (16 * 128 >> 4), id_q, s != 0);
           umma_commit(dq_full);
+          if (more) {
+            if (!(ok = mbar_wait(&q_full[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag, 227))) break;
+            if (!CAP && !(ok = mbar_wait(&lse_full[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag, 228))) break;
+            tc_fence_after();
+            issue_s(j + 1);
+          }
+          // what dP(j+1) needs has normally come by now; waited for here, the waits cost nothing behind S and before dK
+          if (more && !(ok = mbar_wait(do_full, (j + 1) & 1, abort_flag, 224))) break;
+          if (more && !(ok = mbar_wait(delta_full, (j + 1) & 1, abort_flag, 229))) break;
+          if (more && DQ_OVER_DP && !(ok = mbar_wait(dq_empty, j & 1, abort_flag, 225))) break;
+          const uint64_t dq = dQ_m + (j & 1) * (T_BYTES >> 4);
 #pragma unroll
           for (int s = 0; s < 8; ++s)        // reduction over the 128 queries
-            umma_f16(tm_dK, make_smem_desc(aDS + (s >> 2) * (128 * 128) + (s & 3) * 32, 16, 1024),
-                     make_smem_desc(aQ + s * (16 * 128), 128 * 128, 1024), id_v, (j | s) != 0);
+            umma_f16(tm_dK, dDS_k + ((s >> 2) * (128 * 128 >> 4) + (s & 3) * 2), dq + s * (16 * 128 >> 4), id_v,
+                     s == 0 ? j != 0 : 1);
           umma_commit(&q_empty[j & 1]);
         }
-        if (j + 1 < n_iter) {
-          if (!(ok = mbar_wait(do_full, (j + 1) & 1, abort_flag, 224))) break;
-          if (DQ_OVER_DP && j >= 0 && !(ok = mbar_wait(dq_empty, j & 1, abort_flag, 225))) break;
+        if (more) {
+          if (j < 0 && !(ok = mbar_wait(do_full, 0, abort_flag, 224) && mbar_wait(delta_full, 0, abort_flag, 229))) break;
           tc_fence_after();
           issue_dp();
           if (!(ok = mbar_wait(p_full, (j + 1) & 1, abort_flag, 226))) break;
           tc_fence_after();
           issue_dv(j + 1);
         }
-        if (j + 2 < n_iter) {
-          if (!(ok = mbar_wait(&q_full[(j + 2) & 1], ((j + 2) >> 1) & 1, abort_flag, 227))) break;
-          tc_fence_after();
-          issue_s(j + 2);
-        }
       }
       if (ok) umma_commit(acc_full);
     }
-  } else if (warp < 2 + FAB_SOFTMAX_WARPS) {
+  } else if (warp < FAB_SOFTMAX_WARPS) {
     // ------------------------------------------------------------------------- softmax: P and dS
     const int quad = warp & 3;
-    const int half = (warp - 2) >> 2;               // which half of the query columns this warp owns
+    const int half = warp >> 2;                     // which half of the query columns this warp owns
     const int r = quad * 32 + lane;                 // key row inside the tile
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
     const float c = p.scale * 1.4426950408889634f;
@@ -1109,12 +1182,11 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     int h = kvh * rep, qt = qt_first;
     for (int it = 0; it < n_iter && ok; ++it) {
       const uint32_t ph = it & 1;
-      const float4* lse4 = reinterpret_cast<const float4*>(sStat + ph * 256 + half * 64);
-      const float4* dl4 = lse4 + 32;
+      const float4* lse4 = reinterpret_cast<const float4*>(sStat + ph * 128 + half * 64);      // (soft-cap)
       // a tile needs masking only if it touches the end of the queries / keys, the causal diagonal or the window edge
       const bool edge = (qt + 128 > len_q) || (k0 + 128 > len_k) ||
                         (p.causal && (k0 + 127 > qt + off || (p.window > 0 && k0 <= qt + 127 + off - p.window)));
-      if (!(ok = mbar_wait_warp(&stat_full[ph], (it >> 1) & 1, abort_flag, 230))) break;
+      if (CAP && !(ok = mbar_wait_warp(&lse_full[ph], (it >> 1) & 1, abort_flag, 230))) break;
       if (!(ok = mbar_wait_warp(s_full, ph, abort_flag, 231))) break;
       tc_fence_after();
       uint32_t sv[2][32];                           // scores, then P (with soft-cap: the raw scores)
@@ -1138,16 +1210,19 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         uint32_t pk[16];
 #pragma unroll
         for (int g = 0; g < 8; ++g) {
-          const float4 l4 = lse4[q2 * 8 + g];
-          const float ls[4] = {l4.x, l4.y, l4.z, l4.w};
           float pe[4];
+          if constexpr (CAP) {
+            const float4 l4 = lse4[q2 * 8 + g];
+            const float ls[4] = {l4.x, l4.y, l4.z, l4.w};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float s = __uint_as_float(sv[q2][g * 4 + e]);
-            if constexpr (CAP) {
+            for (int e = 0; e < 4; ++e) {
+              const float s = __uint_as_float(sv[q2][g * 4 + e]);
               pe[e] = s == -INFINITY ? 0.f : ex2_approx(cap2 * tanh_fast(s * soc) - ls[e]);
-            } else {
-              pe[e] = ex2_approx(s * c - ls[e]);
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              pe[e] = ex2_approx(__uint_as_float(sv[q2][g * 4 + e]) * c);      // (the score less lse / scale)
               sv[q2][g * 4 + e] = __float_as_uint(pe[e]);
             }
           }
@@ -1166,13 +1241,11 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       tc_fence_after();
 #pragma unroll
       for (int q2 = 0; q2 < 2; ++q2) {
-        uint32_t vd[32];
+        uint32_t vd[32];                            // dP - delta
         tmem_ld_32x32(tm_dP + lane_base + half * 64 + q2 * 32, vd);
         tmem_ld_wait();
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
-          const float4 da = dl4[q2 * 8 + g * 2], db = dl4[q2 * 8 + g * 2 + 1];
-          const float dl[8] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w};
           float ds[8];
           if constexpr (CAP) {
             const float4 la = lse4[q2 * 8 + g * 2], lb = lse4[q2 * 8 + g * 2 + 1];
@@ -1183,12 +1256,12 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
               const float th = tanh_fast(s * soc);
               const float pe = s == -INFINITY ? 0.f : ex2_approx(cap2 * th - ls[e]);
               // d(cap * tanh(scale * s / cap)) / ds = scale * (1 - tanh^2); the scale follows on dQ and dK
-              ds[e] = pe * (__uint_as_float(vd[g * 8 + e]) - dl[e]) * (1.f - th * th);
+              ds[e] = pe * __uint_as_float(vd[g * 8 + e]) * (1.f - th * th);
             }
           } else {
 #pragma unroll
             for (int e = 0; e < 8; ++e)
-              ds[e] = __uint_as_float(sv[q2][g * 8 + e]) * (__uint_as_float(vd[g * 8 + e]) - dl[e]);
+              ds[e] = __uint_as_float(sv[q2][g * 8 + e]) * __uint_as_float(vd[g * 8 + e]);
           }
           uint4 b;
           __nv_bfloat162* b2 = reinterpret_cast<__nv_bfloat162*>(&b);
@@ -1206,49 +1279,58 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     // dK / dV of this key tile (thread = key row)
     constexpr int HC2 = HD / 2;
     if (n_iter > 0 && ok) ok = mbar_wait_warp(acc_full, 0, abort_flag, 233);
-    const size_t row = static_cast<size_t>(ks + k0 + min(r, kr - 1));
-    __nv_bfloat16* dk_row = p.dk + (row * p.KV + kvh) * HD;
-    __nv_bfloat16* dv_row = p.dv + (row * p.KV + kvh) * HD;
-    if (n_iter == 0 || !ok) {
-      if (r < kr)
-        for (int cidx = half * HC2; cidx < half * HC2 + HC2; cidx += 8) {
-          *reinterpret_cast<uint4*>(dk_row + cidx) = make_uint4(0, 0, 0, 0);
-          *reinterpret_cast<uint4*>(dv_row + cidx) = make_uint4(0, 0, 0, 0);
-        }
-    } else {
-      tc_fence_after();
+    // Through shared memory (the Q stages, which nothing reads any more), so that the stores to global memory are whole
+    // rows: a row per thread wrote 32 lines an instruction, 4.0 us a tile.
+    const bool have = n_iter > 0 && ok;
+    tc_fence_after();
 #pragma unroll 1
-      for (int cb = half * HC2; cb < half * HC2 + HC2; cb += 32) {
-        uint32_t a[32], b[32];
+    for (int cb = half * HC2; cb < half * HC2 + HC2; cb += 32) {
+      uint32_t a[32], b[32];
+      if (have) {
         tmem_ld_32x32(tm_dV + lane_base + cb, a);
         tmem_ld_32x32(tm_dK + lane_base + cb, b);
         tmem_ld_wait();
-        if (r < kr) {
+      }
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            uint4 x, y;
-            __nv_bfloat162* x2 = reinterpret_cast<__nv_bfloat162*>(&x);
-            __nv_bfloat162* y2 = reinterpret_cast<__nv_bfloat162*>(&y);
+      for (int g = 0; g < 4; ++g) {
+        uint4 x = make_uint4(0, 0, 0, 0), y = x;
+        if (have) {
+          __nv_bfloat162* x2 = reinterpret_cast<__nv_bfloat162*>(&x);
+          __nv_bfloat162* y2 = reinterpret_cast<__nv_bfloat162*>(&y);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              x2[e] = __floats2bfloat162_rn(__uint_as_float(a[g * 8 + 2 * e]), __uint_as_float(a[g * 8 + 2 * e + 1]));
-              y2[e] = __floats2bfloat162_rn(__uint_as_float(b[g * 8 + 2 * e]) * p.scale,
-                                            __uint_as_float(b[g * 8 + 2 * e + 1]) * p.scale);
-            }
-            *reinterpret_cast<uint4*>(dv_row + cb + g * 8) = x;
-            *reinterpret_cast<uint4*>(dk_row + cb + g * 8) = y;
+          for (int e = 0; e < 4; ++e) {
+            x2[e] = __floats2bfloat162_rn(__uint_as_float(a[g * 8 + 2 * e]), __uint_as_float(a[g * 8 + 2 * e + 1]));
+            y2[e] = __floats2bfloat162_rn(__uint_as_float(b[g * 8 + 2 * e]) * p.scale,
+                                          __uint_as_float(b[g * 8 + 2 * e + 1]) * p.scale);
           }
         }
+        const uint32_t o = sw128_offset(r, cb + g * 8, 128);
+        *reinterpret_cast<uint4*>(sQ + o) = x;
+        *reinterpret_cast<uint4*>(sQ + T_BYTES + o) = y;
       }
     }
-  } else {
+    asm volatile("bar.sync 1, %0;" ::"n"(FAB_SOFTMAX_WARPS * 32) : "memory");
+    constexpr int CH = HD / 8;                      // 16-byte pieces of a row
+#pragma unroll 4
+    for (int i = threadIdx.x; i < 128 * CH; i += FAB_SOFTMAX_WARPS * 32) {
+      const int rr = i / CH, cc = (i % CH) * 8;
+      if (rr < kr) {
+        const size_t at = (static_cast<size_t>(ks + k0 + rr) * p.KV + kvh) * HD + cc;
+        const uint32_t o = sw128_offset(rr, cc, 128);
+        *reinterpret_cast<uint4*>(p.dv + at) = *reinterpret_cast<const uint4*>(sQ + o);
+        *reinterpret_cast<uint4*>(p.dk + at) = *reinterpret_cast<const uint4*>(sQ + T_BYTES + o);
+      }
+    }
+  } else if (warp < 12) {
     // ------------------------------------------------------------------------- dQ drain, 32 query rows a warp
     // Tensor memory -> registers -> fp32 staging in shared memory (blocks of 32 rows x 32 columns, 128-byte swizzle) ->
-    // tiled reduce-adds into the fp32 workspace: L2 sees whole 128-byte lines per reduction.  Each warp is on its own.
+    // tiled reduce-adds into the fp32 workspace: L2 sees whole 128-byte lines per reduction.  Each warp is on its own.  A
+    // tile of hd 128 takes some 4300 cycles to leave, about the rate at which an SM's reductions are taken (16 bytes a
+    // cycle); blocks of 16 rows took 7000, blocks of 64 rows shared by two warps (who then wait for each other) 6500.
     // Rows past the end of the sequence hold exact zeros (their P and dS were masked), so adding them is harmless.
     const int quad = warp & 3;
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
-    uint8_t* stg = sStg + quad * 2 * L::STAGE_BYTES;
+    uint8_t* stg = sStg + quad * L::STAGES * L::STAGE_BYTES;
     // index of this sequence's first query tile (semaphores)
     const int qtile_base = p.dq_sem != nullptr ? tiles_before(p.cu_q, seq, 128) : 0;
     auto stage = [&](int slot, const uint32_t (&v)[32]) {
@@ -1267,23 +1349,23 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         red_add_v4_f32(dst + e, __uint_as_float(v[e]) * p.scale, __uint_as_float(v[e + 1]) * p.scale,
                        __uint_as_float(v[e + 2]) * p.scale, __uint_as_float(v[e + 3]) * p.scale);
     };
+    // In a fixed order, a tile's turn passes on when its additions have been performed.  LAST_FIRST, whose next key tile
+    // comes a step later by itself, looks at that only before the staging block is needed again: waiting at once held this
+    // warp for another 1400 cycles a tile (16 x 1024 tokens 636 us against 613).  IN_STEP, where the next key tile is
+    // waiting, passes on at once (1 x 16384 7240 us against 6990).
+    int* passing = nullptr;
+    auto pass_on = [&]() {
+      if (passing != nullptr) {
+        bulk_wait_all();
+        red_release_gpu_add_s32(passing, 1);
+        passing = nullptr;
+      }
+    };
     int h = kvh * rep, qt = qt_first;
     for (int it = 0; it < n_iter; ++it) {
       if (!mbar_wait_warp(dq_full, it & 1, abort_flag, 235)) break;
       tc_fence_after();
       const bool live = qt + quad * 32 < len_q;
-      // the two halves of the tile's columns go through the same registers; the second is read before the first leaves
-      uint32_t v0[32], v1[32];
-      auto load_half = [&](int col) {
-        tmem_ld_32x32(tm_dQ + lane_base + col, v0);
-        tmem_ld_32x32(tm_dQ + lane_base + col + 32, v1);
-        tmem_ld_wait();
-      };
-      auto release = [&]() {                            // the columns may be written again
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(dq_empty);
-      };
       int* sem = nullptr;
       if (p.dq_sem != nullptr && live)
         // deterministic order, for each 32 rows of a query tile (word 0 of the array is the give-up flag)
@@ -1306,54 +1388,66 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
           __nanosleep(32);
         }
       };
-      if (!live) {
-        release();
-      } else if (p.dq_bulk) {
-        if (lane == 0) bulk_wait_read_all();            // the staging blocks have left
+      // Blocks of 32 columns; the first is staged as soon as it is read, so that three blocks of registers are enough to
+      // empty the columns before anything is waited for.
+      constexpr int NB = HD / 32;
+      uint32_t v[3][32];
+      auto load = [&](int cb) { tmem_ld_32x32(tm_dQ + lane_base + cb * 32, v[cb % 3]); };
+      load(0);
+      load(1);
+      if constexpr (NB > 2) load(2);
+      tmem_ld_wait();
+      if (live && p.dq_bulk) {
+        if (lane == 0) { pass_on(); bulk_wait_read_all(); }      // the last tile has left the staging blocks
         __syncwarp();
-        load_half(0);
-        stage(0, v0);
-        stage(1, v1);
-        if constexpr (HD == 128) load_half(64);
-        release();
-        fence_proxy_async();
+        stage(0, v[0]);
+        if constexpr (NB > 3) { load(3); tmem_ld_wait(); }
+      }
+      if (!live || p.dq_bulk) {
+        tc_fence_before();
         __syncwarp();
-        if (lane == 0) {
-          if (sem != nullptr) wait_turn();
-          tma_reduce_add_2d(&tmDQ, stg, h * HD, qs + qt + quad * 32);
-          tma_reduce_add_2d(&tmDQ, stg + L::STAGE_BYTES, h * HD + 32, qs + qt + quad * 32);
-          bulk_commit();
-        }
-        if constexpr (HD == 128) {
-          if (lane == 0) bulk_wait_read_all();
-          __syncwarp();
-          stage(0, v0);
-          stage(1, v1);
+        if (lane == 0) mbar_arrive(dq_empty);           // the columns may be written again
+      }
+      if (live && p.dq_bulk) {
+#pragma unroll
+        for (int cb = 0; cb < NB; cb += L::STAGES) {
+          if (cb > 0) {
+            if (lane == 0) bulk_wait_read_all();
+            __syncwarp();
+            stage(0, v[cb % 3]);
+          }
+          if constexpr (L::STAGES == 2) stage(1, v[(cb + 1) % 3]);
           fence_proxy_async();
           __syncwarp();
           if (lane == 0) {
-            tma_reduce_add_2d(&tmDQ, stg, h * HD + 64, qs + qt + quad * 32);
-            tma_reduce_add_2d(&tmDQ, stg + L::STAGE_BYTES, h * HD + 96, qs + qt + quad * 32);
+            if (cb == 0 && sem != nullptr) wait_turn();
+#pragma unroll
+            for (int i = 0; i < L::STAGES; ++i)
+              tma_reduce_add_2d(&tmDQ, stg + i * L::STAGE_BYTES, h * HD + (cb + i) * 32, qs + qt + quad * 32);
             bulk_commit();
           }
         }
-        if (lane == 0 && sem != nullptr) {
-          bulk_wait_all();                              // the additions have been performed: the next key tile may add
-          red_release_gpu_add_s32(sem, 1);
+        if (lane == 0) {
+          passing = sem;
+          if (in_step) pass_on();
         }
-      } else {                                          // 16-byte reductions, one row per thread
+      } else if (live) {                                // 16-byte reductions, one row per thread
         const int i = qt + quad * 32 + lane;
         float* dst = p.dq_acc + (static_cast<size_t>(qs + min(i, len_q - 1)) * p.H + h) * HD;
         if (lane == 0 && sem != nullptr) wait_turn();
         __syncwarp();
-#pragma unroll 1
-        for (int col = 0; col < HD; col += 64) {
-          load_half(col);
-          if (col + 64 == HD) release();
-          if (i < len_q) {
-            add_row(dst + col, v0);
-            add_row(dst + col + 32, v1);
-          }
+        if (i < len_q) add_row(dst, v[0]);
+        if constexpr (NB > 3) {
+          __syncwarp();
+          load(3);
+          tmem_ld_wait();
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(dq_empty);
+        if (i < len_q) {
+#pragma unroll
+          for (int cb = 1; cb < NB; ++cb) add_row(dst + cb * 32, v[cb % 3]);
         }
         if (sem != nullptr) {
           __threadfence();
@@ -1363,11 +1457,11 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       }
       next_tile(h, qt);
     }
-    if (p.dq_bulk && lane == 0) bulk_wait_all();        // none of this thread's reduce-adds outlives the kernel
+    if (p.dq_bulk && lane == 0) { pass_on(); bulk_wait_all(); }      // none of this thread's reduce-adds outlives the kernel
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 13) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
@@ -1439,9 +1533,7 @@ int ftb_attn_bwd(const void* dout, const void* q, const void* k, const void* v, 
   BwdParams p;
   p.cu_q = cu_q; p.cu_k = cu_k; p.num_seqs = num_seqs; p.H = H; p.KV = KV; p.dq_bulk = g_dq_bulk;
   p.dq_acc = dq_acc; p.dq_sem = dq_sem; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv; p.lse = lse; p.delta = delta;
-  const long pairs = (long)(H / KV) * ((max_k + 127) / 128);
-  p.order = dq_sem == nullptr ? BWD_FIRST_FIRST
-            : (H > KV && pairs > (hd == 128 ? 128 : 256)) ? BWD_IN_STEP : BWD_LAST_FIRST;
+  p.order = dq_sem == nullptr ? BWD_FIRST_FIRST : max_k > (hd == 128 ? 4096 : 1024) ? BWD_IN_STEP : BWD_LAST_FIRST;
   p.total_q = total_q; p.scale = scale; p.softcap = softcap; p.causal = causal; p.window = window;
   if (softcap > 0.f)
     rc = (hd == 128) ? launch_bwd<128, true>(tq, tdo, tk, tv, tdq, p, max_tiles, stream)
