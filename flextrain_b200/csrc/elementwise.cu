@@ -760,6 +760,59 @@ __global__ void __launch_bounds__(ADAM_THREADS) adamw_kernel(const __grid_consta
   }
 }
 
+// ------------------------------------------------------------------------ sum of squares
+// Sum of the squares of up to SQ_MAX tensors (the gradient norm): one pass that reads every element once, in place of a
+// conversion to fp32, a squaring and a reduction per tensor.  A block adds 16384 elements in fp32 (64 a thread, then a
+// tree) and leaves one partial sum; the second kernel adds the partials of all launches in double, always in the same order.
+// Bound by memory: 0.5 G bf16 elements in 50 tensors 2350 us with three passes a tensor, 205 us (5 TB/s) so.
+constexpr int SQ_MAX = 64;
+constexpr int SQ_THREADS = 256;
+constexpr int SQ_PER_BLOCK = SQ_THREADS * 64;
+struct SqTensor { const void* p; long n; long block_start; int dt, vec; };
+struct SqArgs { SqTensor t[SQ_MAX]; int count; };
+
+__global__ void __launch_bounds__(SQ_THREADS) sumsq_kernel(const __grid_constant__ SqArgs a, float* __restrict__ partial) {
+  __shared__ float sh[SQ_THREADS / 32];
+  int ti = 0;
+#pragma unroll 1
+  for (int i = 1; i < a.count; ++i)
+    if ((long)blockIdx.x >= a.t[i].block_start) ti = i;
+  const SqTensor& t = a.t[ti];
+  const long base = ((long)blockIdx.x - t.block_start) * SQ_PER_BLOCK;
+  float s = 0.f;
+#pragma unroll 4
+  for (int j = 0; j < 8; ++j) {
+    const long i = base + ((long)j * SQ_THREADS + threadIdx.x) * 8;
+    if (t.vec && i + 8 <= t.n) {
+      float f[8];
+      if (t.dt) unpack_raw8<true>(ld_raw8<true>(t.p, i), f);
+      else unpack_raw8<false>(ld_raw8<false>(t.p, i), f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s += f[e] * f[e];
+    } else {
+      for (long e = i; e < i + 8 && e < t.n; ++e) { const float f = ld_any(t.p, e, t.dt); s += f * f; }
+    }
+  }
+  s = block_sum<SQ_THREADS / 32>(s, sh);
+  if (threadIdx.x == 0) partial[blockIdx.x] = s;
+}
+
+__global__ void __launch_bounds__(1024) sumsq_total_kernel(const float* __restrict__ partial, long n, float* __restrict__ out) {
+  __shared__ double sh[32];
+  double s = 0.0;
+  for (long i = threadIdx.x; i < n; i += 1024) s += (double)partial[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = sh[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) out[0] = (float)s;
+  }
+}
+
 // ------------------------------------------------------------------- gated RMSNorm / L2
 __global__ void gated_rmsnorm_fwd_kernel(const bf16* __restrict__ o, const bf16* __restrict__ z,
                                          const float* __restrict__ w, bf16* __restrict__ y, long rows, int D,
@@ -1058,6 +1111,29 @@ int ftb_adamw_multi(int count, void** p, const void** g, void** m, void** v, con
   a.count = count; a.beta1 = beta1; a.beta2 = beta2; a.eps = eps; a.bc1 = bc1; a.bc2 = bc2; a.grad_scale = grad_scale;
   if (blocks == 0) return 0;
   adamw_kernel<<<(unsigned)blocks, ADAM_THREADS, 0, s>>>(a);
+  CHECK_LAUNCH();
+}
+
+// Blocks (partial sums) a tensor of n elements takes in ftb_sumsq.
+long ftb_sumsq_blocks(long n) { return (n + SQ_PER_BLOCK - 1) / SQ_PER_BLOCK; }
+// partial[0 .. blocks) of `count` <= 64 tensors, in order; then ftb_sumsq_total over the partials of all calls.
+int ftb_sumsq(int count, const void** p, const long* n, const int* dt, float* partial, cudaStream_t s) {
+  if (count <= 0) return 0;
+  if (count > SQ_MAX) return -2;
+  SqArgs a;
+  long blocks = 0;
+  for (int i = 0; i < count; ++i) {
+    a.t[i].p = p[i]; a.t[i].n = n[i]; a.t[i].block_start = blocks; a.t[i].dt = dt[i];
+    a.t[i].vec = ((uintptr_t)p[i] & 15) == 0;
+    blocks += ftb_sumsq_blocks(n[i]);
+  }
+  a.count = count;
+  if (blocks == 0) return 0;
+  sumsq_kernel<<<(unsigned)blocks, SQ_THREADS, 0, s>>>(a, partial);
+  CHECK_LAUNCH();
+}
+int ftb_sumsq_total(const float* partial, long n, float* out, cudaStream_t s) {
+  sumsq_total_kernel<<<1, 1024, 0, s>>>(partial, n, out);
   CHECK_LAUNCH();
 }
 

@@ -25,6 +25,7 @@ from typing import Dict, List, Optional, Sequence as Seq
 
 import torch
 
+from .. import ops
 from ..core.activation_schema import ON_DEVICE, ActivationSlot, fetch_home, send_home
 from ..core.layer import ChunkMeta, LayerContext
 from ..core.save_level import (HardwareCost, SaveLevelPlan, TransmissionScheduler, build_dp_tables,
@@ -314,25 +315,19 @@ class ActiveModel:
         bm = self.buffers
         self.streams.synchronize_all()
         dev = self.device
-        rep = torch.zeros((), dtype=torch.float32, device=dev)
-        part = torch.zeros((), dtype=torch.float32, device=dev)
         units = [(self.embed.param_spec, bm.embed_grads()), (self.head.param_spec, bm.head_grads())]
         for l, layer in enumerate(self.layers):
             g = bm.grads(l) if bm.grads_resident else _views(bm.host_g[l], bm.layers[l].g_layout)
             units.append((layer.param_spec, g))
+        rep, part = [], []                                     # replicated tensors, this rank's parts of others
         if getattr(self.embed, "train_encoders", False):       # a trainable vision tower: replicated, counted once
-            for g in self.embed.reduced_encoder_grads(self._encoder_group()).values():
-                rep += g.to(torch.float32).pow(2).sum().to(dev)
+            rep += self.embed.reduced_encoder_grads(self._encoder_group()).values()
         for spec, grads in units:
             for t in spec.trainable():
                 g = grads.get(t.grad_name)
-                if g is None:
-                    continue
-                sq = g.to(torch.float32).pow(2).sum().to(dev)
-                if t.is_local_part:
-                    part += sq
-                else:
-                    rep += sq
+                if g is not None:
+                    (part if t.is_local_part else rep).append(g)
+        rep, part = ops.sum_of_squares(rep, dev), ops.sum_of_squares(part, dev)
         group = self.tp or self.ep
         if group is not None:
             import torch.distributed as dist

@@ -386,6 +386,22 @@ def adamw_multi(params, grads, ms, vs, *, lrs, wds, beta1, beta2, eps, step, gra
                        grad_scale=grad_scale)
 
 
+def sum_of_squares(tensors, device):
+    """Sum of the squares of all elements of ``tensors`` as an fp32 scalar on ``device``; tensors the kernel cannot read
+    there (host gradients, other types or strides) are squared where they are."""
+    out = torch.zeros((), dtype=torch.float32, device=device)
+    ok = [t for t in tensors if t.is_cuda and t.device == out.device and t.is_contiguous() and t.numel()
+          and t.dtype in (torch.bfloat16, torch.float32)]
+    if ok:
+        _count((len(ok) + 63) // 64 + 1)
+        out = _kernels().sum_of_squares(ok)
+    taken = {id(t) for t in ok}
+    for t in tensors:
+        if id(t) not in taken:
+            out = out + t.to(torch.float32).pow(2).sum().to(device)
+    return out
+
+
 def newton_schulz_bf16(u: torch.Tensor, iters: int = 5) -> torch.Tensor:
     """Quintic Newton-Schulz orthogonalisation of one matrix on the tcgen05 GEMM, bf16 iterates with fp32
     accumulation: per iteration ``A = X Xᵀ``, ``B = bA + cA²`` (epilogue ``alpha=c, beta=b``), ``X = aX + BX``

@@ -441,6 +441,26 @@ def adamw_multi(params, grads, ms, vs, *, lrs, wds, beta1, beta2, eps, step, gra
         _check(rc, "ftb_adamw_multi")
 
 
+def sum_of_squares(tensors):
+    """fp32 scalar on the device: the sum of the squares of all ``tensors`` (contiguous, bf16 or fp32), each read once."""
+    lib = load("elementwise")
+    lib.ftb_sumsq_blocks.restype = c_long
+    tensors = [t for t in tensors if t.numel()]
+    blocks = [lib.ftb_sumsq_blocks(c_long(t.numel())) for t in tensors]
+    out = torch.empty((), dtype=torch.float32, device=tensors[0].device)
+    partial = torch.empty(sum(blocks), dtype=torch.float32, device=out.device)
+    at = 0
+    for i0 in range(0, len(tensors), 64):
+        ts = tensors[i0:i0 + 64]
+        n = len(ts)
+        rc = lib.ftb_sumsq(c_int(n), (c_void_p * n)(*[t.data_ptr() for t in ts]), (c_long * n)(*[t.numel() for t in ts]),
+                           (c_int * n)(*[_DT[t.dtype] for t in ts]), c_void_p(partial.data_ptr() + 4 * at), _stream())
+        _check(rc, "ftb_sumsq")
+        at += sum(blocks[i0:i0 + 64])
+    _check(lib.ftb_sumsq_total(_ptr(partial), c_long(at), _ptr(out), _stream()), "ftb_sumsq_total")
+    return out
+
+
 def topk_route(logits, k, mode):
     lib = load("elementwise")
     T, E = logits.shape

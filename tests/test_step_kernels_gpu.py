@@ -40,3 +40,22 @@ def test_adamw_types_tails_and_alignment(pdt, gdt, sdt, shift):
         for a, b, o in zip(got, new, old):
             room = 2.0 ** -20 * (b.float().abs() + o.float().abs()) + (2.0 ** -7 * b.float().abs() if dt == BF16 else 0)
             assert torch.all((a.float() - b.float()).abs() <= room)
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+def test_sum_of_squares_sizes_types_and_alignment(shift):
+    """More tensors than one launch takes, lengths around a group of 8 and a block of 16384, both types, off the 16-byte
+    grid, next to tensors the kernel does not take (host, strided).  Blocks add in fp32 (64 terms a thread and a tree of
+    8 levels: 2^-24 * 72 relative at most, all terms being positive) and the blocks in double."""
+    torch.manual_seed(0)
+    sizes = (1, 7, 8, 9, 16383, 16384, 16385, 40003)
+    ts = [torch.randn(n + shift, device=DEV).to(dt)[shift:] for n in sizes * 5 for dt in (BF16, F32)]
+    ts += [torch.randn(33), torch.randn(64, 32, device=DEV)[:, :7], torch.empty(0, device=DEV)]
+    want = sum(float(t.double().square().sum()) for t in ts)
+    got = float(ops.sum_of_squares(ts, torch.device(DEV, 0)))
+    assert abs(got - want) <= 2.0 ** -24 * 80 * want
+    assert float(ops.sum_of_squares([], torch.device(DEV, 0))) == 0.0
+    ts[3][0] = float("inf")
+    assert float(ops.sum_of_squares(ts, torch.device(DEV, 0))) == float("inf")
+    ts[3][0] = float("nan")
+    assert ops.sum_of_squares(ts, torch.device(DEV, 0)).isnan()
