@@ -8,7 +8,11 @@
 // sequence; sequences x heads x column blocks give thousands of CTAs for packed batches and HV * dv / NC CTAs for
 // one long sequence.  No chunk-level triangular solves are needed.
 //
-// Thread layout (128 threads): ti = tid & 15 owns rows {ti + 16 rr}, tj = tid >> 4 owns columns {tj*CPT + cc}.
+// Thread layout (128 threads): ti = tid & 15 owns the row pairs {2 ti + 32 j, + 1} (one row, ti, at dk = 16), tj = tid >> 4
+// owns columns {tj*CPT + cc}.  The state is kept and updated as pairs of rows in packed fp32 arithmetic (fma.rn.f32x2, one
+// instruction for two fused multiply-adds, each rounded as the scalar one), which halves the instructions to issue: 16384
+// tokens in 512 to 4096 long sequences, 32 heads of 128 x 128: pass F 6.4 -> 5.7 ms, pass R 6.7 -> 6.6 ms, forward 3.6 ms
+// either way.  What bounds them then is the chain of a token (its reductions) in the longest sequences.
 // Reductions over rows (r, o, de) are 4 xor-shuffles inside a half warp; reductions over columns (dq, dk) are
 // accumulated per warp in shared memory over a block of TB tokens and flushed with fp32 atomics once per block.
 //
@@ -80,6 +84,64 @@ __device__ __forceinline__ void all_gather4(float k, int lane, float (&out)[4]) 
   for (int c = 0; c < 4; ++c) out[c] = __shfl_sync(0xffffffffu, k, (lane & 0x13) | (c << 2));
 }
 
+// ---- pairs of fp32
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float sum2(f32x2 v) {
+  float a, b;
+  unpack2(v, a, b);
+  return a + b;
+}
+// The thread's j-th pair of a DK vector; with one row per thread (RPT = 1) the second element does not exist and is 0.
+template <int RPT>
+__device__ __forceinline__ f32x2 load_pair(const float* x, int ti, int j) {
+  if constexpr (RPT == 1) return pack2(x[ti], 0.f);
+  else return *reinterpret_cast<const f32x2*>(x + 2 * ti + 32 * j);
+}
+template <int RPT>
+__device__ __forceinline__ void store_pair(float* x, int ti, int j, f32x2 v) {
+  if constexpr (RPT == 1) x[ti] = __uint_as_float(static_cast<uint32_t>(v));
+  else *reinterpret_cast<f32x2*>(x + 2 * ti + 32 * j) = v;
+}
+// The j-th pair of a column of a (DK, DV) state matrix.
+template <int RPT>
+__device__ __forceinline__ f32x2 load_state(const float* m, int DV, int ti, int j) {
+  if constexpr (RPT == 1) return pack2(m[(size_t)ti * DV], 0.f);
+  const size_t i = 2 * ti + 32 * j;
+  return pack2(m[i * DV], m[(i + 1) * DV]);
+}
+template <int RPT>
+__device__ __forceinline__ void store_state(float* m, int DV, int ti, int j, f32x2 v) {
+  float a, b;
+  unpack2(v, a, b);
+  if constexpr (RPT == 1) { m[(size_t)ti * DV] = a; return; }
+  const size_t i = 2 * ti + 32 * j;
+  m[i * DV] = a;
+  m[(i + 1) * DV] = b;
+}
+__device__ __forceinline__ f32x2 shfl_xor16_add(f32x2 v) {      // sum with the other half warp's pair
+  float a, b;
+  unpack2(v, a, b);
+  a += __shfl_xor_sync(0xffffffffu, a, 16);
+  b += __shfl_xor_sync(0xffffffffu, b, 16);
+  return pack2(a, b);
+}
+
 // Sum over the lanes that hold one token's DK consecutive elements (DK lanes for DK = 16, the whole warp otherwise).
 template <int DK>
 __device__ __forceinline__ float segment_sum(float x) {
@@ -90,23 +152,23 @@ __device__ __forceinline__ float segment_sum(float x) {
 // MODE 0: forward (o, r, final state).  MODE 1: pass F of the backward (dq, dk += S^ dr).
 template <int RPT, int CPT, int MODE>
 __global__ void __launch_bounds__(NT) gdn_forward_kernel(const GdnArgs a) {
-  constexpr int DK = 16 * RPT, NC = 8 * CPT;
-  __shared__ float k_s[TB][DK], q_s[TB][DK], v_s[TB][NC], x_s[TB][NC], y_s[TB][NC];
+  constexpr int DK = 16 * RPT, NC = 8 * CPT, NP = RPT == 1 ? 1 : RPT / 2;
+  __shared__ __align__(16) float k_s[TB][DK], q_s[TB][DK];
+  __shared__ float v_s[TB][NC], x_s[TB][NC], y_s[TB][NC];
   __shared__ float a_s[TB], b_s[TB];
-  __shared__ float acc_q[MODE == 1 ? 4 : 1][TB][MODE == 1 ? DK : 1];
-  __shared__ float acc_k[MODE == 1 ? 4 : 1][TB][MODE == 1 ? DK : 1];
+  __shared__ __align__(16) float acc_q[MODE == 1 ? 4 : 1][TB][MODE == 1 ? DK : 1];
+  __shared__ __align__(16) float acc_k[MODE == 1 ? 4 : 1][TB][MODE == 1 ? DK : 1];
   const int tid = threadIdx.x, ti = tid & 15, tj = tid >> 4, warp = tid >> 5;
   const int col0 = blockIdx.x * NC, hv = blockIdx.y, seq = blockIdx.z;
   const int hk = hv / (a.HV / a.HK);
   const int t0 = a.cu[seq], t1 = a.cu[seq + 1];
-  float S[RPT][CPT];
+  f32x2 S[NP][CPT];
 #pragma unroll
-  for (int rr = 0; rr < RPT; ++rr)
+  for (int j = 0; j < NP; ++j)
 #pragma unroll
-    for (int cc = 0; cc < CPT; ++cc) {
-      const int i = ti + 16 * rr, j = col0 + tj * CPT + cc;
-      S[rr][cc] = a.state_in ? a.state_in[(((size_t)seq * a.HV + hv) * DK + i) * a.DV + j] : 0.f;
-    }
+    for (int cc = 0; cc < CPT; ++cc)
+      S[j][cc] = a.state_in ? load_state<RPT>(a.state_in + ((size_t)seq * a.HV + hv) * DK * a.DV + col0 + tj * CPT + cc,
+                                              a.DV, ti, j) : 0ull;
   for (int tb = t0; tb < t1; tb += TB) {
     const int nt = min(TB, t1 - tb);
     __syncthreads();
@@ -132,17 +194,19 @@ __global__ void __launch_bounds__(NT) gdn_forward_kernel(const GdnArgs a) {
     __syncthreads();
     for (int t = 0; t < nt; ++t) {
       const float at = a_s[t], bt = b_s[t];
-      float kr[RPT], qr[RPT], rj[CPT];
+      const f32x2 at2 = pack2(at, at);
+      f32x2 kr[NP], qr[NP];
+      float rj[CPT];
 #pragma unroll
-      for (int rr = 0; rr < RPT; ++rr) { kr[rr] = k_s[t][ti + 16 * rr]; qr[rr] = q_s[t][ti + 16 * rr]; }
+      for (int j = 0; j < NP; ++j) { kr[j] = load_pair<RPT>(k_s[t], ti, j); qr[j] = load_pair<RPT>(q_s[t], ti, j); }
       {
         float pp[CPT];
 #pragma unroll
         for (int cc = 0; cc < CPT; ++cc) {
-          float p = 0.f;
+          f32x2 p = 0ull;
 #pragma unroll
-          for (int rr = 0; rr < RPT; ++rr) { S[rr][cc] *= at; p += kr[rr] * S[rr][cc]; }
-          pp[cc] = p;
+          for (int j = 0; j < NP; ++j) { S[j][cc] = mul2(S[j][cc], at2); p = fma2(kr[j], S[j][cc], p); }
+          pp[cc] = sum2(p);
         }
         if constexpr (CPT == 4) {
           all_gather4(reduce_scatter4(pp[0], pp[1], pp[2], pp[3], tid & 31), tid & 31, rj);
@@ -152,29 +216,33 @@ __global__ void __launch_bounds__(NT) gdn_forward_kernel(const GdnArgs a) {
         }
       }
       if (MODE == 1) {   // dk += S^ dr  with dr = -beta de   (S holds S^ here)
+        f32x2 dr[CPT];
 #pragma unroll
-        for (int rr = 0; rr < RPT; ++rr) {
-          float p = 0.f;
+        for (int cc = 0; cc < CPT; ++cc) { const float d = -bt * y_s[t][tj * CPT + cc]; dr[cc] = pack2(d, d); }
 #pragma unroll
-          for (int cc = 0; cc < CPT; ++cc) p += S[rr][cc] * (-bt * y_s[t][tj * CPT + cc]);
-          p += __shfl_xor_sync(0xffffffffu, p, 16);
-          if ((tid & 16) == 0) acc_k[warp][t][ti + 16 * rr] = p;
+        for (int j = 0; j < NP; ++j) {
+          f32x2 p = 0ull;
+#pragma unroll
+          for (int cc = 0; cc < CPT; ++cc) p = fma2(S[j][cc], dr[cc], p);
+          p = shfl_xor16_add(p);
+          if ((tid & 16) == 0) store_pair<RPT>(acc_k[warp][t], ti, j, p);
         }
       }
 #pragma unroll
       for (int cc = 0; cc < CPT; ++cc) {
         const float e = bt * (v_s[t][tj * CPT + cc] - rj[cc]);
+        const f32x2 e2 = pack2(e, e);
 #pragma unroll
-        for (int rr = 0; rr < RPT; ++rr) S[rr][cc] += kr[rr] * e;
+        for (int j = 0; j < NP; ++j) S[j][cc] = fma2(kr[j], e2, S[j][cc]);
       }
       if (MODE == 0) {
         float pp[CPT];
 #pragma unroll
         for (int cc = 0; cc < CPT; ++cc) {
-          float p = 0.f;
+          f32x2 p = 0ull;
 #pragma unroll
-          for (int rr = 0; rr < RPT; ++rr) p += qr[rr] * S[rr][cc];
-          pp[cc] = p;
+          for (int j = 0; j < NP; ++j) p = fma2(qr[j], S[j][cc], p);
+          pp[cc] = sum2(p);
         }
         if constexpr (CPT == 4) {
           const float tot = reduce_scatter4(pp[0], pp[1], pp[2], pp[3], tid & 31);
@@ -196,13 +264,17 @@ __global__ void __launch_bounds__(NT) gdn_forward_kernel(const GdnArgs a) {
           }
         }
       } else {            // dq = scale S_t dO
+        f32x2 d_o[CPT];
 #pragma unroll
-        for (int rr = 0; rr < RPT; ++rr) {
-          float p = 0.f;
+        for (int cc = 0; cc < CPT; ++cc) { const float d = x_s[t][tj * CPT + cc]; d_o[cc] = pack2(d, d); }
+        const f32x2 sc2 = pack2(a.scale, a.scale);
 #pragma unroll
-          for (int cc = 0; cc < CPT; ++cc) p += S[rr][cc] * x_s[t][tj * CPT + cc];
-          p += __shfl_xor_sync(0xffffffffu, p, 16);
-          if ((tid & 16) == 0) acc_q[warp][t][ti + 16 * rr] = p * a.scale;
+        for (int j = 0; j < NP; ++j) {
+          f32x2 p = 0ull;
+#pragma unroll
+          for (int cc = 0; cc < CPT; ++cc) p = fma2(S[j][cc], d_o[cc], p);
+          p = mul2(shfl_xor16_add(p), sc2);
+          if ((tid & 16) == 0) store_pair<RPT>(acc_q[warp][t], ti, j, p);
         }
       }
     }
@@ -230,35 +302,33 @@ __global__ void __launch_bounds__(NT) gdn_forward_kernel(const GdnArgs a) {
   }
   if (MODE == 0 && a.state_out) {
 #pragma unroll
-    for (int rr = 0; rr < RPT; ++rr)
+    for (int j = 0; j < NP; ++j)
 #pragma unroll
-      for (int cc = 0; cc < CPT; ++cc) {
-        const int i = ti + 16 * rr, j = col0 + tj * CPT + cc;
-        a.state_out[(((size_t)seq * a.HV + hv) * DK + i) * a.DV + j] = S[rr][cc];
-      }
+      for (int cc = 0; cc < CPT; ++cc)
+        store_state<RPT>(a.state_out + ((size_t)seq * a.HV + hv) * DK * a.DV + col0 + tj * CPT + cc, a.DV, ti, j, S[j][cc]);
   }
 }
 
 // Pass R: reverse in time.  state_in = gradient of the final state (or null), state_out = gradient of the initial one.
 template <int RPT, int CPT>
 __global__ void __launch_bounds__(NT) gdn_reverse_kernel(const GdnArgs a) {
-  constexpr int DK = 16 * RPT, NC = 8 * CPT;
-  __shared__ float k_s[TB][DK], q_s[TB][DK], v_s[TB][NC], x_s[TB][NC], r_s[TB][NC];
+  constexpr int DK = 16 * RPT, NC = 8 * CPT, NP = RPT == 1 ? 1 : RPT / 2;
+  __shared__ __align__(16) float k_s[TB][DK], q_s[TB][DK];
+  __shared__ float v_s[TB][NC], x_s[TB][NC], r_s[TB][NC];
   __shared__ float a_s[TB], b_s[TB];
-  __shared__ float acc_k[4][TB][DK];
+  __shared__ __align__(16) float acc_k[4][TB][DK];
   __shared__ float acc_b[4][TB];
   const int tid = threadIdx.x, ti = tid & 15, tj = tid >> 4, warp = tid >> 5;
   const int col0 = blockIdx.x * NC, hv = blockIdx.y, seq = blockIdx.z;
   const int hk = hv / (a.HV / a.HK);
   const int t0 = a.cu[seq], t1 = a.cu[seq + 1];
-  float dS[RPT][CPT];
+  f32x2 dS[NP][CPT];
 #pragma unroll
-  for (int rr = 0; rr < RPT; ++rr)
+  for (int j = 0; j < NP; ++j)
 #pragma unroll
-    for (int cc = 0; cc < CPT; ++cc) {
-      const int i = ti + 16 * rr, j = col0 + tj * CPT + cc;
-      dS[rr][cc] = a.state_in ? a.state_in[(((size_t)seq * a.HV + hv) * DK + i) * a.DV + j] : 0.f;
-    }
+    for (int cc = 0; cc < CPT; ++cc)
+      dS[j][cc] = a.state_in ? load_state<RPT>(a.state_in + ((size_t)seq * a.HV + hv) * DK * a.DV + col0 + tj * CPT + cc,
+                                               a.DV, ti, j) : 0ull;
   const int nblk = (t1 - t0 + TB - 1) / TB;
   for (int blk = nblk - 1; blk >= 0; --blk) {
     const int tb = t0 + blk * TB;
@@ -284,19 +354,21 @@ __global__ void __launch_bounds__(NT) gdn_reverse_kernel(const GdnArgs a) {
     __syncthreads();
     for (int t = nt - 1; t >= 0; --t) {
       const float at = a_s[t], bt = b_s[t];
-      float kr[RPT], qr[RPT], de[CPT], ej[CPT];
+      f32x2 kr[NP], qr[NP];
+      float de[CPT], ej[CPT];
 #pragma unroll
-      for (int rr = 0; rr < RPT; ++rr) { kr[rr] = k_s[t][ti + 16 * rr]; qr[rr] = q_s[t][ti + 16 * rr]; }
+      for (int j = 0; j < NP; ++j) { kr[j] = load_pair<RPT>(k_s[t], ti, j); qr[j] = load_pair<RPT>(q_s[t], ti, j); }
       float db = 0.f;
       {
         float pp[CPT];
 #pragma unroll
         for (int cc = 0; cc < CPT; ++cc) {
           const float dO = x_s[t][tj * CPT + cc];
-          float p = 0.f;
+          const f32x2 dO2 = pack2(dO, dO);
+          f32x2 p = 0ull;
 #pragma unroll
-          for (int rr = 0; rr < RPT; ++rr) { dS[rr][cc] += qr[rr] * dO; p += kr[rr] * dS[rr][cc]; }
-          pp[cc] = p;
+          for (int j = 0; j < NP; ++j) { dS[j][cc] = fma2(qr[j], dO2, dS[j][cc]); p = fma2(kr[j], dS[j][cc], p); }
+          pp[cc] = sum2(p);
         }
         if constexpr (CPT == 4) {
           all_gather4(reduce_scatter4(pp[0], pp[1], pp[2], pp[3], tid & 31), tid & 31, de);
@@ -318,19 +390,24 @@ __global__ void __launch_bounds__(NT) gdn_reverse_kernel(const GdnArgs a) {
       }
       db += __shfl_xor_sync(0xffffffffu, db, 16);       // every lane of a half warp holds the same db
       if ((tid & 31) == 0) acc_b[warp][t] = db;
+      f32x2 e2[CPT];
 #pragma unroll
-      for (int rr = 0; rr < RPT; ++rr) {
-        float p = 0.f;
+      for (int cc = 0; cc < CPT; ++cc) e2[cc] = pack2(ej[cc], ej[cc]);
 #pragma unroll
-        for (int cc = 0; cc < CPT; ++cc) p += dS[rr][cc] * ej[cc];
-        p += __shfl_xor_sync(0xffffffffu, p, 16);
-        if ((tid & 16) == 0) acc_k[warp][t][ti + 16 * rr] = p;
+      for (int j = 0; j < NP; ++j) {
+        f32x2 p = 0ull;
+#pragma unroll
+        for (int cc = 0; cc < CPT; ++cc) p = fma2(dS[j][cc], e2[cc], p);
+        p = shfl_xor16_add(p);
+        if ((tid & 16) == 0) store_pair<RPT>(acc_k[warp][t], ti, j, p);
       }
+      const f32x2 at2 = pack2(at, at);
 #pragma unroll
       for (int cc = 0; cc < CPT; ++cc) {
         const float dr = -bt * de[cc];
+        const f32x2 dr2 = pack2(dr, dr);
 #pragma unroll
-        for (int rr = 0; rr < RPT; ++rr) dS[rr][cc] = at * (dS[rr][cc] + kr[rr] * dr);
+        for (int j = 0; j < NP; ++j) dS[j][cc] = mul2(at2, fma2(kr[j], dr2, dS[j][cc]));
       }
     }
     __syncthreads();
@@ -355,12 +432,42 @@ __global__ void __launch_bounds__(NT) gdn_reverse_kernel(const GdnArgs a) {
   }
   if (a.state_out) {
 #pragma unroll
-    for (int rr = 0; rr < RPT; ++rr)
+    for (int j = 0; j < NP; ++j)
 #pragma unroll
-      for (int cc = 0; cc < CPT; ++cc) {
-        const int i = ti + 16 * rr, j = col0 + tj * CPT + cc;
-        a.state_out[(((size_t)seq * a.HV + hv) * DK + i) * a.DV + j] = dS[rr][cc];
-      }
+      for (int cc = 0; cc < CPT; ++cc)
+        store_state<RPT>(a.state_out + ((size_t)seq * a.HV + hv) * DK * a.DV + col0 + tj * CPT + cc, a.DV, ti, j, dS[j][cc]);
+  }
+}
+
+// dg[t, h] = sum_{u >= t, same sequence} s[u, h] + extra[seq, h].  A block owns 32 heads of one sequence; its 32 warps take
+// 32 runs of tokens: totals of the runs, their suffix sums in shared memory, then the running sums within each run.  (A
+// cumulative sum over all tokens along the slow axis, as the tensor library does it, kept one thread per head busy: 3.5 ms for
+// 16384 x 32, below 0.02 ms so.)
+__global__ void __launch_bounds__(1024) suffix_sum_kernel(const float* __restrict__ s, const float* __restrict__ extra,
+                                                          const int* __restrict__ cu, float* __restrict__ dg, int H) {
+  __shared__ float tot[32][33];
+  const int lane = threadIdx.x & 31, run = threadIdx.x >> 5;
+  const int h = blockIdx.x * 32 + lane, seq = blockIdx.y;
+  const int t0 = cu[seq], n = cu[seq + 1] - t0;
+  const int per = (n + 31) / 32;
+  const int lo = min(run * per, n), hi = min(lo + per, n);
+  const bool on = h < H;
+  const float* sp = s + (size_t)t0 * H + h;
+  float sum = 0.f;
+  if (on) {
+#pragma unroll 8
+    for (int t = lo; t < hi; ++t) sum += sp[(size_t)t * H];
+  }
+  tot[run][lane] = sum;
+  __syncthreads();
+  if (!on) return;
+  float acc = extra ? extra[(size_t)seq * H + h] : 0.f;
+  for (int r = 31; r > run; --r) acc += tot[r][lane];
+  float* dp = dg + (size_t)t0 * H + h;
+#pragma unroll 8
+  for (int t = hi - 1; t >= lo; --t) {
+    acc += sp[(size_t)t * H];
+    dp[(size_t)t * H] = acc;
   }
 }
 
@@ -403,6 +510,15 @@ extern "C" {
 int ftb_gdn_col_blocks(int nseq, int HV, int DV) {
   const int cpt = cols_per_thread(nseq, HV, DV);
   return cpt ? DV / (8 * cpt) : 0;
+}
+
+// dg (T, H) from the per-token scalars s (T, H); extra (nseq, H) or NULL is added to every token of its sequence.
+int ftb_suffix_sum(const float* s, const float* extra, const int* cu, int nseq, float* dg, int H, cudaStream_t st) {
+  if (nseq <= 0 || H <= 0) return 0;
+  if (nseq > 65535) return -2;
+  suffix_sum_kernel<<<dim3((H + 31) / 32, nseq), 1024, 0, st>>>(s, extra, cu, dg, H);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : -400 - (int)e;
 }
 
 int ftb_gdn(int pass, const void* q, const void* k, const void* v, const float* g, const float* beta, const int* cu,

@@ -181,13 +181,10 @@ def gdn_bwd(q, k, v, g, beta, cu, state_in, final_state, r, d_o, dstate_final=No
     _gdn(2, q, k, v, g, beta, cu, sin, None, None, None, d_o, de, None, None, dq_hv, dk_hv, s, scale)
     # dg_t = sum_{u >= t, same sequence} s_u  (+ <dS_final, S_final>), with the per-token scalar
     # s_u = q_u.dq_u - k_u.(dS'_u e_u) + k_u.(S^_u dr_u) accumulated by the two passes
-    csum = torch.flip(torch.cumsum(torch.flip(s, [0]), 0), [0])            # suffix sums over the whole chunk
-    ends = cu[1:].long()                                                    # first token AFTER each sequence
-    tail = torch.cat([csum, torch.zeros(1, HV, dtype=F32, device=dev)], 0)[ends]       # (S, HV) mass past the end
-    if dstate_final is not None:
-        tail = tail - (dsf * final_state.to(F32)).sum((-1, -2))
-    lens = (cu[1:] - cu[:-1]).long()
-    dg = csum - torch.repeat_interleave(tail, lens, dim=0)
+    extra = (dsf * final_state.to(F32)).sum((-1, -2)).contiguous() if dstate_final is not None else None     # (S, HV)
+    dg = torch.empty(T, HV, dtype=F32, device=dev)
+    _check(load("gdn").ftb_suffix_sum(_ptr(s), _ptr(extra), _ptr(cu), c_int(S), _ptr(dg), c_int(HV), _stream()),
+           "ftb_suffix_sum")
     if rep > 1:
         dq = dq_hv.view(T, HK, rep, DK).sum(2)
         dk = dk_hv.view(T, HK, rep, DK).sum(2)

@@ -204,3 +204,25 @@ def test_gate_prep_fwd_bwd(T, HV):
     dba = la.gate_prep_bwd(ba, dtb, alog, g, dbeta, dg, d_alog, d_dtb)
     assert _rel(dba, baf.grad) < 6e-3
     assert _rel(d_alog, alog_r.grad) < 1e-4 and _rel(d_dtb, dtb_r.grad) < 1e-4
+
+
+@pytest.mark.parametrize("H", [1, 31, 32, 33, 64])
+@pytest.mark.parametrize("with_extra", [False, True])
+def test_suffix_sum_per_sequence(H, with_extra):
+    """Suffix sums of every sequence, at lengths around the 32 runs a block cuts a sequence into (also shorter than 32 and
+    empty), against float64; a sum of n fp32 terms in any order is off by n * 2^-24 of the sum of magnitudes at most."""
+    from flextrain_b200.ops.cuda import _check, _ptr, _stream, load
+    from ctypes import c_int
+    lens = [1, 31, 32, 33, 0, 1000, 65, 2]
+    cu, T = _cu(lens), sum(lens)
+    s = torch.randn(T, H, device=DEV)
+    extra = torch.randn(len(lens), H, device=DEV) if with_extra else None
+    dg = torch.full((T, H), float("nan"), device=DEV)
+    _check(load("gdn").ftb_suffix_sum(_ptr(s), _ptr(extra), _ptr(cu), c_int(len(lens)), _ptr(dg), c_int(H), _stream()), "")
+    off = 0
+    for i, n in enumerate(lens):
+        part = s[off:off + n].double()
+        want = part.flip(0).cumsum(0).flip(0) + (extra[i].double() if with_extra else 0)
+        room = (n + 1) * 2.0 ** -24 * (part.abs().sum(0) + (extra[i].abs() if with_extra else 0))
+        assert torch.all((dg[off:off + n].double() - want).abs() <= room + 1e-12)
+        off += n
