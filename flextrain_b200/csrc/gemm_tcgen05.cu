@@ -117,28 +117,29 @@ __device__ __forceinline__ unsigned long long ld_acquire_gpu_u64(const unsigned 
   return v;
 }
 
-// Grouped tile lookup: tile index -> (group, row tile inside group). Linear walk over the
-// offsets (E <= 256, done by one thread per role per tile; cheap next to a 128xBNxK main loop).
-__device__ __forceinline__ bool grouped_tile(const int* __restrict__ offsets, int num_groups, int tiles_n, int tile,
-                                             int& g, int& row0, int& rows, int& tn) {
-  int acc = 0;
-  for (int e = 0; e < num_groups; ++e) {
-    const int a = offsets[e], b = offsets[e + 1];
-    const int tm_e = (b - a + BM - 1) / BM;
-    const int t_e = tm_e * tiles_n;
-    if (tile < acc + t_e) {
-      const int r = tile - acc;
-      g = e;
-      const int tm = r % tm_e;
-      tn = r / tm_e;
-      row0 = a + tm * BM;
-      rows = min(BM, b - row0);
-      return true;
+// Tiles of the grouped modes in the order a CTA visits them (ascending): the walk over the groups goes on where the last
+// tile left it.
+struct GroupWalk {
+  int e = 0, acc = 0;
+  // rows mode: tile -> group, first row, rows left in the group from there, column tile
+  __device__ __forceinline__ bool rows(const int* __restrict__ offsets, int num_groups, int tile_rows, int tiles_n, int tile,
+                                       int& g, int& row0, int& left, int& tn) {
+    for (; e < num_groups; ++e) {
+      const int a = offsets[e], b = offsets[e + 1];
+      const int tm_e = (b - a + tile_rows - 1) / tile_rows;
+      if (tile < acc + tm_e * tiles_n) {
+        const int r = tile - acc;
+        g = e;
+        tn = r / tm_e;
+        row0 = a + (r - tn * tm_e) * tile_rows;
+        left = b - row0;
+        return true;
+      }
+      acc += tm_e * tiles_n;
     }
-    acc += t_e;
+    return false;
   }
-  return false;
-}
+};
 
 template <int BN, int STAGES, bool A_MN, bool B_MN, int GROUPED, int COMM = 0>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -200,11 +201,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
+      [[maybe_unused]] GroupWalk walk;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         int tm, tn, g = 0, row0, rows;
         int k_lo = 0;
         if constexpr (GROUPED == 1) {
-          if (!grouped_tile(p.offsets, p.num_groups, tiles_n, tile, g, row0, rows, tn)) break;
+          if (!walk.rows(p.offsets, p.num_groups, BM, tiles_n, tile, g, row0, rows, tn)) break;
         } else if constexpr (GROUPED == 2) {
           // per-expert weight gradient: tile = (expert, tm, tn); the reduction runs over the expert's rows
           g = tile / (tiles_m * tiles_n);
@@ -309,10 +311,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
+      [[maybe_unused]] GroupWalk walk;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         if constexpr (GROUPED == 1) {
           int g, row0, rows, tn;
-          if (!grouped_tile(p.offsets, p.num_groups, tiles_n, tile, g, row0, rows, tn)) break;
+          if (!walk.rows(p.offsets, p.num_groups, BM, tiles_n, tile, g, row0, rows, tn)) break;
         }
         if constexpr (GROUPED == 2) {
           const int g = tile / (tiles_m * tiles_n);
@@ -468,12 +471,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
+    [[maybe_unused]] GroupWalk walk;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
       int tm, tn, g = 0, row0, rows;
       char* d_base = reinterpret_cast<char*>(p.D);
       long d_row_shift = 0;
       if constexpr (GROUPED == 1) {
-        if (!grouped_tile(p.offsets, p.num_groups, tiles_n, tile, g, row0, rows, tn)) break;
+        if (!walk.rows(p.offsets, p.num_groups, BM, tiles_n, tile, g, row0, rows, tn)) break;
+        rows = min(BM, rows);
       } else if constexpr (GROUPED == 2) {
         g = tile / (tiles_m * tiles_n);
         tile_coords(tile - g * tiles_m * tiles_n, tiles_m, tiles_n, tm, tn);
@@ -740,9 +745,55 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
 // (tcgen05.commit); loads are plain tiled TMA loads credited to the leader's barrier (no cluster multicast loads).
 // =====================================================================================================
 constexpr int BN2 = 256;
-constexpr int ST2 = 6;
 constexpr int STAGE2_BYTES = 2 * BM * BK * 2;   // A (128 x 64) + B half (128 x 64)
-constexpr int SMEM2_TOTAL = ST2 * STAGE2_BYTES + 256 + 1024;
+// Eight epilogue warps: two for each quadrant of the accumulator's rows, with half of the columns each.  Their staging takes
+// a stage of the operand ring where the gated-FFN epilogues need three buffers.
+constexpr int EPI2_WARPS = 8;
+template <int EPI>
+struct Ring2 {
+  static constexpr int STAGES = EPI == 0 ? 6 : 5;
+  static constexpr int WARP_BYTES = EPI == 0 ? 32 * 128 : 3 * 32 * 64;
+  static constexpr int TOTAL = STAGES * STAGE2_BYTES + EPI2_WARPS * WARP_BYTES + 256 + 1024;
+  static_assert(TOTAL <= 232448, "shared memory of a CTA");
+};
+
+// The accumulator comes out of tensor memory one row per thread.  Stored (or read, for C) from there, an instruction touches
+// 32 rows with 16 bytes of each: 32 passes of the load / store unit, some 4100 cycles for each 128 x 256 bf16 tile and
+// operand, more than the main loop takes when K is below 1024 (a MoE weight gradient reads and writes its tile).  So a warp
+// turns 32 rows over in its own piece of shared memory, 64 or 128 bytes of a row at a time, and moves whole pieces of rows.
+// 16384 x 768 x 768 with C: 55.7 us row by row, 22.8 us so; 9377 x 1024 x 2048 with C 51.5 / 31.0; gated FFN forward
+// 9377 x 3072 x 1024 165 / 104, backward 189 / 110, 16384 x 14336 x 4096 1671 / 1467 (the last three also by twice the
+// epilogue warps).
+// PIECES 16-byte pieces per row; the swizzle keeps both the row-wise and the piece-wise accesses free of bank conflicts.
+template <int PIECES>
+struct Turn {
+  static constexpr int ROWS = 32 / PIECES;          // rows an instruction moves
+  __device__ static __forceinline__ uint4* at(uint8_t* buf, int row, int piece) {
+    const int sw = PIECES == 8 ? (row & 7) : ((row >> 1) & 3);
+    return reinterpret_cast<uint4*>(buf + row * (PIECES * 16) + ((piece ^ sw) << 4));
+  }
+  // pieces of 32 rows from global memory to registers (row r at g + r * ld_bytes), and on to shared memory
+  __device__ static __forceinline__ void fetch(uint4 (&v)[PIECES], const uint8_t* g, size_t ld_bytes, int rows, int pieces,
+                                               int lane) {
+    const int lr = lane / PIECES, lp = lane % PIECES;
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i)
+      if (i * ROWS + lr < rows && lp < pieces) v[i] = *reinterpret_cast<const uint4*>(g + (i * ROWS + lr) * ld_bytes + lp * 16);
+  }
+  __device__ static __forceinline__ void put(uint8_t* buf, const uint4 (&v)[PIECES], int lane) {
+    const int lr = lane / PIECES, lp = lane % PIECES;
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) *at(buf, i * ROWS + lr, lp) = v[i];
+  }
+  // pieces of 32 rows from shared to global memory
+  __device__ static __forceinline__ void store(uint8_t* buf, uint8_t* g, size_t ld_bytes, int rows, int pieces, int lane) {
+    const int lr = lane / PIECES, lp = lane % PIECES;
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i)
+      if (i * ROWS + lr < rows && lp < pieces) *reinterpret_cast<uint4*>(g + (i * ROWS + lr) * ld_bytes + lp * 16) = *at(buf, i * ROWS + lr, lp);
+  }
+};
+
 
 // act(g) and d act / d g of the gate activation (same formulas as the stand-alone SwiGLU / GeGLU kernels)
 __device__ __forceinline__ void glu_act_grad(float g, int kind, float& a, float& da) {
@@ -768,12 +819,14 @@ __device__ __forceinline__ void glu_act_grad(float g, int kind, float& a, float&
 //   2  gated-FFN backward.  The accumulator is dact = dy · W_down; the epilogue reads the saved gate / up values and
 //      writes dgate, dup into D (M x 2F) and the re-emitted activation into glu_act; dact never reaches memory
 //      (flextrain/ops/_kernels/swiglu.py:46-100 reads it back from HBM).
-template <bool A_MN, bool B_MN, int EPI = 0>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
+template <bool A_MN, bool B_MN, int EPI = 0, int GROUPED = 0>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI2_WARPS, 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + ST2 * STAGE2_BYTES);
+  constexpr int ST2 = Ring2<EPI>::STAGES;
+  uint8_t* smem_epi = smem + ST2 * STAGE2_BYTES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem_epi + EPI2_WARPS * Ring2<EPI>::WARP_BYTES);
   uint64_t* empty_bar = full_bar + ST2;
   uint64_t* tfull_bar = empty_bar + ST2;
   uint64_t* tempty_bar = tfull_bar + 2;
@@ -785,14 +838,14 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   const bool leader = cta == 0;
   const int tiles_m = (p.M + 2 * BM - 1) / (2 * BM);
   const int tiles_n = EPI == 1 ? p.glu_F / (BN2 / 2) : (p.N + BN2 - 1) / BN2;
-  const int num_tiles = tiles_m * tiles_n;
-  const int k_blocks = (p.K + BK - 1) / BK;
+  const int num_tiles = GROUPED == 1 ? p.max_tiles : GROUPED == 2 ? p.num_groups * tiles_m * tiles_n : tiles_m * tiles_n;
+  int k_blocks = (p.K + BK - 1) / BK;              // (grouped weight gradients: of the tile's group)
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int s = 0; s < ST2; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], 8); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], 2 * EPI2_WARPS); }
     fence_barrier_init();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
@@ -812,10 +865,24 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
+      [[maybe_unused]] GroupWalk walk;
       for (int tile = pair; tile < num_tiles && ok; tile += n_pairs) {
-        int tm, tn;
-        tile_coords(tile, tiles_m, tiles_n, tm, tn);
-        const int row0 = tm * 2 * BM + static_cast<int>(cta) * BM;      // this CTA's 128 rows of A
+        int tm, tn, g = 0, row0, left, k_lo = 0;
+        if constexpr (GROUPED == 1) {
+          if (!walk.rows(p.offsets, p.num_groups, 2 * BM, tiles_n, tile, g, row0, left, tn)) break;
+        } else {
+          int t = tile;
+          if constexpr (GROUPED == 2) {
+            g = tile / (tiles_m * tiles_n);
+            t -= g * tiles_m * tiles_n;
+            k_lo = p.offsets[g];
+            k_blocks = (p.offsets[g + 1] - k_lo + BK - 1) / BK;
+            if (k_blocks == 0) continue;
+          }
+          tile_coords(t, tiles_m, tiles_n, tm, tn);
+          row0 = tm * 2 * BM;
+        }
+        row0 += static_cast<int>(cta) * BM;                             // this CTA's 128 rows of A
         // this CTA's half of B's N rows (gated forward: 128 gate rows for CTA 0, the matching up rows for CTA 1)
         const int col0 = EPI == 1 ? tn * (BN2 / 2) + static_cast<int>(cta) * p.glu_F
                                   : tn * BN2 + static_cast<int>(cta) * (BN2 / 2);
@@ -824,14 +891,20 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
           uint8_t* sa = smem + stage * STAGE2_BYTES;
           uint8_t* sb = sa + BM * BK * 2;
           if (leader) mbar_expect_tx(&full_bar[stage], 2 * STAGE2_BYTES);
-          const int k0 = kb * BK;
+          const int k0 = k_lo + kb * BK;
           if constexpr (!A_MN) {
             tma_load_2d_2cta(sa, &tmA, &full_bar[stage], k0, row0);
           } else {
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j) tma_load_2d_2cta(sa + j * (64 * BK * 2), &tmA, &full_bar[stage], row0 + j * 64, k0);
           }
-          if constexpr (!B_MN) {
+          if constexpr (GROUPED == 1 && !B_MN) {
+            tma_load_3d_2cta(sb, &tmB, &full_bar[stage], k0, col0, g);
+          } else if constexpr (GROUPED == 1) {
+#pragma unroll
+            for (int j = 0; j < BM / 64; ++j)
+              tma_load_3d_2cta(sb + j * (64 * BK * 2), &tmB, &full_bar[stage], col0 + j * 64, k0, g);
+          } else if constexpr (!B_MN) {
             tma_load_2d_2cta(sb, &tmB, &full_bar[stage], k0, col0);
           } else {
 #pragma unroll
@@ -849,7 +922,17 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
+      [[maybe_unused]] GroupWalk walk;
       for (int tile = pair; tile < num_tiles && ok; tile += n_pairs) {
+        if constexpr (GROUPED == 1) {
+          int g, row0, left, tn;
+          if (!walk.rows(p.offsets, p.num_groups, 2 * BM, tiles_n, tile, g, row0, left, tn)) break;
+        }
+        if constexpr (GROUPED == 2) {
+          const int g = tile / (tiles_m * tiles_n);
+          k_blocks = (p.offsets[g + 1] - p.offsets[g] + BK - 1) / BK;
+          if (k_blocks == 0) continue;
+        }
         if (!(ok = mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag, 60))) break;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * BN2;
@@ -876,174 +959,223 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     }
   } else {
     const int quad = warp & 3;
+    const int part = (warp - 2) >> 2;                  // which half of the columns
+    uint8_t* buf = smem_epi + (warp - 2) * Ring2<EPI>::WARP_BYTES;
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
+    [[maybe_unused]] GroupWalk walk;
     for (int tile = pair; tile < num_tiles && ok; tile += n_pairs) {
-      int tm, tn;
-      tile_coords(tile, tiles_m, tiles_n, tm, tn);
-      const int row0 = tm * 2 * BM + static_cast<int>(cta) * BM;
-      const int rows = min(BM, p.M - row0);
-      const int r_in = quad * 32 + lane;
-      const bool row_ok = r_in < rows;
-      const size_t row = static_cast<size_t>(row0 + r_in);
-      // gated-FFN backward: saved gate / up values of 32 columns, fetched one step ahead of their use (the first
-      // step is issued before the wait for the accumulator, it does not depend on the MMAs)
-      [[maybe_unused]] uint4 xg[4], xu[4];
-      [[maybe_unused]] auto fetch_x13 = [&](int col) {
-        const __nv_bfloat16* xrow = reinterpret_cast<const __nv_bfloat16*>(p.glu_x13) + row * p.glu_ld_x13;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (row_ok && col + 8 * q < p.N) {
-            xg[q] = __ldg(reinterpret_cast<const uint4*>(xrow + col + 8 * q));
-            xu[q] = __ldg(reinterpret_cast<const uint4*>(xrow + p.glu_F + col + 8 * q));
-          }
+      int tm, tn, row0, left;
+      uint8_t* d_base = reinterpret_cast<uint8_t*>(p.D);
+      const uint8_t* c_base = reinterpret_cast<const uint8_t*>(p.C);
+      if constexpr (GROUPED == 1) {
+        int g;
+        if (!walk.rows(p.offsets, p.num_groups, 2 * BM, tiles_n, tile, g, row0, left, tn)) break;
+      } else {
+        int t = tile;
+        if constexpr (GROUPED == 2) {
+          const int g = tile / (tiles_m * tiles_n);
+          t -= g * tiles_m * tiles_n;
+          if ((p.offsets[g + 1] - p.offsets[g] + BK - 1) / BK == 0) continue;    // empty expert: gradient unchanged
+          const size_t skip = static_cast<size_t>(g) * p.M * p.ldd * (p.d_fp32 ? 4 : 2);
+          d_base += skip;
+          c_base += skip;
         }
-      };
-      if constexpr (EPI == 2) fetch_x13(tn * BN2);
-      if (!(ok = mbar_wait(&tfull_bar[acc], acc_phase, abort_flag, 70))) break;
-      tc_fence_after();
+        tile_coords(t, tiles_m, tiles_n, tm, tn);
+        row0 = tm * 2 * BM;
+        left = p.M - row0;
+      }
+      // this warp's 32 rows, and how many of them are rows of the result
+      const int first = static_cast<int>(cta) * BM + quad * 32;
+      const int rows = max(0, min(32, left - first));
+      const size_t row = static_cast<size_t>(row0 + first);
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN2;
       if constexpr (EPI == 1) {
-        __nv_bfloat16* drow = reinterpret_cast<__nv_bfloat16*>(p.D) + row * p.ldd;
-        __nv_bfloat16* arow = reinterpret_cast<__nv_bfloat16*>(p.glu_act) + row * p.glu_ld_act;
+        using T4 = Turn<4>;
+        if (!(ok = mbar_wait(&tfull_bar[acc], acc_phase, abort_flag, 70))) break;
+        tc_fence_after();
+        uint8_t* drow = d_base + row * p.ldd * 2;
+        uint8_t* arow = reinterpret_cast<uint8_t*>(p.glu_act) + row * p.glu_ld_act * 2;
 #pragma unroll 1
-        for (int c = 0; c < BN2 / 2; c += 32) {
+        for (int c = part * (BN2 / 4); c < (part + 1) * (BN2 / 4); c += 32) {
           const int col = tn * (BN2 / 2) + c;
           uint32_t rg[32], ru[32];
           tmem_ld_32x32(taddr + c, rg);
           tmem_ld_32x32(taddr + BN2 / 2 + c, ru);
           tmem_ld_wait();
-          if (row_ok) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
-              uint4 og, ou, oa;
-              __nv_bfloat162* g2 = reinterpret_cast<__nv_bfloat162*>(&og);
-              __nv_bfloat162* u2 = reinterpret_cast<__nv_bfloat162*>(&ou);
-              __nv_bfloat162* a2 = reinterpret_cast<__nv_bfloat162*>(&oa);
+          for (int q = 0; q < 4; ++q) {
+            const int i = 8 * q;
+            uint4 og, ou, oa;
+            __nv_bfloat162* g2 = reinterpret_cast<__nv_bfloat162*>(&og);
+            __nv_bfloat162* u2 = reinterpret_cast<__nv_bfloat162*>(&ou);
+            __nv_bfloat162* a2 = reinterpret_cast<__nv_bfloat162*>(&oa);
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                g2[j] = __floats2bfloat162_rn(__uint_as_float(rg[i + 2 * j]), __uint_as_float(rg[i + 2 * j + 1]));
-                u2[j] = __floats2bfloat162_rn(__uint_as_float(ru[i + 2 * j]), __uint_as_float(ru[i + 2 * j + 1]));
-                // the activation is taken from the ROUNDED gate / up, exactly what the backward will read back
-                const float2 gf = __bfloat1622float2(g2[j]), uf = __bfloat1622float2(u2[j]);
-                float a0, a1, d0, d1;
-                glu_act_grad(gf.x, p.glu_kind, a0, d0);
-                glu_act_grad(gf.y, p.glu_kind, a1, d1);
-                a2[j] = __floats2bfloat162_rn(a0 * uf.x, a1 * uf.y);
-              }
-              *reinterpret_cast<uint4*>(drow + col + i) = og;
-              *reinterpret_cast<uint4*>(drow + p.glu_F + col + i) = ou;
-              *reinterpret_cast<uint4*>(arow + col + i) = oa;
+            for (int j = 0; j < 4; ++j) {
+              g2[j] = __floats2bfloat162_rn(__uint_as_float(rg[i + 2 * j]), __uint_as_float(rg[i + 2 * j + 1]));
+              u2[j] = __floats2bfloat162_rn(__uint_as_float(ru[i + 2 * j]), __uint_as_float(ru[i + 2 * j + 1]));
+              // the activation is taken from the ROUNDED gate / up, exactly what the backward will read back
+              const float2 gf = __bfloat1622float2(g2[j]), uf = __bfloat1622float2(u2[j]);
+              float a0, a1, d0, d1;
+              glu_act_grad(gf.x, p.glu_kind, a0, d0);
+              glu_act_grad(gf.y, p.glu_kind, a1, d1);
+              a2[j] = __floats2bfloat162_rn(a0 * uf.x, a1 * uf.y);
             }
+            *T4::at(buf, lane, q) = og;
+            *T4::at(buf + 2048, lane, q) = ou;
+            *T4::at(buf + 4096, lane, q) = oa;
           }
+          __syncwarp();
+          T4::store(buf, drow + col * 2, p.ldd * 2, rows, 4, lane);
+          T4::store(buf + 2048, drow + (p.glu_F + col) * 2, p.ldd * 2, rows, 4, lane);
+          T4::store(buf + 4096, arow + col * 2, p.glu_ld_act * 2, rows, 4, lane);
+          __syncwarp();
         }
       }
       if constexpr (EPI == 2) {
-        __nv_bfloat16* drow = reinterpret_cast<__nv_bfloat16*>(p.D) + row * p.ldd;
-        __nv_bfloat16* arow = reinterpret_cast<__nv_bfloat16*>(p.glu_act) + row * p.glu_ld_act;
+        using T4 = Turn<4>;
+        // saved gate / up values of 32 columns, fetched one step ahead of their use (the first step is issued before the
+        // wait for the accumulator, it does not depend on the MMAs).  Two steps ahead, with the loop unrolled for it, was
+        // slower: 9377 x 3072 x 1024 141 us against 110.
+        uint4 xg[4] = {}, xu[4] = {};
+        const uint8_t* xrow = reinterpret_cast<const uint8_t*>(p.glu_x13) + row * p.glu_ld_x13 * 2;
+        auto fetch_x13 = [&](int col) {
+          const int pieces = min(4, (p.N - col) >> 3);
+          T4::fetch(xg, xrow + col * 2, p.glu_ld_x13 * 2, rows, pieces, lane);
+          T4::fetch(xu, xrow + (p.glu_F + col) * 2, p.glu_ld_x13 * 2, rows, pieces, lane);
+        };
+        const int c0 = part * (BN2 / 2), c1 = c0 + BN2 / 2;
+        fetch_x13(tn * BN2 + c0);
+        if (!(ok = mbar_wait(&tfull_bar[acc], acc_phase, abort_flag, 70))) break;
+        tc_fence_after();
+        uint8_t* drow = d_base + row * p.ldd * 2;
+        uint8_t* arow = reinterpret_cast<uint8_t*>(p.glu_act) + row * p.glu_ld_act * 2;
 #pragma unroll 1
-        for (int c = 0; c < BN2; c += 32) {
+        for (int c = c0; c < c1; c += 32) {
           const int col = tn * BN2 + c;
           if (col >= p.N) break;
+          const int pieces = min(4, (p.N - col) >> 3);
           uint32_t r[32];
           tmem_ld_32x32(taddr + c, r);
-          uint4 cg[4], cu[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) { cg[q] = xg[q]; cu[q] = xu[q]; }
-          if (c + 32 < BN2 && col + 32 < p.N) fetch_x13(col + 32);
+          T4::put(buf, xg, lane);
+          T4::put(buf + 2048, xu, lane);
+          if (c + 32 < c1 && col + 32 < p.N) fetch_x13(col + 32);
+          __syncwarp();
           tmem_ld_wait();
-          if (row_ok) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const int i = 8 * q;
-              if (col + i < p.N) {
-                const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&cg[q]);
-                const __nv_bfloat162* u2 = reinterpret_cast<const __nv_bfloat162*>(&cu[q]);
-                uint4 odg, odu, oa;
-                __nv_bfloat162* dg2 = reinterpret_cast<__nv_bfloat162*>(&odg);
-                __nv_bfloat162* du2 = reinterpret_cast<__nv_bfloat162*>(&odu);
-                __nv_bfloat162* a2 = reinterpret_cast<__nv_bfloat162*>(&oa);
+          for (int q = 0; q < 4; ++q) {
+            const int i = 8 * q;
+            const uint4 cg = *T4::at(buf, lane, q), cu = *T4::at(buf + 2048, lane, q);
+            const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&cg);
+            const __nv_bfloat162* u2 = reinterpret_cast<const __nv_bfloat162*>(&cu);
+            uint4 odg, odu, oa;
+            __nv_bfloat162* dg2 = reinterpret_cast<__nv_bfloat162*>(&odg);
+            __nv_bfloat162* du2 = reinterpret_cast<__nv_bfloat162*>(&odu);
+            __nv_bfloat162* a2 = reinterpret_cast<__nv_bfloat162*>(&oa);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const float2 gf = __bfloat1622float2(g2[j]), uf = __bfloat1622float2(u2[j]);
-                  const float da0 = __uint_as_float(r[i + 2 * j]) * p.alpha, da1 = __uint_as_float(r[i + 2 * j + 1]) * p.alpha;
-                  float a0, a1, d0, d1;
-                  glu_act_grad(gf.x, p.glu_kind, a0, d0);
-                  glu_act_grad(gf.y, p.glu_kind, a1, d1);
-                  a2[j] = __floats2bfloat162_rn(a0 * uf.x, a1 * uf.y);
-                  dg2[j] = __floats2bfloat162_rn(da0 * uf.x * d0, da1 * uf.y * d1);
-                  du2[j] = __floats2bfloat162_rn(da0 * a0, da1 * a1);
-                }
-                *reinterpret_cast<uint4*>(drow + col + i) = odg;
-                *reinterpret_cast<uint4*>(drow + p.glu_F + col + i) = odu;
-                *reinterpret_cast<uint4*>(arow + col + i) = oa;
-              }
+            for (int j = 0; j < 4; ++j) {
+              const float2 gf = __bfloat1622float2(g2[j]), uf = __bfloat1622float2(u2[j]);
+              const float da0 = __uint_as_float(r[i + 2 * j]) * p.alpha, da1 = __uint_as_float(r[i + 2 * j + 1]) * p.alpha;
+              float a0, a1, d0, d1;
+              glu_act_grad(gf.x, p.glu_kind, a0, d0);
+              glu_act_grad(gf.y, p.glu_kind, a1, d1);
+              a2[j] = __floats2bfloat162_rn(a0 * uf.x, a1 * uf.y);
+              dg2[j] = __floats2bfloat162_rn(da0 * uf.x * d0, da1 * uf.y * d1);
+              du2[j] = __floats2bfloat162_rn(da0 * a0, da1 * a1);
             }
+            *T4::at(buf, lane, q) = odg;
+            *T4::at(buf + 2048, lane, q) = odu;
+            *T4::at(buf + 4096, lane, q) = oa;
           }
+          __syncwarp();
+          T4::store(buf, drow + col * 2, p.ldd * 2, rows, pieces, lane);
+          T4::store(buf + 2048, drow + (p.glu_F + col) * 2, p.ldd * 2, rows, pieces, lane);
+          T4::store(buf + 4096, arow + col * 2, p.glu_ld_act * 2, rows, pieces, lane);
+          __syncwarp();
         }
       }
       if constexpr (EPI == 0) {
+        using T8 = Turn<8>;
+        const int es = p.d_fp32 ? 4 : 2, step = p.d_fp32 ? 32 : 64;     // 128 bytes of a row at a time
+        uint8_t* drow = d_base + row * p.ldd * es;
+        const uint8_t* crow = c_base + row * p.ldc * es;
+        // (bytes in a row's piece: 16 = 8 bf16 or 4 fp32; N is a multiple of 8)
+        auto pieces_at = [&](int col) { return min(8, ((p.N - col) * es) >> 4); };
+        const int c0 = part * (BN2 / 2), c1 = c0 + BN2 / 2;
+        uint4 cv[8] = {};
+        if (p.beta != 0.f)
+          T8::fetch(cv, crow + static_cast<size_t>(tn * BN2 + c0) * es, static_cast<size_t>(p.ldc) * es, rows,
+                    pieces_at(tn * BN2 + c0), lane);
+        if (!(ok = mbar_wait(&tfull_bar[acc], acc_phase, abort_flag, 70))) break;
+        tc_fence_after();
 #pragma unroll 1
-      for (int c = 0; c < BN2; c += 32) {
-        const int col = tn * BN2 + c;
-        if (col >= p.N) break;
-        uint32_t r[32];
-        tmem_ld_32x32(taddr + c, r);
-        tmem_ld_wait();
-        if (row_ok) {
-          float v[32];
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
-          if (p.bias != nullptr) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (col + i < p.N) v[i] += p.bias[col + i];
+        for (int c = c0; c < c1; c += step) {
+          const int col = tn * BN2 + c;
+          if (col >= p.N) break;
+          uint32_t r0[32], r1[32];                     // (32 fp32 columns need the first only)
+          tmem_ld_32x32(taddr + c, r0);
+          if (!p.d_fp32) tmem_ld_32x32(taddr + c + 32, r1);
+          if (p.beta != 0.f) {
+            T8::put(buf, cv, lane);
+            if (c + step < c1 && col + step < p.N)
+              T8::fetch(cv, crow + static_cast<size_t>(col + step) * es, static_cast<size_t>(p.ldc) * es, rows,
+                        pieces_at(col + step), lane);
+            __syncwarp();
           }
-          if (p.d_fp32) {
-            float* dptr = reinterpret_cast<float*>(p.D) + row * p.ldd + col;
-            const float* cptr = reinterpret_cast<const float*>(p.C) + row * p.ldc + col;
+          tmem_ld_wait();
+          auto finish = [&](const uint32_t (&r)[32], int at_col) {
+            float v[32];
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              if (col + i < p.N) {
-                float4 o = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+            for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
+            if (p.bias != nullptr) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                if (col + at_col + i < p.N) v[i] += p.bias[col + at_col + i];
+            }
+            if (p.d_fp32) {
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                float4* at = reinterpret_cast<float4*>(T8::at(buf, lane, q));
+                float4 o = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                 if (p.beta != 0.f) {
-                  const float4 cc = *reinterpret_cast<const float4*>(cptr + i);
+                  const float4 cc = *at;
                   o.x += p.beta * cc.x; o.y += p.beta * cc.y; o.z += p.beta * cc.z; o.w += p.beta * cc.w;
                 }
-                *reinterpret_cast<float4*>(dptr + i) = o;
+                *at = o;
               }
-            }
-          } else {
-            __nv_bfloat16* dptr = reinterpret_cast<__nv_bfloat16*>(p.D) + row * p.ldd + col;
-            const __nv_bfloat16* cptr = reinterpret_cast<const __nv_bfloat16*>(p.C) + row * p.ldc + col;
+            } else {
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
-              if (col + i < p.N) {
+              for (int q = 0; q < 4; ++q) {
+                uint4* at = T8::at(buf, lane, (at_col >> 3) + q);
                 if (p.beta != 0.f) {
-                  const uint4 cc = *reinterpret_cast<const uint4*>(cptr + i);
+                  const uint4 cc = *at;
                   const __nv_bfloat162* c2 = reinterpret_cast<const __nv_bfloat162*>(&cc);
 #pragma unroll
                   for (int j = 0; j < 4; ++j) {
                     const float2 f = __bfloat1622float2(c2[j]);
-                    v[i + 2 * j] += p.beta * f.x;
-                    v[i + 2 * j + 1] += p.beta * f.y;
+                    v[8 * q + 2 * j] += p.beta * f.x;
+                    v[8 * q + 2 * j + 1] += p.beta * f.y;
                   }
                 }
                 uint4 o;
                 __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) o2[j] = __floats2bfloat162_rn(v[i + 2 * j], v[i + 2 * j + 1]);
-                *reinterpret_cast<uint4*>(dptr + i) = o;
+                for (int j = 0; j < 4; ++j) o2[j] = __floats2bfloat162_rn(v[8 * q + 2 * j], v[8 * q + 2 * j + 1]);
+                *at = o;
               }
             }
-          }
+          };
+          finish(r0, 0);
+          if (!p.d_fp32) finish(r1, 32);
+          __syncwarp();
+          T8::store(buf, drow + static_cast<size_t>(col) * es, static_cast<size_t>(p.ldd) * es, rows, pieces_at(col), lane);
+          __syncwarp();
         }
-      }
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_leader(&tempty_bar[acc]);   // 4 warps x 2 CTAs release the accumulator
+      if (lane == 0) mbar_arrive_leader(&tempty_bar[acc]);   // the warps of both CTAs release the accumulator
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
   }
@@ -1057,16 +1189,16 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   }
 }
 
-template <bool A_MN, bool B_MN, int EPI = 0>
+template <bool A_MN, bool B_MN, int EPI = 0, int GROUPED = 0>
 static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t stream) {
-  auto kern = gemm2_kernel<A_MN, B_MN, EPI>;
+  auto kern = gemm2_kernel<A_MN, B_MN, EPI, GROUPED>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring2<EPI>::TOTAL);
     if (e != cudaSuccess) return -300 - static_cast<int>(e);
     configured = true;
   }
-  kern<<<grid, 192, SMEM2_TOTAL, stream>>>(ta, tb, p);
+  kern<<<grid, 64 + 32 * EPI2_WARPS, Ring2<EPI>::TOTAL, stream>>>(ta, tb, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -400 - static_cast<int>(e);
 }
@@ -1386,6 +1518,13 @@ int ftb_gemm_bf16_splitk(const void* A, const void* B, void* D, const void* C, c
   return e == cudaSuccess ? 0 : -400 - static_cast<int>(e);
 }
 
+// Row groups on two-SM tiles (256 rows) where a group has that many rows of the buffer: 16384 x 8 slots over 64 experts,
+// 2048 x 1024: up 642 -> 470 us, down 774 -> 501 us; 8000 x 8 over 128, 2048 x 768: up 275 -> 187, down 383 -> 197.  At 1024
+// x 8 over 64 (128 rows an expert and 128 of padding) 78.5 / 86.5 us on one SM and 80 / 74 on two; at 1024 x 8 over 128
+// (64 rows), where half of every tile is empty, 100 / 97 against 125 / 119, so those stay.  Weight gradients, whose rows are
+// the reduction, always: 64 experts 594 -> 433 us, 128 experts 626 -> 298 us.
+constexpr int GROUPED_TWO_SM_ROWS = 256;
+
 // Grouped GEMM over expert-major rows:  D[rows_g, :] = alpha * A[rows_g, :] * op(B[g]) + beta * C[rows_g, :].
 //   A (total_rows, K) row-major; B (G, N, K) if b_mn_major = 0, (G, K, N) if 1; offsets (G+1) int32 on device.
 //   max_tiles >= sum_g ceil(rows_g/128) * ceil(N/bn); the bound total_rows/128 + G row tiles always suffices.
@@ -1394,6 +1533,7 @@ int ftb_grouped_gemm_bf16(const void* A, const void* B, void* D, const void* C, 
                           int d_fp32, int max_ctas, cudaStream_t stream) {
   if (total_rows <= 0 || N <= 0 || num_groups <= 0) return 0;
   if ((lda & 7) || (N & 7) || (K & 7)) return -2;
+  const bool two_sm = g_use_2cta && N >= 256 && total_rows >= GROUPED_TWO_SM_ROWS * num_groups;
   const int bn = (N <= 128) ? 128 : 256;
   CUtensorMap ta, tb;
   int rc;
@@ -1407,7 +1547,7 @@ int ftb_grouped_gemm_bf16(const void* A, const void* B, void* D, const void* C, 
   if (!b_mn_major) {
     uint64_t dims[3] = {(uint64_t)K, (uint64_t)N, (uint64_t)num_groups};
     uint64_t str[2] = {(uint64_t)K * 2, (uint64_t)K * N * 2};
-    uint32_t box[3] = {BK, (uint32_t)bn, 1};
+    uint32_t box[3] = {BK, (uint32_t)(two_sm ? BM : bn), 1};       // two SMs: half of the 256-wide B tile each
     rc = make_tmap(&tb, B, 3, dims, str, box);
   } else {
     uint64_t dims[3] = {(uint64_t)N, (uint64_t)K, (uint64_t)num_groups};
@@ -1423,6 +1563,15 @@ int ftb_grouped_gemm_bf16(const void* A, const void* B, void* D, const void* C, 
   p.num_groups = num_groups; p.offsets = offsets;
   p.comm_mode = 0; p.world = 1; p.rank = 0; p.panel_rows = 0; p.split_k = 1; p.k_per_split = 0;
   const int tiles_n = (N + bn - 1) / bn;
+  if (two_sm) {
+    p.max_tiles = ((total_rows + 2 * BM - 1) / (2 * BM) + num_groups) * tiles_n;
+    int grid2 = sm_count() & ~1;
+    if (max_ctas > 0 && max_ctas < grid2) grid2 = max_ctas & ~1;
+    if (2 * p.max_tiles < grid2) grid2 = 2 * p.max_tiles;
+    if (grid2 < 2) grid2 = 2;
+    return b_mn_major ? launch2<false, true, 0, 1>(ta, tb, p, grid2, stream)
+                      : launch2<false, false, 0, 1>(ta, tb, p, grid2, stream);
+  }
   p.max_tiles = ((total_rows + BM - 1) / BM + num_groups) * tiles_n;
   int grid = sm_count();
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
@@ -1461,6 +1610,14 @@ int ftb_grouped_wgrad_bf16(const void* dY, const void* X, void* G, const int* of
   p.D = G; p.C = G; p.bias = nullptr; p.d_fp32 = g_fp32;
   p.num_groups = num_groups; p.offsets = offsets; p.max_tiles = 0;
   p.comm_mode = 0; p.world = 1; p.rank = 0; p.panel_rows = 0; p.split_k = 1; p.k_per_split = 0;
+  if (g_use_2cta && N >= 256 && Kd >= 256) {
+    const int tiles2 = num_groups * ((N + 2 * BM - 1) / (2 * BM)) * ((Kd + BN2 - 1) / BN2);
+    int grid2 = sm_count() & ~1;
+    if (max_ctas > 0 && max_ctas < grid2) grid2 = max_ctas & ~1;
+    if (2 * tiles2 < grid2) grid2 = 2 * tiles2;
+    if (grid2 < 2) grid2 = 2;
+    return launch2<true, true, 0, 2>(ta, tb, p, grid2, stream);
+  }
   const int tiles = num_groups * ((N + BM - 1) / BM) * ((Kd + bn - 1) / bn);
   int grid = sm_count();
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
