@@ -838,7 +838,11 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   const bool leader = cta == 0;
   const int tiles_m = (p.M + 2 * BM - 1) / (2 * BM);
   const int tiles_n = EPI == 1 ? p.glu_F / (BN2 / 2) : (p.N + BN2 - 1) / BN2;
-  const int num_tiles = GROUPED == 1 ? p.max_tiles : GROUPED == 2 ? p.num_groups * tiles_m * tiles_n : tiles_m * tiles_n;
+  // split K (plain form): slice sp of the reduction of every tile is a tile of its own, written to slab sp of D
+  const bool split = EPI == 0 && GROUPED == 0 && p.split_k > 1;
+  const int num_tiles = GROUPED == 1 ? p.max_tiles : GROUPED == 2 ? p.num_groups * tiles_m * tiles_n
+                                                                  : tiles_m * tiles_n * (split ? p.split_k : 1);
+  auto slice_blocks = [&](int sp) { return (min(p.K - sp * p.k_per_split, p.k_per_split) + BK - 1) / BK; };
   int k_blocks = (p.K + BK - 1) / BK;              // (grouped weight gradients: of the tile's group)
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
 
@@ -878,6 +882,11 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
             k_lo = p.offsets[g];
             k_blocks = (p.offsets[g + 1] - k_lo + BK - 1) / BK;
             if (k_blocks == 0) continue;
+          } else if (split) {
+            const int sp = tile / (tiles_m * tiles_n);
+            t -= sp * tiles_m * tiles_n;
+            k_lo = sp * p.k_per_split;
+            k_blocks = slice_blocks(sp);
           }
           tile_coords(t, tiles_m, tiles_n, tm, tn);
           row0 = tm * 2 * BM;
@@ -933,6 +942,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
           k_blocks = (p.offsets[g + 1] - p.offsets[g] + BK - 1) / BK;
           if (k_blocks == 0) continue;
         }
+        if (split) k_blocks = slice_blocks(tile / (tiles_m * tiles_n));
         if (!(ok = mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag, 60))) break;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * BN2;
@@ -981,6 +991,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
           const size_t skip = static_cast<size_t>(g) * p.M * p.ldd * (p.d_fp32 ? 4 : 2);
           d_base += skip;
           c_base += skip;
+        } else if (split) {
+          const int sp = tile / (tiles_m * tiles_n);
+          t -= sp * tiles_m * tiles_n;
+          d_base += static_cast<size_t>(sp) * p.M * p.ldd * 4;         // fp32 slabs
         }
         tile_coords(t, tiles_m, tiles_n, tm, tn);
         row0 = tm * 2 * BM;
@@ -1037,7 +1051,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
         using T4 = Turn<4>;
         // saved gate / up values of 32 columns, fetched one step ahead of their use (the first step is issued before the
         // wait for the accumulator, it does not depend on the MMAs).  Two steps ahead, with the loop unrolled for it, was
-        // slower: 9377 x 3072 x 1024 141 us against 110.
+        // slower: 9377 x 3072 x 1024 141 us against 110 to 127.
         uint4 xg[4] = {}, xu[4] = {};
         const uint8_t* xrow = reinterpret_cast<const uint8_t*>(p.glu_x13) + row * p.glu_ld_x13 * 2;
         auto fetch_x13 = [&](int col) {
@@ -1213,6 +1227,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, int splits, v
   const long e = i4 * 4;
   const int m = (int)(e / N), n = (int)(e - (long)m * N);
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
   for (int sl = 0; sl < splits; ++sl) {
     const float4 v = *reinterpret_cast<const float4*>(ws + (size_t)sl * M * N + e);
     acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
@@ -1468,7 +1483,8 @@ int ftb_gemm_bf16_splitk(const void* A, const void* B, void* D, const void* C, c
   if ((lda & 7) || (ldb & 7) || (N & 7) || (reinterpret_cast<uintptr_t>(A) & 15) ||
       (reinterpret_cast<uintptr_t>(B) & 15) || (reinterpret_cast<uintptr_t>(D) & 15))
     return -2;
-  const int bn = (N <= 128) ? 128 : 256;
+  const bool two_sm = g_use_2cta && M >= 512 && N >= 512;
+  const int bn = two_sm ? BM : (N <= 128) ? 128 : 256;        // two SMs: half of the 256-wide B tile each
   int kps = ((K + splits - 1) / splits + BK - 1) / BK * BK;
   splits = (K + kps - 1) / kps;
   CUtensorMap ta, tb;
@@ -1504,11 +1520,18 @@ int ftb_gemm_bf16_splitk(const void* A, const void* B, void* D, const void* C, c
   p.num_groups = 0; p.offsets = nullptr; p.max_tiles = 0;
   p.comm_mode = 0; p.world = 1; p.rank = 0; p.panel_rows = 0;
   p.split_k = splits; p.k_per_split = kps;
-  const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn) * splits;
   int grid = sm_count();
-  if (tiles < grid) grid = tiles;
-  rc = (bn == 256) ? dispatch_major<256, 4, 0>(a_mn_major, b_mn_major, ta, tb, p, grid, stream)
-                   : dispatch_major<128, 6, 0>(a_mn_major, b_mn_major, ta, tb, p, grid, stream);
+  if (two_sm) {
+    const int tiles2 = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN2 - 1) / BN2) * splits;
+    grid = 2 * tiles2 < grid ? 2 * tiles2 : grid & ~1;
+    rc = !a_mn_major ? (!b_mn_major ? launch2<false, false>(ta, tb, p, grid, stream) : launch2<false, true>(ta, tb, p, grid, stream))
+                     : (!b_mn_major ? launch2<true, false>(ta, tb, p, grid, stream) : launch2<true, true>(ta, tb, p, grid, stream));
+  } else {
+    const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn) * splits;
+    if (tiles < grid) grid = tiles;
+    rc = (bn == 256) ? dispatch_major<256, 4, 0>(a_mn_major, b_mn_major, ta, tb, p, grid, stream)
+                     : dispatch_major<128, 6, 0>(a_mn_major, b_mn_major, ta, tb, p, grid, stream);
+  }
   if (rc) return rc;
   const long n4 = (long)M * N / 4;
   splitk_reduce_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, stream>>>(workspace, splits, D, C != nullptr ? C : D,

@@ -7,6 +7,7 @@ never a silent fallback: the CUDA path is the product, the torch path is the CPU
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from ctypes import c_float, c_int, c_long, c_void_p
 from typing import Optional
@@ -124,6 +125,28 @@ def gemm_supported(a: torch.Tensor, b: torch.Tensor, trans_a: bool, trans_b: boo
         and b.data_ptr() % 16 == 0
 
 
+@functools.lru_cache(maxsize=4096)
+def _two_sm_splits(M: int, N: int, K: int) -> int:
+    """Slices of K (fp32 slabs, ordered sum) for a GEMM on two-SM tiles: more than one where 256 x 256 tiles leave many of the
+    74 pairs of SMs idle, in their only wave (weight gradients of narrow layers) or in the last of few (the head's input
+    gradient), and K is long enough to pay for the slabs.
+
+    The times of the rule: a pair does 64 of K in some 512 cycles of 1.75 GHz; a slab is written and read at 4 TB/s; the
+    second launch costs 4 us.  At K = 16384, us without and with its choice: 768 x 768 (9 tiles) 82 / 27, 768 x 2304 (27) 85 /
+    56, 1024 x 4096 (64) 99, not split (113 with two slices); 1024 x 1024 x 9377 49 / 28; 4096 x 1152 x 262144 (80) 2941 / 2250;
+    3001 x 2048 x 128256 (96) 1968 / 1161; 768 x 768 x 1024 20, not split (21 to 23)."""
+    tiles = -(-M // 256) * -(-N // 256)
+    full = K / 64 * 512 / 1.75e3
+    best, least = 1, 0.88 * -(-tiles // 74) * full
+    for s in range(2, 9):
+        if s * M * N * 4 > 128 << 20 or K // s < 256:
+            break
+        us = -(-tiles * s // 74) / s * full + s * M * N * 8 / 4e6 + 4.0
+        if us < least:
+            best, least = s, us
+    return best
+
+
 def gemm(a, b, *, trans_a=False, trans_b=False, alpha=1.0, beta=0.0, c=None, bias=None, out=None, out_dtype=None,
          bn: int = 0):
     """``out = alpha * op(a) @ op(b) + beta * c + bias`` on the tcgen05 kernel.
@@ -149,8 +172,12 @@ def gemm(a, b, *, trans_a=False, trans_b=False, alpha=1.0, beta=0.0, c=None, bia
     # small output, long reduction (rank-r LoRA gradients: M or N = r, K = tokens): a handful of tiles would each walk
     # the whole K on a handful of SMs; split K so that tiles x slices fill the GPU (fp32 slabs + ordered reduce)
     tiles = ((M + 127) // 128) * ((N + (127 if N <= 128 else 255)) // (128 if N <= 128 else 256))
+    splits = 1
     if bn == 0 and tiles <= 40 and K >= 4096 and (N <= 128 or M < 512):
         splits = max(2, min(148 // tiles, K // 512, 64))
+    elif bn == 0 and M >= 512 and N >= 512 and GEMM_MAX_CTAS == 0:
+        splits = _two_sm_splits(M, N, K)
+    if splits > 1:
         ws = torch.empty(splits * M * N, dtype=torch.float32, device=a.device)
         rc = lib.ftb_gemm_bf16_splitk(_ptr(a), _ptr(b), _ptr(out), _ptr(c), _ptr(bias), c_int(M), c_int(N), c_int(K),
                                       c_int(1 if trans_a else 0), c_int(0 if trans_b else 1), c_int(a.stride(0)),

@@ -84,3 +84,24 @@ def test_grouped_two_sm(counts, N, K):
                 want = dy[s].double().t() @ xx[s].double() + (before[e].double() if acc else 0)
                 _close(g[e], want, dy[s].double().abs().t() @ xx[s].double().abs(), cnt[e])
     assert k.device_error_words().get("gemm_tcgen05", 0) == 0
+
+
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N,K", [(512, 512, 4096), (768, 520, 8200), (1000, 776, 16384)])
+@pytest.mark.parametrize("ta,tb", [(True, False), (False, False), (False, True)])
+def test_two_sm_split_k(out_dtype, M, N, K, ta, tb):
+    """Few tiles and a long reduction: slices of K on two-SM tiles, the last one shorter, with C, bias and a strided D."""
+    from flextrain_b200.ops import cuda as k
+    assert k._two_sm_splits(M, N, K) > 1
+    torch.manual_seed(0)
+    a = (torch.randn(K, M, device=DEV) if ta else torch.randn(M, K, device=DEV)).bfloat16()
+    b = (torch.randn(N, K, device=DEV) if tb else torch.randn(K, N, device=DEV)).bfloat16()
+    A, B = (a.t() if ta else a).double(), (b.t() if tb else b).double()
+    prod, mag = A @ B, A.abs() @ B.abs()
+    bias = torch.randn(N, device=DEV)
+    wide = torch.randn(M, N + 24, device=DEV).to(out_dtype)
+    keep = wide.clone()
+    k.gemm(a, b, trans_a=ta, trans_b=tb, alpha=0.5, beta=1.0, bias=bias, out=wide[:, 8:8 + N])
+    _close(wide[:, 8:8 + N], 0.5 * prod + bias.double() + keep[:, 8:8 + N].double(), mag, K)
+    assert torch.equal(wide[:, :8], keep[:, :8]) and torch.equal(wide[:, 8 + N:], keep[:, 8 + N:])
+    assert k.device_error_words().get("gemm_tcgen05", 0) == 0
