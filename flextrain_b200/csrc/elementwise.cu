@@ -760,6 +760,92 @@ __global__ void __launch_bounds__(ADAM_THREADS) adamw_kernel(const __grid_consta
   }
 }
 
+// ------------------------------------------------------------------------------- Muon
+// The elementwise parts of the Muon update for a batch of matrices of one size.  With gf = g * grad_scale and
+// mf = beta * mom + gf, the update is u = gf + beta * mf (Nesterov) or mf, normalised by its Frobenius norm:
+//   muon_norm      partial sums of u^2 per matrix (a block adds 16384 elements)
+//   muon_prepare   mom = mf;  x = u / (||u|| + 1e-7) in bf16, the start of the Newton-Schulz iteration
+//   muon_apply     p = p * (1 - lr * wd) - lr * scale * x
+// u is computed twice rather than kept: its fp32 copy would cost more to write and read than g and mom do.  Bound by
+// memory.  One launch each for up to MUON_MAX matrices, in place of twelve library kernels per matrix.
+constexpr int MUON_MAX = 64;
+constexpr int MUON_THREADS = 256;
+constexpr int MUON_PER_BLOCK = MUON_THREADS * 64;
+struct MuonArgs {
+  const void* g[MUON_MAX];
+  void* m[MUON_MAX];
+  void* p[MUON_MAX];
+  long n;                // elements of a matrix, a multiple of 8
+  long x_stride;         // elements from one matrix to the next in x
+  int g_dt, m_dt, nesterov;
+  float beta, grad_scale, keep, step;
+};
+
+template <bool GF, bool MF>
+__device__ __forceinline__ void muon_update8(const MuonArgs& a, int mat, long i, float (&mf)[8], float (&u)[8]) {
+  float g[8];
+  unpack_raw8<GF>(ld_raw8<GF>(a.g[mat], i), g);
+  unpack_raw8<MF>(ld_raw8<MF>(a.m[mat], i), mf);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float gf = g[j] * a.grad_scale;
+    mf[j] = a.beta * mf[j] + gf;
+    u[j] = a.nesterov ? gf + a.beta * mf[j] : mf[j];
+  }
+}
+
+template <bool GF, bool MF>
+__global__ void __launch_bounds__(MUON_THREADS) muon_norm_kernel(const __grid_constant__ MuonArgs a, float* __restrict__ partial) {
+  __shared__ float sh[MUON_THREADS / 32];
+  const int mat = blockIdx.y;
+  float s = 0.f;
+  for (int k = 0; k < 8; ++k) {
+    const long i = (long)blockIdx.x * MUON_PER_BLOCK + ((long)k * MUON_THREADS + threadIdx.x) * 8;
+    if (i >= a.n) break;
+    float mf[8], u[8];
+    muon_update8<GF, MF>(a, mat, i, mf, u);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s += u[j] * u[j];
+  }
+  s = block_sum<MUON_THREADS / 32>(s, sh);
+  if (threadIdx.x == 0) partial[(long)mat * gridDim.x + blockIdx.x] = s;
+}
+
+template <bool GF, bool MF>
+__global__ void __launch_bounds__(MUON_THREADS) muon_prepare_kernel(const __grid_constant__ MuonArgs a,
+                                                                    const float* __restrict__ partial, bf16* __restrict__ x) {
+  __shared__ float sh[MUON_THREADS / 32];
+  const int mat = blockIdx.y;
+  float s = 0.f;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += MUON_THREADS) s += partial[(long)mat * gridDim.x + b];
+  const float norm = sqrtf(block_sum<MUON_THREADS / 32>(s, sh)) + 1e-7f;
+  for (int k = 0; k < 8; ++k) {
+    const long i = (long)blockIdx.x * MUON_PER_BLOCK + ((long)k * MUON_THREADS + threadIdx.x) * 8;
+    if (i >= a.n) break;
+    float mf[8], u[8];
+    muon_update8<GF, MF>(a, mat, i, mf, u);
+    st_raw8<MF>(a.m[mat], i, mf);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) u[j] = u[j] / norm;
+    *reinterpret_cast<uint4*>(x + mat * a.x_stride + i) = pack8(u);
+  }
+}
+
+__global__ void __launch_bounds__(MUON_THREADS) muon_apply_kernel(const __grid_constant__ MuonArgs a, const bf16* __restrict__ x) {
+  const int mat = blockIdx.y;
+  for (int k = 0; k < 8; ++k) {
+    const long i = (long)blockIdx.x * MUON_PER_BLOCK + ((long)k * MUON_THREADS + threadIdx.x) * 8;
+    if (i >= a.n) break;
+    float p[8], v[8];
+    uint4* pp = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(a.p[mat]) + i);
+    unpack8(*pp, p);
+    unpack8(*reinterpret_cast<const uint4*>(x + mat * a.x_stride + i), v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) p[j] = p[j] * a.keep - a.step * v[j];
+    *pp = pack8(p);
+  }
+}
+
 // ------------------------------------------------------------------------ sum of squares
 // Sum of the squares of up to SQ_MAX tensors (the gradient norm): one pass that reads every element once, in place of a
 // conversion to fp32, a squaring and a reduction per tensor.  A block adds 16384 elements in fp32 (64 a thread, then a
@@ -1111,6 +1197,43 @@ int ftb_adamw_multi(int count, void** p, const void** g, void** m, void** v, con
   a.count = count; a.beta1 = beta1; a.beta2 = beta2; a.eps = eps; a.bc1 = bc1; a.bc2 = bc2; a.grad_scale = grad_scale;
   if (blocks == 0) return 0;
   adamw_kernel<<<(unsigned)blocks, ADAM_THREADS, 0, s>>>(a);
+  CHECK_LAUNCH();
+}
+
+// `count` <= 64 bf16 matrices of n elements each (a multiple of 8, all pointers on 16 bytes); partial: count * blocks floats,
+// blocks = ceil(n / 16384); x: matrix i at x + i * x_stride.  dtype codes as for AdamW.
+int ftb_muon_prepare(int count, const void** g, void** m, long n, long x_stride, int g_dt, int m_dt, float beta, int nesterov,
+                     float grad_scale, float* partial, void* x, cudaStream_t s) {
+  if (count <= 0 || n <= 0) return 0;
+  if (count > MUON_MAX || (n & 7)) return -2;
+  MuonArgs a;
+  for (int i = 0; i < count; ++i) {
+    if (((uintptr_t)g[i] | (uintptr_t)m[i]) & 15) return -2;
+    a.g[i] = g[i]; a.m[i] = m[i]; a.p[i] = nullptr;
+  }
+  a.n = n; a.x_stride = x_stride; a.g_dt = g_dt; a.m_dt = m_dt; a.nesterov = nesterov; a.beta = beta;
+  a.grad_scale = grad_scale; a.keep = 0.f; a.step = 0.f;
+  const dim3 grid((unsigned)((n + MUON_PER_BLOCK - 1) / MUON_PER_BLOCK), count);
+#define FTB_MUON(GF, MF)                                             \
+  muon_norm_kernel<GF, MF><<<grid, MUON_THREADS, 0, s>>>(a, partial); \
+  muon_prepare_kernel<GF, MF><<<grid, MUON_THREADS, 0, s>>>(a, partial, (bf16*)x)
+  if (g_dt && m_dt) { FTB_MUON(true, true); }
+  else if (g_dt) { FTB_MUON(true, false); }
+  else if (m_dt) { FTB_MUON(false, true); }
+  else { FTB_MUON(false, false); }
+#undef FTB_MUON
+  CHECK_LAUNCH();
+}
+int ftb_muon_apply(int count, void** p, const void* x, long n, long x_stride, float keep, float step, cudaStream_t s) {
+  if (count <= 0 || n <= 0) return 0;
+  if (count > MUON_MAX || (n & 7)) return -2;
+  MuonArgs a;
+  for (int i = 0; i < count; ++i) {
+    if ((uintptr_t)p[i] & 15) return -2;
+    a.g[i] = nullptr; a.m[i] = nullptr; a.p[i] = p[i];
+  }
+  a.n = n; a.x_stride = x_stride; a.g_dt = a.m_dt = a.nesterov = 0; a.beta = a.grad_scale = 0.f; a.keep = keep; a.step = step;
+  muon_apply_kernel<<<dim3((unsigned)((n + MUON_PER_BLOCK - 1) / MUON_PER_BLOCK), count), MUON_THREADS, 0, s>>>(a, (const bf16*)x);
   CHECK_LAUNCH();
 }
 

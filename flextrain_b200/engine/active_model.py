@@ -756,11 +756,9 @@ class ActiveModel:
         nL = len(self.layers)
         ringed = not (bm.params_resident and bm.grads_resident and bm.opt_resident)
         if not ringed:
-            for l, layer in enumerate(self.layers):
-                rc |= opt.step(layer.param_spec, bm.params(l), bm.grads(l), bm.opt_state(l), self.step_num, grad_scale)
-                if rc:
-                    return rc
-            return rc
+            from ..optim.base import step_units
+            return step_units(opt, [(layer.param_spec, bm.params(l), bm.grads(l), bm.opt_state(l))
+                                    for l, layer in enumerate(self.layers)], self.step_num, grad_scale)
         # ---- streamed step: prefetch k+depth on inbound, update on compute, write back on outbound
         ring_n = [n for n, res in ((bm.n_p, bm.params_resident), (bm.n_g, bm.grads_resident),
                                    (max(bm.n_o, 2), bm.opt_resident)) if not res]

@@ -374,14 +374,17 @@ def embedding_bwd(dy, tokens, grad_table, scale=1.0):
 # ------------------------------------------------------------------------- optimizers
 def adamw_multi(params, grads, ms, vs, *, lrs, wds, beta1, beta2, eps, step, grad_scale=1.0):
     """Fused AdamW over a list of tensors (one launch per layer on CUDA)."""
-    ok = all(p.is_cuda and p.is_contiguous() and g.is_contiguous() and p.dtype in (torch.bfloat16, torch.float32)
-             and g.dtype in (torch.bfloat16, torch.float32) and m.dtype in (torch.bfloat16, torch.float32)
-             and m.dtype == v.dtype for p, g, m, v in zip(params, grads, ms, vs))
-    if ok and params:
-        _count((len(params) + 23) // 24)
-        return _kernels().adamw_multi(params, grads, ms, vs, lrs=list(lrs), wds=list(wds), beta1=beta1, beta2=beta2,
-                                      eps=eps, step=step, grad_scale=grad_scale)
-    for p, g, m, v, lr, wd in zip(params, grads, ms, vs, lrs, wds):
+    rest = list(zip(params, grads, ms, vs, lrs, wds))
+    ok = [p.is_cuda and p.is_contiguous() and g.is_contiguous() and p.dtype in (torch.bfloat16, torch.float32)
+          and g.dtype in (torch.bfloat16, torch.float32) and m.dtype in (torch.bfloat16, torch.float32)
+          and m.dtype == v.dtype for p, g, m, v, _, _ in rest]
+    if any(ok):
+        P, G, M, V, L, W = map(list, zip(*[r for r, o in zip(rest, ok) if o]))
+        _count((len(P) + 23) // 24)
+        _kernels().adamw_multi(P, G, M, V, lrs=L, wds=W, beta1=beta1, beta2=beta2, eps=eps, step=step,
+                               grad_scale=grad_scale)
+        rest = [r for r, o in zip(rest, ok) if not o]
+    for p, g, m, v, lr, wd in rest:
         ref.adamw_step(p, g, m, v, lr=lr, beta1=beta1, beta2=beta2, eps=eps, weight_decay=wd, step=step,
                        grad_scale=grad_scale)
 
@@ -402,42 +405,46 @@ def sum_of_squares(tensors, device):
     return out
 
 
-def newton_schulz_bf16(u: torch.Tensor, iters: int = 5) -> torch.Tensor:
-    """Quintic Newton-Schulz orthogonalisation of one matrix on the tcgen05 GEMM, bf16 iterates with fp32
-    accumulation: per iteration ``A = X Xᵀ``, ``B = bA + cA²`` (epilogue ``alpha=c, beta=b``), ``X = aX + BX``
-    (epilogue ``beta=a``) — three launches, no elementwise pass (flextrain/ops/_kernels/muon.py:53-61 issues
-    mm / addmm through cuBLAS).  A tall matrix is iterated as ``AᵀA`` on the right, so nothing is transposed."""
-    a, b, c = ref.NS_COEFFS
-    x = (u / (u.norm() + 1e-7)).to(torch.bfloat16).contiguous()
-    tall = x.shape[0] > x.shape[1]
-    for _ in range(iters):
-        if not tall:
-            A = gemm(x, x, trans_b=True)                       # (m, m)
-            B = gemm(A, A, alpha=c, beta=b, c=A)
-            x = gemm(B, x, beta=a, c=x)
-        else:
-            A = gemm(x, x, trans_a=True)                       # (n, n) = XᵀX
-            B = gemm(A, A, alpha=c, beta=b, c=A)
-            x = gemm(x, B, beta=a, c=x)
-    return x
-
-
 def muon_step(p, g, mom, *, lr, beta=0.95, weight_decay=0.0, ns_iters=5, nesterov=True, grad_scale=1.0):
-    """Muon update (flextrain/ops/_kernels/muon.py:16-75).  On CUDA bf16 the Newton-Schulz GEMMs run on the
-    tcgen05 kernel; 3-D tensors (stacked experts) are updated matrix by matrix."""
-    if not (_cuda_bf16(p) and _GEMM_BACKEND == "tcgen05" and p.dim() in (2, 3) and min(p.shape[-2:]) >= 64
-            and p.shape[-1] % 8 == 0 and p.shape[-2] % 8 == 0):
-        return ref.muon_step(p, g, mom, lr=lr, beta=beta, weight_decay=weight_decay, ns_iters=ns_iters,
-                             nesterov=nesterov, grad_scale=grad_scale)
-    gf = g.to(torch.float32) * grad_scale
-    mf = beta * mom.to(torch.float32) + gf
-    mom.copy_(mf.to(mom.dtype))
-    u = gf + beta * mf if nesterov else mf
-    scale = 0.2 * math.sqrt(max(p.shape[-2], p.shape[-1]))
-    mats = [(p, u)] if p.dim() == 2 else [(p[i], u[i]) for i in range(p.shape[0])]
-    for pm, um in mats:
-        x = newton_schulz_bf16(um, ns_iters)
-        pm.copy_((pm.to(torch.float32) * (1.0 - lr * weight_decay) - (lr * scale) * x.to(torch.float32)).to(pm.dtype))
+    """Muon update of one tensor (flextrain/ops/_kernels/muon.py:16-75); 3-D tensors (stacked experts) are batches of
+    matrices."""
+    muon_multi([p], [g], [mom], lr=lr, beta=beta, weight_decay=weight_decay, ns_iters=ns_iters, nesterov=nesterov,
+               grad_scale=grad_scale)
+
+
+MUON_BATCH_ELEMENTS = 64 << 20      # of one batch's iterate: its workspace is four to five buffers of at most this size
+
+
+def muon_multi(ps, gs, moms, *, lr, beta=0.95, weight_decay=0.0, ns_iters=5, nesterov=True, grad_scale=1.0):
+    """Muon update of many tensors.  On CUDA bf16, matrices of one size go through the Newton-Schulz iteration together, as
+    grouped tcgen05 GEMMs: a model's 768 x 768 matrices have 9 output tiles each, for 74 pairs of SMs, and three launches
+    per iteration and matrix took longer to issue than to run (36 matrices of six layers: 630 launches)."""
+    kw = dict(lr=lr, beta=beta, weight_decay=weight_decay, ns_iters=ns_iters, nesterov=nesterov, grad_scale=grad_scale)
+    ready = lambda t: t.is_contiguous() and t.data_ptr() % 16 == 0
+    batches, back = {}, []
+    for p, g, mom in zip(ps, gs, moms):
+        if not (_cuda_bf16(p) and _GEMM_BACKEND == "tcgen05" and p.dim() in (2, 3) and min(p.shape[-2:]) >= 64
+                and p.shape[-1] % 8 == 0 and p.shape[-2] % 8 == 0 and p.numel()):
+            ref.muon_step(p, g, mom, **kw)
+            continue
+        f32 = lambda t: t if t.dtype in (torch.bfloat16, torch.float32) else t.to(torch.float32)
+        src = []
+        for t, written in ((p, True), (f32(g), False), (mom, True)):
+            c = f32(t)
+            c = c if ready(c) else c.clone(memory_format=torch.contiguous_format)
+            if written and c is not t:
+                back.append((t, c))
+            src.append(c)
+        mats = zip(*[t.unbind(0) if t.dim() == 3 else (t,) for t in src])
+        for pm, gm, mm in mats:
+            batches.setdefault((pm.shape, gm.dtype, mm.dtype, pm.device), []).append((pm, gm, mm))
+    for (shape, *_), mats in batches.items():
+        per = max(1, MUON_BATCH_ELEMENTS // (shape[0] * shape[1]))
+        for i in range(0, len(mats), per):
+            _count(3 + 3 * ns_iters)
+            _kernels().muon_batch(*[list(t) for t in zip(*mats[i:i + per])], coeffs=ref.NS_COEFFS, **kw)
+    for t, c in back:
+        t.copy_(c)
 
 
 # -------------------------------------------------------------------------------- MoE

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import math
 import os
 from ctypes import c_float, c_int, c_long, c_void_p
 from typing import Optional
@@ -204,8 +205,9 @@ def gemm(a, b, *, trans_a=False, trans_b=False, alpha=1.0, beta=0.0, c=None, bia
     return out
 
 
-def grouped_gemm(x, w, offsets, *, trans_w=True, out=None, alpha=1.0, beta=0.0):
-    """Expert-major grouped GEMM in one launch. ``x (R,K)``, ``w (E,N,K)`` (``trans_w``) or ``(E,K,N)``."""
+def grouped_gemm(x, w, offsets, *, trans_w=True, out=None, alpha=1.0, beta=0.0, c=None):
+    """Expert-major grouped GEMM in one launch. ``x (R,K)``, ``w (E,N,K)`` (``trans_w``) or ``(E,K,N)``; ``beta`` scales
+    ``c`` (rows as ``out``'s), or ``out`` itself when none is given."""
     lib = load("gemm_tcgen05")
     E = w.shape[0]
     N = w.shape[1] if trans_w else w.shape[2]
@@ -213,7 +215,9 @@ def grouped_gemm(x, w, offsets, *, trans_w=True, out=None, alpha=1.0, beta=0.0):
     assert w.is_contiguous() and x.stride(1) == 1 and offsets.dtype == torch.int32
     if out is None:
         out = torch.empty(x.shape[0], N, dtype=torch.bfloat16, device=x.device)
-    rc = lib.ftb_grouped_gemm_bf16(_ptr(x), _ptr(w), _ptr(out), _ptr(out if beta != 0 else None), _ptr(offsets),
+    assert c is None or (c.shape == out.shape and c.stride() == out.stride() and c.dtype == out.dtype)
+    rc = lib.ftb_grouped_gemm_bf16(_ptr(x), _ptr(w), _ptr(out), _ptr((out if c is None else c) if beta != 0 else None),
+                                   _ptr(offsets),
                                    c_int(E), c_int(x.shape[0]), c_int(N), c_int(K), c_int(0 if trans_w else 1),
                                    c_int(x.stride(0)), c_int(out.stride(0)), c_float(alpha), c_float(beta),
                                    c_int(1 if out.dtype == torch.float32 else 0), c_int(GEMM_MAX_CTAS), _stream())
@@ -466,6 +470,50 @@ def adamw_multi(params, grads, ms, vs, *, lrs, wds, beta1, beta2, eps, step, gra
                                  (c_int * n)(*[_DT[t.dtype] for t in M]), c_float(beta1), c_float(beta2),
                                  c_float(eps), c_float(bc1), c_float(bc2), c_float(grad_scale), _stream())
         _check(rc, "ftb_adamw_multi")
+
+
+def muon_batch(ps, gs, ms, *, lr, beta, weight_decay, ns_iters, nesterov, grad_scale, coeffs):
+    """Muon update of matrices of one size (``ps`` bf16, ``gs`` / ``ms`` of one type each, bf16 or fp32, all contiguous and on
+    16 bytes): the Newton-Schulz iteration of all of them runs as three grouped GEMMs per step, bf16 iterates with fp32
+    accumulation: ``A = X Xᵀ``, ``B = bA + cA²``, ``X = aX + BX`` (epilogues with ``alpha`` and ``beta``).  Tall matrices are
+    iterated as ``AᵀA`` on the right, so nothing is transposed; their rows are padded with zeros to the reduction step."""
+    lib = load("elementwise")
+    (m, n), nb, dev = ps[0].shape, len(ps), ps[0].device
+    a, b, c = coeffs
+    tall = m > n
+    rows = (m + 63) // 64 * 64 if tall else m
+    x = (torch.zeros if rows != m else torch.empty)(nb, rows, n, dtype=torch.bfloat16, device=dev)
+    blocks = (m * n + 16383) // 16384
+    partial = torch.empty(min(nb, 64) * blocks, dtype=torch.float32, device=dev)
+    arr = lambda ts: (c_void_p * len(ts))(*[t.data_ptr() for t in ts])
+    for i in range(0, nb, 64):
+        j = min(i + 64, nb)
+        _check(lib.ftb_muon_prepare(c_int(j - i), arr(gs[i:j]), arr(ms[i:j]), c_long(m * n), c_long(rows * n),
+                                    c_int(_DT[gs[0].dtype]), c_int(_DT[ms[0].dtype]), c_float(beta),
+                                    c_int(1 if nesterov else 0), c_float(grad_scale), _ptr(partial), _ptr(x[i]), _stream()),
+               "ftb_muon_prepare")
+    k = n if tall else m                                       # A and B are (k, k)
+    A = torch.empty(nb, k, k, dtype=torch.bfloat16, device=dev)
+    B, y = torch.empty_like(A), torch.empty_like(x)
+    ofs = torch.arange(0, nb * rows + 1, rows, dtype=torch.int32, device=dev)
+    ofs_k = ofs if k == rows else torch.arange(0, nb * k + 1, k, dtype=torch.int32, device=dev)
+    flat = lambda t: t.view(-1, t.shape[-1])
+    for _ in range(ns_iters):
+        if tall:
+            grouped_wgrad(flat(x), flat(x), ofs, A, accumulate=False)
+        else:
+            grouped_gemm(flat(x), x, ofs, out=flat(A))
+        grouped_gemm(flat(A), A, ofs_k, trans_w=False, out=flat(B), alpha=c, beta=b, c=flat(A))
+        if tall:
+            grouped_gemm(flat(x), B, ofs, trans_w=False, out=flat(y), beta=a, c=flat(x))
+        else:
+            grouped_gemm(flat(B), x, ofs, trans_w=False, out=flat(y), beta=a, c=flat(x))
+        x, y = y, x
+    scale = 0.2 * math.sqrt(max(m, n))
+    for i in range(0, nb, 64):
+        j = min(i + 64, nb)
+        _check(lib.ftb_muon_apply(c_int(j - i), arr(ps[i:j]), _ptr(x[i]), c_long(m * n), c_long(rows * n),
+                                  c_float(1.0 - lr * weight_decay), c_float(lr * scale), _stream()), "ftb_muon_apply")
 
 
 def sum_of_squares(tensors):

@@ -57,21 +57,28 @@ class AdamW:
         return out
 
     def step(self, param_spec, params, grads, state, step_num: int, grad_scale: float = 1.0, only=None) -> int:
+        if self.check_error:
+            G = [grads[t.grad_name] for t in param_spec.trainable() if only is None or t.name in only]
+            if G and not _grads_finite(G):
+                return 1
+        return self.step_units([(param_spec, params, grads, state)], step_num, grad_scale,
+                               only=None if only is None else lambda t: t.name in only)
+
+    def step_units(self, units, step_num: int, grad_scale: float = 1.0, only=None) -> int:
+        """Update of several units (layers) at once, a launch per 24 tensors."""
         P, G, M, V, lrs, wds = [], [], [], [], [], []
-        for t in param_spec.trainable():
-            if only is not None and t.name not in only:
-                continue
-            s = _suffix(t.name)
-            P.append(params[t.name]); G.append(grads[t.grad_name])
-            M.append(state[f"o_adam_m_{s}"]); V.append(state[f"o_adam_v_{s}"])
-            lrs.append(self.lr)
-            wds.append(0.0 if (self.no_decay_1d and len(t.shape) == 1) else self.weight_decay)
-        if not P:
-            return 0
-        if self.check_error and not _grads_finite(G):
-            return 1
-        ops.adamw_multi(P, G, M, V, lrs=lrs, wds=wds, beta1=self.beta1, beta2=self.beta2, eps=self.eps,
-                        step=step_num, grad_scale=grad_scale)
+        for spec, params, grads, state in units:
+            for t in spec.trainable():
+                if only is not None and not only(t):
+                    continue
+                s = _suffix(t.name)
+                P.append(params[t.name]); G.append(grads[t.grad_name])
+                M.append(state[f"o_adam_m_{s}"]); V.append(state[f"o_adam_v_{s}"])
+                lrs.append(self.lr)
+                wds.append(0.0 if (self.no_decay_1d and len(t.shape) == 1) else self.weight_decay)
+        if P:
+            ops.adamw_multi(P, G, M, V, lrs=lrs, wds=wds, beta1=self.beta1, beta2=self.beta2, eps=self.eps,
+                            step=step_num, grad_scale=grad_scale)
         return 0
 
     def flops_per_param(self) -> float:

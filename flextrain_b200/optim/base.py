@@ -52,6 +52,22 @@ def _grads_finite(grads: List[torch.Tensor]) -> bool:
     return float(bad) == 0.0
 
 
+def step_units(opt, units, step_num: int, grad_scale: float = 1.0) -> int:
+    """``opt.step`` over ``units``, a list of ``(param_spec, params, grads, state)``, up to the first that reports an error.
+    An optimizer that can update many units at once says so with a ``step_units`` method next to its ``step``; it is used
+    unless ``step`` has been replaced (by a subclass or on the object) or has to check each unit first."""
+    owner = next((c for c in type(opt).__mro__ if "step" in vars(c)), None)
+    if (owner is not None and "step_units" in vars(owner) and "step" not in getattr(opt, "__dict__", {})
+            and not getattr(opt, "check_error", False)):
+        return int(opt.step_units(units, step_num, grad_scale) or 0)
+    rc = 0
+    for spec, params, grads, state in units:
+        rc |= opt.step(spec, params, grads, state, step_num, grad_scale)
+        if rc:
+            break
+    return rc
+
+
 def _accept_hp_keyword(cls) -> None:
     """``Cls(hp=record)`` is the reference's spelling of ``Cls(record)``."""
     plain = cls.__init__

@@ -87,6 +87,11 @@ class HybridMuonAdamW:
         rc |= self.adamw.step(param_spec, params, grads, state, step_num, grad_scale, only=set(ad))
         return rc
 
+    def step_units(self, units, step_num: int, grad_scale: float = 1.0) -> int:
+        """Update of several units (layers) at once (see :meth:`Muon.step_units`)."""
+        rc = self.muon.step_units(units, step_num, grad_scale, only=uses_muon)
+        return rc | self.adamw.step_units(units, step_num, grad_scale, only=lambda t: not uses_muon(t))
+
     def flops_per_param(self) -> float:
         return 12.0
 

@@ -56,10 +56,15 @@ class Muon:
         todo = [t for t in param_spec.trainable() if only is None or t.name in only]
         if self.check_error and todo and not _grads_finite([grads[t.grad_name] for t in todo]):
             return 1
-        for t in todo:
-            ops.muon_step(params[t.name], grads[t.grad_name], state[f"o_muon_{_suffix(t.name)}"], lr=self.lr,
-                          beta=self.beta, weight_decay=self.weight_decay, ns_iters=self.ns_iters,
-                          nesterov=self.nesterov, grad_scale=grad_scale)
+        return self.step_units([(param_spec, params, grads, state)], step_num, grad_scale, only=lambda t: t in todo)
+
+    def step_units(self, units, step_num: int, grad_scale: float = 1.0, only=None) -> int:
+        """Update of several units (layers) at once: matrices of one size are orthogonalised together across them."""
+        todo = [(params[t.name], grads[t.grad_name], state[f"o_muon_{_suffix(t.name)}"])
+                for spec, params, grads, state in units for t in spec.trainable() if only is None or only(t)]
+        if todo:
+            ops.muon_multi(*map(list, zip(*todo)), lr=self.lr, beta=self.beta, weight_decay=self.weight_decay,
+                           ns_iters=self.ns_iters, nesterov=self.nesterov, grad_scale=grad_scale)
         return 0
 
     def flops_per_param(self) -> float:

@@ -59,3 +59,28 @@ def test_sum_of_squares_sizes_types_and_alignment(shift):
     assert float(ops.sum_of_squares(ts, torch.device(DEV, 0))) == float("inf")
     ts[3][0] = float("nan")
     assert ops.sum_of_squares(ts, torch.device(DEV, 0)).isnan()
+
+
+@pytest.mark.parametrize("nesterov", [True, False])
+@pytest.mark.parametrize("gdt,mdt", [(BF16, BF16), (F32, F32)])
+def test_muon_batches_match_the_reference(nesterov, gdt, mdt):
+    """Matrices of several sizes (wide, tall with a row count that needs padding, square), 2-D and stacked, more of one size
+    than one launch takes, one off the 16-byte grid and one transposed, in one call: momentum as the fp32 reference's to the
+    rounding of its type, and the step within the 2 % that bf16 iterates of five Newton-Schulz steps keep (the reference
+    iterates in fp32; the polynomial's slope at small singular values is 3.4 per step)."""
+    torch.manual_seed(0)
+    shapes = [(256, 512), (328, 64), (200, 200)] + [(64, 72)] * 70 + [(3, 128, 256)]
+    mk = lambda s, dt, k: (torch.randn(*s, device=DEV) * k).to(dt)
+    P, G, M = ([mk(s, dt, k) for s in shapes] for dt, k in ((BF16, 0.05), (gdt, 0.01), (mdt, 0.01)))
+    P[0] = (torch.randn(256 * 512 + 1, device=DEV) * 0.05).to(BF16)[1:].view(256, 512)
+    P[2] = mk((200, 200), BF16, 0.05).t()
+    start = [p.float().clone() for p in P]
+    want = [(p.float().contiguous(), m.float().clone()) for p, m in zip(P, M)]
+    kw = dict(lr=0.02, beta=0.95, weight_decay=0.01, nesterov=nesterov, grad_scale=0.5)
+    ops.muon_multi(P, G, M, **kw)
+    for p, g, m, p0, (pw, mw) in zip(P, G, M, start, want):
+        ref.muon_step(pw, g.float(), mw, **kw)
+        assert torch.all((m.float() - mw).abs() <= (2.0 ** -8 if mdt == BF16 else 2.0 ** -21) * (mw.abs() + g.float().abs()))
+        step, step_want = p.float() - p0, pw - p0
+        cos = torch.nn.functional.cosine_similarity(step.flatten(), step_want.flatten(), dim=0)
+        assert float(cos) > 0.98, (tuple(p.shape), float(cos))
