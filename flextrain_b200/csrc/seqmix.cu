@@ -124,6 +124,178 @@ __global__ void conv1d_bwd_dx_kernel(const float* __restrict__ dpre, const bf16*
   }
 }
 
+// ---- the same three passes with the taps in registers: a thread walks TT tokens of two neighbouring channels and carries the
+// W - 1 inputs (or gradients) around it, so every element is read once, four bytes a lane, eight tokens ahead of their use.
+// The general kernels above read each input W times, two bytes a lane, and look the sequence of every token up; they stay for
+// other widths, odd channel counts and unaligned rows.  Bound by memory.  16384 tokens x 8192 channels, W = 4: forward 833 us
+// before, 170 us so; dpre 1240 us before, 314 us so; dx 930 us before, 154 us so.
+constexpr int CONV_GROUP = 8;
+__device__ __forceinline__ float2 ld2(const bf16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
+
+template <int W>
+struct ConvWalk {                         // ascending tokens: the sequence of the current token and the W - 1 inputs before it
+  int s, a, end;
+  float2 win[W - 1];
+  __device__ __forceinline__ void enter(const bf16* x, long ldx, const bf16* init, const int* cu, int nseq, int D, int t, int d) {
+    s = seq_of(cu, nseq, t);
+    a = cu[s];
+    end = cu[s + 1];
+#pragma unroll
+    for (int j = 0; j < W - 1; ++j) {
+      const int pos = t - a - (W - 1) + j;
+      win[j] = make_float2(conv_input(x, ldx, init, D, W, s, a, pos, d), conv_input(x, ldx, init, D, W, s, a, pos, d + 1));
+    }
+  }
+  __device__ __forceinline__ void shift(float2 v) {
+#pragma unroll
+    for (int j = 0; j + 1 < W - 1; ++j) win[j] = win[j + 1];
+    win[W - 2] = v;
+  }
+};
+template <int W>
+__device__ __forceinline__ void load_taps(float2 (&wr)[W], const bf16* w, int d) {
+#pragma unroll
+  for (int j = 0; j < W; ++j)
+    wr[j] = make_float2(__bfloat162float(w[(long)d * W + j]), __bfloat162float(w[(long)(d + 1) * W + j]));
+}
+
+template <int W, int TT>
+__global__ void __launch_bounds__(128) conv1d_fwd2_kernel(const bf16* __restrict__ x, long ldx, const bf16* __restrict__ w,
+                                                          const bf16* __restrict__ init, const int* __restrict__ cu,
+                                                          int nseq, bf16* __restrict__ y, int T, int D, int act) {
+  const int d = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (d >= D) return;
+  float2 wr[W];
+  load_taps<W>(wr, w, d);
+  const int tb = blockIdx.y * TT, te = min(T, tb + TT);
+  ConvWalk<W> c;
+  c.enter(x, ldx, init, cu, nseq, D, tb, d);
+  for (int t0 = tb; t0 < te; t0 += CONV_GROUP) {
+    float2 in[CONV_GROUP];
+#pragma unroll
+    for (int i = 0; i < CONV_GROUP; ++i)
+      if (t0 + i < te) in[i] = ld2(x + (long)(t0 + i) * ldx + d);
+#pragma unroll
+    for (int i = 0; i < CONV_GROUP; ++i) {
+      const int t = t0 + i;
+      if (t >= te) break;
+      if (t >= c.end) c.enter(x, ldx, init, cu, nseq, D, t, d);
+      float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < W - 1; ++j) { acc.x += wr[j].x * c.win[j].x; acc.y += wr[j].y * c.win[j].y; }
+      acc.x += wr[W - 1].x * in[i].x;
+      acc.y += wr[W - 1].y * in[i].y;
+      c.shift(in[i]);
+      if (act) { acc.x *= sigmoidf(acc.x); acc.y *= sigmoidf(acc.y); }
+      *reinterpret_cast<__nv_bfloat162*>(y + (long)t * D + d) = __floats2bfloat162_rn(acc.x, acc.y);
+    }
+  }
+}
+
+template <int W, int TT>
+__global__ void __launch_bounds__(128) conv1d_bwd_pre2_kernel(const bf16* __restrict__ x, long ldx, const bf16* __restrict__ w,
+                                                              const bf16* __restrict__ init, const int* __restrict__ cu,
+                                                              int nseq, const bf16* __restrict__ dy,
+                                                              float* __restrict__ dpre, float* __restrict__ dw, int T, int D,
+                                                              int act) {
+  const int d = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (d >= D) return;
+  float2 wr[W], gw[W];
+  load_taps<W>(wr, w, d);
+#pragma unroll
+  for (int j = 0; j < W; ++j) gw[j] = make_float2(0.f, 0.f);
+  const int tb = blockIdx.y * TT, te = min(T, tb + TT);
+  ConvWalk<W> c;
+  c.enter(x, ldx, init, cu, nseq, D, tb, d);
+  for (int t0 = tb; t0 < te; t0 += CONV_GROUP) {
+    float2 in[CONV_GROUP], gy[CONV_GROUP];
+#pragma unroll
+    for (int i = 0; i < CONV_GROUP; ++i)
+      if (t0 + i < te) {
+        in[i] = ld2(x + (long)(t0 + i) * ldx + d);
+        gy[i] = ld2(dy + (long)(t0 + i) * D + d);
+      }
+#pragma unroll
+    for (int i = 0; i < CONV_GROUP; ++i) {
+      const int t = t0 + i;
+      if (t >= te) break;
+      if (t >= c.end) c.enter(x, ldx, init, cu, nseq, D, t, d);
+      float2 g = gy[i];
+      if (act) {
+        float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < W - 1; ++j) { acc.x += wr[j].x * c.win[j].x; acc.y += wr[j].y * c.win[j].y; }
+        acc.x += wr[W - 1].x * in[i].x;
+        acc.y += wr[W - 1].y * in[i].y;
+        const float sx = sigmoidf(acc.x), sy = sigmoidf(acc.y);
+        g.x *= sx * (1.f + acc.x * (1.f - sx));
+        g.y *= sy * (1.f + acc.y * (1.f - sy));
+      }
+      *reinterpret_cast<float2*>(dpre + (long)t * D + d) = g;
+#pragma unroll
+      for (int j = 0; j < W - 1; ++j) { gw[j].x += g.x * c.win[j].x; gw[j].y += g.y * c.win[j].y; }
+      gw[W - 1].x += g.x * in[i].x;
+      gw[W - 1].y += g.y * in[i].y;
+      c.shift(in[i]);
+    }
+  }
+  if (dw != nullptr) {
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+      atomicAdd(dw + (long)d * W + j, gw[j].x);
+      atomicAdd(dw + (long)(d + 1) * W + j, gw[j].y);
+    }
+  }
+}
+
+// Descending tokens: win[k] is dpre of token t + 1 + k, zero past the sequence's end.
+template <int W, int TT>
+__global__ void __launch_bounds__(128) conv1d_bwd_dx2_kernel(const float* __restrict__ dpre, const bf16* __restrict__ w,
+                                                             const bf16* __restrict__ dfin, const int* __restrict__ cu,
+                                                             int nseq, bf16* __restrict__ dx, long lddx, int T, int D) {
+  const int d = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (d >= D) return;
+  float2 wr[W], win[W - 1];
+  load_taps<W>(wr, w, d);
+  const int tb = blockIdx.y * TT, te = min(T, tb + TT);
+  int s = seq_of(cu, nseq, te - 1), a = cu[s], end = cu[s + 1];
+  auto at = [&](int t) { return *reinterpret_cast<const float2*>(dpre + (long)t * D + d); };
+#pragma unroll
+  for (int k = 0; k < W - 1; ++k) win[k] = te + k < end ? at(te + k) : make_float2(0.f, 0.f);
+  for (int t0 = te - 1; t0 >= tb; t0 -= CONV_GROUP) {
+    float2 in[CONV_GROUP];
+#pragma unroll
+    for (int i = 0; i < CONV_GROUP; ++i)
+      if (t0 - i >= tb) in[i] = at(t0 - i);
+#pragma unroll
+    for (int i = 0; i < CONV_GROUP; ++i) {
+      const int t = t0 - i;
+      if (t < tb) break;
+      if (t < a) {                                     // the last token of an earlier sequence
+        s = seq_of(cu, nseq, t);
+        a = cu[s];
+        end = cu[s + 1];
+#pragma unroll
+        for (int k = 0; k < W - 1; ++k) win[k] = make_float2(0.f, 0.f);
+      }
+      float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < W - 1; ++j) { acc.x += wr[j].x * win[W - 2 - j].x; acc.y += wr[j].y * win[W - 2 - j].y; }
+      acc.x += wr[W - 1].x * in[i].x;
+      acc.y += wr[W - 1].y * in[i].y;
+      const int m = t - (end - (W - 1));               // (the virtual input of the carried state)
+      if (dfin != nullptr && m >= 0) {
+        acc.x += __bfloat162float(dfin[((long)s * D + d) * (W - 1) + m]);
+        acc.y += __bfloat162float(dfin[((long)s * D + d + 1) * (W - 1) + m]);
+      }
+      *reinterpret_cast<__nv_bfloat162*>(dx + (long)t * lddx + d) = __floats2bfloat162_rn(acc.x, acc.y);
+#pragma unroll
+      for (int k = W - 2; k > 0; --k) win[k] = win[k - 1];
+      win[0] = in[i];
+    }
+  }
+}
+
 __global__ void conv1d_bwd_dinit_kernel(const float* __restrict__ dpre, const bf16* __restrict__ w,
                                         const bf16* __restrict__ dfin, const int* __restrict__ cu, bf16* __restrict__ dinit,
                                         int D, int W) {
@@ -368,10 +540,19 @@ int ftb_gate_prep_bwd(const void* ba, const float* dt_bias, const float* a_log, 
   return e == cudaSuccess ? 0 : -400 - (int)e;
 }
 
+// Rows whose pairs of channels start on their own size: the kernels that walk two channels a thread apply (four taps).
+static bool conv_pairs(int W, int D, const void* a, long lda, const void* b, long ldb) {
+  return W == 4 && D % 2 == 0 && lda % 2 == 0 && ldb % 2 == 0 && (((uintptr_t)a | (uintptr_t)b) & 7) == 0;
+}
+
 int ftb_conv1d_fwd(const void* x, long ldx, const void* w, const void* init, const int* cu, int nseq, void* y, void* fin,
                    int T, int D, int W, int act, cudaStream_t s) {
   if (W > MAXW || W < 2) return -2;
-  if (T > 0) {
+  if (T > 0 && conv_pairs(W, D, x, ldx, y, D)) {
+    dim3 grid((D / 2 + 127) / 128, (T + 63) / 64);
+    conv1d_fwd2_kernel<4, 64><<<grid, 128, 0, s>>>((const bf16*)x, ldx, (const bf16*)w, (const bf16*)init, cu, nseq,
+                                                   (bf16*)y, T, D, act);
+  } else if (T > 0) {
     dim3 grid((D + 127) / 128, (T + 63) / 64);
     conv1d_fwd_kernel<64><<<grid, 128, 0, s>>>((const bf16*)x, ldx, (const bf16*)w, (const bf16*)init, cu, nseq,
                                                (bf16*)y, T, D, W, act);
@@ -388,7 +569,14 @@ int ftb_conv1d_bwd(const void* x, long ldx, const void* w, const void* init, con
                    const void* dfin, float* dpre, void* dx, long lddx, float* dw, void* dinit, int T, int D, int W,
                    int act, cudaStream_t s) {
   if (W > MAXW || W < 2) return -2;
-  if (T > 0) {
+  if (T > 0 && conv_pairs(W, D, x, ldx, dy, D) && conv_pairs(W, D, dx, lddx, dpre, D)) {
+    dim3 grid((D / 2 + 127) / 128, (T + 127) / 128);
+    conv1d_bwd_pre2_kernel<4, 128><<<grid, 128, 0, s>>>((const bf16*)x, ldx, (const bf16*)w, (const bf16*)init, cu, nseq,
+                                                        (const bf16*)dy, dpre, dw, T, D, act);
+    dim3 grid2((D / 2 + 127) / 128, (T + 63) / 64);
+    conv1d_bwd_dx2_kernel<4, 64><<<grid2, 128, 0, s>>>(dpre, (const bf16*)w, (const bf16*)dfin, cu, nseq, (bf16*)dx, lddx,
+                                                       T, D);
+  } else if (T > 0) {
     dim3 grid((D + 127) / 128, (T + 127) / 128);
     conv1d_bwd_pre_kernel<128><<<grid, 128, 0, s>>>((const bf16*)x, ldx, (const bf16*)w, (const bf16*)init, cu, nseq,
                                                     (const bf16*)dy, dpre, dw, T, D, W, act);

@@ -226,3 +226,31 @@ def test_suffix_sum_per_sequence(H, with_extra):
         room = (n + 1) * 2.0 ** -24 * (part.abs().sum(0) + (extra[i].abs() if with_extra else 0))
         assert torch.all((dg[off:off + n].double() - want).abs() <= room + 1e-12)
         off += n
+
+
+@pytest.mark.parametrize("lens", [[1], [3, 64, 65, 2, 1, 1], [127, 129, 500], [8, 8, 8, 300]])
+@pytest.mark.parametrize("with_init", [False, True])
+def test_conv1d_channel_pairs_equal_the_general_kernels(lens, with_init):
+    """Four taps, even channels: the kernels that carry the taps in registers add in the same order as the general ones, which
+    rows off their alignment still take: forward and input gradients agree bit for bit (sequence ends inside and at the edges
+    of a block of 64 / 128 tokens and of a group of 8), the weights' gradient to fp32 sums in another order."""
+    from flextrain_b200.ops import linattn_cuda as la
+    torch.manual_seed(0)
+    T, D, W, S, bf = sum(lens), 258, 4, len(lens), torch.bfloat16
+    cu = _cu(lens)
+    x, dy = torch.randn(T, D, device=DEV).to(bf), torch.randn(T, D, device=DEV).to(bf)
+    w = torch.randn(D, W, device=DEV).to(bf)
+    init, dfin = (torch.randn(S, D, W - 1, device=DEV).to(bf) for _ in range(2))
+    init, dfin = (init, dfin) if with_init else (None, None)
+    odd = torch.empty(T, D + 1, device=DEV, dtype=bf)[:, 1:]
+    odd.copy_(x)
+    got = []
+    for xs in (x, odd):
+        y, fin = la.conv1d_fwd(xs, w, cu, init)
+        dx, dw = torch.empty(T, D, device=DEV, dtype=bf), torch.zeros(D, W, device=DEV)
+        dinit = la.conv1d_bwd(xs, w, cu, init, dy, dfin, dx, dw, want_dinit=with_init)
+        got.append((y, fin, dx, dw, dinit))
+    (y, fin, dx, dw, di), (y1, fin1, dx1, dw1, di1) = got
+    assert torch.equal(y, y1) and torch.equal(fin, fin1) and torch.equal(dx, dx1)
+    assert di is None or torch.equal(di, di1)
+    assert torch.allclose(dw, dw1, rtol=1e-4, atol=1e-4 * float(dw1.abs().max()))
