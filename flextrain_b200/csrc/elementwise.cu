@@ -232,13 +232,22 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const bf16* __r
   }
 }
 
-__global__ void colsum_accum_kernel(const float* __restrict__ partial, float* __restrict__ out, int P, int D,
-                                    int accumulate) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D) return;
+// out[c] (+)= sum over P partial rows.  A block owns 32 columns and adds 32 rows at a time; one thread per column, walking the
+// rows by itself, left all but D / 256 SMs idle: 592 x 1024 28 us, 5 us so.
+__global__ void __launch_bounds__(1024) colsum_accum_kernel(const float* __restrict__ partial, float* __restrict__ out, int P,
+                                                            int D, int accumulate) {
+  __shared__ float sh[32][33];
+  const int lane = threadIdx.x & 31, r = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int p = 0; p < P; ++p) s += partial[(size_t)p * D + c];
-  out[c] = accumulate ? out[c] + s : s;
+  if (c < D) {
+#pragma unroll 4
+    for (int p = r; p < P; p += 32) s += partial[(size_t)p * D + c];
+  }
+  sh[r][lane] = s;
+  __syncthreads();
+  s = warp_sum(sh[lane][r]);                        // warp r adds column r of the block
+  const int o = blockIdx.x * 32 + r;
+  if (lane == 0 && o < D) out[o] = accumulate ? out[o] + s : s;
 }
 
 // Small-D (per-head) RMSNorm: one warp per row of D <= 512 elements (QK-norm, D = head_dim).
@@ -1084,7 +1093,7 @@ int ftb_rmsnorm_bwd(const void* dy, const void* x, const float* w, const float* 
   else if (nv <= 4 * RN_THREADS) FTB_RN_BWD(4);
   else FTB_RN_BWD(8);
 #undef FTB_RN_BWD
-  if (dw) colsum_accum_kernel<<<(D + 255) / 256, 256, 0, s>>>(dw_partial, dw, blocks, D, dw_accumulate);
+  if (dw) colsum_accum_kernel<<<(D + 31) / 32, 1024, 0, s>>>(dw_partial, dw, blocks, D, dw_accumulate);
   CHECK_LAUNCH();
 }
 
