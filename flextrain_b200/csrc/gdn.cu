@@ -12,7 +12,8 @@
 // owns columns {tj*CPT + cc}.  The state is kept and updated as pairs of rows in packed fp32 arithmetic (fma.rn.f32x2, one
 // instruction for two fused multiply-adds, each rounded as the scalar one), which halves the instructions to issue: 16384
 // tokens in 512 to 4096 long sequences, 32 heads of 128 x 128: pass F 6.4 -> 5.7 ms, pass R 6.7 -> 6.6 ms, forward 3.6 ms
-// either way.  What bounds them then is the chain of a token (its reductions) in the longest sequences.
+// either way.  What bounds them then is the chain of a token (its reductions) in the longest sequences; the tokens of the
+// next block are loaded under the current one (16 bytes a thread), which gave 3.7 -> 3.4, 5.7 -> 5.35 and 6.8 -> 6.15 ms.
 // Reductions over rows (r, o, de) are 4 xor-shuffles inside a half warp; reductions over columns (dq, dk) are
 // accumulated per warp in shared memory over a block of TB tokens and flushed with fp32 atomics once per block.
 //
@@ -53,6 +54,7 @@ struct GdnArgs {
   float* sacc;         // (T, HV) fp32       per-token scalar of the gate gradient: q.dq - k.(dS' e) + k.(S^ dr)
   int HK, HV, DV;
   float scale;
+  int vec;             // every tensor of rows starts on 16 bytes
 };
 
 __device__ __forceinline__ float half_warp_sum(float x) {   // over the 16 lanes that share tj
@@ -149,12 +151,82 @@ __device__ __forceinline__ float segment_sum(float x) {
   return half_warp_sum(x);
 }
 
+// One block of TB tokens on its way from global to shared memory: asked for while the block before is computed, a 16-byte
+// piece of k and of q per thread, and a piece of v (threads from 0), of dO (from 32) or of the fp32 rows de / r (from 64).
+__device__ __forceinline__ uint4 load_piece(const bf16* p, int vec) {
+  if (vec) return *reinterpret_cast<const uint4*>(p);
+  uint4 u;
+  bf16* e = reinterpret_cast<bf16*>(&u);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) e[i] = p[i];
+  return u;
+}
+__device__ __forceinline__ uint4 load_piece(const float* p, int vec) {
+  if (vec) return *reinterpret_cast<const uint4*>(p);
+  return make_uint4(__float_as_uint(p[0]), __float_as_uint(p[1]), __float_as_uint(p[2]), __float_as_uint(p[3]));
+}
+__device__ __forceinline__ void put_bf16(float* dst, const uint4& u, float scale) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+  float f[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 v = __bfloat1622float2(h[i]);
+    f[2 * i] = v.x * scale;
+    f[2 * i + 1] = v.y * scale;
+  }
+  reinterpret_cast<float4*>(dst)[0] = make_float4(f[0], f[1], f[2], f[3]);
+  reinterpret_cast<float4*>(dst)[1] = make_float4(f[4], f[5], f[6], f[7]);
+}
+template <int DK, int NC, bool GRAD>
+struct Incoming {
+  uint4 k, q, x;
+  float g, b;
+  __device__ __forceinline__ void fetch(const GdnArgs& a, const float* rows, int tb, int nt, int hk, int hv, int col0) {
+    const int tid = threadIdx.x;
+    if (tid < DK && tid / (DK / 8) < nt) {
+      const size_t off = ((size_t)(tb + tid / (DK / 8)) * a.HK + hk) * DK + tid % (DK / 8) * 8;
+      k = load_piece(a.k + off, a.vec);
+      q = load_piece(a.q + off, a.vec);
+    }
+    const int e = GRAD && tid >= 64 ? (tid - 64) * 4 : (tid & 31) * 8;      // element of the block's TB x NC columns
+    const int t = e / NC, c = e % NC;
+    if (t < nt) {
+      const size_t off = ((size_t)(tb + t) * a.HV + hv) * a.DV + col0 + c;
+      if (tid < 32) x = load_piece(a.v + off, a.vec);
+      else if (GRAD && tid < 64) x = load_piece(a.d_o + off, a.vec);
+      else if (GRAD) x = load_piece(rows + off, a.vec);
+    }
+    if (tid < nt) {
+      g = a.g[(size_t)(tb + tid) * a.HV + hv];
+      b = a.beta[(size_t)(tb + tid) * a.HV + hv];
+    }
+  }
+  __device__ __forceinline__ void put(float* k_s, float* q_s, float* v_s, float* x_s, float* y_s, float* a_s, float* b_s,
+                                      float scale, int nt) {
+    const int tid = threadIdx.x;
+    if (tid < DK && tid / (DK / 8) < nt) {
+      put_bf16(k_s + tid * 8, k, 1.f);
+      put_bf16(q_s + tid * 8, q, scale);
+    }
+    const int e = GRAD && tid >= 64 ? (tid - 64) * 4 : (tid & 31) * 8;
+    if (e / NC < nt) {
+      if (tid < 32) put_bf16(v_s + e, x, 1.f);
+      else if (GRAD && tid < 64) put_bf16(x_s + e, x, 1.f);
+      else if (GRAD) *reinterpret_cast<uint4*>(y_s + e) = x;
+    }
+    if (tid < nt) {
+      a_s[tid] = __expf(g);
+      b_s[tid] = b;
+    }
+  }
+};
+
 // MODE 0: forward (o, r, final state).  MODE 1: pass F of the backward (dq, dk += S^ dr).
 template <int RPT, int CPT, int MODE>
 __global__ void __launch_bounds__(NT) gdn_forward_kernel(const GdnArgs a) {
   constexpr int DK = 16 * RPT, NC = 8 * CPT, NP = RPT == 1 ? 1 : RPT / 2;
   __shared__ __align__(16) float k_s[TB][DK], q_s[TB][DK];
-  __shared__ float v_s[TB][NC], x_s[TB][NC], y_s[TB][NC];
+  __shared__ __align__(16) float v_s[TB][NC], x_s[MODE == 1 ? TB : 1][NC], y_s[MODE == 1 ? TB : 1][NC];
   __shared__ float a_s[TB], b_s[TB];
   __shared__ __align__(16) float acc_q[MODE == 1 ? 4 : 1][TB][MODE == 1 ? DK : 1];
   __shared__ __align__(16) float acc_k[MODE == 1 ? 4 : 1][TB][MODE == 1 ? DK : 1];
@@ -169,29 +241,24 @@ __global__ void __launch_bounds__(NT) gdn_forward_kernel(const GdnArgs a) {
     for (int cc = 0; cc < CPT; ++cc)
       S[j][cc] = a.state_in ? load_state<RPT>(a.state_in + ((size_t)seq * a.HV + hv) * DK * a.DV + col0 + tj * CPT + cc,
                                               a.DV, ti, j) : 0ull;
+  Incoming<DK, NC, MODE == 1> in;
+  if (t0 < t1) in.fetch(a, a.de, t0, min(TB, t1 - t0), hk, hv, col0);
   for (int tb = t0; tb < t1; tb += TB) {
     const int nt = min(TB, t1 - tb);
     __syncthreads();
-    for (int idx = tid; idx < nt * DK; idx += NT) {
-      const int t = idx / DK, i = idx - t * DK;
-      const size_t off = ((size_t)(tb + t) * a.HK + hk) * DK + i;
-      k_s[t][i] = __bfloat162float(a.k[off]);
-      q_s[t][i] = __bfloat162float(a.q[off]) * a.scale;
-    }
-    for (int idx = tid; idx < nt * NC; idx += NT) {
-      const int t = idx / NC, j = idx - t * NC;
-      const size_t off = ((size_t)(tb + t) * a.HV + hv) * a.DV + col0 + j;
-      v_s[t][j] = __bfloat162float(a.v[off]);
-      if (MODE == 1) {
-        x_s[t][j] = __bfloat162float(a.d_o[off]);
-        y_s[t][j] = a.de[off];
-      }
-    }
-    if (tid < nt) {
-      a_s[tid] = __expf(a.g[(size_t)(tb + tid) * a.HV + hv]);
-      b_s[tid] = a.beta[(size_t)(tb + tid) * a.HV + hv];
-    }
+    in.put(&k_s[0][0], &q_s[0][0], &v_s[0][0], &x_s[0][0], &y_s[0][0], a_s, b_s, a.scale, nt);
     __syncthreads();
+    if (tb + TB < t1) in.fetch(a, a.de, tb + TB, min(TB, t1 - tb - TB), hk, hv, col0);
+    // Forward, four columns a thread: the output of a token is reduced over the rows together with the prediction of the next
+    // one (two independent chains of shuffles in place of one after the other).
+    [[maybe_unused]] float last[4] = {0.f, 0.f, 0.f, 0.f}, last_r = 0.f;
+    [[maybe_unused]] auto store_out = [&](int t, float o, float r) {
+      if ((ti & 3) == 0) {                         // lanes 0, 4, 8, 12 of the half warp hold columns 0..3
+        const size_t off = ((size_t)(tb + t) * a.HV + hv) * a.DV + col0 + tj * CPT + (ti >> 2);
+        a.o[off] = __float2bfloat16(o);
+        if (a.r) a.r[off] = r;
+      }
+    };
     for (int t = 0; t < nt; ++t) {
       const float at = a_s[t], bt = b_s[t];
       const f32x2 at2 = pack2(at, at);
@@ -209,7 +276,13 @@ __global__ void __launch_bounds__(NT) gdn_forward_kernel(const GdnArgs a) {
           pp[cc] = sum2(p);
         }
         if constexpr (CPT == 4) {
-          all_gather4(reduce_scatter4(pp[0], pp[1], pp[2], pp[3], tid & 31), tid & 31, rj);
+          const float mine = reduce_scatter4(pp[0], pp[1], pp[2], pp[3], tid & 31);
+          if constexpr (MODE == 0) {
+            const float o = reduce_scatter4(last[0], last[1], last[2], last[3], tid & 31);
+            if (t > 0) store_out(t - 1, o, last_r);
+            last_r = mine;
+          }
+          all_gather4(mine, tid & 31, rj);
         } else {
 #pragma unroll
           for (int cc = 0; cc < CPT; ++cc) rj[cc] = half_warp_sum(pp[cc]);
@@ -245,13 +318,8 @@ __global__ void __launch_bounds__(NT) gdn_forward_kernel(const GdnArgs a) {
           pp[cc] = sum2(p);
         }
         if constexpr (CPT == 4) {
-          const float tot = reduce_scatter4(pp[0], pp[1], pp[2], pp[3], tid & 31);
-          if ((ti & 3) == 0) {                     // lanes 0, 4, 8, 12 of the half warp hold columns 0..3
-            const int cc = ti >> 2;
-            const size_t off = ((size_t)(tb + t) * a.HV + hv) * a.DV + col0 + tj * CPT + cc;
-            a.o[off] = __float2bfloat16(tot);
-            if (a.r) a.r[off] = rj[cc];
-          }
+#pragma unroll
+          for (int cc = 0; cc < 4; ++cc) last[cc] = pp[cc];
         } else {
 #pragma unroll
           for (int cc = 0; cc < CPT; ++cc) {
@@ -278,6 +346,8 @@ __global__ void __launch_bounds__(NT) gdn_forward_kernel(const GdnArgs a) {
         }
       }
     }
+    if constexpr (MODE == 0 && CPT == 4)
+      store_out(nt - 1, reduce_scatter4(last[0], last[1], last[2], last[3], tid & 31), last_r);
     if (MODE == 1) {
       __syncthreads();
       if (tid < TB) a_s[tid] = 0.f;           // reused as the per-token scalar accumulator of this block
@@ -314,7 +384,7 @@ template <int RPT, int CPT>
 __global__ void __launch_bounds__(NT) gdn_reverse_kernel(const GdnArgs a) {
   constexpr int DK = 16 * RPT, NC = 8 * CPT, NP = RPT == 1 ? 1 : RPT / 2;
   __shared__ __align__(16) float k_s[TB][DK], q_s[TB][DK];
-  __shared__ float v_s[TB][NC], x_s[TB][NC], r_s[TB][NC];
+  __shared__ __align__(16) float v_s[TB][NC], x_s[TB][NC], r_s[TB][NC];
   __shared__ float a_s[TB], b_s[TB];
   __shared__ __align__(16) float acc_k[4][TB][DK];
   __shared__ float acc_b[4][TB];
@@ -330,28 +400,15 @@ __global__ void __launch_bounds__(NT) gdn_reverse_kernel(const GdnArgs a) {
       dS[j][cc] = a.state_in ? load_state<RPT>(a.state_in + ((size_t)seq * a.HV + hv) * DK * a.DV + col0 + tj * CPT + cc,
                                                a.DV, ti, j) : 0ull;
   const int nblk = (t1 - t0 + TB - 1) / TB;
+  Incoming<DK, NC, true> in;
+  if (nblk > 0) in.fetch(a, a.r, t0 + (nblk - 1) * TB, t1 - t0 - (nblk - 1) * TB, hk, hv, col0);
   for (int blk = nblk - 1; blk >= 0; --blk) {
     const int tb = t0 + blk * TB;
     const int nt = min(TB, t1 - tb);
     __syncthreads();
-    for (int idx = tid; idx < nt * DK; idx += NT) {
-      const int t = idx / DK, i = idx - t * DK;
-      const size_t off = ((size_t)(tb + t) * a.HK + hk) * DK + i;
-      k_s[t][i] = __bfloat162float(a.k[off]);
-      q_s[t][i] = __bfloat162float(a.q[off]) * a.scale;
-    }
-    for (int idx = tid; idx < nt * NC; idx += NT) {
-      const int t = idx / NC, j = idx - t * NC;
-      const size_t off = ((size_t)(tb + t) * a.HV + hv) * a.DV + col0 + j;
-      v_s[t][j] = __bfloat162float(a.v[off]);
-      x_s[t][j] = __bfloat162float(a.d_o[off]);
-      r_s[t][j] = a.r[off];
-    }
-    if (tid < nt) {
-      a_s[tid] = __expf(a.g[(size_t)(tb + tid) * a.HV + hv]);
-      b_s[tid] = a.beta[(size_t)(tb + tid) * a.HV + hv];
-    }
+    in.put(&k_s[0][0], &q_s[0][0], &v_s[0][0], &x_s[0][0], &r_s[0][0], a_s, b_s, a.scale, nt);
     __syncthreads();
+    if (blk > 0) in.fetch(a, a.r, tb - TB, TB, hk, hv, col0);
     for (int t = nt - 1; t >= 0; --t) {
       const float at = a_s[t], bt = b_s[t];
       f32x2 kr[NP], qr[NP];
@@ -531,6 +588,7 @@ int ftb_gdn(int pass, const void* q, const void* k, const void* v, const float* 
   a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.g = g; a.beta = beta; a.cu = cu;
   a.state_in = state_in; a.state_out = state_out; a.o = (bf16*)o; a.r = r; a.d_o = (const bf16*)d_o; a.de = de;
   a.dv = (bf16*)dv; a.dbeta = dbeta; a.dq = dq; a.dk = dk; a.sacc = sacc; a.HK = HK; a.HV = HV; a.DV = DV; a.scale = scale;
+  a.vec = (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)d_o | (uintptr_t)de | (uintptr_t)r) & 15) == 0;
   switch (DK) {
     case 16: return launch_cols<1>(pass, a, nseq, s);
     case 32: return launch_cols<2>(pass, a, nseq, s);
