@@ -139,12 +139,12 @@ class GQAAttentionBlock:
     def _qk_norm_fwd(self, q, k, params):
         c = self.cfg
         if c.qk_norm == "head":
-            qn, qr = ops.rmsnorm_fwd(q.contiguous(), params["w_q_norm"], c.norm_eps)
-            kn, kr = ops.rmsnorm_fwd(k.contiguous(), params["w_k_norm"], c.norm_eps)
+            qn, qr = ops.rmsnorm_fwd(q, params["w_q_norm"], c.norm_eps)
+            kn, kr = ops.rmsnorm_fwd(k, params["w_k_norm"], c.norm_eps)
         else:
             T = q.shape[0]
-            qn, qr = ops.rmsnorm_fwd(q.reshape(T, -1).contiguous(), params["w_q_norm"], c.norm_eps)
-            kn, kr = ops.rmsnorm_fwd(k.reshape(T, -1).contiguous(), params["w_k_norm"], c.norm_eps)
+            qn, qr = ops.rmsnorm_fwd(q.reshape(T, -1), params["w_q_norm"], c.norm_eps)
+            kn, kr = ops.rmsnorm_fwd(k.reshape(T, -1), params["w_k_norm"], c.norm_eps)
             qn, kn = qn.view(T, c.n_heads, c.head_dim), kn.view(T, c.n_kv_heads, c.head_dim)
         return qn, qr, kn, kr
 
@@ -161,7 +161,7 @@ class GQAAttentionBlock:
         xk = ops.rope(k, pos, inv, out=slot.out("xk", h.device), mrope_sections=sec)
         xv = slot.out("xv", h.device)
         if c.v_norm:
-            vn, vr = ops.rmsnorm_fwd(v.contiguous(), self._unit_gain(h.device), c.norm_eps)
+            vn, vr = ops.rmsnorm_fwd(v, self._unit_gain(h.device), c.norm_eps)
             slot.put("v_rstd", vr)
             xv.copy_(vn)
         else:
@@ -269,8 +269,7 @@ class GQAAttentionBlock:
         dv_dst = dqkv[:, qrows + c.kv_dim:].unflatten(1, (c.n_kv_heads, c.head_dim))
         pre = self._project_qkv(h_fn(), params) if (c.qk_norm or c.v_norm) else None   # pre-norm recompute (one GEMM)
         if c.v_norm:
-            dvp, _ = ops.rmsnorm_bwd(dv.contiguous(), pre[3].contiguous(), self._unit_gain(dxo.device), t["v_rstd"])
-            dv_dst.copy_(dvp.view(T, c.n_kv_heads, c.head_dim))
+            ops.rmsnorm_bwd(dv.contiguous(), pre[3], self._unit_gain(dxo.device), t["v_rstd"], dx_out=dv_dst)
         else:
             dv_dst.copy_(dv)
         if not c.qk_norm:
@@ -283,18 +282,16 @@ class GQAAttentionBlock:
             dqn = ops.rope(dq.contiguous(), pos, inv, inverse=True, mrope_sections=sec)
             dkn = ops.rope(dk.contiguous(), pos, inv, inverse=True, mrope_sections=sec)
             q_pre, _, k_pre, _ = pre
-            if c.qk_norm == "head":
-                dqp, _ = ops.rmsnorm_bwd(dqn, q_pre.contiguous(), params["w_q_norm"], t["q_rstd"],
-                                         dw_out=grads.get("g_q_norm"))
-                dkp, _ = ops.rmsnorm_bwd(dkn, k_pre.contiguous(), params["w_k_norm"], t["k_rstd"],
-                                         dw_out=grads.get("g_k_norm"))
-            else:
-                dqp, _ = ops.rmsnorm_bwd(dqn.view(T, -1), q_pre.reshape(T, -1).contiguous(), params["w_q_norm"],
-                                         t["q_rstd"], dw_out=grads.get("g_q_norm"))
-                dkp, _ = ops.rmsnorm_bwd(dkn.view(T, -1), k_pre.reshape(T, -1).contiguous(), params["w_k_norm"],
-                                         t["k_rstd"], dw_out=grads.get("g_k_norm"))
-            dq_dst.copy_(dqp.view(T, c.n_heads, c.head_dim))
-            dk_dst.copy_(dkp.view(T, c.n_kv_heads, c.head_dim))
+            for dn, x_pre, dst, n in ((dqn, q_pre, dq_dst, "q"), (dkn, k_pre, dk_dst, "k")):
+                if c.qk_norm == "row":              # (a gated projection's heads lie apart, and become rows by a copy)
+                    dn, x_pre = dn.view(T, -1), x_pre.reshape(T, -1)
+                    dst = dst.flatten(1) if not (c.gated and n == "q") else dst
+                if dst.dim() == dn.dim():
+                    ops.rmsnorm_bwd(dn, x_pre, params[f"w_{n}_norm"], t[f"{n}_rstd"], dw_out=grads.get(f"g_{n}_norm"),
+                                    dx_out=dst)
+                else:
+                    dst.copy_(ops.rmsnorm_bwd(dn, x_pre, params[f"w_{n}_norm"], t[f"{n}_rstd"],
+                                              dw_out=grads.get(f"g_{n}_norm"))[0].view(dst.shape))
         dh = self.qkv.dgrad(dqkv, params)
         return dh, dqkv
 

@@ -169,18 +169,52 @@ def bias_grad(dy, gb, *, alpha=1.0, accumulate=True):
 
 
 # --------------------------------------------------------------------------- norms / rope / glu
+def _dense(t):
+    """``t`` contiguous and on 16 bytes, as the vector kernels read it.  (A single row of a wider tensor counts as contiguous
+    wherever it starts.)"""
+    if t is None:
+        return None
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def _gain_ok(w, n: int) -> bool:
+    return w is None or (w.dtype == torch.float32 and w.shape == (n,) and w.is_contiguous() and w.data_ptr() % 16 == 0)
+
+
 def rmsnorm_fwd(x, w, eps):
+    """``(y contiguous, rstd)``.  Views of a wider projection, ``(T, H, hd)`` heads or ``(T, D)`` rows, are read in place."""
     if _cuda_bf16(x) and (w is None or w.dtype == torch.float32):
         _count()
-        return _kernels().rmsnorm_fwd(x.contiguous(), w, eps)
+        k = _kernels()
+        if _gain_ok(w, x.shape[-1]):
+            if k.heads_strided(x):
+                return k.rmsnorm_heads_fwd(x, w, eps)
+            if not x.is_contiguous() and k.rows_strided(x):
+                return k.rmsnorm_rows_fwd(x, w, eps)
+        return k.rmsnorm_fwd(_dense(x), _dense(w), eps)
     return ref.rmsnorm_fwd(x, w, eps)
 
 
-def rmsnorm_bwd(dy, x, w, rstd, *, dx_add=None, emit_y=False, dw_out=None):
-    """Returns ``(dx, y)``; ``dw`` is accumulated into ``dw_out`` (fp32 or grad dtype)."""
+def rmsnorm_bwd(dy, x, w, rstd, *, dx_add=None, emit_y=False, dw_out=None, dx_out=None):
+    """Returns ``(dx, y)``; ``dw`` is accumulated into ``dw_out`` (fp32 or grad dtype).  ``dx_out``, a view of ``dx``'s shape
+    (heads or rows of a wider tensor), is where ``dx`` is written when given."""
+    if dx_out is not None:
+        if (_cuda_bf16(dy, x, dx_out) and _gain_ok(w, x.shape[-1]) and dx_add is None and not emit_y and rstd.is_contiguous()
+                and rstd.dtype == torch.float32
+                and (dw_out is None or (w is not None and dw_out.dtype == torch.float32 and dw_out.is_contiguous()))):
+            k = _kernels()
+            if k.heads_strided(x) and k.heads_strided(dy) and k.heads_strided(dx_out):
+                _count()
+                return k.rmsnorm_heads_bwd(dy, x, w, rstd, dx_out, dw_out), None
+            if k.rows_strided(x) and k.rows_strided(dx_out) and dy.is_contiguous() and k.rows_strided(dy):
+                _count(2)
+                return k.rmsnorm_rows_bwd(dy, x, w, rstd, dx_out, dw_out), None
+        dx, y = rmsnorm_bwd(dy, x, w, rstd, dx_add=dx_add, emit_y=emit_y, dw_out=dw_out)
+        return dx_out.copy_(dx.view(dx_out.shape)), y
     if _cuda_bf16(dy, x) and (w is None or w.dtype == torch.float32) and (dw_out is None or dw_out.dtype == torch.float32):
         _count(2)
-        dx, _, y = _kernels().rmsnorm_bwd(dy.contiguous(), x.contiguous(), w, rstd.contiguous(), dx_add=dx_add,
+        dx, _, y = _kernels().rmsnorm_bwd(_dense(dy), _dense(x), _dense(w), rstd.contiguous(), dx_add=_dense(dx_add),
                                           emit_y=emit_y, dw_out=dw_out)
         return dx, y
     dx, dw = ref.rmsnorm_bwd(dy, x, w, rstd)

@@ -244,6 +244,61 @@ def grouped_wgrad(dy, x, offsets, gw, *, alpha=1.0, accumulate=True):
 
 
 # ------------------------------------------------------------------------ elementwise
+def heads_strided(t: torch.Tensor) -> bool:
+    """``(T, H, hd)`` with heads side by side, any token stride that keeps 16-byte pieces aligned, and a head dim the per-head
+    kernels know."""
+    return (t.dim() == 3 and t.shape[2] in (64, 128, 256) and t.stride(2) == 1 and t.stride(1) == t.shape[2]
+            and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 and t.shape[0] * t.shape[1] < 1 << 31)
+
+
+def rows_strided(t: torch.Tensor) -> bool:
+    """``(T, D)`` rows a multiple of 8 elements apart, on 16 bytes."""
+    return (t.dim() == 2 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.stride(0) >= t.shape[1] and t.shape[1] % 8 == 0
+            and 512 < t.shape[1] <= 16384 and t.data_ptr() % 16 == 0)
+
+
+def rmsnorm_heads_fwd(x, w, eps):
+    lib = load("elementwise")
+    T, H, hd = x.shape
+    y = torch.empty(T, H, hd, dtype=x.dtype, device=x.device)
+    rstd = torch.empty(T, H, dtype=torch.float32, device=x.device)
+    _check(lib.ftb_rmsnorm_heads_fwd(_ptr(x), c_long(x.stride(0)), _ptr(w), _ptr(y), _ptr(rstd), c_int(T), c_int(H), c_int(hd),
+                                     c_float(eps), _stream()), "ftb_rmsnorm_heads_fwd")
+    return y, rstd
+
+
+def rmsnorm_heads_bwd(dy, x, w, rstd, dx, dw_out):
+    """``dx`` (strided as ``x`` may be) is written; the gain's gradient is added to ``dw_out``."""
+    lib = load("elementwise")
+    T, H, hd = x.shape
+    _check(lib.ftb_rmsnorm_heads_bwd(_ptr(dy), c_long(dy.stride(0)), _ptr(x), c_long(x.stride(0)), _ptr(w), _ptr(rstd), _ptr(dx),
+                                     c_long(dx.stride(0)), _ptr(dw_out), c_int(T), c_int(H), c_int(hd), _stream()),
+           "ftb_rmsnorm_heads_bwd")
+    return dx
+
+
+def rmsnorm_rows_fwd(x, w, eps):
+    lib = load("elementwise")
+    T, D = x.shape
+    y = torch.empty(T, D, dtype=x.dtype, device=x.device)
+    rstd = torch.empty(T, dtype=torch.float32, device=x.device)
+    _check(lib.ftb_rmsnorm_fwd_ld(_ptr(x), c_long(x.stride(0)), _ptr(w), _ptr(y), _ptr(rstd), c_int(T), c_int(D), c_float(eps),
+                                  _stream()), "ftb_rmsnorm_fwd_ld")
+    return y, rstd
+
+
+def rmsnorm_rows_bwd(dy, x, w, rstd, dx, dw_out):
+    lib = load("elementwise")
+    T, D = x.shape
+    lib.ftb_rmsnorm_bwd_blocks.restype = c_int
+    part = torch.empty(max(lib.ftb_rmsnorm_bwd_blocks(c_int(T)), 1) * D if dw_out is not None else 0, dtype=torch.float32,
+                       device=x.device)
+    _check(lib.ftb_rmsnorm_bwd_ld(_ptr(dy), _ptr(x), c_long(x.stride(0)), _ptr(w), _ptr(rstd), None, _ptr(dx),
+                                  c_long(dx.stride(0)), None, _ptr(part), _ptr(dw_out), c_int(1), c_int(T), c_int(D),
+                                  _stream()), "ftb_rmsnorm_bwd_ld")
+    return dx
+
+
 def rmsnorm_fwd(x, w, eps):
     lib = load("elementwise")
     D = x.shape[-1]
