@@ -810,13 +810,13 @@ class ActiveModel:
     # ============================================================================= helpers
     def _zero_all_grads(self) -> None:
         bm = self.buffers
-        bm.embed_g.zero_()
-        bm.head_g.zero_()
+        ops.zero_(bm.embed_g)
+        ops.zero_(bm.head_g)
         if getattr(self.embed, "train_encoders", False):
             self.embed.zero_encoder_grads()
         if bm.grads_resident:
             for b in bm.gpu_g:
-                b.zero_()
+                ops.zero_(b)
         self._grads_fresh = {}
 
     def _write_back_losses(self, pending) -> None:

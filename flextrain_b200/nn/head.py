@@ -36,6 +36,9 @@ class LMHead:
         W = params["w_head_proj"]
         per_tok = torch.empty(T, dtype=torch.float32, device=x.device)
         gW = grads.get("g_head_proj")
+        # held-out data with the stock loss: nothing reads the logits' gradient
+        loss_only = (not want_dx and gW is None and type(loss_fn).__call__ is CrossEntropyLoss.__call__
+                     and type(loss_fn).loss_only is CrossEntropyLoss.loss_only)
         for a in range(0, T, self.head_chunk_size):
             b = min(T, a + self.head_chunk_size)
             xa = x[a:b]
@@ -44,7 +47,8 @@ class LMHead:
             sl = TokenSlice(meta.targets[a:b], meta.loss_mask[a:b] if meta.loss_mask is not None else None,
                             meta.extra.get("advantages")[a:b] if meta.extra.get("advantages") is not None else None,
                             meta.extra.get("ref_logprobs")[a:b] if meta.extra.get("ref_logprobs") is not None else None)
-            per_tok[a:b] = apply_loss(loss_fn, logits, sl, loss_scale, self.final_softcap)
+            per_tok[a:b] = (loss_fn.loss_only(logits, sl, self.final_softcap) if loss_only else
+                            apply_loss(loss_fn, logits, sl, loss_scale, self.final_softcap))
             if gW is not None:
                 ops.gemm(logits, hn, trans_a=True, beta=1.0, out=gW)
             if want_dx:

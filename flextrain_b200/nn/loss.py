@@ -112,6 +112,11 @@ class CrossEntropyLoss(_NativeLoss):
         return ops.softmax_ce_(logits, sl.targets, grad_scale=grad_scale, softcap=softcap, loss_mask=sl.loss_mask,
                                ignore_index=self.ignore_index)
 
+    def loss_only(self, logits, sl: TokenSlice, softcap: float = 0.0) -> torch.Tensor:
+        """The losses without the gradient: the logits are read once and not written."""
+        return ops.softmax_ce_loss(logits, sl.targets, softcap=softcap, loss_mask=sl.loss_mask,
+                                   ignore_index=self.ignore_index)
+
 
 class MSELoss(_NativeLoss):
     """Mean-squared error between logits and one-hot targets (regression / debugging head)."""

@@ -390,6 +390,25 @@ def softmax_ce_(logits, targets, *, grad_scale=1.0, softcap=0.0, loss_mask=None,
     return loss
 
 
+def softmax_ce_loss(logits, targets, *, softcap=0.0, loss_mask=None, ignore_index=-100):
+    """Per-token loss only (held-out data): ``logits`` stays as it is."""
+    if _cuda_bf16(logits) and logits.stride(1) == 1:
+        _count()
+        return _kernels().softmax_ce_loss(logits, targets.to(torch.int64), softcap=softcap, loss_mask=loss_mask,
+                                          ignore_index=ignore_index)
+    return ref.softmax_ce_fwd_bwd(logits, targets, grad_scale=1.0, softcap=softcap, loss_mask=loss_mask,
+                                  ignore_index=ignore_index)[0]
+
+
+def zero_(t):
+    """Zeros in place; contiguous CUDA memory as one fill of its bytes.  (The library's fill of an arena, which is bytes to it,
+    stored four bytes a thread: 5 GB of gradients 1.52 ms, 0.83 ms so.)"""
+    if t.is_cuda and t.is_contiguous():
+        _kernels().zero_(t)
+        return t
+    return t.zero_()
+
+
 def embedding_fwd(tokens, table, scale=1.0):
     if _cuda_bf16(table) and table.shape[1] % 8 == 0:
         _count()

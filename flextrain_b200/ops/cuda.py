@@ -494,6 +494,22 @@ def softmax_ce_(logits, targets, *, grad_scale=1.0, softcap=0.0, loss_mask=None,
     return loss
 
 
+def softmax_ce_loss(logits, targets, *, softcap=0.0, loss_mask=None, ignore_index=-100):
+    """Per-token loss (fp32); ``logits`` is only read."""
+    lib = load("elementwise")
+    T, V = logits.shape
+    assert logits.dtype == torch.bfloat16 and logits.stride(1) == 1 and targets.dtype == torch.int64
+    loss = torch.empty(T, dtype=torch.float32, device=logits.device)
+    _check(lib.ftb_softmax_ce_loss(_ptr(logits), _ptr(targets), _ptr(loss_mask), _ptr(loss), c_int(T), c_int(V),
+                                   c_long(logits.stride(0)), c_float(softcap), c_long(ignore_index), _stream()),
+           "ftb_softmax_ce_loss")
+    return loss
+
+
+def zero_(t):
+    _check(load("elementwise").ftb_zero(_ptr(t), c_long(t.numel() * t.element_size()), _stream()), "ftb_zero")
+
+
 def embedding_fwd(tokens, table, scale=1.0):
     lib = load("elementwise")
     T, D = tokens.numel(), table.shape[1]

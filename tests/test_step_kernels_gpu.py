@@ -84,3 +84,25 @@ def test_muon_batches_match_the_reference(nesterov, gdt, mdt):
         step, step_want = p.float() - p0, pw - p0
         cos = torch.nn.functional.cosine_similarity(step.flatten(), step_want.flatten(), dim=0)
         assert float(cos) > 0.98, (tuple(p.shape), float(cos))
+
+
+@pytest.mark.parametrize("V", [8, 1000, 16384, 16392, 32771, 50257])
+@pytest.mark.parametrize("softcap", [0.0, 30.0])
+def test_cross_entropy_batches_and_loss_only(V, softcap):
+    """Vocabularies around what a block reads at once (4 x 512 x 8 = 16384), not a multiple of 8, with ignored and masked
+    rows: loss and gradient as the fp32 reference's, and the loss-only form equal to it bit for bit, logits untouched."""
+    torch.manual_seed(0)
+    T, ld = 37, (V + 15) // 8 * 8
+    z = (torch.randn(T, ld, device=DEV) * 3).to(BF16)[:, :V]
+    tgt = torch.randint(0, V, (T,), device=DEV)
+    tgt[3] = -100
+    mask = torch.ones(T, device=DEV)
+    mask[5] = 0
+    kw = dict(softcap=softcap, loss_mask=mask)
+    before = z.clone()
+    alone = ops.softmax_ce_loss(z, tgt, **kw)
+    assert torch.equal(z, before)
+    lw, dw = ref.softmax_ce_fwd_bwd(z, tgt, grad_scale=0.25, ignore_index=-100, **kw)
+    loss = ops.softmax_ce_(z, tgt, grad_scale=0.25, **kw)
+    assert torch.equal(loss, alone) and torch.allclose(loss, lw, rtol=1e-5, atol=1e-4)      # lse of |z| < 20 in fp32
+    assert torch.all((z.float() - dw.float()).abs() <= 2.0 ** -7 * dw.float().abs() + 1e-6)
