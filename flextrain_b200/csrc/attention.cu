@@ -1255,13 +1255,13 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
               const float s = __uint_as_float(sv[q2][g * 8 + e]);
               const float th = tanh_fast(s * soc);
               const float pe = s == -INFINITY ? 0.f : ex2_approx(cap2 * th - ls[e]);
-              // d(cap * tanh(scale * s / cap)) / ds = scale * (1 - tanh^2); the scale follows on dQ and dK
-              ds[e] = pe * __uint_as_float(vd[g * 8 + e]) * (1.f - th * th);
+              // d(cap * tanh(scale * s / cap)) / ds = scale * (1 - tanh^2)
+              ds[e] = pe * __uint_as_float(vd[g * 8 + e]) * p.scale * (1.f - th * th);
             }
           } else {
 #pragma unroll
             for (int e = 0; e < 8; ++e)
-              ds[e] = __uint_as_float(sv[q2][g * 8 + e]) * __uint_as_float(vd[g * 8 + e]);
+              ds[e] = __uint_as_float(sv[q2][g * 8 + e]) * __uint_as_float(vd[g * 8 + e]) * p.scale;
           }
           uint4 b;
           __nv_bfloat162* b2 = reinterpret_cast<__nv_bfloat162*>(&b);
@@ -1300,8 +1300,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             x2[e] = __floats2bfloat162_rn(__uint_as_float(a[g * 8 + 2 * e]), __uint_as_float(a[g * 8 + 2 * e + 1]));
-            y2[e] = __floats2bfloat162_rn(__uint_as_float(b[g * 8 + 2 * e]) * p.scale,
-                                          __uint_as_float(b[g * 8 + 2 * e + 1]) * p.scale);
+            y2[e] = __floats2bfloat162_rn(__uint_as_float(b[g * 8 + 2 * e]), __uint_as_float(b[g * 8 + 2 * e + 1]));
           }
         }
         const uint32_t o = sw128_offset(r, cb + g * 8, 128);
@@ -1338,16 +1337,13 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         *reinterpret_cast<uint4*>(rowp + ((j ^ (lane & 7)) << 4)) =
-            make_uint4(__float_as_uint(__uint_as_float(v[4 * j]) * p.scale),
-                       __float_as_uint(__uint_as_float(v[4 * j + 1]) * p.scale),
-                       __float_as_uint(__uint_as_float(v[4 * j + 2]) * p.scale),
-                       __float_as_uint(__uint_as_float(v[4 * j + 3]) * p.scale));
+            make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
     };
     auto add_row = [&](float* dst, const uint32_t (&v)[32]) {
 #pragma unroll
       for (int e = 0; e < 32; e += 4)
-        red_add_v4_f32(dst + e, __uint_as_float(v[e]) * p.scale, __uint_as_float(v[e + 1]) * p.scale,
-                       __uint_as_float(v[e + 2]) * p.scale, __uint_as_float(v[e + 3]) * p.scale);
+        red_add_v4_f32(dst + e, __uint_as_float(v[e]), __uint_as_float(v[e + 1]), __uint_as_float(v[e + 2]),
+                       __uint_as_float(v[e + 3]));
     };
     // In a fixed order, a tile's turn passes on when its additions have been performed.  LAST_FIRST, whose next key tile
     // comes a step later by itself, looks at that only before the staging block is needed again: waiting at once held this
