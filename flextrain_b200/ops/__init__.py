@@ -465,7 +465,7 @@ def muon_step(p, g, mom, *, lr, beta=0.95, weight_decay=0.0, ns_iters=5, nestero
                grad_scale=grad_scale)
 
 
-MUON_BATCH_ELEMENTS = 64 << 20      # of one batch's iterate: its workspace is four to five buffers of at most this size
+MUON_BATCH_ELEMENTS = 32 << 20      # of one batch's iterate: its workspace is four buffers of at most this size, in bf16
 
 
 def muon_multi(ps, gs, moms, *, lr, beta=0.95, weight_decay=0.0, ns_iters=5, nesterov=True, grad_scale=1.0):
