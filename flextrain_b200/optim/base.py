@@ -52,13 +52,21 @@ def _grads_finite(grads: List[torch.Tensor]) -> bool:
     return float(bad) == 0.0
 
 
+def _batched(opt) -> bool:
+    """Whether ``opt.step_units`` may take the place of ``opt.step`` on each unit: the two are defined side by side, ``step``
+    has not been replaced (by a subclass or on the object), no unit has to be checked before it is updated, and the same holds
+    for the optimizers that this one delegates to (``inner_optimizers``), whose ``step`` it would pass by as well."""
+    owner = next((c for c in type(opt).__mro__ if "step" in vars(c)), None)
+    return (owner is not None and "step_units" in vars(owner) and "step" not in getattr(opt, "__dict__", {})
+            and not getattr(opt, "check_error", False)
+            and all(_batched(o) for o in getattr(opt, "inner_optimizers", tuple)()))
+
+
 def step_units(opt, units, step_num: int, grad_scale: float = 1.0) -> int:
     """``opt.step`` over ``units``, a list of ``(param_spec, params, grads, state)``, up to the first that reports an error.
     An optimizer that can update many units at once says so with a ``step_units`` method next to its ``step``; it is used
-    unless ``step`` has been replaced (by a subclass or on the object) or has to check each unit first."""
-    owner = next((c for c in type(opt).__mro__ if "step" in vars(c)), None)
-    if (owner is not None and "step_units" in vars(owner) and "step" not in getattr(opt, "__dict__", {})
-            and not getattr(opt, "check_error", False)):
+    where it does the same (:func:`_batched`)."""
+    if _batched(opt):
         return int(opt.step_units(units, step_num, grad_scale) or 0)
     rc = 0
     for spec, params, grads, state in units:

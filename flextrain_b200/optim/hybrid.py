@@ -89,8 +89,13 @@ class HybridMuonAdamW:
 
     def step_units(self, units, step_num: int, grad_scale: float = 1.0) -> int:
         """Update of several units (layers) at once (see :meth:`Muon.step_units`)."""
-        rc = self.muon.step_units(units, step_num, grad_scale, only=uses_muon)
-        return rc | self.adamw.step_units(units, step_num, grad_scale, only=lambda t: not uses_muon(t))
+        mu = {id(t) for spec, *_ in units for names in (self._split(spec)[0],) for t in spec.trainable() if t.name in names}
+        rc = self.muon.step_units(units, step_num, grad_scale, only=lambda t: id(t) in mu)
+        return rc | self.adamw.step_units(units, step_num, grad_scale, only=lambda t: id(t) not in mu)
+
+    def inner_optimizers(self):
+        """The optimizers whose ``step`` this one's ``step`` calls."""
+        return self.muon, self.adamw
 
     def flops_per_param(self) -> float:
         return 12.0
