@@ -1498,7 +1498,10 @@ int ftb_attn_bwd(const void* dout, const void* q, const void* k, const void* v, 
                  int max_tiles, int max_k, cudaStream_t stream) {
   if (total_q <= 0 || num_seqs <= 0) return 0;
   if ((hd != 64 && hd != 128) || H % KV) return -2;
-  if ((q_stride & 7) || (k_stride & 7) || (v_stride & 7) || (do_stride & 7) || (o_stride & 7)) return -2;
+  // (dout and out are read in 16-byte pieces before any tensor map is made; the maps check the others)
+  if ((q_stride & 7) || (k_stride & 7) || (v_stride & 7) || (do_stride & 7) || (o_stride & 7) ||
+      ((reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(out)) & 15))
+    return -2;
   {
     const long threads = (long)total_q * H * (hd / 8);
     (hd == 128 ? fa_delta_kernel<128> : fa_delta_kernel<64>)<<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(

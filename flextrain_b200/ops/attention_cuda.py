@@ -12,15 +12,19 @@ def _strided_ok(t: torch.Tensor) -> bool:
     return t.stride(2) == 1 and t.stride(1) == t.shape[2] and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
 
 
+def _rows(t: torch.Tensor) -> torch.Tensor:
+    """``t`` with rows that the kernels can read (16-byte loads and tensor maps): itself, or a copy.  (A tensor may count as
+    contiguous and start off the 16-byte grid, or have any stride over a dimension of one.)"""
+    if _strided_ok(t):
+        return t
+    c = t.contiguous()
+    return c if _strided_ok(c) else c.clone(memory_format=torch.contiguous_format)
+
+
 def fwd(q, k, v, cu_q, cu_k, max_q, max_k, *, scale, causal=True, window=0, softcap=0.0):
     """``q (Tq,H,hd)``, ``k,v (Tk,KV,hd)`` bf16 (token-strided views allowed). Returns ``(out, lse (H,Tq) fp32)``."""
     lib = load("attention")
-    if not _strided_ok(q):
-        q = q.contiguous()
-    if not _strided_ok(k):
-        k = k.contiguous()
-    if not _strided_ok(v):
-        v = v.contiguous()
+    q, k, v = _rows(q), _rows(k), _rows(v)
     Tq, H, hd = q.shape
     Tk, KV = k.shape[0], k.shape[1]
     nseq = cu_q.numel() - 1
@@ -50,11 +54,7 @@ def bwd(dout, q, k, v, out, lse, cu_q, cu_k, max_q, max_k, *, scale, causal=True
     lib = load("attention")
     if not hasattr(lib, "ftb_attn_bwd"):
         raise NotImplementedError
-    q = q if _strided_ok(q) else q.contiguous()
-    k = k if _strided_ok(k) else k.contiguous()
-    v = v if _strided_ok(v) else v.contiguous()
-    dout = dout if _strided_ok(dout) else dout.contiguous()
-    out = out if _strided_ok(out) else out.contiguous()
+    q, k, v, dout, out = _rows(q), _rows(k), _rows(v), _rows(dout), _rows(out)
     Tq, H, hd = q.shape
     Tk, KV = k.shape[0], k.shape[1]
     nseq = cu_q.numel() - 1

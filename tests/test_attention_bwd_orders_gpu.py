@@ -55,3 +55,24 @@ def test_attention_bwd(hd, name):
         for g in (first, free):
             assert torch.isfinite(g).all()
             assert float((g.float() - w.float()).norm()) <= 2.0 ** -6 * float(w.float().norm()) + 1e-6
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("shift", [2, 4])
+@pytest.mark.parametrize("which", ["dout", "q", "k", "v", "out"])
+def test_operands_off_the_16_byte_grid(which, shift, hd):
+    """A contiguous operand that starts ``shift`` elements past a 16-byte boundary gives the aligned one's bits."""
+    from flextrain_b200 import ops
+    torch.manual_seed(0)
+    cu = torch.tensor([0, 150, 200], dtype=torch.int32, device=DEV)
+    t = {n: torch.randn(200, h, hd, device=DEV).to(torch.bfloat16) for n, h in (("q", 4), ("k", 2), ("v", 2), ("dout", 4))}
+    kw = dict(scale=hd ** -0.5)
+    t["out"], lse = ops.attention_fwd(t["q"], t["k"], t["v"], cu, cu, 150, 150, **kw)
+    run = lambda: ops.attention_bwd(t["dout"], t["q"], t["k"], t["v"], t["out"], lse, cu, cu, 150, 150, **kw)
+    want = run()
+    off = torch.empty(t[which].numel() + shift, dtype=torch.bfloat16, device=DEV)[shift:].view(t[which].shape)
+    t[which] = off.copy_(t[which])
+    assert off.is_contiguous() and off.data_ptr() % 16 == 2 * shift
+    for g, w in zip(run(), want):
+        assert torch.equal(g, w)
+    assert torch.equal(ops.attention_fwd(t["q"], t["k"], t["v"], cu, cu, 150, 150, **kw)[0], t["out"])
