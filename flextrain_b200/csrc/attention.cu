@@ -971,13 +971,13 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   }
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kvh = blockIdx.x;
+  const int kvh = blockIdx.x % p.KV;
   const int rep = p.H / p.KV;
   int seq = 0, k0 = 0;
-  // Blocks are handed out in increasing blockIdx: all heads of a key tile, then the next key tile; see BWD_*.
-  if (!find_tile(p.cu_k, p.num_seqs,
-                 static_cast<int>(p.order == BWD_LAST_FIRST ? gridDim.y - 1 - blockIdx.y : blockIdx.y), TK, seq, k0))
-    return;
+  // Blocks are handed out in increasing blockIdx: all heads of a key tile, then the next key tile; see BWD_*.  (One grid
+  // dimension for both: the second one ends at 65535, fewer than the key tiles of a batch of very many sequences.)
+  const int tile = static_cast<int>(p.order == BWD_LAST_FIRST ? gridDim.x - 1 - blockIdx.x : blockIdx.x) / p.KV;
+  if (!find_tile(p.cu_k, p.num_seqs, tile, TK, seq, k0)) return;
   const int qs = p.cu_q[seq], len_q = p.cu_q[seq + 1] - qs;
   const int ks = p.cu_k[seq], len_k = p.cu_k[seq + 1] - ks;
   const int off = len_k - len_q;
@@ -1474,8 +1474,8 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tdo, const CUten
     if (e != cudaSuccess) return -300 - static_cast<int>(e);
     configured = true;
   }
-  dim3 grid(p.KV, tiles);
-  kern<<<grid, FAB_THREADS, SMEM, s>>>(tq, tdo, tk, tv, tdq, p);
+  if (static_cast<long>(p.KV) * tiles > 0x7fffffffL) return -2;
+  kern<<<static_cast<unsigned>(p.KV * tiles), FAB_THREADS, SMEM, s>>>(tq, tdo, tk, tv, tdq, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -400 - static_cast<int>(e);
 }

@@ -76,3 +76,22 @@ def test_operands_off_the_16_byte_grid(which, shift, hd):
     for g, w in zip(run(), want):
         assert torch.equal(g, w)
     assert torch.equal(ops.attention_fwd(t["q"], t["k"], t["v"], cu, cu, 150, 150, **kw)[0], t["out"])
+
+
+@pytest.mark.parametrize("deterministic", [False, True])
+def test_more_key_tiles_than_the_second_grid_dimension_holds(deterministic):
+    """66000 sequences of one token: every query sees its own key alone, so out = v, dv = dout, and dq and dk are what is left
+    of dP - delta: two fp32 sums of the same 64 products of at most 25 in size, one of them as three bf16 terms, which differ by
+    2^-20 of the sum of the sizes at most; times a key or query (at most 5) and the scale."""
+    from flextrain_b200.ops import attention_cuda as fa
+    from flextrain_b200.ops import cuda as kk
+    torch.manual_seed(0)
+    n, hd = 66000, 64
+    q, k, v, do = (torch.randn(n, 1, hd, device=DEV).to(torch.bfloat16) for _ in range(4))
+    cu = torch.arange(n + 1, dtype=torch.int32, device=DEV)
+    out, lse = fa.fwd(q, k, v, cu, cu, 1, 1, scale=hd ** -0.5)
+    dq, dk, dv = fa.bwd(do, q, k, v, out, lse, cu, cu, 1, 1, scale=hd ** -0.5, deterministic=deterministic)
+    assert kk.device_error_words().get("attention", 0) == 0
+    assert torch.equal(out, v) and torch.equal(dv, do)
+    room = 2.0 ** -20 * 64 * 25 * 5 * hd ** -0.5
+    assert float(dq.float().abs().max()) <= room and float(dk.float().abs().max()) <= room
