@@ -1178,6 +1178,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     const float cap2 = p.softcap * 1.4426950408889634f;
     const float soc = CAP ? p.scale / p.softcap : 0.f;
     const int win = min(p.window, 1 << 29);
+    constexpr float HIDDEN = -3.402823466e38f;      // (with soft-cap) finite: its product with a scale of 0 is a number
     bool ok = true;
     int h = kvh * rep, qt = qt_first;
     for (int it = 0; it < n_iter && ok; ++it) {
@@ -1199,11 +1200,13 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         const int first = p.causal ? kj - off - qt : 0;
         const int lo = (kj < len_k ? first : 1 << 30) - half * 64;
         const int hi = min(len_q - qt, (p.causal && win > 0) ? first + win : 128) - half * 64;
+        // infinitely far on the side where the exponential is 0 (soft-cap: a value that is looked for)
+        const uint32_t hidden = __float_as_uint(CAP ? HIDDEN : copysignf(INFINITY, -c));
 #pragma unroll
         for (int q2 = 0; q2 < 2; ++q2)
 #pragma unroll
           for (int e = 0; e < 32; ++e)
-            if (q2 * 32 + e < lo || q2 * 32 + e >= hi) sv[q2][e] = 0xff800000u;        // -inf: exponential 0
+            if (q2 * 32 + e < lo || q2 * 32 + e >= hi) sv[q2][e] = hidden;
       }
 #pragma unroll
       for (int q2 = 0; q2 < 2; ++q2) {
@@ -1217,7 +1220,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const float s = __uint_as_float(sv[q2][g * 4 + e]);
-              pe[e] = s == -INFINITY ? 0.f : ex2_approx(cap2 * tanh_fast(s * soc) - ls[e]);
+              pe[e] = s == HIDDEN ? 0.f : ex2_approx(cap2 * tanh_fast(s * soc) - ls[e]);
             }
           } else {
 #pragma unroll
@@ -1254,7 +1257,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             for (int e = 0; e < 8; ++e) {
               const float s = __uint_as_float(sv[q2][g * 8 + e]);
               const float th = tanh_fast(s * soc);
-              const float pe = s == -INFINITY ? 0.f : ex2_approx(cap2 * th - ls[e]);
+              const float pe = s == HIDDEN ? 0.f : ex2_approx(cap2 * th - ls[e]);
               // d(cap * tanh(scale * s / cap)) / ds = scale * (1 - tanh^2)
               ds[e] = pe * __uint_as_float(vd[g * 8 + e]) * p.scale * (1.f - th * th);
             }
@@ -1534,7 +1537,10 @@ int ftb_attn_bwd(const void* dout, const void* q, const void* k, const void* v, 
   p.dq_acc = dq_acc; p.dq_sem = dq_sem; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv; p.lse = lse; p.delta = delta;
   p.order = dq_sem == nullptr ? BWD_FIRST_FIRST : max_k > (hd == 128 ? 4096 : 1024) ? BWD_IN_STEP : BWD_LAST_FIRST;
   p.total_q = total_q; p.scale = scale; p.softcap = softcap; p.causal = causal; p.window = window;
-  if (softcap > 0.f)
+  // The plain form divides lse by the scale.  A scale of 0 (or so small that the quotient leaves fp32) takes the soft-cap form,
+  // which subtracts lse after scaling: a cap of 1 leaves scores that are all next to 0 as they are.
+  if (!(softcap > 0.f) && fabsf(scale) < 1e-20f) p.softcap = 1.f;
+  if (p.softcap > 0.f)
     rc = (hd == 128) ? launch_bwd<128, true>(tq, tdo, tk, tv, tdq, p, max_tiles, stream)
                      : launch_bwd<64, true>(tq, tdo, tk, tv, tdq, p, max_tiles, stream);
   else

@@ -95,3 +95,19 @@ def test_more_key_tiles_than_the_second_grid_dimension_holds(deterministic):
     assert torch.equal(out, v) and torch.equal(dv, do)
     room = 2.0 ** -20 * 64 * 25 * 5 * hd ** -0.5
     assert float(dq.float().abs().max()) <= room and float(dk.float().abs().max()) <= room
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("scale", [0.0, 1e-30, -0.1])
+def test_unusual_scales(scale, hd):
+    """Uniform attention (a scale of 0) and scores that fall as the product grows, against the fp32 reference and its lse, with
+    the bound of the other cases."""
+    from flextrain_b200.ops import attention_cuda as fa
+    torch.manual_seed(2)
+    cu = torch.tensor([0, 150, 450], dtype=torch.int32, device=DEV)
+    q, do, k, v = (torch.randn(450, h, hd, device=DEV).to(torch.bfloat16) for h in (4, 4, 2, 2))
+    o, lse = ref.attention_fwd(q, k, v, cu, cu, scale=scale)
+    want = ref.attention_bwd(do, q, k, v, o, lse, cu, cu, scale=scale)
+    for g, w in zip(fa.bwd(do, q, k, v, o.to(torch.bfloat16), lse.contiguous(), cu, cu, 300, 300, scale=scale), want):
+        assert torch.isfinite(g).all()
+        assert float((g.float() - w.float()).norm()) <= 2.0 ** -6 * float(w.float().norm()) + 1e-6
