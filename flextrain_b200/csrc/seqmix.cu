@@ -33,7 +33,7 @@ __device__ __forceinline__ int seq_of(const int* __restrict__ cu, int nseq, int 
 __device__ __forceinline__ float conv_input(const bf16* __restrict__ x, long ldx, const bf16* __restrict__ init, int D,
                                             int W, int seq, int a, int pos, int d) {
   if (pos >= 0) return __bfloat162float(x[(long)(a + pos) * ldx + d]);
-  if (init == nullptr) return 0.f;
+  if (init == nullptr || pos < -(W - 1)) return 0.f;      // (a token before the first sequence reaches further back)
   return __bfloat162float(init[((long)seq * D + d) * (W - 1) + (W - 1) + pos]);
 }
 
@@ -127,7 +127,8 @@ __global__ void conv1d_bwd_dx_kernel(const float* __restrict__ dpre, const bf16*
 // ---- the same three passes with the taps in registers: a thread walks TT tokens of two neighbouring channels and carries the
 // W - 1 inputs (or gradients) around it, so every element is read once, four bytes a lane, eight tokens ahead of their use.
 // The general kernels above read each input W times, two bytes a lane, and look the sequence of every token up; they stay for
-// other widths, odd channel counts and unaligned rows.  Bound by memory.  16384 tokens x 8192 channels, W = 4: forward 833 us
+// other widths, odd channel counts and unaligned rows.  Tokens before the first sequence or after the last (padding) belong to
+// the nearest one, as in the general kernels, but are no part of its inputs or of its end.  Bound by memory.  16384 tokens x 8192 channels, W = 4: forward 833 us
 // before, 170 us so; dpre 1240 us before, 314 us so; dx 930 us before, 154 us so.
 constexpr int CONV_GROUP = 8;
 __device__ __forceinline__ float2 ld2(const bf16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
@@ -179,7 +180,8 @@ __global__ void __launch_bounds__(128) conv1d_fwd2_kernel(const bf16* __restrict
     for (int i = 0; i < CONV_GROUP; ++i) {
       const int t = t0 + i;
       if (t >= te) break;
-      if (t >= c.end) c.enter(x, ldx, init, cu, nseq, D, t, d);
+      if (t >= c.end || t == c.a) c.enter(x, ldx, init, cu, nseq, D, t, d);
+      if (t < c.a) in[i] = make_float2(0.f, 0.f);
       float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
       for (int j = 0; j < W - 1; ++j) { acc.x += wr[j].x * c.win[j].x; acc.y += wr[j].y * c.win[j].y; }
@@ -219,7 +221,8 @@ __global__ void __launch_bounds__(128) conv1d_bwd_pre2_kernel(const bf16* __rest
     for (int i = 0; i < CONV_GROUP; ++i) {
       const int t = t0 + i;
       if (t >= te) break;
-      if (t >= c.end) c.enter(x, ldx, init, cu, nseq, D, t, d);
+      if (t >= c.end || t == c.a) c.enter(x, ldx, init, cu, nseq, D, t, d);
+      if (t < c.a) in[i] = make_float2(0.f, 0.f);
       float2 g = gy[i];
       if (act) {
         float2 acc = make_float2(0.f, 0.f);
@@ -261,7 +264,7 @@ __global__ void __launch_bounds__(128) conv1d_bwd_dx2_kernel(const float* __rest
   int s = seq_of(cu, nseq, te - 1), a = cu[s], end = cu[s + 1];
   auto at = [&](int t) { return *reinterpret_cast<const float2*>(dpre + (long)t * D + d); };
 #pragma unroll
-  for (int k = 0; k < W - 1; ++k) win[k] = te + k < end ? at(te + k) : make_float2(0.f, 0.f);
+  for (int k = 0; k < W - 1; ++k) win[k] = te + k >= a && te + k < end ? at(te + k) : make_float2(0.f, 0.f);
   for (int t0 = te - 1; t0 >= tb; t0 -= CONV_GROUP) {
     float2 in[CONV_GROUP];
 #pragma unroll
@@ -271,20 +274,21 @@ __global__ void __launch_bounds__(128) conv1d_bwd_dx2_kernel(const float* __rest
     for (int i = 0; i < CONV_GROUP; ++i) {
       const int t = t0 - i;
       if (t < tb) break;
-      if (t < a) {                                     // the last token of an earlier sequence
+      if (t < a && s > 0) {                            // the last token of an earlier sequence
         s = seq_of(cu, nseq, t);
         a = cu[s];
         end = cu[s + 1];
 #pragma unroll
         for (int k = 0; k < W - 1; ++k) win[k] = make_float2(0.f, 0.f);
       }
+      if (t < a || t >= end) in[i] = make_float2(0.f, 0.f);
       float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
       for (int j = 0; j < W - 1; ++j) { acc.x += wr[j].x * win[W - 2 - j].x; acc.y += wr[j].y * win[W - 2 - j].y; }
       acc.x += wr[W - 1].x * in[i].x;
       acc.y += wr[W - 1].y * in[i].y;
       const int m = t - (end - (W - 1));               // (the virtual input of the carried state)
-      if (dfin != nullptr && m >= 0) {
+      if (dfin != nullptr && m >= 0 && m < W - 1) {
         acc.x += __bfloat162float(dfin[((long)s * D + d) * (W - 1) + m]);
         acc.y += __bfloat162float(dfin[((long)s * D + d + 1) * (W - 1) + m]);
       }

@@ -230,14 +230,16 @@ def test_suffix_sum_per_sequence(H, with_extra):
 
 @pytest.mark.parametrize("lens", [[1], [3, 64, 65, 2, 1, 1], [127, 129, 500], [8, 8, 8, 300]])
 @pytest.mark.parametrize("with_init", [False, True])
-def test_conv1d_channel_pairs_equal_the_general_kernels(lens, with_init):
+@pytest.mark.parametrize("before,after", [(0, 0), (0, 1), (0, 75), (5, 0), (130, 9)])
+def test_conv1d_channel_pairs_equal_the_general_kernels(lens, with_init, before, after):
     """Four taps, even channels: the kernels that carry the taps in registers add in the same order as the general ones, which
     rows off their alignment still take: forward and input gradients agree bit for bit (sequence ends inside and at the edges
-    of a block of 64 / 128 tokens and of a group of 8), the weights' gradient to fp32 sums in another order."""
+    of a block of 64 / 128 tokens and of a group of 8), the weights' gradient to fp32 sums in another order.  Also with tokens
+    before the first sequence and after the last, whose values must not reach the sequences."""
     from flextrain_b200.ops import linattn_cuda as la
     torch.manual_seed(0)
-    T, D, W, S, bf = sum(lens), 258, 4, len(lens), torch.bfloat16
-    cu = _cu(lens)
+    T, D, W, S, bf = before + sum(lens) + after, 258, 4, len(lens), torch.bfloat16
+    cu = _cu(lens) + before
     x, dy = torch.randn(T, D, device=DEV).to(bf), torch.randn(T, D, device=DEV).to(bf)
     w = torch.randn(D, W, device=DEV).to(bf)
     init, dfin = (torch.randn(S, D, W - 1, device=DEV).to(bf) for _ in range(2))
@@ -254,3 +256,10 @@ def test_conv1d_channel_pairs_equal_the_general_kernels(lens, with_init):
     assert torch.equal(y, y1) and torch.equal(fin, fin1) and torch.equal(dx, dx1)
     assert di is None or torch.equal(di, di1)
     assert torch.allclose(dw, dw1, rtol=1e-4, atol=1e-4 * float(dw1.abs().max()))
+    if before or after:                            # the sequences by themselves
+        own = slice(before, before + sum(lens))
+        y2, fin2 = la.conv1d_fwd(x[own], w, cu - before, init)
+        dx2 = torch.empty_like(x[own])
+        di2 = la.conv1d_bwd(x[own], w, cu - before, init, dy[own], dfin, dx2, None, want_dinit=with_init)
+        assert torch.equal(y[own], y2) and torch.equal(fin, fin2) and torch.equal(dx[own], dx2)
+        assert di is None or torch.equal(di, di2)
