@@ -34,6 +34,13 @@ typedef __nv_bfloat16 bf16;
 constexpr int TB = 8;            // tokens staged per block
 constexpr int NT = 128;          // threads per CTA
 
+// error word, read by the host after a step (3: bounds check)
+static __device__ int g_error_word = 0;
+static __device__ int g_error_where = 0;
+__device__ __forceinline__ void set_error(int code, int where) {
+  if (atomicCAS(&g_error_word, 0, code) == 0) g_error_where = where;
+}
+
 struct GdnArgs {
   const bf16* q;       // (T, HK, DK)
   const bf16* k;       // (T, HK, DK)
@@ -499,10 +506,11 @@ __global__ void __launch_bounds__(NT) gdn_reverse_kernel(const GdnArgs a) {
 // dg[t, h] = sum_{u >= t, same sequence} s[u, h] + extra[seq, h].  A block owns 32 heads of one sequence; its 32 warps take
 // 32 runs of tokens: totals of the runs, their suffix sums in shared memory, then the running sums within each run.  (A
 // cumulative sum over all tokens along the slow axis, as the tensor library does it, kept one thread per head busy: 3.5 ms for
-// 16384 x 32, below 0.02 ms so.)
+// 16384 x 32, below 0.02 ms so.)  T >= 0: the sequences have to cover the T tokens; if they do not, the error word says so.
 __global__ void __launch_bounds__(1024) suffix_sum_kernel(const float* __restrict__ s, const float* __restrict__ extra,
-                                                          const int* __restrict__ cu, float* __restrict__ dg, int H) {
+                                                          const int* __restrict__ cu, int T, float* __restrict__ dg, int H) {
   __shared__ float tot[32][33];
+  if (T >= 0 && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && (cu[0] != 0 || cu[gridDim.y] != T)) set_error(3, 300);
   const int lane = threadIdx.x & 31, run = threadIdx.x >> 5;
   const int h = blockIdx.x * 32 + lane, seq = blockIdx.y;
   const int t0 = cu[seq], n = cu[seq + 1] - t0;
@@ -569,13 +577,29 @@ int ftb_gdn_col_blocks(int nseq, int HV, int DV) {
   return cpt ? DV / (8 * cpt) : 0;
 }
 
-// dg (T, H) from the per-token scalars s (T, H); extra (nseq, H) or NULL is added to every token of its sequence.
-int ftb_suffix_sum(const float* s, const float* extra, const int* cu, int nseq, float* dg, int H, cudaStream_t st) {
-  if (nseq <= 0 || H <= 0) return 0;
+// dg (T, H) from the per-token scalars s (T, H); extra (nseq, H) or NULL is added to every token of its sequence.  T: tokens
+// that the sequences have to cover, or -1.
+int ftb_gate_sum(const float* s, const float* extra, const int* cu, int nseq, int T, float* dg, int H, cudaStream_t st) {
+  if (nseq <= 0 || H <= 0) return T > 0 ? -2 : 0;
   if (nseq > 65535) return -2;
-  suffix_sum_kernel<<<dim3((H + 31) / 32, nseq), 1024, 0, st>>>(s, extra, cu, dg, H);
+  suffix_sum_kernel<<<dim3((H + 31) / 32, nseq), 1024, 0, st>>>(s, extra, cu, T, dg, H);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -400 - (int)e;
+}
+int ftb_suffix_sum(const float* s, const float* extra, const int* cu, int nseq, float* dg, int H, cudaStream_t st) {
+  return ftb_gate_sum(s, extra, cu, nseq, -1, dg, H, st);
+}
+
+int ftb_gdn_error(void) {
+  int h[2] = {0, 0};
+  cudaMemcpyFromSymbol(&h[0], g_error_word, sizeof(int));
+  cudaMemcpyFromSymbol(&h[1], g_error_where, sizeof(int));
+  if (h[0] != 0) {
+    int z = 0;
+    cudaMemcpyToSymbol(g_error_word, &z, sizeof(int));
+    cudaMemcpyToSymbol(g_error_where, &z, sizeof(int));
+  }
+  return h[0] * 1000 + h[1];
 }
 
 int ftb_gdn(int pass, const void* q, const void* k, const void* v, const float* g, const float* beta, const int* cu,

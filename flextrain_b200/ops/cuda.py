@@ -100,7 +100,7 @@ def device_error_words() -> dict:
     """Read (and clear) the error word of each loaded kernel library: ``{lib: code*1000 + where}``."""
     out = {}
     for name, fn in (("gemm_tcgen05", "ftb_gemm_error"), ("attention", "ftb_attn_error"), ("comm", "ftb_comm_error"),
-                     ("moe", "ftb_moe_error")):
+                     ("moe", "ftb_moe_error"), ("gdn", "ftb_gdn_error")):
         lib = _libs.get(name)
         if lib is not None and hasattr(lib, fn):
             f = getattr(lib, fn)

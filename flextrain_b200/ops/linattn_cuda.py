@@ -160,7 +160,8 @@ def gdn_fwd(q, k, v, g, beta, cu, state_in=None, scale=None, want_r=False):
 
 def gdn_bwd(q, k, v, g, beta, cu, state_in, final_state, r, d_o, dstate_final=None, scale=None):
     """Backward of :func:`gdn_fwd`.  Returns ``(dq (T,HK,dk) fp32, dk (T,HK,dk) fp32, dv (T,HV,dv) bf16,
-    dg (T,HV) fp32, dbeta (T,HV) fp32, dstate_in (S,HV,dk,dv) fp32)``."""
+    dg (T,HV) fp32, dbeta (T,HV) fp32, dstate_in (S,HV,dk,dv) fp32)``.  The sequences of ``cu`` have to cover all T tokens:
+    the library's error word (``device_error_words``) reports it when they do not."""
     T, HK, DK = q.shape
     HV, DV = v.shape[1], v.shape[2]
     S = cu.numel() - 1
@@ -182,9 +183,9 @@ def gdn_bwd(q, k, v, g, beta, cu, state_in, final_state, r, d_o, dstate_final=No
     # dg_t = sum_{u >= t, same sequence} s_u  (+ <dS_final, S_final>), with the per-token scalar
     # s_u = q_u.dq_u - k_u.(dS'_u e_u) + k_u.(S^_u dr_u) accumulated by the two passes
     extra = (dsf * final_state.to(F32)).sum((-1, -2)).contiguous() if dstate_final is not None else None     # (S, HV)
-    dg = torch.empty(T, HV, dtype=F32, device=dev)
-    _check(load("gdn").ftb_suffix_sum(_ptr(s), _ptr(extra), _ptr(cu), c_int(S), _ptr(dg), c_int(HV), _stream()),
-           "ftb_suffix_sum")
+    dg = torch.zeros(T, HV, dtype=F32, device=dev)
+    _check(load("gdn").ftb_gate_sum(_ptr(s), _ptr(extra), _ptr(cu), c_int(S), c_int(T), _ptr(dg), c_int(HV), _stream()),
+           "ftb_gate_sum")
     if rep > 1:
         dq = dq_hv.view(T, HK, rep, DK).sum(2)
         dk = dk_hv.view(T, HK, rep, DK).sum(2)

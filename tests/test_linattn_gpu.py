@@ -263,3 +263,24 @@ def test_conv1d_channel_pairs_equal_the_general_kernels(lens, with_init, before,
         di2 = la.conv1d_bwd(x[own], w, cu - before, init, dy[own], dfin, dx2, None, want_dinit=with_init)
         assert torch.equal(y[own], y2) and torch.equal(fin, fin2) and torch.equal(dx[own], dx2)
         assert di is None or torch.equal(di, di2)
+
+
+@pytest.mark.parametrize("ends,covered", [([0, 64, 70], True), ([0, 64], False), ([2, 64, 70], False)])
+def test_gdn_backward_reports_sequences_that_leave_tokens_out(ends, covered):
+    """The gate's gradient was put together from the sequences' lengths, which had to add up to the tokens; the kernel that took
+    its place says through the error word when they do not.  Tokens of no sequence get a gradient of 0."""
+    from flextrain_b200.ops import linattn_cuda as la
+    from flextrain_b200.ops.cuda import device_error_words
+    torch.manual_seed(0)
+    T, H, D = 70, 2, 16
+    cu = torch.tensor(ends, dtype=torch.int32, device=DEV)
+    q, k, v, do = (torch.randn(T, H, D, device=DEV).to(BF) for _ in range(4))
+    k = F.normalize(k.float(), dim=-1).to(BF)
+    g, beta = -torch.rand(T, H, device=DEV), torch.rand(T, H, device=DEV)
+    o, fin, r = la.gdn_fwd(q, k, v, g, beta, cu, want_r=True)
+    device_error_words()
+    dg = la.gdn_bwd(q, k, v, g, beta, cu, None, fin, r, do)[3]
+    assert device_error_words()["gdn"] == (0 if covered else 3300)
+    assert device_error_words()["gdn"] == 0
+    assert torch.isfinite(dg).all()
+    assert float(dg[:ends[0]].abs().sum() + dg[ends[-1]:].abs().sum()) == 0.0
