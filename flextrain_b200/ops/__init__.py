@@ -494,8 +494,7 @@ def muon_multi(ps, gs, moms, *, lr, beta=0.95, weight_decay=0.0, ns_iters=5, nes
     for (shape, *_), mats in batches.items():
         per = max(1, MUON_BATCH_ELEMENTS // (shape[0] * shape[1]))
         for i in range(0, len(mats), per):
-            _count(3 + 3 * ns_iters)
-            _kernels().muon_batch(*[list(t) for t in zip(*mats[i:i + per])], coeffs=ref.NS_COEFFS, **kw)
+            _count(_kernels().muon_batch(*[list(t) for t in zip(*mats[i:i + per])], coeffs=ref.NS_COEFFS, **kw))
     for t, c in back:
         t.copy_(c)
 

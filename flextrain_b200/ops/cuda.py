@@ -153,6 +153,18 @@ def _two_sm_splits(M: int, N: int, K: int) -> int:
     return best
 
 
+def _k_splits(M: int, N: int, K: int, bn: int = 0) -> int:
+    """Slices of K that :func:`gemm` cuts a product into."""
+    # small output, long reduction (rank-r LoRA gradients: M or N = r, K = tokens): a handful of tiles would each walk
+    # the whole K on a handful of SMs; split K so that tiles x slices fill the GPU (fp32 slabs + ordered reduce)
+    tiles = ((M + 127) // 128) * ((N + (127 if N <= 128 else 255)) // (128 if N <= 128 else 256))
+    if bn == 0 and tiles <= 40 and K >= 4096 and (N <= 128 or M < 512):
+        return max(2, min(148 // tiles, K // 512, 64))
+    if bn == 0 and M >= 512 and N >= 512 and GEMM_MAX_CTAS == 0:
+        return _two_sm_splits(M, N, K)
+    return 1
+
+
 def gemm(a, b, *, trans_a=False, trans_b=False, alpha=1.0, beta=0.0, c=None, bias=None, out=None, out_dtype=None,
          bn: int = 0):
     """``out = alpha * op(a) @ op(b) + beta * c + bias`` on the tcgen05 kernel.
@@ -175,14 +187,7 @@ def gemm(a, b, *, trans_a=False, trans_b=False, alpha=1.0, beta=0.0, c=None, bia
         assert c.dtype == out.dtype and c.stride(1) == 1
     if bias is not None:
         assert bias.dtype == torch.float32
-    # small output, long reduction (rank-r LoRA gradients: M or N = r, K = tokens): a handful of tiles would each walk
-    # the whole K on a handful of SMs; split K so that tiles x slices fill the GPU (fp32 slabs + ordered reduce)
-    tiles = ((M + 127) // 128) * ((N + (127 if N <= 128 else 255)) // (128 if N <= 128 else 256))
-    splits = 1
-    if bn == 0 and tiles <= 40 and K >= 4096 and (N <= 128 or M < 512):
-        splits = max(2, min(148 // tiles, K // 512, 64))
-    elif bn == 0 and M >= 512 and N >= 512 and GEMM_MAX_CTAS == 0:
-        splits = _two_sm_splits(M, N, K)
+    splits = _k_splits(M, N, K, bn)
     if splits > 1:
         ws = torch.empty(splits * M * N, dtype=torch.float32, device=a.device)
         rc = lib.ftb_gemm_bf16_splitk(_ptr(a), _ptr(b), _ptr(out), _ptr(c), _ptr(bias), c_int(M), c_int(N), c_int(K),
@@ -548,11 +553,21 @@ def adamw_multi(params, grads, ms, vs, *, lrs, wds, beta1, beta2, eps, step, gra
         _check(rc, "ftb_adamw_multi")
 
 
+def _gram_alone(nb: int, k: int, length: int) -> bool:
+    """Whether ``nb`` products of a (k, length) matrix with itself are faster one after the other, each with its reduction cut
+    into slices, than as one grouped product, whose tiles walk the whole length: a tile does 64 of it in 0.43 us (64 x 65536:
+    440 us on one SM of 148), a product of its own takes the slice's time and 10 us for its two launches."""
+    splits = _k_splits(k, k, length)
+    whole = length / 64 * 0.43
+    return splits > 1 and nb * (whole / splits + 10.0) < whole
+
+
 def muon_batch(ps, gs, ms, *, lr, beta, weight_decay, ns_iters, nesterov, grad_scale, coeffs):
     """Muon update of matrices of one size (``ps`` bf16, ``gs`` / ``ms`` of one type each, bf16 or fp32, all contiguous and on
     16 bytes): the Newton-Schulz iteration of all of them runs as three grouped GEMMs per step, bf16 iterates with fp32
     accumulation: ``A = X Xᵀ``, ``B = bA + cA²``, ``X = aX + BX`` (epilogues with ``alpha`` and ``beta``).  Tall matrices are
-    iterated as ``AᵀA`` on the right, so nothing is transposed; their rows are padded with zeros to the reduction step."""
+    iterated as ``AᵀA`` on the right, so nothing is transposed; their rows are padded with zeros to the reduction step.
+    ``A`` of few, very long matrices is computed matrix by matrix (:func:`_gram_alone`).  Returns the number of launches."""
     lib = load("elementwise")
     (m, n), nb, dev = ps[0].shape, len(ps), ps[0].device
     a, b, c = coeffs
@@ -574,8 +589,12 @@ def muon_batch(ps, gs, ms, *, lr, beta, weight_decay, ns_iters, nesterov, grad_s
     ofs = torch.arange(0, nb * rows + 1, rows, dtype=torch.int32, device=dev)
     ofs_k = ofs if k == rows else torch.arange(0, nb * k + 1, k, dtype=torch.int32, device=dev)
     flat = lambda t: t.view(-1, t.shape[-1])
+    alone = _gram_alone(nb, k, max(m, n))
     for _ in range(ns_iters):
-        if tall:
+        if alone:
+            for xi, Ai in zip(x, A):
+                gemm(xi, xi, trans_a=tall, trans_b=not tall, out=Ai)
+        elif tall:
             grouped_wgrad(flat(x), flat(x), ofs, A, accumulate=False)
         else:
             grouped_gemm(flat(x), x, ofs, out=flat(A))
@@ -590,6 +609,7 @@ def muon_batch(ps, gs, ms, *, lr, beta, weight_decay, ns_iters, nesterov, grad_s
         j = min(i + 64, nb)
         _check(lib.ftb_muon_apply(c_int(j - i), arr(ps[i:j]), _ptr(x[i]), c_long(m * n), c_long(rows * n),
                                   c_float(1.0 - lr * weight_decay), c_float(lr * scale), _stream()), "ftb_muon_apply")
+    return 3 * ((nb + 63) // 64) + ns_iters * (2 + (2 * nb if alone else 1))
 
 
 def sum_of_squares(tensors):

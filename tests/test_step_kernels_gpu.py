@@ -86,6 +86,20 @@ def test_muon_batches_match_the_reference(nesterov, gdt, mdt):
         assert float(cos) > 0.98, (tuple(p.shape), float(cos))
 
 
+@pytest.mark.parametrize("shape", [(64, 4096), (4104, 64), (2, 64, 65536), (30, 64, 8192), (128, 20000), (20000, 512)])
+def test_muon_long_matrices(shape):
+    """Few matrices with a long side, whose products with themselves are cut along it, and as many as are not: the step within
+    the 2 % of the batches above."""
+    torch.manual_seed(0)
+    p, g, m = ((torch.randn(*shape, device=DEV) * k).to(BF16) for k in (0.05, 0.01, 0.01))
+    start, pw, mw = p.float(), p.float(), m.float()
+    kw = dict(lr=0.02, beta=0.95, weight_decay=0.01)
+    ops.muon_step(p, g, m, **kw)
+    ref.muon_step(pw, g.float(), mw, **kw)
+    for a, b in zip((p.float() - start).view(-1, *shape[-2:]), (pw - start).view(-1, *shape[-2:])):
+        assert float(torch.nn.functional.cosine_similarity(a.flatten(), b.flatten(), dim=0)) > 0.98
+
+
 @pytest.mark.parametrize("V", [8, 1000, 16384, 16392, 32771, 50257])
 @pytest.mark.parametrize("softcap", [0.0, 30.0])
 def test_cross_entropy_batches_and_loss_only(V, softcap):
