@@ -465,6 +465,20 @@ def muon_step(p, g, mom, *, lr, beta=0.95, weight_decay=0.0, ns_iters=5, nestero
                grad_scale=grad_scale)
 
 
+def newton_schulz_bf16(u: torch.Tensor, iters: int = 5) -> torch.Tensor:
+    """Quintic Newton-Schulz orthogonalisation of one matrix on the tcgen05 GEMM (:func:`muon_multi` iterates many together):
+    bf16 iterates with fp32 accumulation, per iteration ``A = X Xᵀ``, ``B = bA + cA²`` (epilogue ``alpha=c, beta=b``),
+    ``X = aX + BX`` (epilogue ``beta=a``).  A tall matrix is iterated as ``AᵀA`` on the right, so nothing is transposed."""
+    a, b, c = ref.NS_COEFFS
+    x = (u / (u.norm() + 1e-7)).to(torch.bfloat16).contiguous()
+    tall = x.shape[0] > x.shape[1]
+    for _ in range(iters):
+        A = gemm(x, x, trans_a=tall, trans_b=not tall)
+        B = gemm(A, A, alpha=c, beta=b, c=A)
+        x = gemm(x, B, beta=a, c=x) if tall else gemm(B, x, beta=a, c=x)
+    return x
+
+
 MUON_BATCH_ELEMENTS = 32 << 20      # of one batch's iterate: its workspace is four buffers of at most this size, in bf16
 
 
