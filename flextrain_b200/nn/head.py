@@ -37,7 +37,8 @@ class LMHead:
         per_tok = torch.empty(T, dtype=torch.float32, device=x.device)
         gW = grads.get("g_head_proj")
         # held-out data with the stock loss: nothing reads the logits' gradient
-        loss_only = (not want_dx and gW is None and type(loss_fn).__call__ is CrossEntropyLoss.__call__
+        loss_only = (not want_dx and gW is None and isinstance(loss_fn, CrossEntropyLoss) and loss_fn._native
+                     and type(loss_fn).__call__ is CrossEntropyLoss.__call__
                      and type(loss_fn).loss_only is CrossEntropyLoss.loss_only)
         for a in range(0, T, self.head_chunk_size):
             b = min(T, a + self.head_chunk_size)

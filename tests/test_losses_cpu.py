@@ -141,3 +141,26 @@ def test_builtin_losses_answer_to_the_reference_call_and_names():
     onehot = torch.zeros_like(p).scatter_(1, labels.clamp(min=0).unsqueeze(1), 1.0)
     torch.testing.assert_close(dz, (p - onehot) * (labels != -100).unsqueeze(1))       # unscaled, as the reference says
     assert GRPOLoss(kl_coef=0.3).kl_beta == 0.3
+
+
+class _Borrowed:
+    """Not a subclass: takes the stock loss's call alone."""
+    ignore_index = -100
+    __call__ = ft.CrossEntropyLoss.__call__
+
+
+class _Computed(ft.CrossEntropyLoss):
+    """The stock loss in the ``compute`` style, doubled."""
+    _native = False
+
+    def compute(self, logits, token_slice, *, loss_scale=1.0, per_token_loss_out=None):
+        per_token_loss_out.copy_(2.0 * self(logits, token_slice, 1.0))
+        return logits, {}
+
+
+@pytest.mark.parametrize("loss,factor", [(_Borrowed(), 1.0), (_Computed(), 2.0), (ft.CrossEntropyLoss(), 1.0)])
+def test_evaluate_takes_losses_built_from_the_stock_one(loss, factor):
+    """Held-out data takes a short way with the stock loss; what borrows from it or changes it does not."""
+    want = build_tiny(dims=DIMS).evaluate(_seqs())
+    got = build_tiny(dims=DIMS).evaluate(_seqs(), loss_fn=loss)
+    assert abs(got.loss_sum - factor * want.loss_sum) <= 1e-5 * abs(want.loss_sum)
