@@ -6,7 +6,7 @@ import torch
 
 import flextrain_b200 as ft
 from flextrain_b200.bench.naive import clone_params, naive_forward
-from flextrain_b200.nn.loss import GRPOLoss, MSELoss
+from flextrain_b200.nn.loss import CrossEntropyLoss, GRPOLoss, MSELoss
 from conftest import build_tiny
 
 DIMS = dict(vocab_size=256, n_layers=2, d_model=64, n_heads=4, n_kv_heads=2, head_dim=16, expert_dim=128, ffn_dim=128,
@@ -146,10 +146,10 @@ def test_builtin_losses_answer_to_the_reference_call_and_names():
 class _Borrowed:
     """Not a subclass: takes the stock loss's call alone."""
     ignore_index = -100
-    __call__ = ft.CrossEntropyLoss.__call__
+    __call__ = CrossEntropyLoss.__call__
 
 
-class _Computed(ft.CrossEntropyLoss):
+class _Computed(CrossEntropyLoss):
     """The stock loss in the ``compute`` style, doubled."""
     _native = False
 
@@ -158,7 +158,7 @@ class _Computed(ft.CrossEntropyLoss):
         return logits, {}
 
 
-@pytest.mark.parametrize("loss,factor", [(_Borrowed(), 1.0), (_Computed(), 2.0), (ft.CrossEntropyLoss(), 1.0)])
+@pytest.mark.parametrize("loss,factor", [(_Borrowed(), 1.0), (_Computed(), 2.0), (CrossEntropyLoss(), 1.0)])
 def test_evaluate_takes_losses_built_from_the_stock_one(loss, factor):
     """Held-out data takes a short way with the stock loss; what borrows from it or changes it does not."""
     want = build_tiny(dims=DIMS).evaluate(_seqs())
