@@ -674,7 +674,7 @@ rope_inv_freq = ref.rope_inv_freq
 # ``timing_report()`` aggregates them by (op, shape): the per-kernel time table of a training step without a
 # profiler attached.  The events add host work, so a throughput number taken with it on is not a benchmark value.
 _TIMED_OPS = ("gemm", "gemm_glu_fwd", "gemm_glu_bwd", "rmsnorm_fwd", "rmsnorm_bwd", "rope", "glu_fwd", "glu_bwd", "glu_bwd_weighted", "attention_fwd",
-              "attention_bwd", "softmax_ce_", "embedding_fwd", "embedding_bwd", "adamw_multi", "topk_route",
+              "attention_bwd", "softmax_ce_", "softmax_ce_loss", "embedding_fwd", "embedding_bwd", "adamw_multi", "topk_route",
               "topk_route_bwd", "gather_rows", "moe_combine", "grouped_gemm", "grouped_wgrad", "l2norm_fwd",
               "gated_rmsnorm_fwd", "bias_grad")
 _timing_events: list = []

@@ -164,3 +164,10 @@ def test_evaluate_takes_losses_built_from_the_stock_one(loss, factor):
     want = build_tiny(dims=DIMS).evaluate(_seqs())
     got = build_tiny(dims=DIMS).evaluate(_seqs(), loss_fn=loss)
     assert abs(got.loss_sum - factor * want.loss_sum) <= 1e-5 * abs(want.loss_sum)
+
+
+def test_the_op_timing_table_names_the_ops_that_run():
+    """Both forms of the cross entropy are in the table, and every name in it is an op."""
+    from flextrain_b200 import ops
+    assert {"softmax_ce_", "softmax_ce_loss"} <= set(ops._TIMED_OPS)
+    assert all(callable(getattr(ops, n, None)) for n in ops._TIMED_OPS)
