@@ -148,6 +148,11 @@ def baseline_model_memory(layers, embed, head, optimizer, probe_tokens: int = 40
     return ModelMemory(lp, lm, lg, lo, eh, af, at, flops, head_flops, [r / max(flops, 1e-9) for r in redo])
 
 
+# Temporaries that no shape below stands for: the fp32 slabs of a GEMM with a cut reduction while a chunk is in flight, and a
+# batch of the Muon iteration during the update, when the chunk's own temporaries are free.
+WORKSPACE_ALLOWANCE = 256 << 20
+
+
 def _workspace_bytes(layers, head, chunk: int, act_bytes: int = 2, head_rows: Optional[int] = None) -> int:
     """Transient GPU memory while one chunk is in flight: residual stream in/out, the widest projection output
     and its gradient, attention workspace, and one head micro-chunk of logits."""
@@ -166,7 +171,7 @@ def _workspace_bytes(layers, head, chunk: int, act_bytes: int = 2, head_rows: Op
         widest = max(widest, w)
     per_tok = (4 * d + 2 * widest) * act_bytes
     head_ws = min(chunk, head_rows or head.head_chunk_size) * head.vocab_size * act_bytes * 2
-    return chunk * per_tok + head_ws + (256 << 20)
+    return chunk * per_tok + head_ws + WORKSPACE_ALLOWANCE
 
 
 def determine_working_set_config(*, layers, embed, head, optimizer, max_seq_len: int, max_global_batch_tokens: int,

@@ -479,7 +479,15 @@ def newton_schulz_bf16(u: torch.Tensor, iters: int = 5) -> torch.Tensor:
     return x
 
 
-MUON_BATCH_ELEMENTS = 32 << 20      # of one batch's iterate: its workspace is four buffers of at most this size, in bf16
+# Elements of one batch's iterate: its workspace is four buffers of at most this size, in bf16, which is what a plan sets aside
+# for temporaries.  (A matrix that is larger by itself is a batch of one: 8 bytes an element, in place of 16 and more when its
+# momentum and update were kept in fp32.)
+MUON_BATCH_ELEMENTS = 32 << 20
+
+
+def _muon_batch_size(m: int, n: int) -> int:
+    """Matrices of one batch (the rows of tall ones are padded to the reduction step)."""
+    return max(1, MUON_BATCH_ELEMENTS // ((m + 63) // 64 * 64 * n if m > n else m * n))
 
 
 def muon_multi(ps, gs, moms, *, lr, beta=0.95, weight_decay=0.0, ns_iters=5, nesterov=True, grad_scale=1.0):
@@ -506,7 +514,7 @@ def muon_multi(ps, gs, moms, *, lr, beta=0.95, weight_decay=0.0, ns_iters=5, nes
         for pm, gm, mm in mats:
             batches.setdefault((pm.shape, gm.dtype, mm.dtype, pm.device), []).append((pm, gm, mm))
     for (shape, *_), mats in batches.items():
-        per = max(1, MUON_BATCH_ELEMENTS // (shape[0] * shape[1]))
+        per = _muon_batch_size(*shape)
         for i in range(0, len(mats), per):
             _count(_kernels().muon_batch(*[list(t) for t in zip(*mats[i:i + per])], coeffs=ref.NS_COEFFS, **kw))
     for t, c in back:

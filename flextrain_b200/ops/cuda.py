@@ -131,6 +131,10 @@ def gemm_supported(a: torch.Tensor, b: torch.Tensor, trans_a: bool, trans_b: boo
         and b.data_ptr() % 16 == 0
 
 
+# Most that the fp32 slabs of one cut GEMM take: half of what a plan sets aside for temporaries besides its layers' own.
+GEMM_SLAB_BYTES = 128 << 20
+
+
 @functools.lru_cache(maxsize=4096)
 def _two_sm_splits(M: int, N: int, K: int) -> int:
     """Slices of K (fp32 slabs, ordered sum) for a GEMM on two-SM tiles: more than one where 256 x 256 tiles leave many of the
@@ -145,7 +149,7 @@ def _two_sm_splits(M: int, N: int, K: int) -> int:
     full = K / 64 * 512 / 1.75e3
     best, least = 1, 0.88 * -(-tiles // 74) * full
     for s in range(2, 9):
-        if s * M * N * 4 > 128 << 20 or K // s < 256:
+        if s * M * N * 4 > GEMM_SLAB_BYTES or K // s < 256:
             break
         us = -(-tiles * s // 74) / s * full + s * M * N * 8 / 4e6 + 4.0
         if us < least:
