@@ -128,8 +128,8 @@ __global__ void conv1d_bwd_dx_kernel(const float* __restrict__ dpre, const bf16*
 // W - 1 inputs (or gradients) around it, so every element is read once, four bytes a lane, eight tokens ahead of their use.
 // The general kernels above read each input W times, two bytes a lane, and look the sequence of every token up; they stay for
 // other widths, odd channel counts and unaligned rows.  Tokens before the first sequence or after the last (padding) belong to
-// the nearest one, as in the general kernels, but are no part of its inputs or of its end.  Bound by memory.  16384 tokens x 8192 channels, W = 4: forward 833 us
-// before, 170 us so; dpre 1240 us before, 314 us so; dx 930 us before, 154 us so.
+// the nearest one, as in the general kernels, but their values are no part of it.  Bound by memory.  16384 tokens x 8192
+// channels, W = 4: forward 833 us before, 170 us so; dpre 1240 us before, 314 us so; dx 930 us before, 154 us so.
 constexpr int CONV_GROUP = 8;
 __device__ __forceinline__ float2 ld2(const bf16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
 
@@ -142,10 +142,10 @@ struct ConvWalk {                         // ascending tokens: the sequence of t
     a = cu[s];
     end = cu[s + 1];
 #pragma unroll
-    for (int j = 0; j < W - 1; ++j) {
-      const int pos = t - a - (W - 1) + j;
-      win[j] = make_float2(conv_input(x, ldx, init, D, W, s, a, pos, d), conv_input(x, ldx, init, D, W, s, a, pos, d + 1));
-    }
+    for (int j = 0; j < W - 1; ++j) win[j] = input(x, ldx, init, D, t - a - (W - 1) + j, d);
+  }
+  __device__ __forceinline__ float2 input(const bf16* x, long ldx, const bf16* init, int D, int pos, int d) const {
+    return make_float2(conv_input(x, ldx, init, D, W, s, a, pos, d), conv_input(x, ldx, init, D, W, s, a, pos, d + 1));
   }
   __device__ __forceinline__ void shift(float2 v) {
 #pragma unroll
@@ -180,8 +180,8 @@ __global__ void __launch_bounds__(128) conv1d_fwd2_kernel(const bf16* __restrict
     for (int i = 0; i < CONV_GROUP; ++i) {
       const int t = t0 + i;
       if (t >= te) break;
-      if (t >= c.end || t == c.a) c.enter(x, ldx, init, cu, nseq, D, t, d);
-      if (t < c.a) in[i] = make_float2(0.f, 0.f);
+      if (t >= c.end) c.enter(x, ldx, init, cu, nseq, D, t, d);
+      if (t < c.a) in[i] = c.input(x, ldx, init, D, t - c.a, d);
       float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
       for (int j = 0; j < W - 1; ++j) { acc.x += wr[j].x * c.win[j].x; acc.y += wr[j].y * c.win[j].y; }
@@ -221,8 +221,8 @@ __global__ void __launch_bounds__(128) conv1d_bwd_pre2_kernel(const bf16* __rest
     for (int i = 0; i < CONV_GROUP; ++i) {
       const int t = t0 + i;
       if (t >= te) break;
-      if (t >= c.end || t == c.a) c.enter(x, ldx, init, cu, nseq, D, t, d);
-      if (t < c.a) in[i] = make_float2(0.f, 0.f);
+      if (t >= c.end) c.enter(x, ldx, init, cu, nseq, D, t, d);
+      if (t < c.a) in[i] = c.input(x, ldx, init, D, t - c.a, d);
       float2 g = gy[i];
       if (act) {
         float2 acc = make_float2(0.f, 0.f);
