@@ -33,8 +33,14 @@ __device__ __forceinline__ int seq_of(const int* __restrict__ cu, int nseq, int 
 __device__ __forceinline__ float conv_input(const bf16* __restrict__ x, long ldx, const bf16* __restrict__ init, int D,
                                             int W, int seq, int a, int pos, int d) {
   if (pos >= 0) return __bfloat162float(x[(long)(a + pos) * ldx + d]);
-  if (init == nullptr || pos < -(W - 1)) return 0.f;      // (a token before the first sequence reaches further back)
+  if (init == nullptr) return 0.f;
   return __bfloat162float(init[((long)seq * D + d) * (W - 1) + (W - 1) + pos]);
+}
+
+// the same for any token: one before the first sequence reaches further back than the carried state
+__device__ __forceinline__ float conv_input_any(const bf16* __restrict__ x, long ldx, const bf16* __restrict__ init, int D,
+                                                int W, int seq, int a, int pos, int d) {
+  return pos < -(W - 1) ? 0.f : conv_input(x, ldx, init, D, W, seq, a, pos, d);
 }
 
 // y[t, d] = act( sum_j w[d, j] * in(pos - (W-1) + j) ),  thread = channel, block row = TT tokens
@@ -50,7 +56,7 @@ __global__ void conv1d_fwd_kernel(const bf16* __restrict__ x, long ldx, const bf
   for (int t = tb; t < min(T, tb + TT); ++t) {
     const int s = seq_of(cu, nseq, t), a = cu[s], pos = t - a;
     float acc = 0.f;
-    for (int j = 0; j < W; ++j) acc += wr[j] * conv_input(x, ldx, init, D, W, s, a, pos - (W - 1) + j, d);
+    for (int j = 0; j < W; ++j) acc += wr[j] * conv_input_any(x, ldx, init, D, W, s, a, pos - (W - 1) + j, d);
     y[(long)t * D + d] = __float2bfloat16(act ? acc * sigmoidf(acc) : acc);
   }
 }
@@ -83,7 +89,7 @@ __global__ void conv1d_bwd_pre_kernel(const bf16* __restrict__ x, long ldx, cons
   for (int t = tb; t < min(T, tb + TT); ++t) {
     const int s = seq_of(cu, nseq, t), a = cu[s], pos = t - a;
     float in[MAXW], acc = 0.f;
-    for (int j = 0; j < W; ++j) { in[j] = conv_input(x, ldx, init, D, W, s, a, pos - (W - 1) + j, d); acc += wr[j] * in[j]; }
+    for (int j = 0; j < W; ++j) { in[j] = conv_input_any(x, ldx, init, D, W, s, a, pos - (W - 1) + j, d); acc += wr[j] * in[j]; }
     float g = __bfloat162float(dy[(long)t * D + d]);
     if (act) {
       const float sg = sigmoidf(acc);
@@ -127,9 +133,10 @@ __global__ void conv1d_bwd_dx_kernel(const float* __restrict__ dpre, const bf16*
 // ---- the same three passes with the taps in registers: a thread walks TT tokens of two neighbouring channels and carries the
 // W - 1 inputs (or gradients) around it, so every element is read once, four bytes a lane, eight tokens ahead of their use.
 // The general kernels above read each input W times, two bytes a lane, and look the sequence of every token up; they stay for
-// other widths, odd channel counts and unaligned rows.  Tokens before the first sequence or after the last (padding) belong to
-// the nearest one, as in the general kernels, but their values are no part of it.  Bound by memory.  16384 tokens x 8192
-// channels, W = 4: forward 833 us before, 170 us so; dpre 1240 us before, 314 us so; dx 930 us before, 154 us so.
+// other widths, odd channel counts and unaligned rows.  A block that holds tokens before the first sequence or after the last
+// (padding) looks its tokens up one by one, as in the general kernels: tested for each token, that cost the other blocks 15 %,
+// and 10 % where it took the backward above 96 registers, so it has functions of its own there.  Bound by memory.  16384 tokens x 8192 channels, W = 4: forward 833 us before, 170 us so; dpre 1240 us before, 314 us so; dx
+// 930 us before, 154 us so.
 constexpr int CONV_GROUP = 8;
 __device__ __forceinline__ float2 ld2(const bf16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
 
@@ -142,10 +149,10 @@ struct ConvWalk {                         // ascending tokens: the sequence of t
     a = cu[s];
     end = cu[s + 1];
 #pragma unroll
-    for (int j = 0; j < W - 1; ++j) win[j] = input(x, ldx, init, D, t - a - (W - 1) + j, d);
-  }
-  __device__ __forceinline__ float2 input(const bf16* x, long ldx, const bf16* init, int D, int pos, int d) const {
-    return make_float2(conv_input(x, ldx, init, D, W, s, a, pos, d), conv_input(x, ldx, init, D, W, s, a, pos, d + 1));
+    for (int j = 0; j < W - 1; ++j) {
+      const int pos = t - a - (W - 1) + j;
+      win[j] = make_float2(conv_input(x, ldx, init, D, W, s, a, pos, d), conv_input(x, ldx, init, D, W, s, a, pos, d + 1));
+    }
   }
   __device__ __forceinline__ void shift(float2 v) {
 #pragma unroll
@@ -160,8 +167,37 @@ __device__ __forceinline__ void load_taps(float2 (&wr)[W], const bf16* w, int d)
     wr[j] = make_float2(__bfloat162float(w[(long)d * W + j]), __bfloat162float(w[(long)(d + 1) * W + j]));
 }
 
+// One token by itself: its inputs and their product with the taps.
+template <int W>
+__device__ __forceinline__ float2 conv_token(float2 (&in)[W], const float2 (&wr)[W], const bf16* x, long ldx, const bf16* init,
+                                             const int* cu, int nseq, int D, int t, int d) {
+  const int s = seq_of(cu, nseq, t), a = cu[s];
+  float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+    const int pos = t - a - (W - 1) + j;
+    in[j] = make_float2(conv_input_any(x, ldx, init, D, W, s, a, pos, d), conv_input_any(x, ldx, init, D, W, s, a, pos, d + 1));
+    acc.x += wr[j].x * in[j].x;
+    acc.y += wr[j].y * in[j].y;
+  }
+  return acc;
+}
+template <int W>
+__device__ __forceinline__ void add_taps(float* dw, const float2 (&gw)[W], int d) {
+  if (dw == nullptr) return;
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+    atomicAdd(dw + (long)d * W + j, gw[j].x);
+    atomicAdd(dw + (long)(d + 1) * W + j, gw[j].y);
+  }
+}
+__device__ __forceinline__ float2 act_grad(float2 g, float2 pre) {
+  const float sx = sigmoidf(pre.x), sy = sigmoidf(pre.y);
+  return make_float2(g.x * (sx * (1.f + pre.x * (1.f - sx))), g.y * (sy * (1.f + pre.y * (1.f - sy))));
+}
+
 template <int W, int TT>
-__global__ void __launch_bounds__(128) conv1d_fwd2_kernel(const bf16* __restrict__ x, long ldx, const bf16* __restrict__ w,
+__global__ void __launch_bounds__(128, 8) conv1d_fwd2_kernel(const bf16* __restrict__ x, long ldx, const bf16* __restrict__ w,
                                                           const bf16* __restrict__ init, const int* __restrict__ cu,
                                                           int nseq, bf16* __restrict__ y, int T, int D, int act) {
   const int d = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
@@ -169,6 +205,15 @@ __global__ void __launch_bounds__(128) conv1d_fwd2_kernel(const bf16* __restrict
   float2 wr[W];
   load_taps<W>(wr, w, d);
   const int tb = blockIdx.y * TT, te = min(T, tb + TT);
+  if (tb < cu[0]) {
+#pragma unroll 1
+    for (int t = tb; t < te; ++t) {
+      float2 in[W], acc = conv_token<W>(in, wr, x, ldx, init, cu, nseq, D, t, d);
+      if (act) { acc.x *= sigmoidf(acc.x); acc.y *= sigmoidf(acc.y); }
+      *reinterpret_cast<__nv_bfloat162*>(y + (long)t * D + d) = __floats2bfloat162_rn(acc.x, acc.y);
+    }
+    return;
+  }
   ConvWalk<W> c;
   c.enter(x, ldx, init, cu, nseq, D, tb, d);
   for (int t0 = tb; t0 < te; t0 += CONV_GROUP) {
@@ -181,7 +226,6 @@ __global__ void __launch_bounds__(128) conv1d_fwd2_kernel(const bf16* __restrict
       const int t = t0 + i;
       if (t >= te) break;
       if (t >= c.end) c.enter(x, ldx, init, cu, nseq, D, t, d);
-      if (t < c.a) in[i] = c.input(x, ldx, init, D, t - c.a, d);
       float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
       for (int j = 0; j < W - 1; ++j) { acc.x += wr[j].x * c.win[j].x; acc.y += wr[j].y * c.win[j].y; }
@@ -192,6 +236,27 @@ __global__ void __launch_bounds__(128) conv1d_fwd2_kernel(const bf16* __restrict
       *reinterpret_cast<__nv_bfloat162*>(y + (long)t * D + d) = __floats2bfloat162_rn(acc.x, acc.y);
     }
   }
+}
+
+// dpre and the taps' gradient of a block with padding, one token at a time
+template <int W>
+__device__ __noinline__ void conv1d_pre_block(const bf16* x, long ldx, const bf16* w, const bf16* init, const int* cu, int nseq,
+                                              const bf16* dy, float* dpre, float* dw, int tb, int te, int D, int d, int act) {
+  float2 wr[W], gw[W];
+  load_taps<W>(wr, w, d);
+#pragma unroll
+  for (int j = 0; j < W; ++j) gw[j] = make_float2(0.f, 0.f);
+#pragma unroll 1
+  for (int t = tb; t < te; ++t) {
+    float2 in[W];
+    const float2 pre = conv_token<W>(in, wr, x, ldx, init, cu, nseq, D, t, d);
+    float2 g = ld2(dy + (long)t * D + d);
+    if (act) g = act_grad(g, pre);
+    *reinterpret_cast<float2*>(dpre + (long)t * D + d) = g;
+#pragma unroll
+    for (int j = 0; j < W; ++j) { gw[j].x += g.x * in[j].x; gw[j].y += g.y * in[j].y; }
+  }
+  add_taps<W>(dw, gw, d);
 }
 
 template <int W, int TT>
@@ -207,6 +272,10 @@ __global__ void __launch_bounds__(128) conv1d_bwd_pre2_kernel(const bf16* __rest
 #pragma unroll
   for (int j = 0; j < W; ++j) gw[j] = make_float2(0.f, 0.f);
   const int tb = blockIdx.y * TT, te = min(T, tb + TT);
+  if (tb < cu[0]) {
+    conv1d_pre_block<W>(x, ldx, w, init, cu, nseq, dy, dpre, dw, tb, te, D, d, act);
+    return;
+  }
   ConvWalk<W> c;
   c.enter(x, ldx, init, cu, nseq, D, tb, d);
   for (int t0 = tb; t0 < te; t0 += CONV_GROUP) {
@@ -222,7 +291,6 @@ __global__ void __launch_bounds__(128) conv1d_bwd_pre2_kernel(const bf16* __rest
       const int t = t0 + i;
       if (t >= te) break;
       if (t >= c.end) c.enter(x, ldx, init, cu, nseq, D, t, d);
-      if (t < c.a) in[i] = c.input(x, ldx, init, D, t - c.a, d);
       float2 g = gy[i];
       if (act) {
         float2 acc = make_float2(0.f, 0.f);
@@ -230,9 +298,7 @@ __global__ void __launch_bounds__(128) conv1d_bwd_pre2_kernel(const bf16* __rest
         for (int j = 0; j < W - 1; ++j) { acc.x += wr[j].x * c.win[j].x; acc.y += wr[j].y * c.win[j].y; }
         acc.x += wr[W - 1].x * in[i].x;
         acc.y += wr[W - 1].y * in[i].y;
-        const float sx = sigmoidf(acc.x), sy = sigmoidf(acc.y);
-        g.x *= sx * (1.f + acc.x * (1.f - sx));
-        g.y *= sy * (1.f + acc.y * (1.f - sy));
+        g = act_grad(g, acc);
       }
       *reinterpret_cast<float2*>(dpre + (long)t * D + d) = g;
 #pragma unroll
@@ -242,11 +308,22 @@ __global__ void __launch_bounds__(128) conv1d_bwd_pre2_kernel(const bf16* __rest
       c.shift(in[i]);
     }
   }
-  if (dw != nullptr) {
+  add_taps<W>(dw, gw, d);
+}
+
+// dx of a block with padding
+template <int W>
+__device__ __noinline__ void conv1d_dx_block(const float* dpre, const bf16* w, const bf16* dfin, const int* cu, int nseq, bf16* dx,
+                                             long lddx, int tb, int te, int D, int d) {
+#pragma unroll 1
+  for (int c = d; c < d + 2; ++c) {
+    float wr[W];
 #pragma unroll
-    for (int j = 0; j < W; ++j) {
-      atomicAdd(dw + (long)d * W + j, gw[j].x);
-      atomicAdd(dw + (long)(d + 1) * W + j, gw[j].y);
+    for (int j = 0; j < W; ++j) wr[j] = __bfloat162float(w[(long)c * W + j]);
+#pragma unroll 1
+    for (int t = tb; t < te; ++t) {
+      const int s = seq_of(cu, nseq, t), a = cu[s], L = cu[s + 1] - a;
+      dx[(long)t * lddx + c] = __float2bfloat16(conv_dinput(dpre, wr, dfin, D, W, s, a, L, t - a, c));
     }
   }
 }
@@ -261,10 +338,14 @@ __global__ void __launch_bounds__(128) conv1d_bwd_dx2_kernel(const float* __rest
   float2 wr[W], win[W - 1];
   load_taps<W>(wr, w, d);
   const int tb = blockIdx.y * TT, te = min(T, tb + TT);
+  if (tb < cu[0] || te > cu[nseq]) {
+    conv1d_dx_block<W>(dpre, w, dfin, cu, nseq, dx, lddx, tb, te, D, d);
+    return;
+  }
   int s = seq_of(cu, nseq, te - 1), a = cu[s], end = cu[s + 1];
   auto at = [&](int t) { return *reinterpret_cast<const float2*>(dpre + (long)t * D + d); };
 #pragma unroll
-  for (int k = 0; k < W - 1; ++k) win[k] = te + k >= a && te + k < end ? at(te + k) : make_float2(0.f, 0.f);
+  for (int k = 0; k < W - 1; ++k) win[k] = te + k < end ? at(te + k) : make_float2(0.f, 0.f);
   for (int t0 = te - 1; t0 >= tb; t0 -= CONV_GROUP) {
     float2 in[CONV_GROUP];
 #pragma unroll
@@ -274,21 +355,20 @@ __global__ void __launch_bounds__(128) conv1d_bwd_dx2_kernel(const float* __rest
     for (int i = 0; i < CONV_GROUP; ++i) {
       const int t = t0 - i;
       if (t < tb) break;
-      if (t < a && s > 0) {                            // the last token of an earlier sequence
+      if (t < a) {                                     // the last token of an earlier sequence
         s = seq_of(cu, nseq, t);
         a = cu[s];
         end = cu[s + 1];
 #pragma unroll
         for (int k = 0; k < W - 1; ++k) win[k] = make_float2(0.f, 0.f);
       }
-      if (t < a || t >= end) in[i] = make_float2(0.f, 0.f);
       float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
       for (int j = 0; j < W - 1; ++j) { acc.x += wr[j].x * win[W - 2 - j].x; acc.y += wr[j].y * win[W - 2 - j].y; }
       acc.x += wr[W - 1].x * in[i].x;
       acc.y += wr[W - 1].y * in[i].y;
       const int m = t - (end - (W - 1));               // (the virtual input of the carried state)
-      if (dfin != nullptr && m >= 0 && m < W - 1) {
+      if (dfin != nullptr && m >= 0) {
         acc.x += __bfloat162float(dfin[((long)s * D + d) * (W - 1) + m]);
         acc.y += __bfloat162float(dfin[((long)s * D + d + 1) * (W - 1) + m]);
       }
