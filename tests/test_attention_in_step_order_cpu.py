@@ -2,12 +2,12 @@
 host like the first: key tiles ascending, query tiles descending with the heads of the group inside, a CTA waiting for the
 key tiles below its own that touch the query tile.  With any number of resident CTAs every wait must be satisfiable by CTAs
 handed out before, every counter must end at the number of key tiles that touch its query tile, and the additions must come
-in strictly ascending key-tile order."""
+in strictly ascending key-tile order.  Here a turn passes on at once."""
 import random
 
 import pytest
 
-from test_attention_order_cpu import TQ, replay
+from test_attention_order_cpu import TQ, replay, row_groups
 
 
 def ctas_in_dispatch_order(lens_q, lens_k, causal, window, rep, grid_slack=3):
@@ -33,7 +33,7 @@ def ctas_in_dispatch_order(lens_q, lens_k, causal, window, rep, grid_slack=3):
         its, qt, h = [], i_lo + (n_qt - 1) * TQ, 0
         for _ in range(n_qt * rep):
             j_lo = max(0, qt + off - window + 1) // TQ if causal and window > 0 else 0
-            its.append(((qtile_base[seq] + qt // TQ, h), k0 // TQ - j_lo, k0 // TQ))
+            its.append(((qtile_base[seq] + qt // TQ, h), k0 // TQ - j_lo, k0 // TQ, row_groups(len_q - qt)))
             h += 1
             if h == rep:
                 h, qt = 0, qt - TQ
@@ -51,8 +51,8 @@ def test_in_step_order_is_satisfiable_and_ascending(seed):
     window = rng.choice((0, 0, 1, 100, 128, 129, 300)) if causal else 0
     ctas = ctas_in_dispatch_order(lens_q, lens_k, causal, window, rng.choice((1, 2, 4)))
     for resident in (1, 2, 5, 1000):
-        done, sem, order = replay(ctas, resident)
+        done, sem, order = replay(ctas, resident, late=False)
         assert done
         for key, tiles in order.items():
             assert tiles == sorted(set(tiles)) and sem[key] == len(tiles)
-        assert sum(map(len, order.values())) == sum(len(c[2]) for c in ctas)
+        assert sum(map(len, order.values())) == sum(groups for c in ctas for *_, groups in c[2])
