@@ -805,11 +805,13 @@ namespace ftb {
 //   IN_STEP      key tiles ascending, query tiles descending with the heads of the group inside: all key tiles of a
 //                sequence walk the same (query tile, head) list in step, the short ones leave it early.  The longest CTAs
 //                come first; the price is a wait per key tile at the start and additions that meet at the same addresses.
-// With a fixed order, LAST_FIRST against IN_STEP, us: head dim 128, 32 / 8 heads: 16 x 1024 tokens 614 / 635, 4 x 4096
-// 2033 / 2056, 2 x 8192 4253 / 3824, 1 x 16384 9406 / 8411; 16 / 16 heads: 4 x 4096 1061 / 1165, 2 x 8192 1930 / 1892,
-// 1 x 16384 4183 / 3702; 16 / 8 heads: 2 x 8192 1943 / 2043, 1 x 16384 4146 / 3860.  Head dim 64, 32 / 8 heads: 8 x 2048
-// 808 / 774, 1 x 16384 5826 / 5054.  So IN_STEP where the longest sequence has more than 4096 keys (1024 at head dim 64,
-// whose tile pairs are shorter).
+// With a fixed order, LAST_FIRST against IN_STEP, causal, us of this kernel, all taken in turn on one GPU.  Head dim 128,
+// 32 / 8 heads: 16 x 1024 tokens 609 / 636, 4 x 4096 2041 / 1940, 2 x 8192 4347 / 3607, 1 x 16384 9013 / 7018; 16 / 8 heads:
+// 4 x 4096 1043 / 1054, 2 x 8192 1967 / 1925, 1 x 16384 4272 / 3635; 16 / 16 heads: 4 x 4096 1030 / 1154, 2 x 8192 1927 / 2037,
+// 1 x 16384 4175 / 3765.  Head dim 64, 32 / 8 heads: 16 x 1024 468 / 462, 8 x 2048 810 / 756, 1 x 16384 5810 / 4866; 16 / 16
+// heads: 16 x 1024 291 / 311, 8 x 2048 453 / 471, 2 x 8192 1399 / 1403.  The more heads share a key, the earlier IN_STEP wins; it
+// is taken where the longest sequence has more than 4096 keys (1024 at head dim 64, whose tile pairs are shorter), where the two
+// differ by 5 to 7 % either way.
 constexpr int BWD_FIRST_FIRST = 0, BWD_LAST_FIRST = 1, BWD_IN_STEP = 2;
 
 struct BwdParams {
@@ -818,7 +820,7 @@ struct BwdParams {
   int num_seqs;
   int H, KV;
   float* dq_acc;            // (Tq, H, HD) fp32, zero-initialised by the caller
-  int* dq_sem;              // deterministic mode: one counter per (query tile, head), zeroed by the caller; else NULL
+  int* dq_sem;              // deterministic mode: a flag and one counter per (query tile, head, 32 rows), zeroed; else NULL
   int order;                // BWD_*: the order of the key tiles over the grid and of the query tiles in a CTA
   int dq_bulk;              // 1: dQ tiles leave through shared memory as tiled reduce-adds; 0: per-thread vector reductions
   __nv_bfloat16* dk;        // (Tk, KV, HD) contiguous
@@ -877,8 +879,8 @@ __global__ void fa_delta_kernel(const __nv_bfloat16* __restrict__ dout, long do_
 // core subtracts them: one more step of 16 in the reduction, whose A rows are (1, 1, 1, 0 ...) and whose B rows hold
 // -lse / scale (or -delta) as the sum of three bf16 (24 bits, as exact as the fp32 value).
 // Causal, 32 / 8 heads of 128, dQ in any order: 16 x 1024 tokens 771 us with one chain S, dP -> softmax -> dV, dK, dQ ->
-// drain per tile pair, 506 us so; 1 x 16384 9160 us (600 TFLOP/s) before, 5510 us (997) so.  With dQ in a fixed order 926 ->
-// 613 us and 12300 -> 6990 us.
+// drain per tile pair, 514 us so; 1 x 16384 9160 us (600 TFLOP/s) before, 5710 us (963) so.  With dQ in a fixed order 926 ->
+// 609 us and 12300 -> 7018 us.
 constexpr int FAB_THREADS = 448;
 constexpr int FAB_SOFTMAX_WARPS = 8;
 
@@ -1350,8 +1352,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     };
     // In a fixed order, a tile's turn passes on when its additions have been performed.  LAST_FIRST, whose next key tile
     // comes a step later by itself, looks at that only before the staging block is needed again: waiting at once held this
-    // warp for another 1400 cycles a tile (16 x 1024 tokens 636 us against 613).  IN_STEP, where the next key tile is
-    // waiting, passes on at once (1 x 16384 7240 us against 6990).
+    // warp for another 1400 cycles a tile (16 x 1024 tokens 4 % more).  IN_STEP, where the next key tile is
+    // waiting, passes on at once (1 x 16384: later, 4 % more).
     int* passing = nullptr;
     auto pass_on = [&]() {
       if (passing != nullptr) {

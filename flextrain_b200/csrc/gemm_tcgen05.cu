@@ -1470,11 +1470,12 @@ int ftb_gemm_glu_bwd(const void* dY, const void* W2, const void* x13, void* dx13
   return launch2<false, true, 2>(ta, tb, p, grid, stream);
 }
 
-// Split-K variant for small outputs with a long reduction (the rank-r LoRA gradients: M or N = r, K = tokens): the K
-// range is cut into `splits` slices so that tiles x splits work items fill the GPU instead of a handful of CTAs each
-// walking the whole K.  Every slice writes alpha * partial into its own fp32 slab of `workspace` (splits x M x N
-// floats, supplied by the caller) and a second kernel adds the slabs (+ beta * C + bias) into D in the output type:
-// fixed summation order, no atomics.  Same operand rules as ftb_gemm_bf16; one-SM kernel only.
+// Split-K variant for outputs of few tiles with a long reduction (the rank-r LoRA gradients: M or N = r, K = tokens; weight
+// gradients of narrow layers; the head's input gradient): the K range is cut into `splits` slices so that tiles x splits work
+// items fill the GPU instead of a handful of CTAs each walking the whole K.  Every slice writes alpha * partial into its own
+// fp32 slab of `workspace` (splits x M x N floats, supplied by the caller) and a second kernel adds the slabs (+ beta * C +
+// bias) into D in the output type: fixed summation order, no atomics.  Same operand rules as ftb_gemm_bf16, and the same tiles:
+// two SMs where M and N reach 512, else one.
 int ftb_gemm_bf16_splitk(const void* A, const void* B, void* D, const void* C, const float* bias, int M, int N, int K,
                          int a_mn_major, int b_mn_major, int lda, int ldb, int ldd, int ldc, float alpha, float beta,
                          int d_fp32, int splits, float* workspace, cudaStream_t stream) {

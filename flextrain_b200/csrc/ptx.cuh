@@ -260,13 +260,14 @@ __device__ __forceinline__ void tma_load_2d_2cta(void* smem_dst, const CUtensorM
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(smem_u32(bar) & PEER_BIT_MASK)
       : "memory");
 }
-// 256-row MMA across the pair: each CTA contributes 128 rows of A and half of B's N; issued by the leader only.
+// the same for a 3-D map (one matrix of a stack)
 __device__ __forceinline__ void tma_load_3d_2cta(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y, int z) {
   asm volatile(
       "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar) & PEER_BIT_MASK)
       : "memory");
 }
+// 256-row MMA across the pair: each CTA contributes 128 rows of A and half of B's N; issued by the leader only.
 __device__ __forceinline__ void umma_f16_2cta(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                               uint32_t accumulate) {
   asm volatile(
