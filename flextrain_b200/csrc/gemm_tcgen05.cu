@@ -754,8 +754,19 @@ struct Ring2 {
   static constexpr int STAGES = EPI == 0 ? 6 : 5;
   static constexpr int WARP_BYTES = EPI == 0 ? 32 * 128 : 3 * 32 * 64;
   static constexpr int TOTAL = STAGES * STAGE2_BYTES + EPI2_WARPS * WARP_BYTES + 256 + 1024;
-  static_assert(TOTAL <= 232448, "shared memory of a CTA");
+  // of the SM's 228 KB, of which every block takes 1 KB: one more block without shared memory has room
+  static_assert(TOTAL + 2 * 1024 <= 228 * 1024, "shared memory of a CTA and of a block beside it");
 };
+// The kernel is compiled as if for 512 threads: 128 registers, so that the collectives of a data-parallel step (256 threads of
+// 34 to 40 registers) and AdamW (52) run beside it on their own stream.  Its ten warps put three on two of the SM's four
+// partitions; at the 168 registers that 320 threads may have these filled a partition's 16384, and the streams took turns.  40
+// products of 16384 x 4096 x 4096 (14.1 ms) with 40 reductions of 64 M gradients (5.8 ms) 20.4 ms at 168 registers, 18.5 ms so;
+// with 40 AdamW updates of 64 M (8.8 ms) 25.2 and 21.0 ms.  The products alone take the same time: the epilogue handles 32
+// columns of its 64 after the other 32.
+// The gated-FFN backward and the grouped weight gradient, which are bound by their epilogues, keep 168: at 128 they took 2 to 4 %
+// longer (9377 x 3072 x 1024: 101 to 103 us, 103 to 105 at 128).
+template <int EPI, int GROUPED>
+constexpr int GEMM2_BOUND = EPI == 2 || GROUPED == 2 ? 64 + 32 * EPI2_WARPS : 512;
 
 // The accumulator comes out of tensor memory one row per thread.  Stored (or read, for C) from there, an instruction touches
 // 32 rows with 16 bytes of each: 32 passes of the load / store unit, some 4100 cycles for each 128 x 256 bf16 tile and
@@ -820,7 +831,7 @@ __device__ __forceinline__ void glu_act_grad(float g, int kind, float& a, float&
 //      writes dgate, dup into D (M x 2F) and the re-emitted activation into glu_act; dact never reaches memory
 //      (flextrain/ops/_kernels/swiglu.py:46-100 reads it back from HBM).
 template <bool A_MN, bool B_MN, int EPI = 0, int GROUPED = 0>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI2_WARPS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM2_BOUND<EPI, GROUPED>, 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1127,9 +1138,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
         for (int c = c0; c < c1; c += step) {
           const int col = tn * BN2 + c;
           if (col >= p.N) break;
-          uint32_t r0[32], r1[32];                     // (32 fp32 columns need the first only)
-          tmem_ld_32x32(taddr + c, r0);
-          if (!p.d_fp32) tmem_ld_32x32(taddr + c + 32, r1);
+          uint32_t r[32];
+          tmem_ld_32x32(taddr + c, r);
           if (p.beta != 0.f) {
             T8::put(buf, cv, lane);
             if (c + step < c1 && col + step < p.N)
@@ -1180,8 +1190,12 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
               }
             }
           };
-          finish(r0, 0);
-          if (!p.d_fp32) finish(r1, 32);
+          finish(r, 0);
+          if (!p.d_fp32) {                             // (32 fp32 columns are a whole piece)
+            tmem_ld_32x32(taddr + c + 32, r);
+            tmem_ld_wait();
+            finish(r, 32);
+          }
           __syncwarp();
           T8::store(buf, drow + static_cast<size_t>(col) * es, static_cast<size_t>(p.ldd) * es, rows, pieces_at(col), lane);
           __syncwarp();

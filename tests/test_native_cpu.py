@@ -388,3 +388,22 @@ def test_hand_built_working_set_in_the_reference_form():
                         max_global_batch_tokens=256, max_gpu_mem_bytes=8 << 30, max_host_mem_bytes=16 << 30,
                         device="cpu", plan_only=True)
     assert plan.available_gpu_memory_bytes == 8 << 30 and plan.available_host_memory_bytes == 16 << 30
+
+
+def test_a_collective_fits_beside_the_two_sm_gemm():
+    """A block of 256 threads of the collectives' kernels or of AdamW has the registers it needs on an SM whose GEMM block (ten
+    warps; the gated-FFN backward and the grouped weight gradient apart, which hold more) is running: each of the four partitions has 16384, for up to three warps of the GEMM and two of the other, in steps of
+    8 a thread."""
+    import re
+    from flextrain_b200 import build
+    regs = {}
+    for lib in ("gemm_tcgen05", "comm", "elementwise"):
+        log = build.LIB / f"{lib}.ptxas.log"
+        if not log.exists():
+            pytest.skip("the library was not built here")
+        for name, n in re.findall(r"Compiling entry function '(\S+)'.*?Used (\d+) registers", log.read_text(), re.S):
+            regs[name] = (int(n) + 7) // 8 * 8
+    gemm = [n for k, n in regs.items() if "gemm2_kernel" in k and "ELi2E" not in k]
+    beside = [n for k, n in regs.items() if any(w in k for w in ("reduce_scatter", "push_kernel", "12adamw_kernel"))]
+    assert len(gemm) == 7 and len(beside) >= 4
+    assert 32 * (3 * max(gemm) + 2 * max(beside)) <= 16384
