@@ -135,8 +135,8 @@ __global__ void conv1d_bwd_dx_kernel(const float* __restrict__ dpre, const bf16*
 // The general kernels above read each input W times, two bytes a lane, and look the sequence of every token up; they stay for
 // other widths, odd channel counts and unaligned rows.  A block that holds tokens before the first sequence or after the last
 // (padding) looks its tokens up one by one, as in the general kernels: tested for each token, that cost the other blocks 15 %,
-// and 10 % where it took the backward above 96 registers, so it has functions of its own there.  Bound by memory.  16384 tokens x 8192 channels, W = 4: forward 833 us before, 170 us so; dpre 1240 us before, 314 us so; dx
-// 930 us before, 154 us so.
+// and 10 % where it took the backward above 96 registers, so it has functions of its own there.  Bound by memory.  16384 tokens
+// x 8192 channels, W = 4: forward 833 us before, 170 us so; dpre 1240 us before, 314 us so; dx 930 us before, 154 us so.
 constexpr int CONV_GROUP = 8;
 __device__ __forceinline__ float2 ld2(const bf16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
 
