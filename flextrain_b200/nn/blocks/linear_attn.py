@@ -15,8 +15,9 @@ The only tensors kept per chunk are the boundary states, which is the reference'
 Two implementations of the same math:
 
 * **CUDA (bf16)**: hand-written forward and backward, no autograd: tcgen05 GEMMs for the projections, the conv1d /
-  L2-norm / gated-RMSNorm kernels of ``csrc/seqmix.cu`` and the recurrent delta-rule kernels of ``csrc/gdn.cu``
-  (forward pass; backward = one reverse pass for the state adjoint + one forward-direction pass for the
+  L2-norm / gated-RMSNorm kernels of ``csrc/seqmix.cu`` and the delta-rule kernels of ``csrc/gdn_chunk.cu``
+  (heads of 128 x 128, in chunks on the tensor cores) or ``csrc/gdn.cu`` (other sizes, token by token; backward = one reverse
+  pass for the state adjoint + one forward-direction pass for the
   state-dependent terms; the gate gradient is a suffix sum of per-token scalars).
 * **Reference (any device / dtype)**: the fp32 PyTorch formulation under autograd; it is the CPU path and the oracle
   the CUDA path is tested against.  ``FTB_GDN_BACKEND=reference`` forces it.
@@ -131,7 +132,7 @@ class GatedDeltaNetBlock:
         qkv_c, conv_fin = la.conv1d_fwd(qkv, p["w_lin_conv"], cu, conv_in, activation=True)
         qn, q_rn = la.l2norm_heads_fwd(qkv_c[:, : c.key_dim], c.n_k_heads, c.head_k_dim)
         kn, k_rn = la.l2norm_heads_fwd(qkv_c[:, c.key_dim: 2 * c.key_dim], c.n_k_heads, c.head_k_dim)
-        v = qkv_c[:, 2 * c.key_dim:].contiguous().view(T, c.n_v_heads, c.head_v_dim)
+        v = qkv_c[:, 2 * c.key_dim:].unflatten(1, (c.n_v_heads, c.head_v_dim))
         # gates in one launch straight from the bf16 projection (flextrain/ops/_kernels/gate_prep.py:29-80)
         beta, g = la.gate_prep_fwd(ba.contiguous(), p["w_lin_dt_bias"].to(f32), p["w_lin_A_log"].to(f32))
         o, fin, r = la.gdn_fwd(qn, kn, v, g, beta, cu, state_in, want_r=want_r)
@@ -167,16 +168,16 @@ class GatedDeltaNetBlock:
                                    params["w_lin_norm"].to(f32), dqkvz[:, c.conv_dim:], dwn, c.n_v_heads,
                                    c.head_v_dim, c.norm_eps)
         acc("g_lin_norm", dwn)
-        # ---- recurrence
-        dq, dk, dv, dg, dbeta, dstate_in = la.gdn_bwd(s["qn"], s["kn"], s["v"], s["g"], s["beta"], cu, ctx.lin_state_in,
-                                                      s["fin"], s["r"], d_o, dstate_final=ctx.lin_dstate_in)
-        # ---- L2 norms and conv
+        # ---- recurrence (dv straight into its columns)
         dqkv_c = torch.empty(T, c.conv_dim, dtype=h.dtype, device=h.device)
+        dq, dk, _, dg, dbeta, dstate_in = la.gdn_bwd(s["qn"], s["kn"], s["v"], s["g"], s["beta"], cu, ctx.lin_state_in, s["fin"],
+                                                     s["r"], d_o, dstate_final=ctx.lin_dstate_in,
+                                                     dv_out=dqkv_c[:, 2 * c.key_dim:].unflatten(1, (c.n_v_heads, c.head_v_dim)))
+        # ---- L2 norms and conv
         la.l2norm_heads_bwd(dq.contiguous(), s["qkv_c"][:, : c.key_dim], s["q_rn"], dqkv_c[:, : c.key_dim],
                             c.n_k_heads, c.head_k_dim)
         la.l2norm_heads_bwd(dk.contiguous(), s["qkv_c"][:, c.key_dim: 2 * c.key_dim], s["k_rn"],
                             dqkv_c[:, c.key_dim: 2 * c.key_dim], c.n_k_heads, c.head_k_dim)
-        dqkv_c[:, 2 * c.key_dim:].copy_(dv.view(T, c.value_dim))
         dwc = torch.zeros(c.conv_dim, c.conv_width, dtype=f32, device=h.device)
         dconv_in = la.conv1d_bwd(s["qkvz"][:, : c.conv_dim], params["w_lin_conv"], cu, ctx.lin_conv_in, dqkv_c,
                                  ctx.lin_dconv_in, dqkvz[:, : c.conv_dim], dwc, want_dinit=ctx.lin_conv_in is not None)

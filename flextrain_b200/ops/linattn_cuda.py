@@ -143,9 +143,25 @@ def _gdn(pass_, q, k, v, g, beta, cu, state_in, state_out, o, r, d_o, de, dv, db
     _check(rc, f"ftb_gdn(pass {pass_})")
 
 
+def _chunked(q: torch.Tensor, v: torch.Tensor, *rest: torch.Tensor) -> bool:
+    """Heads of 128 x 128 on 16 bytes run in chunks on the tensor cores (``csrc/gdn_chunk.cu``); see there for the figures."""
+    return q.shape[2] == 128 and v.shape[2] == 128 and all(t.data_ptr() % 16 == 0 for t in (q, v, *rest))
+
+
+def _head_rows(x: torch.Tensor) -> bool:
+    """``(T, H, D)`` with the heads of a token side by side: a view of a wider projection, or contiguous."""
+    return x.stride(2) == 1 and x.stride(1) == x.shape[2] and x.stride(0) % 8 == 0
+
+
+def _chunk_work(T: int, S: int, HV: int, device) -> torch.Tensor:
+    lib = load("gdn_chunk")
+    lib.ftb_gdn_chunk_bytes.restype = c_long
+    return torch.empty(lib.ftb_gdn_chunk_bytes(c_long(T), c_int(S), c_int(HV)), dtype=torch.uint8, device=device)
+
+
 def gdn_fwd(q, k, v, g, beta, cu, state_in=None, scale=None, want_r=False):
-    """``q,k (T,HK,dk)``, ``v (T,HV,dv)`` bf16 contiguous; ``g, beta (T,HV)`` fp32; ``state_in (S,HV,dk,dv)`` fp32.
-    Returns ``(o (T,HV,dv) bf16, final_state fp32, r or None)``."""
+    """``q,k (T,HK,dk)``, ``v (T,HV,dv)`` bf16 contiguous (``v`` may be a view of a wider projection); ``g, beta (T,HV)`` fp32;
+    ``state_in (S,HV,dk,dv)`` fp32.  Returns ``(o (T,HV,dv) bf16, final_state fp32, r or None)``."""
     T, HK, DK = q.shape
     HV, DV = v.shape[1], v.shape[2]
     S = cu.numel() - 1
@@ -154,39 +170,62 @@ def gdn_fwd(q, k, v, g, beta, cu, state_in=None, scale=None, want_r=False):
     fin = torch.empty(S, HV, DK, DV, dtype=F32, device=q.device)
     r = torch.empty(T, HV, DV, dtype=F32, device=q.device) if want_r else None
     sin = state_in.to(F32).contiguous() if state_in is not None else None
-    _gdn(0, q, k, v, g, beta, cu, sin, fin, o, r, None, None, None, None, None, None, None, scale)
+    if _chunked(q, v, k) and _head_rows(v):
+        work = _chunk_work(T, S, HV, q.device)
+        rc = load("gdn_chunk").ftb_gdn_chunk_fwd(
+            _ptr(q), _ptr(k), _ptr(v), c_long(v.stride(0)), _ptr(g), _ptr(beta), _ptr(cu), c_int(S), c_long(T), _ptr(sin), _ptr(fin),
+            _ptr(o), _ptr(r), _ptr(work), c_int(HK), c_int(HV), c_float(scale), _stream())
+        _check(rc, "ftb_gdn_chunk_fwd")
+        return o, fin, r
+    _gdn(0, q, k, v.contiguous(), g, beta, cu, sin, fin, o, r, None, None, None, None, None, None, None, scale)
     return o, fin, r
 
 
-def gdn_bwd(q, k, v, g, beta, cu, state_in, final_state, r, d_o, dstate_final=None, scale=None):
+def gdn_bwd(q, k, v, g, beta, cu, state_in, final_state, r, d_o, dstate_final=None, scale=None, dv_out=None,
+            sum_heads=True):
     """Backward of :func:`gdn_fwd`.  Returns ``(dq (T,HK,dk) fp32, dk (T,HK,dk) fp32, dv (T,HV,dv) bf16,
-    dg (T,HV) fp32, dbeta (T,HV) fp32, dstate_in (S,HV,dk,dv) fp32)``.  The sequences of ``cu`` have to cover all T tokens:
-    the library's error word (``device_error_words``) reports it when they do not."""
+    dg (T,HV) fp32, dbeta (T,HV) fp32, dstate_in (S,HV,dk,dv) fp32)``.  ``dv_out``: where to write ``dv`` (a view of a wider
+    tensor, its heads side by side).  ``sum_heads=False`` leaves ``dq`` and ``dk`` per value head, ``(T,HV,dk)``.  The
+    sequences of ``cu`` have to cover all T tokens: the library's error word (``device_error_words``) reports it when they do
+    not."""
     T, HK, DK = q.shape
     HV, DV = v.shape[1], v.shape[2]
     S = cu.numel() - 1
     rep = HV // HK
     scale = scale if scale is not None else DK ** -0.5
     dev = q.device
-    de = torch.empty(T, HV, DV, dtype=F32, device=dev)
-    dv = torch.empty(T, HV, DV, dtype=BF, device=dev)
-    dbeta = torch.zeros(T, HV, dtype=F32, device=dev)
-    dk_hv = torch.zeros(T, HV, DK, dtype=F32, device=dev)
-    s = torch.zeros(T, HV, dtype=F32, device=dev)
-    dstate_in = torch.empty(S, HV, DK, DV, dtype=F32, device=dev)
     dsf = dstate_final.to(F32).contiguous() if dstate_final is not None else None
-    d_o = d_o.contiguous()
-    _gdn(1, q, k, v, g, beta, cu, dsf, dstate_in, None, r, d_o, de, dv, dbeta, None, dk_hv, s, scale)
-    dq_hv = torch.zeros(T, HV, DK, dtype=F32, device=dev)
     sin = state_in.to(F32).contiguous() if state_in is not None else None
-    _gdn(2, q, k, v, g, beta, cu, sin, None, None, None, d_o, de, None, None, dq_hv, dk_hv, s, scale)
+    d_o = d_o.contiguous()
+    chunked = _chunked(q, v, k, r, d_o) and _head_rows(v)
+    new = torch.empty if chunked and S > 0 else torch.zeros          # (the recurrent kernels add into these)
+    de = torch.empty(T, HV, DV, dtype=F32, device=dev)
+    dv = dv_out
+    if dv is None or not (chunked and _head_rows(dv) and dv.data_ptr() % 16 == 0):
+        dv = torch.empty(T, HV, DV, dtype=BF, device=dev)
+    dbeta, s = (new(T, HV, dtype=F32, device=dev) for _ in range(2))
+    dq_hv, dk_hv = (new(T, HV, DK, dtype=F32, device=dev) for _ in range(2))
+    dstate_in = torch.empty(S, HV, DK, DV, dtype=F32, device=dev)
+    if chunked:
+        work = _chunk_work(T, S, HV, dev)
+        rc = load("gdn_chunk").ftb_gdn_chunk_bwd(
+            _ptr(q), _ptr(k), _ptr(v), c_long(v.stride(0)), _ptr(g), _ptr(beta), _ptr(cu), c_int(S), c_long(T), _ptr(sin), _ptr(dsf),
+            _ptr(dstate_in), _ptr(r), _ptr(d_o), _ptr(de), _ptr(dv), c_long(dv.stride(0)), _ptr(dbeta), _ptr(dq_hv), _ptr(dk_hv),
+            _ptr(s), _ptr(work), c_int(HK), c_int(HV), c_float(scale), _stream())
+        _check(rc, "ftb_gdn_chunk_bwd")
+    else:
+        v = v.contiguous()
+        _gdn(1, q, k, v, g, beta, cu, dsf, dstate_in, None, r, d_o, de, dv, dbeta, None, dk_hv, s, scale)
+        _gdn(2, q, k, v, g, beta, cu, sin, None, None, None, d_o, de, None, None, dq_hv, dk_hv, s, scale)
+    if dv_out is not None and dv is not dv_out:
+        dv = dv_out.copy_(dv)
     # dg_t = sum_{u >= t, same sequence} s_u  (+ <dS_final, S_final>), with the per-token scalar
     # s_u = q_u.dq_u - k_u.(dS'_u e_u) + k_u.(S^_u dr_u) accumulated by the two passes
     extra = (dsf * final_state.to(F32)).sum((-1, -2)).contiguous() if dstate_final is not None else None     # (S, HV)
     dg = torch.zeros(T, HV, dtype=F32, device=dev)
     _check(load("gdn").ftb_gate_sum(_ptr(s), _ptr(extra), _ptr(cu), c_int(S), c_int(T), _ptr(dg), c_int(HV), _stream()),
            "ftb_gate_sum")
-    if rep > 1:
+    if rep > 1 and sum_heads:
         dq = dq_hv.view(T, HK, rep, DK).sum(2)
         dk = dk_hv.view(T, HK, rep, DK).sum(2)
     else:
