@@ -14,6 +14,9 @@
 //
 // A grouped variant (one launch for all experts of an MoE layer, tile list built on the device
 // from the expert offsets) shares the same pipeline; see ftb_grouped_gemm_bf16.
+#include <map>
+#include <mutex>
+
 #include "ptx.cuh"
 
 namespace ftb {
@@ -24,6 +27,9 @@ constexpr int UMMA_K = 16;
 constexpr int NUM_THREADS = 256;   // warps 0-5: TMA / MMA / epilogue; warps 6-7: peer-panel pull (TP all-gather mode)
 constexpr int MAX_RANKS = 8;
 constexpr int GROUP_M = 16;  // tile rasterisation: GROUP_M row-tiles share a sweep over N (L2 reuse)
+constexpr int GROUP2_M = 8;  // the same, in 256 rows, where the two-SM kernel gives out tiles by die, see TilesOfPair
+
+constexpr int MAX_PAIRS = 80;
 
 struct GemmParams {
   int M, N, K;
@@ -41,6 +47,9 @@ struct GemmParams {
   // split-K (plain mode only): the K range is cut into split_k slices of k_per_split elements; slice s of every output
   // tile is a work item of its own and lands in D + s * M * ldd (an fp32 workspace), to be summed by splitk_reduce.
   int split_k, k_per_split;
+  // two-SM kernel: which tiles a pair takes, see TilesOfPair
+  int die_pairs;             // pairs of SMs on the first die; 0: pairs take tiles in the order of their blocks
+  unsigned char pair_of[MAX_PAIRS];
   // gated-FFN epilogues of the two-SM kernel (EPI 1 / 2, see gemm2_kernel)
   int glu_F, glu_kind;       // F = ffn width (columns of one half); kind 0 SwiGLU, 1 GeGLU(tanh)
   void* glu_act;             // (M, F) bf16: activation output
@@ -88,11 +97,11 @@ constexpr int RS_STAGE_BYTES = 4 * 32 * 256;
 // All-gather mode: two shared-memory buffers of this size carry the remote panels (peer -> shared -> local staging).
 constexpr int PULL_CHUNK_BYTES = 16384;
 
-__device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
-  const int per_group = GROUP_M * tiles_n;
+__device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& tm, int& tn, int GM = GROUP_M) {
+  const int per_group = GM * tiles_n;
   const int g = tile / per_group;
-  const int first_m = g * GROUP_M;
-  const int gm = min(GROUP_M, tiles_m - first_m);
+  const int first_m = g * GM;
+  const int gm = min(GM, tiles_m - first_m);
   const int r = tile - g * per_group;
   tm = first_m + r % gm;
   tn = r / gm;
@@ -745,15 +754,22 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
 // (tcgen05.commit); loads are plain tiled TMA loads credited to the leader's barrier (no cluster multicast loads).
 // =====================================================================================================
 constexpr int BN2 = 256;
-constexpr int STAGE2_BYTES = 2 * BM * BK * 2;   // A (128 x 64) + B half (128 x 64)
-// Eight epilogue warps: two for each quadrant of the accumulator's rows, with half of the columns each.  Their staging takes
-// a stage of the operand ring where the gated-FFN epilogues need three buffers.
+constexpr int DIES_K = 4096, WIDE_K = 8192;     // from these K on: tiles by die (TilesOfPair), tiles of 512 x 256 (Ring2)
+// Eight epilogue warps: two for each quadrant of the accumulator's rows, with half of the columns each.
 constexpr int EPI2_WARPS = 8;
-template <int EPI>
+// TM = 2: a tile of 512 x 256, 256 rows of A for each CTA.  A byte of B then serves twice the rows: 96 KB per 64 of K and
+// 512 x 256 outputs where two tiles of 256 x 256 take 128 KB, out of L2 and into shared memory, and that is power the tensor
+// cores get (see TilesOfPair).  The two accumulators of a tile fill tensor memory, so reading them out overlaps the next tile
+// by four steps of K only; it pays from K = 8192 on, and where the tile costs no wave.  Sustained TFLOP/s of products at the power limit,
+// in the order of blocks: 8192^3 1217 -> 1300, 16384 x 4096 x 14336 1228 -> 1293, input gradients 16384 x 4096 x 28672 1166 ->
+// 1274, 4096 x 4096 x 128256 1116 -> 1295, weight gradient 28672 x 4096 x 16384 1135 -> 1155; at K = 4096 no gain (1298, 1296).
+template <int EPI, int TM>
 struct Ring2 {
-  static constexpr int STAGES = EPI == 0 ? 6 : 5;
+  static constexpr int STAGES = TM == 2 ? 4 : EPI == 0 ? 6 : 5;
+  static constexpr int A_BYTES = TM * BM * BK * 2;                       // A (TM x 128 rows x 64)
+  static constexpr int STAGE_BYTES = A_BYTES + BM * BK * 2;              // + B half (128 x 64)
   static constexpr int WARP_BYTES = EPI == 0 ? 32 * 128 : 3 * 32 * 64;
-  static constexpr int TOTAL = STAGES * STAGE2_BYTES + EPI2_WARPS * WARP_BYTES + 256 + 1024;
+  static constexpr int TOTAL = STAGES * STAGE_BYTES + EPI2_WARPS * WARP_BYTES + 256 + 1024;
   // of the SM's 228 KB, of which every block takes 1 KB: one more block without shared memory has room
   static_assert(TOTAL + 2 * 1024 <= 228 * 1024, "shared memory of a CTA and of a block beside it");
 };
@@ -806,6 +822,43 @@ struct Turn {
 };
 
 
+// Which tiles a pair of SMs takes.  The GPU is two dies, each with its own half of L2: a panel of an operand crosses the link
+// between them once for each die whose SMs read it, and again whenever it has left that half.  Blocks are dealt out in the
+// order of SM numbers, which alternates between the dies, so that with consecutive tiles on consecutive blocks every panel of a
+// wave went to both.  The host measures once which pair is on which die (measure_dies) and numbers the pairs die by die; each
+// die works through a contiguous half of the tiles, 2048 rows at a time, where a wave of its 37 pairs reads few panels.
+//
+// A product runs at the power limit, and what its panels cost in power the tensor cores do not get (the same kernels reach
+// 2140 TFLOP/s on zeros).  16384 x 4096 x 14336 with 256 x 256 tiles: 3.7 -> 2.5 GB from memory, 118 -> 73 M sectors between the
+// dies.  Sustained TFLOP/s, blocks in order and groups of 4096 rows / so, tiles of 512 x 256 from K = 8192 on both times: 8192^3
+// 1300 / 1382; 16384 x 4096 x 14336 1293 / 1367; input gradient 16384 x 4096 x 28672 1274 / 1363; weight gradients 28672 x 4096 x
+// 16384 1155 / 1245, 128256 x 4096 x 4096 1176 / 1248; 16384 x 6144 x 4096 1298 / 1330; gated FFN forward 16384 x 14336 x 4096
+// 1257 / 1302.  (Another GPU, with 35 and 39 pairs on its dies: 2 to 4 % more.)  Groups of 1536 or 2560 rows: 2 to 6 % less.
+// Short products, below K = 4096, are bound by their outputs and keep the order of blocks, as do the experts' tiles, which
+// differ in length.
+struct TilesOfPair {
+  int first, step, end;
+  int rows;                                      // row tiles that share a sweep over N
+  __device__ __forceinline__ TilesOfPair(const GemmParams& p, int num_tiles, int group) {
+    const int n = gridDim.x >> 1;
+    first = blockIdx.x >> 1;
+    step = n;
+    end = num_tiles;
+    rows = p.die_pairs ? group : GROUP_M;
+    if (p.die_pairs == 0) return;
+    first = p.pair_of[first];
+    if (num_tiles < 2 * n) return;
+    const int half = static_cast<int>(static_cast<long>(num_tiles) * p.die_pairs / n);
+    if (first < p.die_pairs) {
+      end = half;
+      step = p.die_pairs;
+    } else {
+      first += half - p.die_pairs;
+      step = n - p.die_pairs;
+    }
+  }
+};
+
 // act(g) and d act / d g of the gate activation (same formulas as the stand-alone SwiGLU / GeGLU kernels)
 __device__ __forceinline__ void glu_act_grad(float g, int kind, float& a, float& da) {
   if (kind == 0) {
@@ -830,14 +883,16 @@ __device__ __forceinline__ void glu_act_grad(float g, int kind, float& a, float&
 //   2  gated-FFN backward.  The accumulator is dact = dy · W_down; the epilogue reads the saved gate / up values and
 //      writes dgate, dup into D (M x 2F) and the re-emitted activation into glu_act; dact never reaches memory
 //      (flextrain/ops/_kernels/swiglu.py:46-100 reads it back from HBM).
-template <bool A_MN, bool B_MN, int EPI = 0, int GROUPED = 0>
+template <bool A_MN, bool B_MN, int EPI = 0, int GROUPED = 0, int TM = 1>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM2_BOUND<EPI, GROUPED>, 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  constexpr int ST2 = Ring2<EPI>::STAGES;
-  uint8_t* smem_epi = smem + ST2 * STAGE2_BYTES;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem_epi + EPI2_WARPS * Ring2<EPI>::WARP_BYTES);
+  using R2 = Ring2<EPI, TM>;
+  static_assert(TM == 1 || (EPI == 0 && GROUPED == 0), "wide tiles: plain products");
+  constexpr int ST2 = R2::STAGES, TILE_M = 2 * TM * BM;
+  uint8_t* smem_epi = smem + ST2 * R2::STAGE_BYTES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem_epi + EPI2_WARPS * R2::WARP_BYTES);
   uint64_t* empty_bar = full_bar + ST2;
   uint64_t* tfull_bar = empty_bar + ST2;
   uint64_t* tempty_bar = tfull_bar + 2;
@@ -847,7 +902,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();
   const bool leader = cta == 0;
-  const int tiles_m = (p.M + 2 * BM - 1) / (2 * BM);
+  const int tiles_m = (p.M + TILE_M - 1) / TILE_M;
   const int tiles_n = EPI == 1 ? p.glu_F / (BN2 / 2) : (p.N + BN2 - 1) / BN2;
   // split K (plain form): slice sp of the reduction of every tile is a tile of its own, written to slab sp of D
   const bool split = EPI == 0 && GROUPED == 0 && p.split_k > 1;
@@ -855,7 +910,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                                                                   : tiles_m * tiles_n * (split ? p.split_k : 1);
   auto slice_blocks = [&](int sp) { return (min(p.K - sp * p.k_per_split, p.k_per_split) + BK - 1) / BK; };
   int k_blocks = (p.K + BK - 1) / BK;              // (grouped weight gradients: of the tile's group)
-  const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+  const TilesOfPair mine(p, num_tiles, GROUP2_M / TM);
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -881,7 +936,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       uint32_t phase = 0;
       bool ok = true;
       [[maybe_unused]] GroupWalk walk;
-      for (int tile = pair; tile < num_tiles && ok; tile += n_pairs) {
+      for (int tile = mine.first; tile < mine.end && ok; tile += mine.step) {
         int tm, tn, g = 0, row0, left, k_lo = 0;
         if constexpr (GROUPED == 1) {
           if (!walk.rows(p.offsets, p.num_groups, 2 * BM, tiles_n, tile, g, row0, left, tn)) break;
@@ -899,24 +954,25 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
             k_lo = sp * p.k_per_split;
             k_blocks = slice_blocks(sp);
           }
-          tile_coords(t, tiles_m, tiles_n, tm, tn);
-          row0 = tm * 2 * BM;
+          tile_coords(t, tiles_m, tiles_n, tm, tn, mine.rows);
+          row0 = tm * TILE_M;
         }
-        row0 += static_cast<int>(cta) * BM;                             // this CTA's 128 rows of A
+        row0 += static_cast<int>(cta) * (TM * BM);                      // this CTA's rows of A
         // this CTA's half of B's N rows (gated forward: 128 gate rows for CTA 0, the matching up rows for CTA 1)
         const int col0 = EPI == 1 ? tn * (BN2 / 2) + static_cast<int>(cta) * p.glu_F
                                   : tn * BN2 + static_cast<int>(cta) * (BN2 / 2);
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (!(ok = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, 50))) break;
-          uint8_t* sa = smem + stage * STAGE2_BYTES;
-          uint8_t* sb = sa + BM * BK * 2;
-          if (leader) mbar_expect_tx(&full_bar[stage], 2 * STAGE2_BYTES);
+          uint8_t* sa = smem + stage * R2::STAGE_BYTES;
+          uint8_t* sb = sa + R2::A_BYTES;
+          if (leader) mbar_expect_tx(&full_bar[stage], 2 * R2::STAGE_BYTES);
           const int k0 = k_lo + kb * BK;
           if constexpr (!A_MN) {
-            tma_load_2d_2cta(sa, &tmA, &full_bar[stage], k0, row0);
+#pragma unroll
+            for (int h = 0; h < TM; ++h) tma_load_2d_2cta(sa + h * (BM * BK * 2), &tmA, &full_bar[stage], k0, row0 + h * BM);
           } else {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j) tma_load_2d_2cta(sa + j * (64 * BK * 2), &tmA, &full_bar[stage], row0 + j * 64, k0);
+            for (int j = 0; j < TM * BM / 64; ++j) tma_load_2d_2cta(sa + j * (64 * BK * 2), &tmA, &full_bar[stage], row0 + j * 64, k0);
           }
           if constexpr (GROUPED == 1 && !B_MN) {
             tma_load_3d_2cta(sb, &tmB, &full_bar[stage], k0, col0, g);
@@ -943,7 +999,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       uint32_t acc_phase = 0;
       bool ok = true;
       [[maybe_unused]] GroupWalk walk;
-      for (int tile = pair; tile < num_tiles && ok; tile += n_pairs) {
+      for (int tile = mine.first; tile < mine.end && ok; tile += mine.step) {
         if constexpr (GROUPED == 1) {
           int g, row0, left, tn;
           if (!walk.rows(p.offsets, p.num_groups, 2 * BM, tiles_n, tile, g, row0, left, tn)) break;
@@ -954,14 +1010,11 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
           if (k_blocks == 0) continue;
         }
         if (split) k_blocks = slice_blocks(tile / (tiles_m * tiles_n));
-        if (!(ok = mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag, 60))) break;
-        tc_fence_after();
-        const uint32_t tmem_d = tmem_base + acc * BN2;
-        for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!(ok = mbar_wait(&full_bar[stage], phase, abort_flag, 61))) break;
-          tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * STAGE2_BYTES);
-          const uint32_t sb = sa + BM * BK * 2;
+        // the four steps of a stage for the upper (h = 0) or lower 128 rows of each CTA's A
+        auto multiply = [&](int st, int kb, int h) {
+          const uint32_t sa = smem_u32(smem + st * R2::STAGE_BYTES) + h * (BM * BK * 2);
+          const uint32_t sb = smem_u32(smem + st * R2::STAGE_BYTES) + R2::A_BYTES;
+          const uint32_t tmem_d = tmem_base + (TM == 2 ? h : acc) * BN2;
 #pragma unroll
           for (int kk = 0; kk < BK / UMMA_K; ++kk) {
             const uint64_t ad = A_MN ? make_smem_desc(sa + kk * (UMMA_K * 128), 64 * BK * 2, 1024)
@@ -970,23 +1023,54 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                                      : make_smem_desc(sb + kk * (UMMA_K * 2), 16, 1024);
             umma_f16_2cta(tmem_d, ad, bd, idesc, (kb | kk) != 0);
           }
+        };
+        if (!(ok = mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag, 60))) break;
+        tc_fence_after();
+        int kb = 0;
+        if constexpr (TM == 2) {
+          // The tile fills tensor memory.  Its upper half is read out first: as many steps as the ring holds start on that half
+          // while the lower one is still being read.
+          const int ahead = min(ST2, k_blocks), stage0 = stage;
+          const uint32_t phase0 = phase;
+          int st = stage0;
+          uint32_t ph = phase0;
+          for (int i = 0; i < ahead; ++i) {
+            if (!(ok = mbar_wait(&full_bar[st], ph, abort_flag, 61))) break;
+            tc_fence_after();
+            multiply(st, i, 0);
+            if (++st == ST2) { st = 0; ph ^= 1; }
+          }
+          if (!ok || !(ok = mbar_wait(&tempty_bar[1], acc_phase ^ 1, abort_flag, 62))) break;
+          tc_fence_after();
+          for (; kb < ahead; ++kb) {
+            multiply(stage, kb, 1);
+            umma_commit_2cta(&empty_bar[stage], 3);
+            if (++stage == ST2) { stage = 0; phase ^= 1; }
+          }
+        }
+        for (; kb < k_blocks; ++kb) {
+          if (!(ok = mbar_wait(&full_bar[stage], phase, abort_flag, 61))) break;
+          tc_fence_after();
+#pragma unroll
+          for (int h = 0; h < TM; ++h) multiply(stage, kb, h);
           umma_commit_2cta(&empty_bar[stage], 3);   // frees this stage in both CTAs
           if (++stage == ST2) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
         umma_commit_2cta(&tfull_bar[acc], 3);       // accumulator ready in both CTAs
-        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        if (TM == 2) acc_phase ^= 1;
+        else if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
   } else {
     const int quad = warp & 3;
     const int part = (warp - 2) >> 2;                  // which half of the columns
-    uint8_t* buf = smem_epi + (warp - 2) * Ring2<EPI>::WARP_BYTES;
+    uint8_t* buf = smem_epi + (warp - 2) * R2::WARP_BYTES;
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
     [[maybe_unused]] GroupWalk walk;
-    for (int tile = pair; tile < num_tiles && ok; tile += n_pairs) {
+    for (int tile = mine.first; tile < mine.end && ok; tile += mine.step) {
       int tm, tn, row0, left;
       uint8_t* d_base = reinterpret_cast<uint8_t*>(p.D);
       const uint8_t* c_base = reinterpret_cast<const uint8_t*>(p.C);
@@ -1007,15 +1091,17 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
           t -= sp * tiles_m * tiles_n;
           d_base += static_cast<size_t>(sp) * p.M * p.ldd * 4;         // fp32 slabs
         }
-        tile_coords(t, tiles_m, tiles_n, tm, tn);
-        row0 = tm * 2 * BM;
+        tile_coords(t, tiles_m, tiles_n, tm, tn, mine.rows);
+        row0 = tm * TILE_M;
         left = p.M - row0;
       }
+#pragma unroll 1
+      for (int h = 0; h < TM && ok; ++h) {
       // this warp's 32 rows, and how many of them are rows of the result
-      const int first = static_cast<int>(cta) * BM + quad * 32;
+      const int first = static_cast<int>(cta) * (TM * BM) + h * BM + quad * 32;
       const int rows = max(0, min(32, left - first));
       const size_t row = static_cast<size_t>(row0 + first);
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN2;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + (TM == 2 ? h : acc) * BN2;
       if constexpr (EPI == 1) {
         using T4 = Turn<4>;
         if (!(ok = mbar_wait(&tfull_bar[acc], acc_phase, abort_flag, 70))) break;
@@ -1203,8 +1289,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_leader(&tempty_bar[acc]);   // the warps of both CTAs release the accumulator
-      if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+      if (lane == 0) mbar_arrive_leader(&tempty_bar[TM == 2 ? h : acc]);   // the warps of both CTAs release the accumulator
+      }
+      if (TM == 2) acc_phase ^= 1;
+      else if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
   }
 
@@ -1217,18 +1305,134 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   }
 }
 
-template <bool A_MN, bool B_MN, int EPI = 0, int GROUPED = 0>
+// ------------------------------------------------------------------------------------------------ dies
+// Latency of atomics on 32 words spread over memory, from one SM of every pair: a word's home is on one of the dies, and its
+// latency from there is some 270 cycles, from the other 650.  Pairs with the same pattern are on the same die.
+constexpr int PROBE_WORDS = 32, PROBE_STRIDE = 4096;                       // 16 KB apart
+static __device__ unsigned g_probe_word[PROBE_WORDS * PROBE_STRIDE];
+static __device__ float g_probe_cycles[MAX_PAIRS * PROBE_WORDS];
+
+__global__ void __cluster_dims__(2, 1, 1) die_probe_kernel() {
+  if (threadIdx.x != 0 || (blockIdx.x & 1)) return;
+  for (int a = 0; a < PROBE_WORDS; ++a) {
+    unsigned* w = g_probe_word + a * PROBE_STRIDE;
+    unsigned v, zero = 0;                                                  // (each atomic waits for the one before)
+    long long t0 = 0, t1;
+    for (int i = 0; i < 20; ++i) {
+      if (i == 4) asm volatile("mov.u64 %0, %%clock64;" : "=l"(t0) : "r"(zero) : "memory");
+      asm volatile("atom.relaxed.gpu.global.add.u32 %0, [%1], %2;" : "=r"(v) : "l"(w), "r"(zero) : "memory");
+      zero = v >> 31;
+    }
+    asm volatile("mov.u64 %0, %%clock64;" : "=l"(t1) : "r"(zero) : "memory");
+    g_probe_cycles[(blockIdx.x >> 1) * PROBE_WORDS + a] = static_cast<float>(t1 - t0);
+  }
+}
+
+struct DieMap {
+  int pairs = 0, first_die = 0;                 // first_die = 0: not known, or not two dies
+  unsigned char pair_of[MAX_PAIRS] = {};
+};
+
+// `cycles` (pairs x PROBE_WORDS) -> numbers of the pairs, die by die.  Patterns that are not clearly those of two dies of about
+// the same size give none.
+static DieMap dies_from_latencies(const float* cycles, int pairs) {
+  DieMap m;
+  m.pairs = pairs;
+  bool other[MAX_PAIRS];
+  float ref[PROBE_WORDS];
+  int count[2] = {0, 0};
+  for (int p = 0; p < pairs; ++p) {
+    float x[PROBE_WORDS], mean = 0.f, dot = 0.f, xx = 0.f, rr = 0.f;
+    for (int a = 0; a < PROBE_WORDS; ++a) mean += cycles[p * PROBE_WORDS + a] / PROBE_WORDS;
+    for (int a = 0; a < PROBE_WORDS; ++a) x[a] = cycles[p * PROBE_WORDS + a] - mean;
+    if (p == 0)
+      for (int a = 0; a < PROBE_WORDS; ++a) ref[a] = x[a];
+    for (int a = 0; a < PROBE_WORDS; ++a) { dot += x[a] * ref[a]; xx += x[a] * x[a]; rr += ref[a] * ref[a]; }
+    if (!(dot * dot > 0.5f * xx * rr)) return m;
+    other[p] = dot < 0.f;
+    ++count[other[p]];
+  }
+  if (4 * count[0] < pairs || 4 * count[1] < pairs) return m;
+  int next[2] = {0, count[0]};
+  for (int p = 0; p < pairs; ++p) m.pair_of[p] = static_cast<unsigned char>(next[other[p]]++);
+  m.first_die = count[0];
+  return m;
+}
+
+// Of the current device, measured at its first two-SM launch outside a graph capture (a fifth of a millisecond; the stream is
+// waited for).  What it gives only orders the tiles: any answer is a correct one.
+static DieMap measure_dies(cudaStream_t stream) {
+  static std::mutex lock;
+  static std::map<int, DieMap> known;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> hold(lock);
+  auto it = known.find(dev);
+  if (it != known.end()) return it->second;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return DieMap();
+  }
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int pairs = sms / 2;
+  DieMap m;
+  if (pairs >= 2 && pairs <= MAX_PAIRS) {
+    constexpr int ALONE = 160 * 1024;            // shared memory, so that every block has an SM of its own, as the products' have
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);  // (another thread's capture is not disturbed by the wait)
+    float cycles[MAX_PAIRS * PROBE_WORDS];
+    if (cudaFuncSetAttribute(die_probe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ALONE) == cudaSuccess) {
+      die_probe_kernel<<<2 * pairs, 64, ALONE, stream>>>();
+      if (cudaGetLastError() == cudaSuccess &&
+          cudaMemcpyFromSymbolAsync(cycles, g_probe_cycles, sizeof(float) * pairs * PROBE_WORDS, 0, cudaMemcpyDeviceToHost, stream) ==
+              cudaSuccess &&
+          cudaStreamSynchronize(stream) == cudaSuccess)
+        m = dies_from_latencies(cycles, pairs);
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  }
+  known[dev] = m;
+  return m;
+}
+
+template <bool A_MN, bool B_MN, int EPI = 0, int GROUPED = 0, int TM = 1>
 static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t stream) {
-  auto kern = gemm2_kernel<A_MN, B_MN, EPI, GROUPED>;
+  auto kern = gemm2_kernel<A_MN, B_MN, EPI, GROUPED, TM>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring2<EPI>::TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring2<EPI, TM>::TOTAL);
     if (e != cudaSuccess) return -300 - static_cast<int>(e);
     configured = true;
   }
-  kern<<<grid, 64 + 32 * EPI2_WARPS, Ring2<EPI>::TOTAL, stream>>>(ta, tb, p);
+  GemmParams q = p;
+  const DieMap dies = measure_dies(stream);
+  q.die_pairs = 2 * dies.pairs == grid && GROUPED == 0 && p.K >= DIES_K ? dies.first_die : 0;
+  for (int i = 0; i < MAX_PAIRS; ++i) q.pair_of[i] = dies.pair_of[i];
+  kern<<<grid, 64 + 32 * EPI2_WARPS, Ring2<EPI, TM>::TOTAL, stream>>>(ta, tb, q);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -400 - static_cast<int>(e);
+}
+
+// Plain products (and slices of one) on 256 x 256 tiles, or on 512 x 256.
+static int launch2_major(int a_mn, int b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int most, cudaStream_t s) {
+  const int slices = p.split_k > 1 ? p.split_k : 1, k = p.split_k > 1 ? p.k_per_split : p.K;
+  const int columns = (p.N + BN2 - 1) / BN2 * slices;
+  const int tiles = (p.M + 2 * BM - 1) / (2 * BM) * columns, wide = (p.M + 4 * BM - 1) / (4 * BM) * columns;
+  const int pairs = most / 2 > 0 ? most / 2 : 1;
+  if (k >= WIDE_K && 2 * ((wide + pairs - 1) / pairs) <= (tiles + pairs - 1) / pairs) {
+    const int grid = 2 * (wide < pairs ? wide : pairs);
+    if (!a_mn && !b_mn) return launch2<false, false, 0, 0, 2>(ta, tb, p, grid, s);
+    if (!a_mn && b_mn) return launch2<false, true, 0, 0, 2>(ta, tb, p, grid, s);
+    if (a_mn && !b_mn) return launch2<true, false, 0, 0, 2>(ta, tb, p, grid, s);
+    return launch2<true, true, 0, 0, 2>(ta, tb, p, grid, s);
+  }
+  const int grid = 2 * (tiles < pairs ? tiles : pairs);
+  if (!a_mn && !b_mn) return launch2<false, false>(ta, tb, p, grid, s);
+  if (!a_mn && b_mn) return launch2<false, true>(ta, tb, p, grid, s);
+  if (a_mn && !b_mn) return launch2<true, false>(ta, tb, p, grid, s);
+  return launch2<true, true>(ta, tb, p, grid, s);
 }
 
 // D[m, n] = sum_s ws[s][m, n] + beta * C[m, n] + bias[n], four columns per thread (N % 8 == 0).
@@ -1294,6 +1498,22 @@ static int sm_count() {
 
 extern "C" {
 
+// Numbers of `pairs` pairs of SMs from the latencies of their atomics (pairs x 32): pair_of[pairs]; returns the pairs of the
+// first die, or 0.
+int ftb_gemm_dies_from_latencies(const float* cycles, int pairs, unsigned char* pair_of) {
+  if (pairs < 1 || pairs > MAX_PAIRS) return 0;
+  const DieMap m = dies_from_latencies(cycles, pairs);
+  for (int i = 0; i < pairs; ++i) pair_of[i] = m.pair_of[i];
+  return m.first_die;
+}
+// What was measured of the current device: the numbers of its pairs and how many are on the first die (0: not known yet).
+int ftb_gemm_dies(unsigned char* pair_of, int* pairs, cudaStream_t stream) {
+  const DieMap m = measure_dies(stream);
+  *pairs = m.pairs;
+  for (int i = 0; i < m.pairs; ++i) pair_of[i] = m.pair_of[i];
+  return m.first_die;
+}
+
 // D = alpha*op(A)*op(B) + beta*C + bias.   A, B bf16.  D/C bf16 (d_fp32=0) or fp32 (d_fp32=1).
 //   a_mn_major = 0: A stored (M, K) row-major, leading dim lda;  1: A stored (K, M), leading dim lda.
 //   b_mn_major = 0: B stored (N, K) row-major, leading dim ldb;  1: B stored (K, N), leading dim ldb.
@@ -1342,15 +1562,9 @@ int ftb_gemm_bf16(const void* A, const void* B, void* D, const void* C, const fl
     p2.D = D; p2.C = (C != nullptr) ? C : D; p2.bias = bias; p2.d_fp32 = d_fp32;
     p2.num_groups = 0; p2.offsets = nullptr; p2.max_tiles = 0;
     p2.comm_mode = 0; p2.world = 1; p2.rank = 0; p2.panel_rows = 0; p2.split_k = 1; p2.k_per_split = 0;
-    const int tiles2 = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN2 - 1) / BN2);
     int grid2 = sm_count() & ~1;
     if (max_ctas > 0 && max_ctas < grid2) grid2 = max_ctas & ~1;
-    if (2 * tiles2 < grid2) grid2 = 2 * tiles2;
-    if (grid2 < 2) grid2 = 2;
-    if (!a_mn_major && !b_mn_major) return launch2<false, false>(ta2, tb2, p2, grid2, stream);
-    if (!a_mn_major && b_mn_major) return launch2<false, true>(ta2, tb2, p2, grid2, stream);
-    if (a_mn_major && !b_mn_major) return launch2<true, false>(ta2, tb2, p2, grid2, stream);
-    return launch2<true, true>(ta2, tb2, p2, grid2, stream);
+    return launch2_major(a_mn_major, b_mn_major, ta2, tb2, p2, grid2, stream);
   }
   if (bn != 128 && bn != 256) bn = (N <= 128) ? 128 : 256;
   CUtensorMap ta, tb;
@@ -1537,10 +1751,7 @@ int ftb_gemm_bf16_splitk(const void* A, const void* B, void* D, const void* C, c
   p.split_k = splits; p.k_per_split = kps;
   int grid = sm_count();
   if (two_sm) {
-    const int tiles2 = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN2 - 1) / BN2) * splits;
-    grid = 2 * tiles2 < grid ? 2 * tiles2 : grid & ~1;
-    rc = !a_mn_major ? (!b_mn_major ? launch2<false, false>(ta, tb, p, grid, stream) : launch2<false, true>(ta, tb, p, grid, stream))
-                     : (!b_mn_major ? launch2<true, false>(ta, tb, p, grid, stream) : launch2<true, true>(ta, tb, p, grid, stream));
+    rc = launch2_major(a_mn_major, b_mn_major, ta, tb, p, grid & ~1, stream);
   } else {
     const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn) * splits;
     if (tiles < grid) grid = tiles;
