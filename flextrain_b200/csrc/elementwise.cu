@@ -233,6 +233,172 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const bf16* __r
   }
 }
 
+// Forward of rows of up to 2048 elements: a warp per row, NV 16-byte pieces a lane, no barriers.  A block per row, as above, leaves
+// most of its 256 threads without a piece there (96 of 768 / 8) and has one row in flight between two barriers.
+// us, block per row / so, forward: 16384 x 768 22.7 / 9.9, 9377 x 1024 14.6 / 8.2, 16384 x 2048 28.7 / 25.4; backward with its sum
+// of dw: 58.6 / 28.6, 37.9 / 22.6, 79.3 / 66.5, 8192 x 1152 36.6 / 24.7, 16384 x 3072 98.2 / 89.3.
+template <int NV>
+__global__ void __launch_bounds__(RN_THREADS) rmsnorm_warp_fwd_kernel(const bf16* __restrict__ x, const float* __restrict__ w,
+                                                                      bf16* __restrict__ y, float* __restrict__ rstd_out, int T,
+                                                                      int D, float eps, long ldx) {
+  const int lane = threadIdx.x & 31, nv = D >> 3, step = gridDim.x * (RN_THREADS / 32);
+  for (int row = blockIdx.x * (RN_THREADS / 32) + (threadIdx.x >> 5); row < T; row += step) {
+    const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * ldx);
+    uint4 v[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int i = lane + j * 32;
+      v[j] = i < nv ? xr[i] : make_uint4(0, 0, 0, 0);
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      float f[8];
+      unpack8(v[j], f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss += f[e] * f[e];
+    }
+    const float r = rsqrtf(warp_sum(ss) / (float)D + eps);
+    if (lane == 0 && rstd_out) rstd_out[row] = r;
+    uint4* yr = reinterpret_cast<uint4*>(y + (size_t)row * D);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int i = lane + j * 32;
+      if (i < nv) {
+        float f[8];
+        unpack8(v[j], f);
+        if (w) {
+          const float4 w0 = reinterpret_cast<const float4*>(w)[2 * i];
+          const float4 w1 = reinterpret_cast<const float4*>(w)[2 * i + 1];
+          f[0] *= r * w0.x; f[1] *= r * w0.y; f[2] *= r * w0.z; f[3] *= r * w0.w;
+          f[4] *= r * w1.x; f[5] *= r * w1.y; f[6] *= r * w1.z; f[7] *= r * w1.w;
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) f[e] *= r;
+        }
+        yr[i] = pack8(f);
+      }
+    }
+  }
+}
+
+// The backward of rows of up to 3072: WPR warps to a row (one up to 768 elements, two up to 1536, four), which meet once a row.  NV
+// stays at three: the operands of a row, the gain and the sums of dw are in registers together, and two blocks an SM have to
+// keep enough rows on their way (a warp for 2048 took 241 registers and 88 us).  The groups of a block add up their parts of dw
+// one after the other (a fixed order).
+template <int NV, int WPR>
+__global__ void __launch_bounds__(RN_THREADS, 2) rmsnorm_warp_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
+                                                                      const float* __restrict__ w, const float* __restrict__ rstd,
+                                                                      const bf16* __restrict__ dx_add, bf16* __restrict__ dx,
+                                                                      bf16* __restrict__ y_out, float* __restrict__ dw_partial, int T,
+                                                                      int D, long ldx, long lddx) {
+  constexpr int LANES = 32 * WPR, GROUPS = RN_THREADS / LANES;
+  __shared__ __align__(16) float dw_s[NV * LANES * 8];
+  __shared__ float dot_s[2][RN_THREADS / 32];
+  const int lane = threadIdx.x % LANES, group = threadIdx.x / LANES, nv = D >> 3, step = gridDim.x * GROUPS;
+  int turn = 0;
+  float dwacc[NV][8];
+#pragma unroll
+  for (int j = 0; j < NV; ++j)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) dwacc[j][e] = 0.f;
+  auto gain = [&](int i, float (&wf)[8]) {
+    if (w) {
+      const float4 w0 = reinterpret_cast<const float4*>(w)[2 * i];
+      const float4 w1 = reinterpret_cast<const float4*>(w)[2 * i + 1];
+      wf[0] = w0.x; wf[1] = w0.y; wf[2] = w0.z; wf[3] = w0.w; wf[4] = w1.x; wf[5] = w1.y; wf[6] = w1.z; wf[7] = w1.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) wf[e] = 1.f;
+    }
+  };
+  for (int row = blockIdx.x * GROUPS + group; row < T; row += step) {
+    const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * ldx);
+    const uint4* gr = reinterpret_cast<const uint4*>(dy + (size_t)row * D);
+    const uint4* ar = reinterpret_cast<const uint4*>(dx_add + (size_t)row * D);
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    uint4 xv[NV], gv[NV], av[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int i = lane + j * LANES;
+      xv[j] = i < nv ? xr[i] : zero;
+      gv[j] = i < nv ? gr[i] : zero;
+      if (dx_add) av[j] = i < nv ? ar[i] : zero;
+    }
+    const float r = rstd[row];
+    float dot = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int i = lane + j * LANES;
+      if (i < nv) {
+        float xf[8], gf[8], wf[8];
+        unpack8(xv[j], xf);
+        unpack8(gv[j], gf);
+        gain(i, wf);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float xh = xf[e] * r;
+          dwacc[j][e] += gf[e] * xh;
+          dot += gf[e] * wf[e] * xh;
+        }
+      }
+    }
+    dot = warp_sum(dot);
+    if constexpr (WPR > 1) {                       // (two buffers: the next row's sums do not meet this row's readers)
+      if ((threadIdx.x & 31) == 0) dot_s[turn][threadIdx.x >> 5] = dot;
+      asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(LANES) : "memory");
+      dot = 0.f;
+#pragma unroll
+      for (int u = 0; u < WPR; ++u) dot += dot_s[turn][group * WPR + u];
+      turn ^= 1;
+    }
+    dot /= (float)D;
+    uint4* dxr = reinterpret_cast<uint4*>(dx + (size_t)row * lddx);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int i = lane + j * LANES;
+      if (i < nv) {
+        float xf[8], gf[8], wf[8], o[8];
+        unpack8(xv[j], xf);
+        unpack8(gv[j], gf);
+        gain(i, wf);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = (gf[e] * wf[e] - xf[e] * r * dot) * r;
+        if (dx_add) {
+          float a[8];
+          unpack8(av[j], a);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) o[e] += a[e];
+        }
+        dxr[i] = pack8(o);
+        if (y_out) {
+          float yv[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) yv[e] = xf[e] * r * wf[e];
+          reinterpret_cast<uint4*>(y_out + (size_t)row * D)[i] = pack8(yv);
+        }
+      }
+    }
+  }
+  if (dw_partial) {
+    for (int t = 0; t < GROUPS; ++t) {
+      if (group == t) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+          float4* s = reinterpret_cast<float4*>(dw_s + (lane + j * LANES) * 8);
+          float4 a = t ? s[0] : make_float4(0.f, 0.f, 0.f, 0.f), b = t ? s[1] : make_float4(0.f, 0.f, 0.f, 0.f);
+          a.x += dwacc[j][0]; a.y += dwacc[j][1]; a.z += dwacc[j][2]; a.w += dwacc[j][3];
+          b.x += dwacc[j][4]; b.y += dwacc[j][5]; b.z += dwacc[j][6]; b.w += dwacc[j][7];
+          s[0] = a;
+          s[1] = b;
+        }
+      }
+      __syncthreads();
+    }
+    for (int c = threadIdx.x; c < D; c += RN_THREADS) dw_partial[(size_t)blockIdx.x * D + c] = dw_s[c];
+  }
+}
+
 // out[c] (+)= sum over P partial rows.  A block owns 32 columns and adds 32 rows at a time; one thread per column, walking the
 // rows by itself, left all but D / 256 SMs idle: 592 x 1024 28 us, 5 us so.
 __global__ void __launch_bounds__(1024) colsum_accum_kernel(const float* __restrict__ partial, float* __restrict__ out, int P,
@@ -1191,9 +1357,26 @@ int ftb_rmsnorm_fwd_ld(const void* x, long ldx, const float* w, void* y, float* 
   const int nv = D / 8;
 #define FTB_RN_FWD(MV) \
   rmsnorm_fwd_kernel<MV><<<grid_rows(T, 148 * 8), RN_THREADS, 0, s>>>((const bf16*)x, w, (bf16*)y, rstd, T, D, eps, ldx)
-  if (nv <= 2 * RN_THREADS) FTB_RN_FWD(2);
-  else if (nv <= 4 * RN_THREADS) FTB_RN_FWD(4);
-  else FTB_RN_FWD(8);
+#define FTB_RN_WARP(NV)                                                                                                \
+  case NV:                                                                                                             \
+    rmsnorm_warp_fwd_kernel<NV><<<grid_rows((T + 7L) / 8, 148 * 8), RN_THREADS, 0, s>>>((const bf16*)x, w, (bf16*)y, rstd, T, \
+                                                                                        D, eps, ldx);                  \
+    break
+  switch ((nv + 31) / 32) {
+    FTB_RN_WARP(1);
+    FTB_RN_WARP(2);
+    FTB_RN_WARP(3);
+    FTB_RN_WARP(4);
+    FTB_RN_WARP(5);
+    FTB_RN_WARP(6);
+    FTB_RN_WARP(7);
+    FTB_RN_WARP(8);
+    default:
+      if (nv <= 2 * RN_THREADS) FTB_RN_FWD(2);
+      else if (nv <= 4 * RN_THREADS) FTB_RN_FWD(4);
+      else FTB_RN_FWD(8);
+  }
+#undef FTB_RN_WARP
 #undef FTB_RN_FWD
   CHECK_LAUNCH();
 }
@@ -1210,14 +1393,28 @@ int ftb_rmsnorm_bwd_ld(const void* dy, const void* x, long ldx, const float* w, 
                        cudaStream_t s) {
   if (T == 0) return 0;
   if (D % 8 || ldx % 8 || lddx % 8 || D > 8 * RN_THREADS * RN_MAXV) return -2;
-  const int blocks = ftb_rmsnorm_bwd_blocks(T);
+  int blocks = ftb_rmsnorm_bwd_blocks(T);
   const int nv = D / 8;
 #define FTB_RN_BWD(MV)                                                                                              \
   rmsnorm_bwd_kernel<MV><<<blocks, RN_THREADS, 0, s>>>((const bf16*)dy, (const bf16*)x, w, rstd, (const bf16*)dx_add, \
                                                        (bf16*)dx, (bf16*)y_out, dw ? dw_partial : nullptr, T, D, ldx, lddx)
-  if (nv <= 2 * RN_THREADS) FTB_RN_BWD(2);
+#define FTB_RN_WARP(NV, WPR)                                                                                                          \
+  do {                                                                                                                                \
+    blocks = grid_rows((T + 8L / WPR - 1) / (8 / WPR), 148 * 2);                                                                      \
+    rmsnorm_warp_bwd_kernel<NV, WPR><<<blocks, RN_THREADS, 0, s>>>((const bf16*)dy, (const bf16*)x, w, rstd, (const bf16*)dx_add,     \
+                                                                   (bf16*)dx, (bf16*)y_out, dw ? dw_partial : nullptr, T, D, ldx, lddx); \
+  } while (0)
+  if (nv <= 32) FTB_RN_WARP(1, 1);
+  else if (nv <= 64) FTB_RN_WARP(2, 1);
+  else if (nv <= 96) FTB_RN_WARP(3, 1);
+  else if (nv <= 128) FTB_RN_WARP(2, 2);
+  else if (nv <= 192) FTB_RN_WARP(3, 2);
+  else if (nv <= 256) FTB_RN_WARP(2, 4);
+  else if (nv <= 384) FTB_RN_WARP(3, 4);
+  else if (nv <= 2 * RN_THREADS) FTB_RN_BWD(2);
   else if (nv <= 4 * RN_THREADS) FTB_RN_BWD(4);
   else FTB_RN_BWD(8);
+#undef FTB_RN_WARP
 #undef FTB_RN_BWD
   if (dw) colsum_accum_kernel<<<(D + 31) / 32, 1024, 0, s>>>(dw_partial, dw, blocks, D, dw_accumulate);
   CHECK_LAUNCH();
