@@ -136,8 +136,7 @@ class GatedDeltaNetBlock:
         # gates in one launch straight from the bf16 projection (flextrain/ops/_kernels/gate_prep.py:29-80)
         beta, g = la.gate_prep_fwd(ba.contiguous(), p["w_lin_dt_bias"].to(f32), p["w_lin_A_log"].to(f32))
         o, fin, r = la.gdn_fwd(qn, kn, v, g, beta, cu, state_in, want_r=want_r)
-        z = z2d.contiguous().view(T * c.n_v_heads, c.head_v_dim)
-        on = ops.gated_rmsnorm_fwd(o.view(T * c.n_v_heads, c.head_v_dim), z, p["w_lin_norm"].to(f32), c.norm_eps)
+        on = la.gated_rmsnorm_fwd(o, z2d, p["w_lin_norm"].to(f32), c.norm_eps)
         return dict(qkvz=qkvz, qkv_c=qkv_c, conv_fin=conv_fin, qn=qn, kn=kn, q_rn=q_rn, k_rn=k_rn, v=v, ba=ba,
                     beta=beta, g=g, o=o, fin=fin, r=r, on=on.view(T, c.value_dim))
 
@@ -171,12 +170,12 @@ class GatedDeltaNetBlock:
         # ---- recurrence (dv straight into its columns)
         dqkv_c = torch.empty(T, c.conv_dim, dtype=h.dtype, device=h.device)
         dq, dk, _, dg, dbeta, dstate_in = la.gdn_bwd(s["qn"], s["kn"], s["v"], s["g"], s["beta"], cu, ctx.lin_state_in, s["fin"],
-                                                     s["r"], d_o, dstate_final=ctx.lin_dstate_in,
+                                                     s["r"], d_o, dstate_final=ctx.lin_dstate_in, sum_heads=False,
                                                      dv_out=dqkv_c[:, 2 * c.key_dim:].unflatten(1, (c.n_v_heads, c.head_v_dim)))
         # ---- L2 norms and conv
-        la.l2norm_heads_bwd(dq.contiguous(), s["qkv_c"][:, : c.key_dim], s["q_rn"], dqkv_c[:, : c.key_dim],
+        la.l2norm_heads_bwd(dq, s["qkv_c"][:, : c.key_dim], s["q_rn"], dqkv_c[:, : c.key_dim],
                             c.n_k_heads, c.head_k_dim)
-        la.l2norm_heads_bwd(dk.contiguous(), s["qkv_c"][:, c.key_dim: 2 * c.key_dim], s["k_rn"],
+        la.l2norm_heads_bwd(dk, s["qkv_c"][:, c.key_dim: 2 * c.key_dim], s["k_rn"],
                             dqkv_c[:, c.key_dim: 2 * c.key_dim], c.n_k_heads, c.head_k_dim)
         dwc = torch.zeros(c.conv_dim, c.conv_width, dtype=f32, device=h.device)
         dconv_in = la.conv1d_bwd(s["qkvz"][:, : c.conv_dim], params["w_lin_conv"], cu, ctx.lin_conv_in, dqkv_c,

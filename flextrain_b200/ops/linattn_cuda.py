@@ -72,18 +72,40 @@ def l2norm_heads_fwd(x2d: torch.Tensor, H: int, D: int, eps: float = 1e-6) -> Tu
     return y, rn
 
 
+def _vec_rows(D: int, *rows2d: torch.Tensor) -> bool:
+    """Rows that the 16-byte kernels of ``csrc/seqmix.cu`` take (``vec_rows`` there)."""
+    return D in (64, 128, 256) and all(t.data_ptr() % 16 == 0 and t.stride(0) % 8 == 0 for t in rows2d)
+
+
 def l2norm_heads_bwd(dy: torch.Tensor, x2d: torch.Tensor, rnorm: torch.Tensor, dx_out2d: torch.Tensor, H: int, D: int
                      ) -> None:
-    """``dy (T,H,D)`` fp32 → gradient of the pre-norm values written into ``dx_out2d (T, >=H*D)``."""
+    """``dy (T,H,D)`` fp32 → gradient of the pre-norm values written into ``dx_out2d (T, >=H*D)``.  A ``dy`` of ``rep`` rows per
+    head, ``(T,H*rep,D)``, is added up over them."""
     lib = load("seqmix")
     T = x2d.shape[0]
     assert dy.dtype == F32 and dy.is_contiguous()
-    rc = lib.ftb_l2norm_strided_bwd(_ptr(dy), _ptr(x2d), c_long(_rows_ld(x2d)), _ptr(rnorm), _ptr(dx_out2d),
-                                    c_long(_rows_ld(dx_out2d)), c_long(T), c_int(H), c_int(D), _stream())
-    _check(rc, "ftb_l2norm_strided_bwd")
+    rep = dy.shape[1] // H if dy.dim() == 3 else 1
+    if rep > 1 and not (_vec_rows(D, x2d, dx_out2d) and dy.data_ptr() % 16 == 0):
+        dy, rep = dy.view(T, H, rep, D).sum(2), 1
+    rc = lib.ftb_l2norm_rep_bwd(_ptr(dy), c_int(rep), _ptr(x2d), c_long(_rows_ld(x2d)), _ptr(rnorm), _ptr(dx_out2d),
+                                c_long(_rows_ld(dx_out2d)), c_long(T), c_int(H), c_int(D), _stream())
+    _check(rc, "ftb_l2norm_rep_bwd")
 
 
-# ------------------------------------------------------------------------------------- gated RMSNorm backward
+# ---------------------------------------------------------------------------------------------- gated RMSNorm
+def gated_rmsnorm_fwd(o: torch.Tensor, z2d: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
+    """``o (T,H,D)`` contiguous, ``z2d (T, H*D)`` a row-strided view, ``w (D)`` fp32 → ``rmsnorm(o) * w * silu(z)``, contiguous."""
+    T, H, D = o.shape
+    if not (_vec_rows(D, z2d) and o.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
+        from .. import ops
+        return ops.gated_rmsnorm_fwd(o.view(T * H, D), z2d.contiguous().view(T * H, D), w, eps).view(T, H, D)
+    y = torch.empty_like(o)
+    rc = load("seqmix").ftb_gated_rmsnorm_strided_fwd(_ptr(o), _ptr(z2d), c_long(_rows_ld(z2d)), c_int(H), _ptr(w), _ptr(y),
+                                                      c_long(T), c_int(D), c_float(eps), _stream())
+    _check(rc, "ftb_gated_rmsnorm_strided_fwd")
+    return y
+
+
 def gated_rmsnorm_bwd(dy: torch.Tensor, o: torch.Tensor, z2d: torch.Tensor, w: torch.Tensor, dz_out2d: torch.Tensor,
                       dw: Optional[torch.Tensor], H: int, D: int, eps: float) -> torch.Tensor:
     """``dy, o (T,H,D)`` contiguous; ``z2d`` / ``dz_out2d`` are row-strided ``(T, H*D)`` views.  Returns ``d_o``."""

@@ -41,3 +41,33 @@ def test_rmsnorm_rows_by_warps(D, T):
     want = R * (G - X * R * (G * X * R).mean(-1, keepdim=True))
     size = R * (G.abs() + (X * R).abs() * (G * X * R).abs().mean(-1, keepdim=True))
     assert near(dx, want, want.abs() * 2.0 ** -8 + size * (D + 32) * 2.0 ** -23)
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("T,H", [(1, 1), (5, 3), (700, 4)])
+def test_l2_and_gated_norm_rows(D, T, H):
+    """The 16-byte kernels against the general ones (rows one element off the grid), and the heads that share a key head.  Two
+    roundings to bf16 of values that differ in the last bits of fp32: one unit in 2^-7 of each at most."""
+    from flextrain_b200.ops import linattn_cuda as la
+    torch.manual_seed(0)
+    x, z = _randn(T, H * D + 8), _randn(T, H * D + 16)
+    off = lambda t: torch.empty(t.shape[0], t.shape[1] + 1, device=DEV, dtype=t.dtype)[:, 1:].copy_(t)
+    (y, rn), (y1, rn1) = (la.l2norm_heads_fwd(t, H, D) for t in (x, off(x)))
+    assert torch.allclose(rn, rn1, rtol=1e-6) and torch.allclose(y.float(), y1.float(), rtol=2.0 ** -7, atol=1e-6)
+    dy = torch.randn(T, 2 * H, D, device=DEV)
+    dx, dx1 = torch.empty_like(x), torch.empty_like(x)
+    la.l2norm_heads_bwd(dy, x, rn, dx[:, :H * D], H, D)
+    la.l2norm_heads_bwd(dy.view(T, H, 2, D).sum(2), off(x), rn, dx1[:, :H * D], H, D)
+    assert torch.allclose(dx[:, :H * D].float(), dx1[:, :H * D].float(), rtol=2.0 ** -7, atol=1e-5)
+    la.l2norm_heads_bwd(dy, off(x), rn, dx1[:, :H * D], H, D)                      # general rows, two heads a key head
+    assert torch.allclose(dx[:, :H * D].float(), dx1[:, :H * D].float(), rtol=2.0 ** -7, atol=1e-5)
+    o, w, g = _randn(T, H, D), torch.rand(D, device=DEV) + 0.5, _randn(T, H, D)
+    a, b = (la.gated_rmsnorm_fwd(o, t[:, :H * D], w, 1e-6) for t in (z, off(z)))
+    assert torch.allclose(a.float(), b.float(), rtol=2.0 ** -7, atol=1e-6)
+    got = []
+    for zz in (z, off(z)):
+        dz, dw = torch.empty(T, H * D, device=DEV, dtype=BF), torch.ones(D, device=DEV)
+        got.append((la.gated_rmsnorm_bwd(g, o, zz[:, :H * D], w, dz, dw, H, D, 1e-6), dz, dw))
+    for u, v in zip(got[0][:2], got[1][:2]):
+        assert torch.allclose(u.float(), v.float(), rtol=2.0 ** -7, atol=1e-5)
+    assert torch.allclose(got[0][2], got[1][2], rtol=1e-4, atol=T * H * 2.0 ** -20)
