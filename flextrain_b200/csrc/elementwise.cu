@@ -668,6 +668,76 @@ __global__ void rope_full_vec_kernel(const bf16* __restrict__ x, long in_stride,
   }
 }
 
+// Q, K and V of a projection in one pass: Q and K rotated (full rotary, one position axis), V copied, each (T, H, hd) with a token
+// stride of its own.  Forward from the projection into the saved activations, and inverse from the attention's gradients (dQ
+// still in fp32 as the kernel accumulated it) into the projection's gradient.  A block takes 512 / hd tokens, so that every
+// thread works out one (sin, cos); a block per token left most threads of a narrow model idle, and V went by a library copy of
+// two bytes an access.
+// us, rotation of each, copy of V and rounding of dQ / so: 16384 x (32 + 2 x 8) x 128 97.5 / 65.5 forward, 156 / 82.3 backward; (6 + 2 x
+// 6) x 128 54.1 / 31.1 and 67.4 / 32.5; (32 + 2 x 8) x 64 55.4 / 42.0 and 86.1 / 44.1.
+template <typename TQ>
+__global__ void __launch_bounds__(256) rope_qkv_kernel(const TQ* __restrict__ q, long q_is, bf16* __restrict__ qo, long q_os, int HQ,
+                                                       const bf16* __restrict__ k, long k_is, bf16* __restrict__ ko, long k_os,
+                                                       const bf16* __restrict__ v, long v_is, bf16* __restrict__ vo, long v_os, int HK,
+                                                       int HV, const int* __restrict__ pos, const float* __restrict__ inv_freq, int T,
+                                                       int hd, int inverse) {
+  __shared__ float sn[256], cs[256];             // [token][pair]
+  const int half = hd >> 1, t0 = blockIdx.x * (256 / half);
+  {
+    const int t = t0 + threadIdx.x / half;
+    if (t < T) {
+      float s, c;
+      sincosf((float)pos[t] * inv_freq[threadIdx.x % half], &s, &c);
+      sn[threadIdx.x] = inverse ? -s : s;
+      cs[threadIdx.x] = c;
+    }
+  }
+  __syncthreads();
+  const int per_head = half >> 3, heads = HQ + HK + HV, units = heads * per_head, n = min(256 / half, T - t0);
+  auto load_bf = [](const bf16* p, float (&f)[8]) { unpack8(*reinterpret_cast<const uint4*>(p), f); };
+  for (int idx = threadIdx.x; idx < n * units; idx += 256) {
+    const int tt = idx / units, u = idx - tt * units, h = u / per_head, c = (u - h * per_head) << 3;
+    const long t = t0 + tt;
+    if (h >= HQ + HK) {
+      const long at = (long)(h - HQ - HK) * hd + c;
+      const uint4 a = *reinterpret_cast<const uint4*>(v + t * v_is + at), b = *reinterpret_cast<const uint4*>(v + t * v_is + at + half);
+      *reinterpret_cast<uint4*>(vo + t * v_os + at) = a;
+      *reinterpret_cast<uint4*>(vo + t * v_os + at + half) = b;
+      continue;
+    }
+    float a[8], b[8], ra[8], rb[8];
+    bf16* o;
+    if (h >= HQ) {
+      const bf16* p = k + t * k_is + (long)(h - HQ) * hd + c;
+      o = ko + t * k_os + (long)(h - HQ) * hd + c;
+      load_bf(p, a);
+      load_bf(p + half, b);
+    } else {
+      const TQ* p = q + t * q_is + (long)h * hd + c;
+      o = qo + t * q_os + (long)h * hd + c;
+      if constexpr (sizeof(TQ) == 4) {
+#pragma unroll
+        for (int e = 0; e < 8; e += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(p + e), y = *reinterpret_cast<const float4*>(p + half + e);
+          a[e] = x.x; a[e + 1] = x.y; a[e + 2] = x.z; a[e + 3] = x.w;
+          b[e] = y.x; b[e + 1] = y.y; b[e + 2] = y.z; b[e + 3] = y.w;
+        }
+      } else {
+        load_bf(p, a);
+        load_bf(p + half, b);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float s1 = sn[tt * half + c + e], c1 = cs[tt * half + c + e];
+      ra[e] = a[e] * c1 - b[e] * s1;
+      rb[e] = b[e] * c1 + a[e] * s1;
+    }
+    *reinterpret_cast<uint4*>(o) = pack8(ra);
+    *reinterpret_cast<uint4*>(o + half) = pack8(rb);
+  }
+}
+
 // ------------------------------------------------------------------------ SwiGLU / GeGLU
 __device__ __forceinline__ void act_and_grad(float g, int kind, float& a, float& da) {
   if (kind == 0) {
@@ -1490,6 +1560,26 @@ int ftb_rope(const void* x, long in_stride, void* out, long out_stride, const in
   threads = threads > 512 ? 512 : ((threads + 31) / 32) * 32;
   rope_kernel<<<T, threads, 0, s>>>((const bf16*)x, in_stride, (bf16*)out, out_stride, pos, inv_freq, T, H, hd,
                                     half_rot, inverse, pos_stride, sec_h, sec_w);
+  CHECK_LAUNCH();
+}
+
+// One launch for the heads of a projection (see the kernel).  HQ, HK, HV may be 0.  -2: not what the kernel takes.
+int ftb_rope_qkv(const void* q, int q_fp32, long q_is, void* qo, long q_os, int HQ, const void* k, long k_is, void* ko, long k_os,
+                 int HK, const void* v, long v_is, void* vo, long v_os, int HV, const int* pos, const float* inv_freq, int T, int hd,
+                 int inverse, cudaStream_t s) {
+  if (T <= 0 || HQ + HK + HV == 0) return 0;
+  if (hd != 64 && hd != 128 && hd != 256) return -2;
+  const void* base[6] = {HQ ? q : nullptr, HQ ? qo : nullptr, HK ? k : nullptr, HK ? ko : nullptr, HV ? v : nullptr, HV ? vo : nullptr};
+  const long ld[6] = {q_is, q_os, k_is, k_os, v_is, v_os};
+  for (int i = 0; i < 6; ++i)
+    if (base[i] && (((uintptr_t)base[i] & 15) || ld[i] % 8)) return -2;
+  const unsigned blocks = (T + 512 / hd - 1) / (512 / hd);
+  if (q_fp32)
+    rope_qkv_kernel<float><<<blocks, 256, 0, s>>>((const float*)q, q_is, (bf16*)qo, q_os, HQ, (const bf16*)k, k_is, (bf16*)ko, k_os,
+                                                  (const bf16*)v, v_is, (bf16*)vo, v_os, HK, HV, pos, inv_freq, T, hd, inverse);
+  else
+    rope_qkv_kernel<bf16><<<blocks, 256, 0, s>>>((const bf16*)q, q_is, (bf16*)qo, q_os, HQ, (const bf16*)k, k_is, (bf16*)ko, k_os,
+                                                 (const bf16*)v, v_is, (bf16*)vo, v_os, HK, HV, pos, inv_freq, T, hd, inverse);
   CHECK_LAUNCH();
 }
 

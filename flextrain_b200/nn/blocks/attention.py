@@ -158,19 +158,14 @@ class GQAAttentionBlock:
             slot.put("k_rstd", kr)
         inv = self._inv_freq(h.device)
         pos, sec = meta.positions, c.rope.mrope_sections
-        xk = ops.rope(k, pos, inv, out=slot.out("xk", h.device), mrope_sections=sec)
-        xv = slot.out("xv", h.device)
+        xk, xv = slot.out("xk", h.device), slot.out("xv", h.device)
+        xq = slot.out("xq", h.device) if want_q else None
         if c.v_norm:
-            vn, vr = ops.rmsnorm_fwd(v, self._unit_gain(h.device), c.norm_eps)
+            v, vr = ops.rmsnorm_fwd(v, self._unit_gain(h.device), c.norm_eps)
             slot.put("v_rstd", vr)
-            xv.copy_(vn)
-        else:
-            xv.copy_(v)
-        xq = None
-        if want_q:
-            xq = ops.rope(q, pos, inv, out=slot.out("xq", h.device), mrope_sections=sec)
-            if c.gated:
-                slot.put("xgate", gate.contiguous() if slot.buffer is None else gate)
+        ops.rope_qkv(q if want_q else None, k, v, pos, inv, q_out=xq, k_out=xk, v_out=xv, mrope_sections=sec)
+        if want_q and c.gated:
+            slot.put("xgate", gate.contiguous() if slot.buffer is None else gate)
         return xq, xk, xv
 
     def _kv_for_attention(self, meta: ChunkMeta, xk, xv, ctx: LayerContext, *, write: bool):
@@ -251,7 +246,7 @@ class GQAAttentionBlock:
         dq, dk, dv = ops.attention_bwd(dattn.view(T, c.n_heads, c.head_dim), t["xq"], K, V,
                                        attn_raw.view(T, c.n_heads, c.head_dim), t["softmax_lse"], meta.cu_seqlens_q,
                                        meta.cu_seqlens_k, meta.max_seqlen_q, meta.max_seqlen_k, scale=self.scale,
-                                       causal=c.causal, window=c.window, softcap=c.softcap)
+                                       causal=c.causal, window=c.window, softcap=c.softcap, dq_fp32=True)
         if meta.has_prior or (ctx.kv_window is not None and ctx.kv_window.dk is not None and any(meta.has_more_chunks)):
             dk, dv = self._cross_chunk_dkv(dk, dv, meta, ctx)
         # inverse RoPE, then QK-norm backward, assembling dqkv in projection-row order
@@ -267,20 +262,17 @@ class GQAAttentionBlock:
             dq_dst = dqkv[:, :qrows].unflatten(1, (c.n_heads, c.head_dim))
         dk_dst = dqkv[:, qrows: qrows + c.kv_dim].unflatten(1, (c.n_kv_heads, c.head_dim))
         dv_dst = dqkv[:, qrows + c.kv_dim:].unflatten(1, (c.n_kv_heads, c.head_dim))
+        dv_src, dv_rope = (None, None) if c.v_norm else (dv, dv_dst)
+        if c.qk_norm:
+            dqn, dkn = torch.empty_like(t["xq"]), torch.empty_like(dk)
+            ops.rope_qkv(dq, dk, dv_src, pos, inv, q_out=dqn, k_out=dkn, v_out=dv_rope, inverse=True, mrope_sections=sec)
+        else:
+            ops.rope_qkv(dq, dk, dv_src, pos, inv, q_out=dq_dst, k_out=dk_dst, v_out=dv_rope, inverse=True, mrope_sections=sec)
+        del dq                                                                          # (fp32: the largest tensor here)
         pre = self._project_qkv(h_fn(), params) if (c.qk_norm or c.v_norm) else None   # pre-norm recompute (one GEMM)
         if c.v_norm:
             ops.rmsnorm_bwd(dv.contiguous(), pre[3], self._unit_gain(dxo.device), t["v_rstd"], dx_out=dv_dst)
-        else:
-            dv_dst.copy_(dv)
-        if not c.qk_norm:
-            if c.gated:
-                dq_dst.copy_(ops.rope(dq.contiguous(), pos, inv, inverse=True, mrope_sections=sec))
-            else:
-                ops.rope(dq, pos, inv, out=dq_dst, inverse=True, mrope_sections=sec)
-            ops.rope(dk, pos, inv, out=dk_dst, inverse=True, mrope_sections=sec)
-        else:
-            dqn = ops.rope(dq.contiguous(), pos, inv, inverse=True, mrope_sections=sec)
-            dkn = ops.rope(dk.contiguous(), pos, inv, inverse=True, mrope_sections=sec)
+        if c.qk_norm:
             q_pre, _, k_pre, _ = pre
             for dn, x_pre, dst, n in ((dqn, q_pre, dq_dst, "q"), (dkn, k_pre, dk_dst, "k")):
                 if c.qk_norm == "row":              # (a gated projection's heads lie apart, and become rows by a copy)

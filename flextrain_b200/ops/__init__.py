@@ -244,6 +244,34 @@ def rope(x, positions, inv_freq, *, out=None, inverse=False, mrope_sections=None
     return out
 
 
+def rope_qkv_fused(_heads, *args):
+    """The fused kernel itself (GPU only); ``rope_qkv`` is the entry that falls back."""
+    return _kernels().rope_qkv(*args)
+
+
+def rope_qkv(q, k, v, positions, inv_freq, *, q_out, k_out, v_out, inverse=False, mrope_sections=None):
+    """``q`` and ``k`` rotated into ``q_out`` and ``k_out``, ``v`` copied into ``v_out`` (pairs may be None); one launch where the
+    heads allow it.  ``q`` may be fp32 (the attention backward's accumulators)."""
+    if (k is not None and _cuda_bf16(k)) or (k is None and q is not None and q.is_cuda):
+        kn = _kernels()
+        pos = positions.to(torch.int32).contiguous()
+        if kn.rope_qkv_supported(q, k, v, q_out, k_out, v_out, pos, inv_freq, mrope_sections):
+            _count()
+            rope_qkv_fused(k if k is not None else q, q, k, v, pos, inv_freq, q_out, k_out, v_out, inverse)
+            return
+    for x, o in ((q, q_out), (k, k_out)):
+        if x is None:
+            continue
+        if x.dtype != o.dtype:
+            x = x.to(o.dtype)
+        if o.stride(1) == o.shape[2]:
+            rope(x, positions, inv_freq, out=o, inverse=inverse, mrope_sections=mrope_sections)
+        else:
+            o.copy_(rope(x.contiguous(), positions, inv_freq, inverse=inverse, mrope_sections=mrope_sections))
+    if v is not None:
+        v_out.copy_(v)
+
+
 def glu_fwd(gate, up, kind="swiglu"):
     if _cuda_bf16(gate, up):
         _count()
@@ -354,15 +382,16 @@ def attention_fwd(q, k, v, cu_q, cu_k, max_q, max_k, *, scale, causal=True, wind
     return ref.attention_fwd(q, k, v, cu_q, cu_k, scale=scale, causal=causal, window=window, softcap=softcap)
 
 
-def attention_bwd(dout, q, k, v, out, lse, cu_q, cu_k, max_q, max_k, *, scale, causal=True, window=0, softcap=0.0):
-    """Returns ``(dq, dk, dv)``; dk/dv span all visible keys."""
+def attention_bwd(dout, q, k, v, out, lse, cu_q, cu_k, max_q, max_k, *, scale, causal=True, window=0, softcap=0.0,
+                  dq_fp32=False):
+    """Returns ``(dq, dk, dv)``; dk/dv span all visible keys.  ``dq_fp32``: ``dq`` may come as the fp32 sums themselves."""
     be = _attn_backend_for(q)
     if be == "ftb" and hasattr(_kernels().load("attention"), "ftb_attn_bwd"):
         from . import attention_cuda
         _count(3)
         _used("attention_bwd", "ftb")
         return attention_cuda.bwd(dout, q, k, v, out, lse, cu_q, cu_k, max_q, max_k, scale=scale, causal=causal,
-                                  window=window, softcap=softcap)
+                                  window=window, softcap=softcap, dq_fp32=dq_fp32)
     if q.is_cuda:
         _fallback("attention_bwd", f"backend {be}, head_dim {q.shape[-1]}, dtype {q.dtype}")
     if be in ("library", "ftb") and not softcap:
@@ -681,8 +710,8 @@ rope_inv_freq = ref.rope_inv_freq
 # ``FTB_OP_TIMING=1`` brackets every leaf op of this module with CUDA events on the current stream and
 # ``timing_report()`` aggregates them by (op, shape): the per-kernel time table of a training step without a
 # profiler attached.  The events add host work, so a throughput number taken with it on is not a benchmark value.
-_TIMED_OPS = ("gemm", "gemm_glu_fwd", "gemm_glu_bwd", "rmsnorm_fwd", "rmsnorm_bwd", "rope", "glu_fwd", "glu_bwd", "glu_bwd_weighted", "attention_fwd",
-              "attention_bwd", "softmax_ce_", "softmax_ce_loss", "embedding_fwd", "embedding_bwd", "adamw_multi", "topk_route",
+_TIMED_OPS = ("gemm", "gemm_glu_fwd", "gemm_glu_bwd", "rmsnorm_fwd", "rmsnorm_bwd", "rope", "rope_qkv_fused", "glu_fwd", "glu_bwd",
+              "glu_bwd_weighted", "attention_fwd", "attention_bwd", "softmax_ce_", "softmax_ce_loss", "embedding_fwd", "embedding_bwd", "adamw_multi", "topk_route",
               "topk_route_bwd", "gather_rows", "moe_combine", "grouped_gemm", "grouped_wgrad", "l2norm_fwd",
               "gated_rmsnorm_fwd", "bias_grad")
 _timing_events: list = []

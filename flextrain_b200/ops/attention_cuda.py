@@ -48,8 +48,8 @@ def deterministic_default() -> bool:
 
 
 def bwd(dout, q, k, v, out, lse, cu_q, cu_k, max_q, max_k, *, scale, causal=True, window=0, softcap=0.0,
-        deterministic=None):
-    """Returns ``(dq, dk, dv)``; dk / dv cover all keys.  ``deterministic`` (default: :func:`deterministic_default`)
+        deterministic=None, dq_fp32=False):
+    """Returns ``(dq, dk, dv)``; dk / dv cover all keys.  ``dq_fp32``: ``dq`` as the fp32 sums, not rounded.  ``deterministic`` (default: :func:`deterministic_default`)
     orders the key tiles' additions to every query tile, so two runs give bit-identical dQ (dK / dV always are)."""
     lib = load("attention")
     if not hasattr(lib, "ftb_attn_bwd"):
@@ -59,7 +59,6 @@ def bwd(dout, q, k, v, out, lse, cu_q, cu_k, max_q, max_k, *, scale, causal=True
     Tk, KV = k.shape[0], k.shape[1]
     nseq = cu_q.numel() - 1
     dq_acc = torch.zeros(Tq, H, hd, dtype=torch.float32, device=q.device)
-    dq = torch.empty(Tq, H, hd, dtype=q.dtype, device=q.device)
     dk = torch.empty(Tk, KV, hd, dtype=q.dtype, device=q.device)
     dv = torch.empty(Tk, KV, hd, dtype=q.dtype, device=q.device)
     delta = torch.empty(H, Tq, dtype=torch.float32, device=q.device)
@@ -68,11 +67,10 @@ def bwd(dout, q, k, v, out, lse, cu_q, cu_k, max_q, max_k, *, scale, causal=True
     det = deterministic_default() if deterministic is None else bool(deterministic)
     sem = torch.zeros(1 + (Tq // 128 + nseq) * H * 4, dtype=torch.int32, device=q.device) if det else None
     rc = lib.ftb_attn_bwd(_ptr(dout), _ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(lse), _ptr(delta), _ptr(dq_acc),
-                          _ptr(sem), _ptr(dq), _ptr(dk), _ptr(dv), _ptr(cu_q), _ptr(cu_k), c_int(nseq), c_int(Tq), c_int(Tk),
+                          _ptr(sem), None, _ptr(dk), _ptr(dv), _ptr(cu_q), _ptr(cu_k), c_int(nseq), c_int(Tq), c_int(Tk),
                           c_int(H), c_int(KV), c_int(hd), c_long(q.stride(0)), c_long(k.stride(0)),
                           c_long(v.stride(0)), c_long(dout.stride(0)), c_long(out.stride(0)), c_float(scale),
                           c_float(float(softcap or 0.0)), c_int(1 if causal else 0), c_int(int(window or 0)),
                           c_int(Tk // 128 + nseq), c_int(int(max_k)), _stream())
     _check(rc, "ftb_attn_bwd")
-    dq.copy_(dq_acc)
-    return dq, dk, dv
+    return dq_acc if dq_fp32 else dq_acc.to(q.dtype), dk, dv

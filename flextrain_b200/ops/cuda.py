@@ -377,6 +377,35 @@ def rope(x, positions, inv_freq, *, out=None, inverse=False, mrope_sections=None
     return out
 
 
+def rope_qkv_supported(q, k, v, q_out, k_out, v_out, positions, inv_freq, mrope_sections) -> bool:
+    """Full rotary over one position axis, bf16 heads of 64, 128 or 256 side by side on 16 bytes (``q`` may be fp32)."""
+    if mrope_sections is not None or positions.dim() != 1 or inv_freq.dtype != torch.float32:
+        return False
+    hd = 2 * inv_freq.numel()
+    if hd not in (64, 128, 256):
+        return False
+    for t in (q, k, v, q_out, k_out, v_out):
+        if t is None:
+            continue
+        if not (t.is_cuda and (t.dtype == torch.bfloat16 or (t is q and t.dtype == torch.float32)) and t.shape[2] == hd
+                and t.stride(2) == 1 and t.stride(1) == hd and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0):
+            return False
+    return True
+
+
+def rope_qkv(q, k, v, positions, inv_freq, q_out, k_out, v_out, inverse=False):
+    lib = load("elementwise")
+    some = next(t for t in (k, q, v) if t is not None)
+    args = []
+    for t, o in ((q, q_out), (k, k_out), (v, v_out)):
+        args.append((_ptr(t), c_long(t.stride(0) if t is not None else 0), _ptr(o), c_long(o.stride(0) if t is not None else 0),
+                     c_int(t.shape[1] if t is not None else 0)))
+    qa, ka, va = args
+    _check(lib.ftb_rope_qkv(qa[0], c_int(1 if q is not None and q.dtype == torch.float32 else 0), *qa[1:], *ka, *va, _ptr(positions),
+                            _ptr(inv_freq), c_int(some.shape[0]), c_int(some.shape[2]), c_int(1 if inverse else 0), _stream()),
+           "ftb_rope_qkv")
+
+
 _KIND = {"swiglu": 0, "geglu": 1}
 
 

@@ -43,6 +43,37 @@ def test_rmsnorm_rows_by_warps(D, T):
     assert near(dx, want, want.abs() * 2.0 ** -8 + size * (D + 32) * 2.0 ** -23)
 
 
+@pytest.mark.parametrize("hd,HQ,HK", [(64, 3, 1), (128, 6, 2), (256, 2, 2)])
+@pytest.mark.parametrize("T", [1, 5, 301])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_rope_qkv_equals_its_parts(hd, HQ, HK, T, inverse):
+    """One launch for Q, K and V against the rotation of each and a copy: the same bits; fp32 queries against rounded ones within
+    the rounding of the input."""
+    from flextrain_b200 import ops
+    torch.manual_seed(0)
+    qkv = _randn(T, (HQ + 2 * HK) * hd)
+    q, k, v = (t.unflatten(1, (-1, hd)) for t in qkv.split([HQ * hd, HK * hd, HK * hd], 1))
+    pos = torch.randint(0, 5000, (T,), device=DEV)
+    inv = 1.0 / 10000 ** (torch.arange(hd // 2, device=DEV) / (hd // 2))
+    want = [ops.rope(t.contiguous(), pos, inv, inverse=inverse) for t in (q.clone(), k.clone())] + [v]
+    out = torch.full((T, (HQ + 2 * HK) * hd + 8), 3.0, device=DEV, dtype=BF)
+    dst = [t.unflatten(1, (-1, hd)) for t in out[:, :-8].split([HQ * hd, HK * hd, HK * hd], 1)]
+    before = ops.launch_count()
+    ops.rope_qkv(q, k, v, pos, inv, q_out=dst[0], k_out=dst[1], v_out=dst[2], inverse=inverse)
+    assert ops.launch_count() == before + 1
+    assert all(torch.equal(a, b) for a, b in zip(dst, want)) and bool((out[:, -8:] == 3.0).all())
+    some = torch.empty(T, HK, hd, device=DEV, dtype=BF)
+    ops.rope_qkv(None, k, None, pos, inv, q_out=None, k_out=some, v_out=None, inverse=inverse)
+    assert torch.equal(some, want[1])
+    got = torch.empty(T, HQ, hd, device=DEV, dtype=BF)
+    ops.rope_qkv(q.float().contiguous(), k, v, pos, inv, q_out=got, k_out=some, v_out=torch.empty_like(some), inverse=inverse)
+    assert torch.equal(got, want[0])
+    odd = torch.empty(T * HK * hd + 1, device=DEV, dtype=BF)[1:].view(T, HK, hd).copy_(k)      # off the grid: by parts
+    ops.rope_qkv(q, odd, v, pos, inv, q_out=got, k_out=some, v_out=dst[2], inverse=inverse)
+    near = lambda a, b: torch.allclose(a.float(), b.float(), rtol=2.0 ** -7, atol=1e-3)         # (other roundings in fp32)
+    assert near(some, want[1]) and near(got, want[0])
+
+
 @pytest.mark.parametrize("D", [64, 128, 256])
 @pytest.mark.parametrize("T,H", [(1, 1), (5, 3), (700, 4)])
 def test_l2_and_gated_norm_rows(D, T, H):
