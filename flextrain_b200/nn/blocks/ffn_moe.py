@@ -140,10 +140,7 @@ class MoEFFN:
     def _experts_fwd(self, h, params, plan, x_up_out=None):
         F = self.cfg.expert_dim
         xs = ops.gather_rows(h, plan.row_src, idx_div=self.cfg.top_k)
-        up = ops.grouped_gemm(xs, self.weight(params, "w_up"), plan.offsets)
-        if x_up_out is not None and x_up_out.data_ptr() != up.data_ptr():
-            x_up_out.copy_(up)
-            up = x_up_out
+        up = ops.grouped_gemm(xs, self.weight(params, "w_up"), plan.offsets, out=x_up_out)
         act = ops.glu_fwd(up[:, F:], up[:, :F], self.cfg.kind)
         return xs, up, act
 
