@@ -74,6 +74,17 @@ __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool on) {
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
+// The next chunk's rows (64 of 128 elements of `es` bytes) on their way to L2.
+__device__ __forceinline__ void prefetch_rows(const char* src, long row_bytes, int es, int n, int tid) {
+  const int lines = es;                          // 128-byte lines in a row of 128 elements
+  for (int i = tid; i < C * lines; i += NT) {
+    const int r = i / lines;
+    if (r < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + r * row_bytes + (i - r * lines) * 128));
+  }
+}
+__device__ __forceinline__ void red_add4(float* p, float x, float y, float z, float w) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
 __device__ __forceinline__ void ldsm(uint32_t (&r)[4], uint32_t a) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
@@ -536,32 +547,66 @@ constexpr int kRevStage = 3 * kTile + 2 * kTri * 4;
 constexpr int kRevSmem = 2 * kRevStage + kRedR + sizeof(Gates) + 8 * C * 4;  // (the planes lie in the parts' place)
 static_assert(2 * 3 * kTri * 2 <= kRedR, "planes");
 
-// y = v - r of the warp's 16 value columns as accumulator tiles (rows = value columns, columns = the 8 tokens from i0).
-__device__ __forceinline__ void load_y_t(float (&y)[4], const Args& a, int t, int i0, int n, long vs, int hv, int col, int lane) {
+// y = v - r of the warp's 16 value columns as accumulator tiles (rows = value columns, columns = the chunk's tokens): asked for in
+// one go, all of it on its way at once, and put together where it is used.
+struct ColumnsOfY {
+  float r[8][4];
+  uint32_t v[8][2];
+  __device__ __forceinline__ void ask(const Args& a, int t, int n, long vs, int hv, int col, int lane) {
+    const int c = hv * DV + col + (lane >> 2);
+    const unsigned short* vp = reinterpret_cast<const unsigned short*>(a.v);
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const int i = i0 + (lane & 3) * 2 + (e & 1);
-    const int c = hv * DV + col + (lane >> 2) + (e >> 1) * 8;
-    y[e] = i < n ? __bfloat162float(a.v[(long)(t + i) * a.v_ts + c]) - a.r[(long)(t + i) * vs + c] : 0.f;
-  }
-}
-// Rows of an fp32 (T, HV, 128) tensor (or of y) as an A operand: tokens i0 .. i0 + 15 x 16 columns from col, times `f` per row.
-template <bool Y>
-__device__ __forceinline__ void load_rows_a(uint32_t (&s)[3][4], const Args& a, const float* x, const float* f, int t, int i0, int n,
-                                            long vs, int hv, int col, int lane) {
+    for (int nb = 0; nb < 8; ++nb)
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const int i = i0 + (lane >> 2) + (e & 1) * 8;
-    const int c = hv * DV + col + (lane & 3) * 2 + (e >> 1) * 8;
-    float2 u = make_float2(0.f, 0.f);
-    if (i < n) {
-      u = *reinterpret_cast<const float2*>(x + (long)(t + i) * vs + c);
-      if (Y) {
-        const float2 v = bf2(*reinterpret_cast<const uint32_t*>(a.v + (long)(t + i) * a.v_ts + c));
-        u = make_float2(v.x - u.x, v.y - u.y);
+      for (int h = 0; h < 2; ++h) {
+        const int i = nb * 8 + (lane & 3) * 2 + h;
+        const long ra = (long)(t + i) * vs + c, va = (long)(t + i) * a.v_ts + c;
+        const bool on = i < n;
+        r[nb][h] = on ? a.r[ra] : 0.f;
+        r[nb][2 + h] = on ? a.r[ra + 8] : 0.f;
+        v[nb][h] = on ? (uint32_t)vp[va] | (uint32_t)vp[va + 8] << 16 : 0u;
       }
-      if (f) { u.x *= f[i]; u.y *= f[i]; }
+  }
+  __device__ __forceinline__ void get(float (&y)[4], int nb) const {
+    const float2 v0 = bf2(v[nb][0]), v1 = bf2(v[nb][1]);
+    y[0] = v0.x - r[nb][0];
+    y[1] = v1.x - r[nb][1];
+    y[2] = v0.y - r[nb][2];
+    y[3] = v1.y - r[nb][3];
+  }
+};
+// The same columns with the tokens as rows, as A operands of 16 tokens x 16 columns, times beta.
+struct RowsOfY {
+  float2 r[4][4];
+  uint32_t v[4][4];
+  __device__ __forceinline__ void ask(const Args& a, int t, int n, long vs, int hv, int col, int lane) {
+#pragma unroll
+    for (int tt = 0; tt < 4; ++tt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = tt * 16 + (lane >> 2) + (e & 1) * 8;
+        const int c = hv * DV + col + (lane & 3) * 2 + (e >> 1) * 8;
+        r[tt][e] = i < n ? *reinterpret_cast<const float2*>(a.r + (long)(t + i) * vs + c) : make_float2(0.f, 0.f);
+        v[tt][e] = i < n ? *reinterpret_cast<const uint32_t*>(a.v + (long)(t + i) * a.v_ts + c) : 0u;
+      }
+  }
+  __device__ __forceinline__ void get(uint32_t (&s)[3][4], const float* bet, int tt, int lane) const {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 x = bf2(v[tt][e]);
+      const float b = bet[tt * 16 + (lane >> 2) + (e & 1) * 8];
+      split3((x.x - r[tt][e].x) * b, (x.y - r[tt][e].y) * b, s[0][e], s[1][e], s[2][e]);
     }
+  }
+};
+// fp32 rows of 128 in shared memory: the 16-byte piece c of row r lies at piece c ^ (r & 7).
+__device__ __forceinline__ uint32_t row32_at(int r, int c) { return r * 512 + ((c ^ (r & 7)) << 4); }
+// 16 rows x 16 columns of them as an A operand, three terms.
+__device__ __forceinline__ void rows_a(uint32_t (&s)[3][4], const char* rows, int i0, int col, int lane) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int c = col + (lane & 3) * 2 + (e >> 1) * 8;
+    const float2 u = *reinterpret_cast<const float2*>(rows + row32_at(i0 + (lane >> 2) + (e & 1) * 8, c >> 2) + (c & 3) * 4);
     split3(u.x, u.y, s[0][e], s[1][e], s[2][e]);
   }
 }
@@ -618,6 +663,12 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_reverse_kernel(const Args a) 
     make_gates(gt, a, slot0 + c, t, n, hv, tid);
     split_tri(planes_t, reinterpret_cast<const float*>(stage + 3 * kTile), tid);
     split_tri(planes_p, reinterpret_cast<const float*>(stage + 3 * kTile) + kTri, tid);
+    ColumnsOfY columns;
+    columns.ask(a, t, n, vs, hv, warp * 16, lane);
+    if (c > 0) {
+      prefetch_rows(reinterpret_cast<const char*>(a.r + (long)(t - C) * vs + hv * DV), vs * 4, 4, C, tid);
+      prefetch_rows(reinterpret_cast<const char*>(a.v + (long)(t - C) * a.v_ts + hv * DV), a.v_ts * 2, 2, C, tid);
+    }
     float R[8][4] = {};
 #pragma unroll
     for (int kb = 0; kb < 8; ++kb) {
@@ -651,7 +702,7 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_reverse_kernel(const Args a) 
 #pragma unroll
     for (int nb = 0; nb < 8; ++nb) {               // rhs . y over the warp's columns, then rhs <- -beta rhs
       float y[4];
-      load_y_t(y, a, t, nb * 8, n, vs, hv, warp * 16, lane);
+      columns.get(y, nb);
       float2 p = make_float2(R[nb][0] * y[0] + R[nb][2] * y[2], R[nb][1] * y[1] + R[nb][3] * y[3]);
 #pragma unroll
       for (int m = 4; m < 32; m <<= 1) {
@@ -665,6 +716,8 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_reverse_kernel(const Args a) 
       R[nb][2] *= -b.x;
       R[nb][3] *= -b.y;
     }
+    RowsOfY rows;
+    rows.ask(a, t, n, vs, hv, warp * 16, lane);
     float Z[8][4] = {};                            // dR^T
 #pragma unroll
     for (int jb = 0; jb < 4; ++jb) {
@@ -694,7 +747,7 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_reverse_kernel(const Args a) 
     {
       uint32_t s[4][3][4];
 #pragma unroll
-      for (int tt = 0; tt < 4; ++tt) load_rows_a<true>(s[tt], a, a.r, gt->bet, t, tt * 16, n, vs, hv, warp * 16, lane);
+      for (int tt = 0; tt < 4; ++tt) rows.get(s[tt], gt->bet, tt, lane);
       float kd = 0.f;                              // the thread's part of k . dk of its row
       const int row = tid >> 2, c8 = (tid & 3) * 8;
 #pragma unroll
@@ -793,14 +846,15 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_reverse_kernel(const Args a) 
 // W1 and W2 of the chunk from products over all value columns (warps share the ten lower blocks), then dQ and dK, 16 key
 // columns at a time: every warp its 16 value columns of the state's part, and one block column of W1 (warps 0-3) or W2 (4-7).
 constexpr int kPartLd = 20;
-constexpr int kParts = 2 * 8 * C * kPartLd * 4;                              // dQ and dK; the planes of Y lie in their place
+constexpr int kParts = 2 * 8 * C * kPartLd * 4;                              // dQ and dK; Y (planes) and dR lie in their place
 constexpr int kFinStage = 3 * kTile;
 constexpr int kFinSmem = 2 * kFinStage + kParts + 2 * 3 * kTri * 2 + sizeof(Gates) + C * 8 + 2 * 4 * C * 4;
-static_assert(3 * kTile <= kParts, "planes of Y");
+static_assert(3 * kTile + C * 512 <= kParts, "planes of Y, dR");
 
 __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
   extern __shared__ __align__(128) char sm[];
   char* y_s = sm + 2 * kFinStage;
+  char* dr_s = y_s + 3 * kTile;                                    // dR as it is, fp32
   float* parts = reinterpret_cast<float*>(y_s);
   char* w1_s = y_s + kParts;
   char* w2_s = w1_s + 3 * kTri * 2;
@@ -829,29 +883,52 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
   for (int c = 0; c < nc; ++c) {
     cp_wait_all();
     __syncthreads();
-    if (c + 1 < nc) fetch(c + 1);
     const uint32_t k_s = smem_addr(sm + (c & 1) * kFinStage), q_s = k_s + kTile, d_s = k_s + 2 * kTile;
     const int t = t0 + c * C, n = min(C, t1 - t);
+#pragma unroll
+    for (int i = tid; i < C * 32; i += NT) {
+      const int r = i >> 5, p = i & 31;
+      cp16(smem_addr(dr_s) + row32_at(r, p), a.dr + (long)(t + (r < n ? r : 0)) * vs + hv * DV + p * 4, r < n);
+    }
+    cp_commit();
+    if (c + 1 < nc) {
+      fetch(c + 1);
+      const int m = min(C, t1 - t - C);
+      prefetch_rows(reinterpret_cast<const char*>(a.r + (long)(t + C) * vs + hv * DV), vs * 4, 4, m, tid);
+      prefetch_rows(reinterpret_cast<const char*>(a.dr + (long)(t + C) * vs + hv * DV), vs * 4, 4, m, tid);
+      prefetch_rows(reinterpret_cast<const char*>(a.v + (long)(t + C) * a.v_ts + hv * DV), a.v_ts * 2, 2, m, tid);
+    } else {
+      cp_commit();
+    }
     make_gates(gt, a, slot0 + c, t, n, hv, tid);
     if (tid < C) gs[tid] = a.gsum[((slot0 + c) * a.HV + hv) * C + tid];
     for (int i = tid; i < 2 * 4 * C; i += NT) col1[i] = 0.f;
-    for (int i = tid; i < C * 16; i += NT) {       // y as three planes of (64, 128)
-      const int r = i >> 4, c8 = i & 15;
-      uint32_t p[3][4] = {};
-      if (r < n) {
+    {                                              // y as three planes of (64, 128)
+      uint4 vv[4];
+      float4 ra[4], rb[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = tid + u * NT, r = i >> 4, c8 = i & 15;
         const long at = (long)(t + r) * vs + hv * DV + c8 * 8;
-        const uint4 vv = *reinterpret_cast<const uint4*>(a.v + (long)(t + r) * a.v_ts + hv * DV + c8 * 8);
-        const float4 r0 = *reinterpret_cast<const float4*>(a.r + at), r1 = *reinterpret_cast<const float4*>(a.r + at + 4);
-        const float2 v0 = bf2(vv.x), v1 = bf2(vv.y), v2 = bf2(vv.z), v3 = bf2(vv.w);
-        split3(v0.x - r0.x, v0.y - r0.y, p[0][0], p[1][0], p[2][0]);
-        split3(v1.x - r0.z, v1.y - r0.w, p[0][1], p[1][1], p[2][1]);
-        split3(v2.x - r1.x, v2.y - r1.y, p[0][2], p[1][2], p[2][2]);
-        split3(v3.x - r1.z, v3.y - r1.w, p[0][3], p[1][3], p[2][3]);
+        vv[u] = r < n ? *reinterpret_cast<const uint4*>(a.v + (long)(t + r) * a.v_ts + hv * DV + c8 * 8) : make_uint4(0, 0, 0, 0);
+        ra[u] = r < n ? *reinterpret_cast<const float4*>(a.r + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+        rb[u] = r < n ? *reinterpret_cast<const float4*>(a.r + at + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
-      for (int j = 0; j < 3; ++j)
-        *reinterpret_cast<uint4*>(y_s + j * kTile + tile_at(r, c8)) = make_uint4(p[j][0], p[j][1], p[j][2], p[j][3]);
+      for (int u = 0; u < 4; ++u) {
+        const int i = tid + u * NT, r = i >> 4, c8 = i & 15;
+        uint32_t p[3][4];
+        const float2 v0 = bf2(vv[u].x), v1 = bf2(vv[u].y), v2 = bf2(vv[u].z), v3 = bf2(vv[u].w);
+        split3(v0.x - ra[u].x, v0.y - ra[u].y, p[0][0], p[1][0], p[2][0]);
+        split3(v1.x - ra[u].z, v1.y - ra[u].w, p[0][1], p[1][1], p[2][1]);
+        split3(v2.x - rb[u].x, v2.y - rb[u].y, p[0][2], p[1][2], p[2][2]);
+        split3(v3.x - rb[u].z, v3.y - rb[u].w, p[0][3], p[1][3], p[2][3]);
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          *reinterpret_cast<uint4*>(y_s + j * kTile + tile_at(r, c8)) = make_uint4(p[j][0], p[j][1], p[j][2], p[j][3]);
+      }
     }
+    asm volatile("cp.async.wait_group 1;" ::: "memory");           // dR; the next chunk's tiles may still be on their way
     __syncthreads();
     // blocks 0..9 of W2 on warps 0-4 (two each), blocks of W1 on warps 5-7
     const bool second = warp < 5;
@@ -868,7 +945,7 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
         for (int p = 0; p < 3; ++p) ldsm(y[p], smem_addr(y_s) + p * kTile + tile_rc(jb * 16, kb * 2, lane));
         if (second) {
           uint32_t s[3][4];
-          load_rows_a<false>(s, a, a.dr, nullptr, t, ib * 16, n, vs, hv, kb * 16, lane);
+          rows_a(s, dr_s, ib * 16, kb * 16, lane);
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const uint32_t bb[3][2] = {{y[0][2 * e], y[0][2 * e + 1]}, {y[1][2 * e], y[1][2 * e + 1]}, {y[2][2 * e], y[2][2 * e + 1]}};
@@ -921,7 +998,7 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
     }
     uint32_t dr[4][3][4];
 #pragma unroll
-    for (int tt = 0; tt < 4; ++tt) load_rows_a<false>(dr[tt], a, a.dr, nullptr, t, tt * 16, n, vs, hv, warp * 16, lane);
+    for (int tt = 0; tt < 4; ++tt) rows_a(dr[tt], dr_s, tt * 16, warp * 16, lane);
     __syncthreads();                               // W1, W2 are there; the parts take the place of y
     float sc = 0.f;
     const int which = tid >> 7, row = (tid & 127) >> 1, c8 = (tid & 1) * 8;      // 128 threads add up dQ, 128 dK
@@ -1017,16 +1094,18 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
       }
       if (row < n) {
         float4* p = reinterpret_cast<float4*>((which ? a.dk : a.dq) + ((long)(t + row) * a.HV + hv) * DK + np * 16 + c8);
-        if (which) {
-          const float4 u = p[0], v = p[1];
-          x[0] += u.x; x[1] += u.y; x[2] += u.z; x[3] += u.w;
-          x[4] += v.x; x[5] += v.y; x[6] += v.z; x[7] += v.w;
+        if (which) {                               // to what pass R wrote, one addition: no order to depend on
+          red_add4(reinterpret_cast<float*>(p), x[0], x[1], x[2], x[3]);
+          red_add4(reinterpret_cast<float*>(p + 1), x[4], x[5], x[6], x[7]);
+        } else {
+          p[0] = make_float4(x[0], x[1], x[2], x[3]);
+          p[1] = make_float4(x[4], x[5], x[6], x[7]);
         }
-        p[0] = make_float4(x[0], x[1], x[2], x[3]);
-        p[1] = make_float4(x[4], x[5], x[6], x[7]);
       }
       __syncthreads();
     }
+    ColumnsOfY columns;
+    columns.ask(a, t, n, vs, hv, warp * 16, lane);
     // per-token scalars: q.dq + k.(W2 K + S^ dr) - k.(W1^T Q + W2^T K), the last by the column sums (k.dk has it with the sign turned)
     sc += __shfl_xor_sync(0xffffffffu, sc, 1);
     float* sums = parts;                           // [2][64]
@@ -1052,7 +1131,7 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int i = (2 * tb + h) * 8;
-        load_y_t(x[h], a, t, i, n, vs, hv, warp * 16, lane);
+        columns.get(x[h], 2 * tb + h);
         const float2 d = *reinterpret_cast<const float2*>(gt->dec + i + (lane & 3) * 2);
         const float2 b = *reinterpret_cast<const float2*>(gt->bet + i + (lane & 3) * 2);
         x[h][0] = x[h][0] * b.x * d.x;
