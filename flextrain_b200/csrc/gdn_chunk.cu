@@ -16,7 +16,9 @@
 // Precision.  q, k, v, dO are bf16 and enter the products as they are.  Everything the recurrence keeps in fp32 (state,
 // inverse, Y, dR, decayed products) enters as the sum of three bf16 terms, cut so that the sum is the fp32 number itself; of
 // the nine products of two such operands the six largest are formed, which leaves out 2^-24 of the result.  Sums are fp32
-// throughout, G is summed in fp64 (differences of it are taken), the inverse is a forward substitution in fp32.
+// throughout, G is summed in fp64 (differences of it are taken), the inverse is a forward substitution in fp32.  The tensor
+// cores cut off what they add to an accumulator below its last bit, so a product over 16 has an accumulator of its own, which
+// starts at zero and takes the smaller terms first, and is added to the sum in fp32, rounded to nearest.
 //
 // Why mma.sync and not tcgen05: the chain of a sequence is state -> prediction -> solve -> state.  A warp owns 16 of the 128
 // value columns, which never meet those of another warp, and holds its slice of the state transposed as the accumulators of
@@ -24,6 +26,12 @@
 // registers: no round trip through shared or tensor memory and no barrier between its products.  Shared memory holds only
 // what the warps share (K, Q, the inverse).  The backward products that sum over value columns (dQ, dK) are added up over
 // the eight warps through shared memory.
+//
+// Measured, ms, token by token (gdn.cu) / so, 32 heads: 16 x 1024 tokens forward 2.19 / 1.05, backward 7.98 / 5.1; one sequence of
+// 16384 7.5 / 3.2 and 25.4 / 18.5; 300 sequences of 33, mostly half-empty chunks, 1.60 / 1.29 and 5.16 / 5.33.  Errors against fp64 (2-norm, gates as a
+// model's): final state 4.8e-8 / 6.9e-8, dq 1.16e-7 / 1.13e-7, dk 1.54e-7 / 1.14e-7, dg 1.0e-5 / 5.5e-6; with slow decay (0.01 a token) 2.0e-6 /
+// 1.4e-7, 1.6e-6 / 1.8e-7, 2.0e-6 / 2.3e-7.  What bounds it now: mma.sync at 537 TFLOP/s, reached to two thirds forward and a third
+// backward, where the warps meet sixteen times a chunk.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -53,7 +61,7 @@ struct Args {
   float* dq;               // (T, HV, 128)  pass F
   float* dk;               // (T, HV, 128)  pass R writes the part of X, pass F adds the rest
   float* sacc;             // (T, HV)       q.dq - k.(dS' e) + k.(S^ dr), as in gdn.cu: pass R writes, pass F adds
-  float* tri_t;            // (slots, HV, 10, 16, 16)  (I + L B)^-1
+  float* tri_t;            // (slots, HV, 10, 16, 16)  (I + L B)^-1 - I  (the identity is added in fp32)
   float* tri_p;            // (slots, HV, 10, 16, 16)  P
   double* gsum;            // (slots, HV, 64)          G in powers of two
   int* order;              // (nseq)  sequences, longest first
@@ -108,6 +116,12 @@ __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint3
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+__device__ __forceinline__ void mma_zero(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+
 // Two fp32 numbers as three packed pairs of bf16 whose sum they are (each term is the upper half of what the ones before leave).
 __device__ __forceinline__ void split3(float x, float y, uint32_t& t0, uint32_t& t1, uint32_t& t2) {
   const uint32_t xu = __float_as_uint(x), yu = __float_as_uint(y);
@@ -125,14 +139,44 @@ __device__ __forceinline__ void split_a(const float (&lo)[4], const float (&hi)[
   split3(hi[0], hi[1], a[0][2], a[1][2], a[2][2]);
   split3(hi[2], hi[3], a[0][3], a[1][3], a[2][3]);
 }
-// c += a b with both operands in three terms, the smallest products first.
-__device__ __forceinline__ void mma6(float (&c)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2]) {
-  mma(c, a[2], b[0][0], b[0][1]);
-  mma(c, a[0], b[2][0], b[2][1]);
-  mma(c, a[1], b[1][0], b[1][1]);
-  mma(c, a[1], b[0][0], b[0][1]);
-  mma(c, a[0], b[1][0], b[1][1]);
-  mma(c, a[0], b[0][0], b[0][1]);
+__device__ __forceinline__ void add4(float (&c)[4], const float (&d)[4]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) c[e] += d[e];
+}
+// c += a b, the smaller products first: a in three terms, b as it is
+__device__ __forceinline__ void prod3(float (&c)[4], const uint32_t (&a)[3][4], uint32_t b0, uint32_t b1) {
+  float d[4];
+  mma_zero(d, a[2], b0, b1);
+  mma(d, a[1], b0, b1);
+  mma(d, a[0], b0, b1);
+  add4(c, d);
+}
+// a as it is, b in three terms
+__device__ __forceinline__ void prod3(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[3][2]) {
+  float d[4];
+  mma_zero(d, a, b[2][0], b[2][1]);
+  mma(d, a, b[1][0], b[1][1]);
+  mma(d, a, b[0][0], b[0][1]);
+  add4(c, d);
+}
+// both in three terms
+__device__ __forceinline__ void prod6(float (&c)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2]) {
+  float d[4];
+  mma_zero(d, a[2], b[0][0], b[0][1]);
+  mma(d, a[0], b[2][0], b[2][1]);
+  mma(d, a[1], b[1][0], b[1][1]);
+  mma(d, a[1], b[0][0], b[0][1]);
+  mma(d, a[0], b[1][0], b[1][1]);
+  mma(d, a[0], b[0][0], b[0][1]);
+  add4(c, d);
+}
+// the fragments of two neighbouring tiles in three planes: those of tile e
+__device__ __forceinline__ void pick(uint32_t (&b)[3][2], const uint32_t (&planes)[3][4], int e) {
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+    b[p][0] = planes[p][2 * e];
+    b[p][1] = planes[p][2 * e + 1];
+  }
 }
 __device__ __forceinline__ float2 bf2(uint32_t u) {
   return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
@@ -140,6 +184,23 @@ __device__ __forceinline__ float2 bf2(uint32_t u) {
 __device__ __forceinline__ uint32_t pack_bf(float x, float y) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
   return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// 2^x for a difference of sums: the whole part goes into the exponent, 2^f, |f| <= 1/2, by its series (the term of f^8 is below
+// 6e-9).  The hardware's approximation is off by 2^-22, and rounding x to fp32 first would cost another |x| 2^-25.
+__device__ __forceinline__ float exp2_of(double x) {
+  if (x < -126.0) return 0.f;
+  if (x > 127.0) return x > 128.0 ? __int_as_float(0x7f800000) : exp2f((float)x);
+  const float n = rintf((float)x), f = (float)(x - (double)n);
+  float p = 1.52527338e-5f;                        // ln(2)^k / k!, k = 7 .. 0
+  p = p * f + 1.54035304e-4f;
+  p = p * f + 1.33335581e-3f;
+  p = p * f + 9.61812911e-3f;
+  p = p * f + 5.55041087e-2f;
+  p = p * f + 2.40226507e-1f;
+  p = p * f + 6.93147181e-1f;
+  p = p * f + 1.f;
+  return p * __int_as_float(((int)n + 127) << 23);
 }
 
 // ---- shared-memory tiles.  (64, 128) bf16 with 256-byte rows: the 16-byte piece c of row r lies at piece c ^ (r & 7).
@@ -185,7 +246,7 @@ __device__ __forceinline__ void split_tri(char* planes, const float* src, int ti
 constexpr int kLd = 68;                                           // floats in a row of L B
 constexpr int kPrepSmem = 2 * C * 256 + 2 * C * kLd * 4 + 2 * C * 8 + 2 * C * 4;
 
-__global__ void __launch_bounds__(128) gdn_prep_kernel(const Args a) {
+__global__ void __launch_bounds__(128, 3) gdn_prep_kernel(const Args a) {
   extern __shared__ __align__(128) char sm[];
   char* k_s = sm;
   char* q_s = sm + C * 256;
@@ -287,7 +348,7 @@ __global__ void __launch_bounds__(128) gdn_prep_kernel(const Args a) {
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int i = warp * 16 + (lane >> 2) + (e >> 1) * 8, j = nb * 8 + (lane & 3) * 2 + (e & 1);
-            const float d = i >= j ? exp2f((float)(gs[h * C + i] - gs[h * C + j])) : 0.f;
+            const float d = i >= j ? exp2_of(gs[h * C + i] - gs[h * C + j]) : 0.f;
             lb[(h * C + i) * kLd + j] = i > j ? d * kk[nb][e] * bs[h * C + j] : 0.f;
             a.tri_p[at + blk_of(warp, nb >> 1) * 256 + (i & 15) * 16 + (j & 15)] = i >= j ? a.scale * d * qk[nb][e] : 0.f;
           }
@@ -313,7 +374,7 @@ __global__ void __launch_bounds__(128) gdn_prep_kernel(const Args a) {
       float* out = a.tri_t + ((long)slot * a.HV + hk * rep + h0 + h) * kTri;
 #pragma unroll
       for (int i = 0; i < C; ++i)
-        if ((j >> 4) <= (i >> 4)) out[blk_of(i >> 4, j >> 4) * 256 + (i & 15) * 16 + (j & 15)] = y[i];
+        if ((j >> 4) <= (i >> 4)) out[blk_of(i >> 4, j >> 4) * 256 + (i & 15) * 16 + (j & 15)] = i == j ? 0.f : y[i];
     }
   }
 }
@@ -332,10 +393,10 @@ __device__ __forceinline__ void make_gates(Gates* s, const Args& a, long slot, i
   if (tid < C) {
     const double* gs = a.gsum + (slot * a.HV + hv) * C;
     const double gi = gs[tid], gc = gs[C - 1];
-    s->gam[tid] = exp2f((float)gi);
-    s->dec[tid] = exp2f((float)(gc - gi));
+    s->gam[tid] = exp2_of(gi);
+    s->dec[tid] = exp2_of(gc - gi);
     s->bet[tid] = tid < n ? a.beta[(long)(t0 + tid) * a.HV + hv] : 0.f;
-    if (tid == 0) s->end = exp2f((float)gc);
+    if (tid == 0) s->end = exp2_of(gc);
   }
 }
 
@@ -360,11 +421,8 @@ __device__ __forceinline__ void state_times_tile(float (&acc)[8][4], const uint3
   for (int np = 0; np < 4; ++np) {
     uint32_t b[4];
     ldsm(b, tile + tile_rc(np * 16, kb * 2, lane));
-#pragma unroll
-    for (int p = 2; p >= 0; --p) {
-      mma(acc[2 * np], s[p], b[0], b[1]);
-      mma(acc[2 * np + 1], s[p], b[2], b[3]);
-    }
+    prod3(acc[2 * np], s, b[0], b[1]);
+    prod3(acc[2 * np + 1], s, b[2], b[3]);
   }
 }
 // state^T (16 x 128) += x^T (16 x 16 tokens of block tb, three terms) X (those tokens of the tile).
@@ -373,28 +431,26 @@ __device__ __forceinline__ void state_add(float (&st)[16][4], const uint32_t (&x
   for (int np = 0; np < 8; ++np) {
     uint32_t b[4];
     ldsm_t(b, tile + tile_cr(tb * 16, np * 2, lane));
-#pragma unroll
-    for (int p = 2; p >= 0; --p) {
-      mma(st[2 * np], x[p], b[0], b[1]);
-      mma(st[2 * np + 1], x[p], b[2], b[3]);
-    }
+    prod3(st[2 * np], x, b[0], b[1]);
+    prod3(st[2 * np + 1], x, b[2], b[3]);
   }
 }
 // acc^T (16 x 64 tokens i) += x^T (16 x 64 tokens j) M^T for the lower triangular M (three planes of blocks): columns j <= i.
+// acc may be x: a block is read before anything is added to it.
 __device__ __forceinline__ void tri_times(float (&acc)[8][4], const float (&x)[8][4], uint32_t planes, int lane) {
 #pragma unroll
-  for (int jb = 0; jb < 4; ++jb) {
+  for (int jb = 3; jb >= 0; --jb) {
     uint32_t s[3][4];
     split_a(x[2 * jb], x[2 * jb + 1], s);
 #pragma unroll
     for (int ib = jb; ib < 4; ++ib) {
-      uint32_t b[3][4];
+      uint32_t b[3][4], bb[3][2];
 #pragma unroll
       for (int p = 0; p < 3; ++p) ldsm(b[p], planes + p * kTri * 2 + blk_of(ib, jb) * 512 + blk_rc(lane));
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const uint32_t bb[3][2] = {{b[0][2 * e], b[0][2 * e + 1]}, {b[1][2 * e], b[1][2 * e + 1]}, {b[2][2 * e], b[2][2 * e + 1]}};
-        mma6(acc[2 * ib + e], s, bb);
+        pick(bb, b, e);
+        prod6(acc[2 * ib + e], s, bb);
       }
     }
   }
@@ -481,8 +537,8 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_forward_kernel(const Args a) 
         O[nb][3] *= a.scale * gm.y;
       }
     }
-    float Y[8][4] = {};
-    tri_times(Y, R, smem_addr(planes_t), lane);
+    tri_times(R, R, smem_addr(planes_t), lane);
+    float (&Y)[8][4] = R;
     if (a.r) {
 #pragma unroll
       for (int np = 0; np < 4; ++np) {
@@ -690,14 +746,16 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_reverse_kernel(const Args a) 
       uint32_t x[4];
       ldsm_t(x, d_s + tile_rc(jb * 16, warp * 2, lane));
 #pragma unroll
-      for (int ib = 0; ib <= jb; ++ib)
+      for (int ib = 0; ib <= jb; ++ib) {
+        uint32_t b[3][4], bb[3][2];
 #pragma unroll
-        for (int p = 2; p >= 0; --p) {
-          uint32_t b[4];
-          ldsm_t(b, smem_addr(planes_p) + p * kTri * 2 + blk_of(jb, ib) * 512 + blk_cr(lane));
-          mma(R[2 * ib], x, b[0], b[1]);
-          mma(R[2 * ib + 1], x, b[2], b[3]);
+        for (int p = 0; p < 3; ++p) ldsm_t(b[p], smem_addr(planes_p) + p * kTri * 2 + blk_of(jb, ib) * 512 + blk_cr(lane));
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          pick(bb, b, e);
+          prod3(R[2 * ib + e], x, bb);
         }
+      }
     }
 #pragma unroll
     for (int nb = 0; nb < 8; ++nb) {               // rhs . y over the warp's columns, then rhs <- -beta rhs
@@ -716,25 +774,25 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_reverse_kernel(const Args a) 
       R[nb][2] *= -b.x;
       R[nb][3] *= -b.y;
     }
-    RowsOfY rows;
-    rows.ask(a, t, n, vs, hv, warp * 16, lane);
-    float Z[8][4] = {};                            // dR^T
 #pragma unroll
-    for (int jb = 0; jb < 4; ++jb) {
+    for (int jb = 0; jb < 4; ++jb) {               // dR^T, block by block in place (block jb is read before anything is added to it)
       uint32_t s[3][4];
       split_a(R[2 * jb], R[2 * jb + 1], s);
 #pragma unroll
       for (int ib = 0; ib <= jb; ++ib) {
-        uint32_t b[3][4];
+        uint32_t b[3][4], bb[3][2];
 #pragma unroll
         for (int p = 0; p < 3; ++p) ldsm_t(b[p], smem_addr(planes_t) + p * kTri * 2 + blk_of(jb, ib) * 512 + blk_cr(lane));
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const uint32_t bb[3][2] = {{b[0][2 * e], b[0][2 * e + 1]}, {b[1][2 * e], b[1][2 * e + 1]}, {b[2][2 * e], b[2][2 * e + 1]}};
-          mma6(Z[2 * ib + e], s, bb);
+          pick(bb, b, e);
+          prod6(R[2 * ib + e], s, bb);
         }
       }
     }
+    float (&Z)[8][4] = R;
+    RowsOfY rows;
+    rows.ask(a, t, n, vs, hv, warp * 16, lane);
 #pragma unroll
     for (int nb = 0; nb < 8; ++nb) {
       const int i = nb * 8 + (lane & 3) * 2;
@@ -759,7 +817,7 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_reverse_kernel(const Args a) 
 #pragma unroll
           for (int tt = 0; tt < 4; ++tt) {
             float acc[4] = {};
-            mma6(acc, s[tt], b);
+            prod6(acc, s[tt], b);
             float* p = red + (warp * C + tt * 16 + (lane >> 2)) * kRedLd + u * 8 + (lane & 3) * 2;
             *reinterpret_cast<float2*>(p) = make_float2(acc[0], acc[1]);
             *reinterpret_cast<float2*>(p + 8 * kRedLd) = make_float2(acc[2], acc[3]);
@@ -843,12 +901,12 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_reverse_kernel(const Args a) 
 }
 
 // ================================================================================================ backward, forward in time
-// W1 and W2 of the chunk from products over all value columns (warps share the ten lower blocks), then dQ and dK, 16 key
-// columns at a time: every warp its 16 value columns of the state's part, and one block column of W1 (warps 0-3) or W2 (4-7).
+// W1 and W2 of the chunk from products over all value columns (warps share the ten lower blocks; the diagonal of W1 stays in
+// fp32, aside), then dQ and dK, 16 key columns at a time: every warp its 16 value columns of the state's part, and one block column of W1 (warps 0-3) or W2 (4-7).
 constexpr int kPartLd = 20;
 constexpr int kParts = 2 * 8 * C * kPartLd * 4;                              // dQ and dK; Y (planes) and dR lie in their place
 constexpr int kFinStage = 3 * kTile;
-constexpr int kFinSmem = 2 * kFinStage + kParts + 2 * 3 * kTri * 2 + sizeof(Gates) + C * 8 + 2 * 4 * C * 4;
+constexpr int kFinSmem = 2 * kFinStage + kParts + 2 * 3 * kTri * 2 + sizeof(Gates) + C * 8 + 2 * 4 * C * 4 + C * 4;
 static_assert(3 * kTile + C * 512 <= kParts, "planes of Y, dR");
 
 __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
@@ -859,9 +917,10 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
   char* w1_s = y_s + kParts;
   char* w2_s = w1_s + 3 * kTri * 2;
   double* gs = reinterpret_cast<double*>(w2_s + 3 * kTri * 2);     // [64]
-  float* col1 = reinterpret_cast<float*>(gs + C);                  // [4][64] column sums of W1 o QK^T, by block row
+  float* col1 = reinterpret_cast<float*>(gs + C);                  // [4][64] column sums of W1 o QK^T without its diagonal, by block row
   float* col2 = col1 + 4 * C;                                      // [4][64] of D o KK^T o (dR Y^T)
   Gates* gt = reinterpret_cast<Gates*>(col2 + 4 * C);
+  float* diag = reinterpret_cast<float*>(gt + 1);                  // [64] the diagonal of W1
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int hv = blockIdx.x, seq = a.order[blockIdx.y];
   const int hk = hv / (a.HV / a.HK);
@@ -943,20 +1002,21 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
         uint32_t y[3][4], f[4], b[4];
 #pragma unroll
         for (int p = 0; p < 3; ++p) ldsm(y[p], smem_addr(y_s) + p * kTile + tile_rc(jb * 16, kb * 2, lane));
+        uint32_t bb[3][2];
         if (second) {
           uint32_t s[3][4];
           rows_a(s, dr_s, ib * 16, kb * 16, lane);
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const uint32_t bb[3][2] = {{y[0][2 * e], y[0][2 * e + 1]}, {y[1][2 * e], y[1][2 * e + 1]}, {y[2][2 * e], y[2][2 * e + 1]}};
-            mma6(m[e], s, bb);
+            pick(bb, y, e);
+            prod6(m[e], s, bb);
           }
         } else {
           ldsm(f, d_s + tile_cr(ib * 16, kb * 2, lane));
 #pragma unroll
-          for (int p = 2; p >= 0; --p) {
-            mma(m[0], f, y[p][0], y[p][1]);
-            mma(m[1], f, y[p][2], y[p][3]);
+          for (int e = 0; e < 2; ++e) {
+            pick(bb, y, e);
+            prod3(m[e], f, bb);
           }
         }
         ldsm(f, (second ? k_s : q_s) + tile_cr(ib * 16, kb * 2, lane));
@@ -973,8 +1033,10 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
         for (int h = 0; h < 2; ++h) {
           const int i = ib * 16 + (lane >> 2) + h * 8, j = jb * 16 + e * 8 + (lane & 3) * 2;
           float d0 = 0.f, d1 = 0.f;
-          if (second ? i > j : i >= j) d0 = exp2f((float)(gs[i] - gs[j]));
-          if (second ? i > j + 1 : i >= j + 1) d1 = exp2f((float)(gs[i] - gs[j + 1]));
+          if (i > j) d0 = exp2_of(gs[i] - gs[j]);
+          if (i > j + 1) d1 = exp2_of(gs[i] - gs[j + 1]);
+          if (!second && i == j) diag[i] = (m[e][2 * h]) * (a.scale * gt->bet[i]);
+          if (!second && i == j + 1) diag[i] = (m[e][2 * h + 1]) * (a.scale * gt->bet[i]);
           d0 *= m[e][2 * h];
           d1 *= m[e][2 * h + 1];
           if (!second) { d0 *= a.scale * gt->bet[j]; d1 *= a.scale * gt->bet[j + 1]; }
@@ -1003,35 +1065,11 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
     float sc = 0.f;
     const int which = tid >> 7, row = (tid & 127) >> 1, c8 = (tid & 1) * 8;      // 128 threads add up dQ, 128 dK
     const int jb = warp & 3;
+    const float w_ii = diag[row];
     const uint32_t w_s = smem_addr(warp < 4 ? w1_s : w2_s);
 #pragma unroll
     for (int np = 0; np < 8; ++np) {
-      float q2[2][4][4], k2[2][4][4];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        uint32_t b[3][2];
-        state_b(b, S[2 * np + e]);
-#pragma unroll
-        for (int tt = 0; tt < 4; ++tt) {
-          uint32_t f[4];
-          ldsm(f, d_s + tile_cr(tt * 16, warp * 2, lane));
-#pragma unroll
-          for (int j = 0; j < 4; ++j) q2[e][tt][j] = k2[e][tt][j] = 0.f;
-          mma(q2[e][tt], f, b[2][0], b[2][1]);
-          mma(q2[e][tt], f, b[1][0], b[1][1]);
-          mma(q2[e][tt], f, b[0][0], b[0][1]);
-          mma6(k2[e][tt], dr[tt], b);
-          const float g0 = gt->gam[tt * 16 + (lane >> 2)], g1 = gt->gam[tt * 16 + (lane >> 2) + 8];
-          k2[e][tt][0] *= g0;
-          k2[e][tt][1] *= g0;
-          k2[e][tt][2] *= g1;
-          k2[e][tt][3] *= g1;
-          q2[e][tt][0] *= a.scale * g0;
-          q2[e][tt][1] *= a.scale * g0;
-          q2[e][tt][2] *= a.scale * g1;
-          q2[e][tt][3] *= a.scale * g1;
-        }
-      }
+      float q2[2][4][4] = {}, k2[2][4][4] = {};
       uint32_t kf[4], qf[4];
       ldsm_t(kf, k_s + tile_cr(jb * 16, np * 2, lane));
       if (warp < 4) ldsm_t(qf, q_s + tile_cr(jb * 16, np * 2, lane));
@@ -1040,28 +1078,45 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
         for (int j = 0; j < 4; ++j) qf[j] = kf[j];
 #pragma unroll
       for (int tt = 0; tt < 4; ++tt) {
+        uint32_t w[3][4];
         if (tt >= jb) {                            // W1 K into dQ, W2 K into dK
 #pragma unroll
-          for (int p = 2; p >= 0; --p) {
-            uint32_t w[4];
-            ldsm(w, w_s + p * kTri * 2 + blk_of(tt, jb) * 512 + blk_cr(lane));
-            if (warp < 4) {
-              mma(q2[0][tt], w, kf[0], kf[1]);
-              mma(q2[1][tt], w, kf[2], kf[3]);
-            } else {
-              mma(k2[0][tt], w, kf[0], kf[1]);
-              mma(k2[1][tt], w, kf[2], kf[3]);
-            }
+          for (int p = 0; p < 3; ++p) ldsm(w[p], w_s + p * kTri * 2 + blk_of(tt, jb) * 512 + blk_cr(lane));
+          if (warp < 4) {
+            prod3(q2[0][tt], w, kf[0], kf[1]);
+            prod3(q2[1][tt], w, kf[2], kf[3]);
+          } else {
+            prod3(k2[0][tt], w, kf[0], kf[1]);
+            prod3(k2[1][tt], w, kf[2], kf[3]);
           }
         }
         if (tt <= jb) {                            // W1^T Q and W2^T K into dK
 #pragma unroll
-          for (int p = 2; p >= 0; --p) {
-            uint32_t w[4];
-            ldsm_t(w, w_s + p * kTri * 2 + blk_of(jb, tt) * 512 + blk_rc(lane));
-            mma(k2[0][tt], w, qf[0], qf[1]);
-            mma(k2[1][tt], w, qf[2], qf[3]);
-          }
+          for (int p = 0; p < 3; ++p) ldsm_t(w[p], w_s + p * kTri * 2 + blk_of(jb, tt) * 512 + blk_rc(lane));
+          prod3(k2[0][tt], w, qf[0], qf[1]);
+          prod3(k2[1][tt], w, qf[2], qf[3]);
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {                // the state's part
+        uint32_t b[3][2];
+        state_b(b, S[2 * np + e]);
+#pragma unroll
+        for (int tt = 0; tt < 4; ++tt) {
+          uint32_t f[4];
+          ldsm(f, d_s + tile_cr(tt * 16, warp * 2, lane));
+          float u[4] = {}, v[4] = {};
+          prod3(u, f, b);
+          prod6(v, dr[tt], b);
+          const float g0 = gt->gam[tt * 16 + (lane >> 2)], g1 = gt->gam[tt * 16 + (lane >> 2) + 8];
+          q2[e][tt][0] += u[0] * (a.scale * g0);
+          q2[e][tt][1] += u[1] * (a.scale * g0);
+          q2[e][tt][2] += u[2] * (a.scale * g1);
+          q2[e][tt][3] += u[3] * (a.scale * g1);
+          k2[e][tt][0] += v[0] * g0;
+          k2[e][tt][1] += v[1] * g0;
+          k2[e][tt][2] += v[2] * g1;
+          k2[e][tt][3] += v[3] * g1;
         }
       }
 #pragma unroll
@@ -1084,13 +1139,17 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
         x[0] += u.x; x[1] += u.y; x[2] += u.z; x[3] += u.w;
         x[4] += v.x; x[5] += v.y; x[6] += v.z; x[7] += v.w;
       }
-      uint32_t kr[4];
-      asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(kr[0]), "=r"(kr[1]), "=r"(kr[2]), "=r"(kr[3])
+      uint32_t own[4], other[4];                   // the row of q (dQ) or k (dK), and the other one, which the diagonal multiplies
+      asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(own[0]), "=r"(own[1]), "=r"(own[2]), "=r"(own[3])
                    : "r"((which ? k_s : q_s) + tile_at(row, np * 2 + (tid & 1))) : "memory");
+      asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(other[0]), "=r"(other[1]), "=r"(other[2]), "=r"(other[3])
+                   : "r"((which ? q_s : k_s) + tile_at(row, np * 2 + (tid & 1))) : "memory");
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float2 f = bf2(kr[e]);
+        const float2 f = bf2(own[e]), g = bf2(other[e]);
         sc += f.x * x[2 * e] + f.y * x[2 * e + 1];
+        x[2 * e] += w_ii * g.x;
+        x[2 * e + 1] += w_ii * g.y;
       }
       if (row < n) {
         float4* p = reinterpret_cast<float4*>((which ? a.dk : a.dq) + ((long)(t + row) * a.HV + hv) * DK + np * 16 + c8);
@@ -1106,7 +1165,8 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
     }
     ColumnsOfY columns;
     columns.ask(a, t, n, vs, hv, warp * 16, lane);
-    // per-token scalars: q.dq + k.(W2 K + S^ dr) - k.(W1^T Q + W2^T K), the last by the column sums (k.dk has it with the sign turned)
+    // per-token scalars: q.dq + k.(W2 K + S^ dr) - k.(W1^T Q + W2^T K), the last by the column sums (k.dk has it with the sign
+    // turned).  The diagonal of W1 has no part in them (q.dq and k.dk have the same from it) and would only cancel.
     sc += __shfl_xor_sync(0xffffffffu, sc, 1);
     float* sums = parts;                           // [2][64]
     if ((tid & 1) == 0) sums[which * C + row] = sc;

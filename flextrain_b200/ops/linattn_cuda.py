@@ -165,9 +165,11 @@ def _gdn(pass_, q, k, v, g, beta, cu, state_in, state_out, o, r, d_o, de, dv, db
     _check(rc, f"ftb_gdn(pass {pass_})")
 
 
-def _chunked(q: torch.Tensor, v: torch.Tensor, *rest: torch.Tensor) -> bool:
-    """Heads of 128 x 128 on 16 bytes run in chunks on the tensor cores (``csrc/gdn_chunk.cu``); see there for the figures."""
-    return q.shape[2] == 128 and v.shape[2] == 128 and all(t.data_ptr() % 16 == 0 for t in (q, v, *rest))
+def _chunked(S: int, q: torch.Tensor, v: torch.Tensor, *rest: torch.Tensor) -> bool:
+    """Heads of 128 x 128 on 16 bytes run in chunks of 64 tokens on the tensor cores (``csrc/gdn_chunk.cu``, with the figures);
+    sequences of fewer than 40 tokens on average leave their chunks too empty for that and go token by token."""
+    return (q.shape[2] == 128 and v.shape[2] == 128 and q.shape[0] >= 40 * S
+            and all(t.data_ptr() % 16 == 0 for t in (q, v, *rest)))
 
 
 def _head_rows(x: torch.Tensor) -> bool:
@@ -192,7 +194,7 @@ def gdn_fwd(q, k, v, g, beta, cu, state_in=None, scale=None, want_r=False):
     fin = torch.empty(S, HV, DK, DV, dtype=F32, device=q.device)
     r = torch.empty(T, HV, DV, dtype=F32, device=q.device) if want_r else None
     sin = state_in.to(F32).contiguous() if state_in is not None else None
-    if _chunked(q, v, k) and _head_rows(v):
+    if _chunked(S, q, v, k) and _head_rows(v):
         work = _chunk_work(T, S, HV, q.device)
         rc = load("gdn_chunk").ftb_gdn_chunk_fwd(
             _ptr(q), _ptr(k), _ptr(v), c_long(v.stride(0)), _ptr(g), _ptr(beta), _ptr(cu), c_int(S), c_long(T), _ptr(sin), _ptr(fin),
@@ -219,7 +221,7 @@ def gdn_bwd(q, k, v, g, beta, cu, state_in, final_state, r, d_o, dstate_final=No
     dsf = dstate_final.to(F32).contiguous() if dstate_final is not None else None
     sin = state_in.to(F32).contiguous() if state_in is not None else None
     d_o = d_o.contiguous()
-    chunked = _chunked(q, v, k, r, d_o) and _head_rows(v)
+    chunked = _chunked(S, q, v, k, r, d_o) and _head_rows(v)
     new = torch.empty if chunked and S > 0 else torch.zeros          # (the recurrent kernels add into these)
     de = torch.empty(T, HV, DV, dtype=F32, device=dev)
     dv = dv_out

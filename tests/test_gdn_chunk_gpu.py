@@ -43,8 +43,9 @@ def _rel(a, b):
 
 
 @pytest.mark.parametrize("lens,HK,HV,decay,with_state", [
-    ([1], 1, 1, 0.2, True),
+    ([1], 1, 1, 0.2, True),                        # token by token
     ([63, 64, 65, 1, 17], 2, 4, 0.2, True),
+    ([40], 1, 1, 0.2, True),                       # the shortest that goes in a chunk
     ([128, 0, 129], 1, 3, 0.2, True),              # an empty sequence, an odd number of value heads
     ([200], 2, 2, 0.0, False),                     # no decay at all
     ([150, 90], 1, 2, 5.0, True),                  # strong decay: most of a chunk forgotten inside it
