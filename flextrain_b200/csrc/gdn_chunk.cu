@@ -90,8 +90,8 @@ __device__ __forceinline__ void prefetch_rows(const char* src, long row_bytes, i
     if (r < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + r * row_bytes + (i - r * lines) * 128));
   }
 }
-__device__ __forceinline__ void red_add4(float* p, float x, float y, float z, float w) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+__device__ __forceinline__ void red_add2(float* p, float x, float y) {
+  asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(x), "f"(y) : "memory");
 }
 __device__ __forceinline__ void ldsm(uint32_t (&r)[4], uint32_t a) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -902,25 +902,26 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_reverse_kernel(const Args a) 
 
 // ================================================================================================ backward, forward in time
 // W1 and W2 of the chunk from products over all value columns (warps share the ten lower blocks; the diagonal of W1 stays in
-// fp32, aside), then dQ and dK, 16 key columns at a time: every warp its 16 value columns of the state's part, and one block column of W1 (warps 0-3) or W2 (4-7).
-constexpr int kPartLd = 20;
-constexpr int kParts = 2 * 8 * C * kPartLd * 4;                              // dQ and dK; Y (planes) and dR lie in their place
-constexpr int kFinStage = 3 * kTile;
-constexpr int kFinSmem = 2 * kFinStage + kParts + 2 * 3 * kTri * 2 + sizeof(Gates) + C * 8 + 2 * 4 * C * 4 + C * 4;
-static_assert(3 * kTile + C * 512 <= kParts, "planes of Y, dR");
+// fp32, aside), then dQ and dK: a warp has 16 tokens and 64 key columns of both, and sums over all value columns by itself.  The
+// state goes through shared memory for that, as three planes of bf16; its place is that of Y, which is done with by then.  (With
+// every warp multiplying its own value columns, and the parts of dQ and dK added up over the warps, 16 key columns at a time,
+// the warps met sixteen times a chunk and moved 1 MB through shared memory: 3.0 ms for 16 x 1024 tokens, 32 heads.)
+constexpr int kPlane = DV * 256;                                             // (128 value columns, 128 key columns) bf16
+constexpr int kFinSmem = 3 * kTile + 3 * kPlane + C * 512 + 2 * 3 * kTri * 2 + sizeof(Gates) + C * 8 + 2 * 4 * C * 4 + 3 * C * 4;
+static_assert(3 * kTile <= 3 * kPlane, "planes of Y in the state's place");
 
 __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
   extern __shared__ __align__(128) char sm[];
-  char* y_s = sm + 2 * kFinStage;
-  char* dr_s = y_s + 3 * kTile;                                    // dR as it is, fp32
-  float* parts = reinterpret_cast<float*>(y_s);
-  char* w1_s = y_s + kParts;
+  char* st_s = sm + 3 * kTile;                                     // planes of the state, or of Y
+  char* dr_s = st_s + 3 * kPlane;                                  // dR as it is, fp32
+  char* w1_s = dr_s + C * 512;
   char* w2_s = w1_s + 3 * kTri * 2;
   double* gs = reinterpret_cast<double*>(w2_s + 3 * kTri * 2);     // [64]
   float* col1 = reinterpret_cast<float*>(gs + C);                  // [4][64] column sums of W1 o QK^T without its diagonal, by block row
   float* col2 = col1 + 4 * C;                                      // [4][64] of D o KK^T o (dR Y^T)
   Gates* gt = reinterpret_cast<Gates*>(col2 + 4 * C);
   float* diag = reinterpret_cast<float*>(gt + 1);                  // [64] the diagonal of W1
+  float* sums = diag + C;                                          // [2][64] q.dq + k.dk by halves of the key columns
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int hv = blockIdx.x, seq = a.order[blockIdx.y];
   const int hk = hv / (a.HV / a.HK);
@@ -928,37 +929,23 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
   const long slot0 = first_slot(a.cu, seq);
   const long qs = (long)a.HK * DK, vs = (long)a.HV * DV;
   const int nc = (t1 - t0 + C - 1) / C;
+  const uint32_t k_s = smem_addr(sm), q_s = k_s + kTile, d_s = k_s + 2 * kTile, w1 = smem_addr(w1_s), w2 = smem_addr(w2_s);
   auto fetch = [&](int c) {
-    const uint32_t st = smem_addr(sm) + (c & 1) * kFinStage;
     const int t = t0 + c * C, n = min(C, t1 - t);
-    load_tile(st, a.k + (long)t * qs + hk * DK, qs, n, tid, NT);
-    load_tile(st + kTile, a.q + (long)t * qs + hk * DK, qs, n, tid, NT);
-    load_tile(st + 2 * kTile, a.d_o + (long)t * vs + hv * DV, vs, n, tid, NT);
+    load_tile(k_s, a.k + (long)t * qs + hk * DK, qs, n, tid, NT);
+    load_tile(q_s, a.q + (long)t * qs + hk * DK, qs, n, tid, NT);
+    load_tile(d_s, a.d_o + (long)t * vs + hv * DV, vs, n, tid, NT);
+    for (int i = tid; i < C * 32; i += NT) {
+      const int r = i >> 5, p = i & 31;
+      cp16(smem_addr(dr_s) + row32_at(r, p), a.dr + (long)(t + (r < n ? r : 0)) * vs + hv * DV + p * 4, r < n);
+    }
     cp_commit();
   };
   float S[16][4];
   load_state(S, a.state_in ? a.state_in + ((size_t)seq * a.HV + hv) * DK * DV : nullptr, warp * 16, lane);
   if (nc > 0) fetch(0);
   for (int c = 0; c < nc; ++c) {
-    cp_wait_all();
-    __syncthreads();
-    const uint32_t k_s = smem_addr(sm + (c & 1) * kFinStage), q_s = k_s + kTile, d_s = k_s + 2 * kTile;
     const int t = t0 + c * C, n = min(C, t1 - t);
-#pragma unroll
-    for (int i = tid; i < C * 32; i += NT) {
-      const int r = i >> 5, p = i & 31;
-      cp16(smem_addr(dr_s) + row32_at(r, p), a.dr + (long)(t + (r < n ? r : 0)) * vs + hv * DV + p * 4, r < n);
-    }
-    cp_commit();
-    if (c + 1 < nc) {
-      fetch(c + 1);
-      const int m = min(C, t1 - t - C);
-      prefetch_rows(reinterpret_cast<const char*>(a.r + (long)(t + C) * vs + hv * DV), vs * 4, 4, m, tid);
-      prefetch_rows(reinterpret_cast<const char*>(a.dr + (long)(t + C) * vs + hv * DV), vs * 4, 4, m, tid);
-      prefetch_rows(reinterpret_cast<const char*>(a.v + (long)(t + C) * a.v_ts + hv * DV), a.v_ts * 2, 2, m, tid);
-    } else {
-      cp_commit();
-    }
     make_gates(gt, a, slot0 + c, t, n, hv, tid);
     if (tid < C) gs[tid] = a.gsum[((slot0 + c) * a.HV + hv) * C + tid];
     for (int i = tid; i < 2 * 4 * C; i += NT) col1[i] = 0.f;
@@ -984,11 +971,21 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
         split3(v3.x - rb[u].z, v3.y - rb[u].w, p[0][3], p[1][3], p[2][3]);
 #pragma unroll
         for (int j = 0; j < 3; ++j)
-          *reinterpret_cast<uint4*>(y_s + j * kTile + tile_at(r, c8)) = make_uint4(p[j][0], p[j][1], p[j][2], p[j][3]);
+          *reinterpret_cast<uint4*>(st_s + j * kTile + tile_at(r, c8)) = make_uint4(p[j][0], p[j][1], p[j][2], p[j][3]);
       }
     }
-    asm volatile("cp.async.wait_group 1;" ::: "memory");           // dR; the next chunk's tiles may still be on their way
+    cp_wait_all();
     __syncthreads();
+    if (c + 1 < nc) {                              // the next chunk's rows come closer meanwhile
+      const int m = min(C, t1 - t - C);
+      const long at = (long)(t + C) * vs + hv * DV, kt = (long)(t + C) * qs + hk * DK;
+      prefetch_rows(reinterpret_cast<const char*>(a.r + at), vs * 4, 4, m, tid);
+      prefetch_rows(reinterpret_cast<const char*>(a.dr + at), vs * 4, 4, m, tid);
+      prefetch_rows(reinterpret_cast<const char*>(a.v + (long)(t + C) * a.v_ts + hv * DV), a.v_ts * 2, 2, m, tid);
+      prefetch_rows(reinterpret_cast<const char*>(a.d_o + at), vs * 2, 2, m, tid);
+      prefetch_rows(reinterpret_cast<const char*>(a.k + kt), qs * 2, 2, m, tid);
+      prefetch_rows(reinterpret_cast<const char*>(a.q + kt), qs * 2, 2, m, tid);
+    }
     // blocks 0..9 of W2 on warps 0-4 (two each), blocks of W1 on warps 5-7
     const bool second = warp < 5;
     const int b_lo = second ? warp * 2 : (warp - 5) * 3, b_hi = second ? b_lo + 2 : (warp == 7 ? 10 : b_lo + 3);
@@ -999,10 +996,9 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
       float m[2][4] = {}, x[2][4] = {};            // (dO or dR) Y^T and (Q or K) K^T
 #pragma unroll
       for (int kb = 0; kb < 8; ++kb) {
-        uint32_t y[3][4], f[4], b[4];
+        uint32_t y[3][4], f[4], b[4], bb[3][2];
 #pragma unroll
-        for (int p = 0; p < 3; ++p) ldsm(y[p], smem_addr(y_s) + p * kTile + tile_rc(jb * 16, kb * 2, lane));
-        uint32_t bb[3][2];
+        for (int p = 0; p < 3; ++p) ldsm(y[p], smem_addr(st_s) + p * kTile + tile_rc(jb * 16, kb * 2, lane));
         if (second) {
           uint32_t s[3][4];
           rows_a(s, dr_s, ib * 16, kb * 16, lane);
@@ -1035,8 +1031,8 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
           float d0 = 0.f, d1 = 0.f;
           if (i > j) d0 = exp2_of(gs[i] - gs[j]);
           if (i > j + 1) d1 = exp2_of(gs[i] - gs[j + 1]);
-          if (!second && i == j) diag[i] = (m[e][2 * h]) * (a.scale * gt->bet[i]);
-          if (!second && i == j + 1) diag[i] = (m[e][2 * h + 1]) * (a.scale * gt->bet[i]);
+          if (!second && i == j) diag[i] = m[e][2 * h] * (a.scale * gt->bet[i]);
+          if (!second && i == j + 1) diag[i] = m[e][2 * h + 1] * (a.scale * gt->bet[i]);
           d0 *= m[e][2 * h];
           d1 *= m[e][2 * h + 1];
           if (!second) { d0 *= a.scale * gt->bet[j]; d1 *= a.scale * gt->bet[j + 1]; }
@@ -1058,126 +1054,122 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
         if (lane < 4) *reinterpret_cast<float2*>(col + e * 8 + lane * 2) = cs;
       }
     }
-    uint32_t dr[4][3][4];
+    __syncthreads();                               // W1, W2 are there; the state takes the place of y
 #pragma unroll
-    for (int tt = 0; tt < 4; ++tt) rows_a(dr[tt], dr_s, tt * 16, warp * 16, lane);
-    __syncthreads();                               // W1, W2 are there; the parts take the place of y
-    float sc = 0.f;
-    const int which = tid >> 7, row = (tid & 127) >> 1, c8 = (tid & 1) * 8;      // 128 threads add up dQ, 128 dK
-    const int jb = warp & 3;
-    const float w_ii = diag[row];
-    const uint32_t w_s = smem_addr(warp < 4 ? w1_s : w2_s);
+    for (int nb = 0; nb < 16; ++nb)
 #pragma unroll
-    for (int np = 0; np < 8; ++np) {
-      float q2[2][4][4] = {}, k2[2][4][4] = {};
-      uint32_t kf[4], qf[4];
-      ldsm_t(kf, k_s + tile_cr(jb * 16, np * 2, lane));
-      if (warp < 4) ldsm_t(qf, q_s + tile_cr(jb * 16, np * 2, lane));
-      else
+      for (int h = 0; h < 2; ++h) {
+        uint32_t p0, p1, p2;
+        split3(S[nb][2 * h], S[nb][2 * h + 1], p0, p1, p2);
+        char* at = st_s + tile_at(warp * 16 + (lane >> 2) + h * 8, nb) + (lane & 3) * 4;
+        *reinterpret_cast<uint32_t*>(at) = p0;
+        *reinterpret_cast<uint32_t*>(at + kPlane) = p1;
+        *reinterpret_cast<uint32_t*>(at + 2 * kPlane) = p2;
+      }
+    __syncthreads();
+    {
+      const int tt = warp & 3, half = warp >> 2;   // 16 tokens, 64 key columns
+      float q2[8][4] = {}, k2[8][4] = {};
+#pragma unroll 1
+      for (int kb = 0; kb < 8; ++kb) {             // the state's part: 16 value columns a time
+        uint32_t f[4], d[3][4];
+        ldsm(f, d_s + tile_cr(tt * 16, kb * 2, lane));
+        rows_a(d, dr_s, tt * 16, kb * 16, lane);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) qf[j] = kf[j];
+        for (int np = 0; np < 4; ++np) {
+          uint32_t b[3][4], bb[3][2];
 #pragma unroll
-      for (int tt = 0; tt < 4; ++tt) {
-        uint32_t w[3][4];
-        if (tt >= jb) {                            // W1 K into dQ, W2 K into dK
+          for (int p = 0; p < 3; ++p) ldsm_t(b[p], smem_addr(st_s) + p * kPlane + tile_cr(kb * 16, half * 8 + np * 2, lane));
 #pragma unroll
-          for (int p = 0; p < 3; ++p) ldsm(w[p], w_s + p * kTri * 2 + blk_of(tt, jb) * 512 + blk_cr(lane));
-          if (warp < 4) {
-            prod3(q2[0][tt], w, kf[0], kf[1]);
-            prod3(q2[1][tt], w, kf[2], kf[3]);
-          } else {
-            prod3(k2[0][tt], w, kf[0], kf[1]);
-            prod3(k2[1][tt], w, kf[2], kf[3]);
+          for (int e = 0; e < 2; ++e) {
+            pick(bb, b, e);
+            prod3(q2[2 * np + e], f, bb);
+            prod6(k2[2 * np + e], d, bb);
           }
         }
-        if (tt <= jb) {                            // W1^T Q and W2^T K into dK
+      }
+      const int r0 = tt * 16 + (lane >> 2);        // the thread's rows: r0 and r0 + 8
+      const float g0 = gt->gam[r0], g1 = gt->gam[r0 + 8];
 #pragma unroll
-          for (int p = 0; p < 3; ++p) ldsm_t(w[p], w_s + p * kTri * 2 + blk_of(jb, tt) * 512 + blk_rc(lane));
-          prod3(k2[0][tt], w, qf[0], qf[1]);
-          prod3(k2[1][tt], w, qf[2], qf[3]);
+      for (int nb = 0; nb < 8; ++nb) {
+        q2[nb][0] *= a.scale * g0;
+        q2[nb][1] *= a.scale * g0;
+        q2[nb][2] *= a.scale * g1;
+        q2[nb][3] *= a.scale * g1;
+        k2[nb][0] *= g0;
+        k2[nb][1] *= g0;
+        k2[nb][2] *= g1;
+        k2[nb][3] *= g1;
+      }
+#pragma unroll 1
+      for (int jb = 0; jb <= tt; ++jb) {           // W1 K into dQ, W2 K into dK
+        uint32_t x[3][4], z[3][4];
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+          ldsm(x[p], w1 + p * kTri * 2 + blk_of(tt, jb) * 512 + blk_cr(lane));
+          ldsm(z[p], w2 + p * kTri * 2 + blk_of(tt, jb) * 512 + blk_cr(lane));
+        }
+#pragma unroll
+        for (int np = 0; np < 4; ++np) {
+          uint32_t b[4];
+          ldsm_t(b, k_s + tile_cr(jb * 16, half * 8 + np * 2, lane));
+          prod3(q2[2 * np], x, b[0], b[1]);
+          prod3(q2[2 * np + 1], x, b[2], b[3]);
+          prod3(k2[2 * np], z, b[0], b[1]);
+          prod3(k2[2 * np + 1], z, b[2], b[3]);
         }
       }
+#pragma unroll 1
+      for (int jb = tt; jb < 4; ++jb) {            // W1^T Q and W2^T K into dK
+        uint32_t x[3][4], z[3][4];
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {                // the state's part
-        uint32_t b[3][2];
-        state_b(b, S[2 * np + e]);
+        for (int p = 0; p < 3; ++p) {
+          ldsm_t(x[p], w1 + p * kTri * 2 + blk_of(jb, tt) * 512 + blk_rc(lane));
+          ldsm_t(z[p], w2 + p * kTri * 2 + blk_of(jb, tt) * 512 + blk_rc(lane));
+        }
 #pragma unroll
-        for (int tt = 0; tt < 4; ++tt) {
-          uint32_t f[4];
-          ldsm(f, d_s + tile_cr(tt * 16, warp * 2, lane));
-          float u[4] = {}, v[4] = {};
-          prod3(u, f, b);
-          prod6(v, dr[tt], b);
-          const float g0 = gt->gam[tt * 16 + (lane >> 2)], g1 = gt->gam[tt * 16 + (lane >> 2) + 8];
-          q2[e][tt][0] += u[0] * (a.scale * g0);
-          q2[e][tt][1] += u[1] * (a.scale * g0);
-          q2[e][tt][2] += u[2] * (a.scale * g1);
-          q2[e][tt][3] += u[3] * (a.scale * g1);
-          k2[e][tt][0] += v[0] * g0;
-          k2[e][tt][1] += v[1] * g0;
-          k2[e][tt][2] += v[2] * g1;
-          k2[e][tt][3] += v[3] * g1;
+        for (int np = 0; np < 4; ++np) {
+          uint32_t b[4];
+          ldsm_t(b, q_s + tile_cr(jb * 16, half * 8 + np * 2, lane));
+          prod3(k2[2 * np], x, b[0], b[1]);
+          prod3(k2[2 * np + 1], x, b[2], b[3]);
+          ldsm_t(b, k_s + tile_cr(jb * 16, half * 8 + np * 2, lane));
+          prod3(k2[2 * np], z, b[0], b[1]);
+          prod3(k2[2 * np + 1], z, b[2], b[3]);
         }
       }
+      // out, with the diagonal of W1; q.dq + k.dk without it (it has no part in the gate's scalars and would only cancel)
 #pragma unroll
-      for (int tt = 0; tt < 4; ++tt)
+      for (int h = 0; h < 2; ++h) {
+        const int r = r0 + h * 8;
+        const float w_ii = diag[r];
+        float sc = 0.f;
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          float* p = parts + (warp * C + tt * 16 + (lane >> 2)) * kPartLd + e * 8 + (lane & 3) * 2;
-          *reinterpret_cast<float2*>(p) = make_float2(q2[e][tt][0], q2[e][tt][1]);
-          *reinterpret_cast<float2*>(p + 8 * kPartLd) = make_float2(q2[e][tt][2], q2[e][tt][3]);
-          p += 8 * C * kPartLd;
-          *reinterpret_cast<float2*>(p) = make_float2(k2[e][tt][0], k2[e][tt][1]);
-          *reinterpret_cast<float2*>(p + 8 * kPartLd) = make_float2(k2[e][tt][2], k2[e][tt][3]);
+        for (int nb = 0; nb < 8; ++nb) {
+          const uint32_t at = tile_at(r, half * 8 + nb) + (lane & 3) * 4;
+          uint32_t qu, ku;
+          asm volatile("ld.shared.b32 %0, [%1];" : "=r"(qu) : "r"(q_s + at) : "memory");
+          asm volatile("ld.shared.b32 %0, [%1];" : "=r"(ku) : "r"(k_s + at) : "memory");
+          const float2 qf = bf2(qu), kf = bf2(ku);
+          float2 dq = make_float2(q2[nb][2 * h], q2[nb][2 * h + 1]), dk = make_float2(k2[nb][2 * h], k2[nb][2 * h + 1]);
+          sc += (qf.x * dq.x + qf.y * dq.y) + (kf.x * dk.x + kf.y * dk.y);
+          dq.x += w_ii * kf.x;
+          dq.y += w_ii * kf.y;
+          dk.x += w_ii * qf.x;
+          dk.y += w_ii * qf.y;
+          if (r < n) {
+            const long o = ((long)(t + r) * a.HV + hv) * DK + half * 64 + nb * 8 + (lane & 3) * 2;
+            *reinterpret_cast<float2*>(a.dq + o) = dq;
+            red_add2(a.dk + o, dk.x, dk.y);        // to what pass R wrote, one addition: no order to depend on
+          }
         }
-      __syncthreads();
-      float x[8] = {};
-#pragma unroll
-      for (int w = 0; w < 8; ++w) {
-        const float4* p = reinterpret_cast<const float4*>(parts + ((which * 8 + w) * C + row) * kPartLd + c8);
-        const float4 u = p[0], v = p[1];
-        x[0] += u.x; x[1] += u.y; x[2] += u.z; x[3] += u.w;
-        x[4] += v.x; x[5] += v.y; x[6] += v.z; x[7] += v.w;
+        sc += __shfl_xor_sync(0xffffffffu, sc, 1);
+        sc += __shfl_xor_sync(0xffffffffu, sc, 2);
+        if ((lane & 3) == 0) sums[half * C + r] = sc;
       }
-      uint32_t own[4], other[4];                   // the row of q (dQ) or k (dK), and the other one, which the diagonal multiplies
-      asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(own[0]), "=r"(own[1]), "=r"(own[2]), "=r"(own[3])
-                   : "r"((which ? k_s : q_s) + tile_at(row, np * 2 + (tid & 1))) : "memory");
-      asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(other[0]), "=r"(other[1]), "=r"(other[2]), "=r"(other[3])
-                   : "r"((which ? q_s : k_s) + tile_at(row, np * 2 + (tid & 1))) : "memory");
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 f = bf2(own[e]), g = bf2(other[e]);
-        sc += f.x * x[2 * e] + f.y * x[2 * e + 1];
-        x[2 * e] += w_ii * g.x;
-        x[2 * e + 1] += w_ii * g.y;
-      }
-      if (row < n) {
-        float4* p = reinterpret_cast<float4*>((which ? a.dk : a.dq) + ((long)(t + row) * a.HV + hv) * DK + np * 16 + c8);
-        if (which) {                               // to what pass R wrote, one addition: no order to depend on
-          red_add4(reinterpret_cast<float*>(p), x[0], x[1], x[2], x[3]);
-          red_add4(reinterpret_cast<float*>(p + 1), x[4], x[5], x[6], x[7]);
-        } else {
-          p[0] = make_float4(x[0], x[1], x[2], x[3]);
-          p[1] = make_float4(x[4], x[5], x[6], x[7]);
-        }
-      }
-      __syncthreads();
     }
     ColumnsOfY columns;
     columns.ask(a, t, n, vs, hv, warp * 16, lane);
-    // per-token scalars: q.dq + k.(W2 K + S^ dr) - k.(W1^T Q + W2^T K), the last by the column sums (k.dk has it with the sign
-    // turned).  The diagonal of W1 has no part in them (q.dq and k.dk have the same from it) and would only cancel.
-    sc += __shfl_xor_sync(0xffffffffu, sc, 1);
-    float* sums = parts;                           // [2][64]
-    if ((tid & 1) == 0) sums[which * C + row] = sc;
-    __syncthreads();
-    if (tid < n) {
-      const float c1 = col1[tid] + col1[C + tid] + col1[2 * C + tid] + col1[3 * C + tid];
-      const float c2 = col2[tid] + col2[C + tid] + col2[2 * C + tid] + col2[3 * C + tid];
-      const long at = (long)(t + tid) * a.HV + hv;
-      a.dbeta[at] += c2;
-      a.sacc[at] += sums[tid] + (sums[C + tid] - 2.f * (c1 + gt->bet[tid] * c2));
-    }
     // S <- exp(G_C) S + (exp(G_C - G) K)^T B Y
     const float end = gt->end;
 #pragma unroll
@@ -1202,6 +1194,17 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
       split_a(x[0], x[1], s);
       state_add(S, s, k_s, tb, lane);
     }
+    __syncthreads();                               // the tiles, the state's planes and the sums are done with, or there
+    if (c + 1 < nc) fetch(c + 1);
+    // per-token scalars: q.dq + k.(W2 K + S^ dr) - k.(W1^T Q + W2^T K), the last by the column sums (k.dk has it with the sign turned)
+    if (tid < n) {
+      const float c1 = col1[tid] + col1[C + tid] + col1[2 * C + tid] + col1[3 * C + tid];
+      const float c2 = col2[tid] + col2[C + tid] + col2[2 * C + tid] + col2[3 * C + tid];
+      const long at = (long)(t + tid) * a.HV + hv;
+      a.dbeta[at] += c2;
+      a.sacc[at] += (sums[tid] + sums[C + tid]) - 2.f * (c1 + gt->bet[tid] * c2);
+    }
+    __syncthreads();
   }
 }
 
