@@ -24,14 +24,15 @@
 // value columns, which never meet those of another warp, and holds its slice of the state transposed as the accumulators of
 // m16n8k16; these are, register for register, the A operand of the next product, so the whole chain stays in one warp's
 // registers: no round trip through shared or tensor memory and no barrier between its products.  Shared memory holds only
-// what the warps share (K, Q, the inverse).  The backward products that sum over value columns (dQ, dK) are added up over
-// the eight warps through shared memory.
+// what the warps share (K, Q, the inverse).  The backward products that sum over value columns (dQ, dK) are the exception: there
+// the state goes through shared memory once a chunk, and a warp owns tokens.
 //
-// Measured, ms, token by token (gdn.cu) / so, 32 heads: 16 x 1024 tokens forward 2.19 / 1.05, backward 7.98 / 5.1; one sequence of
-// 16384 7.5 / 3.2 and 25.4 / 18.5; 300 sequences of 33, mostly half-empty chunks, 1.60 / 1.29 and 5.16 / 5.33.  Errors against fp64 (2-norm, gates as a
-// model's): final state 4.8e-8 / 6.9e-8, dq 1.16e-7 / 1.13e-7, dk 1.54e-7 / 1.14e-7, dg 1.0e-5 / 5.5e-6; with slow decay (0.01 a token) 2.0e-6 /
-// 1.4e-7, 1.6e-6 / 1.8e-7, 2.0e-6 / 2.3e-7.  What bounds it now: mma.sync at 537 TFLOP/s, reached to two thirds forward and a third
-// backward, where the warps meet sixteen times a chunk.
+// Measured, ms, token by token (gdn.cu) / so, 32 heads: 16 x 1024 tokens forward 2.19 / 1.00, backward 7.98 / 4.12; one sequence
+// of 16384 7.5 / 3.2 and 25.4 / 14.8; two of 8192 4.6 / 1.7 and 15.1 / 7.7; 512 tokens 0.22 / 0.12 and 0.81 / 0.49; 300 sequences of
+// 33, mostly half-empty chunks, 1.60 / 1.29 and 5.16 / 5.33.  Errors against fp64 (2-norm, gates as a model's): final state 4.8e-8
+// / 6.9e-8, dq 1.16e-7 / 1.13e-7, dk 1.54e-7 / 1.14e-7, dg 1.0e-5 / 4.4e-6; with slow decay (0.01 a token) 2.0e-6 / 1.4e-7, 1.6e-6
+// / 1.8e-7, 2.0e-6 / 2.3e-7.  What bounds it now: the chain of a sequence, product after product; mma.sync (537 TFLOP/s) is in
+// use for about half of the time.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>

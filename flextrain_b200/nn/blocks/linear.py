@@ -177,15 +177,18 @@ class LinearGroup:
                     ops.linear_wgrad(dy[:, r0:r0 + g.shape[0]], x, g, alpha=alpha)
                     r0 += g.shape[0]
         else:
-            r0 = 0
+            r0, adapters = 0, []
             for n, gname in zip(self.names, gnames):
                 rows = params[n].shape[0]
                 dyn = dy[:, r0:r0 + rows]
                 if gname in grads:
                     ops.linear_wgrad(dyn, x, grads[gname], alpha=alpha)
-                if n in self.lora_names:
-                    self._lora_wgrad(n, dyn, x, params, grads, alpha)
+                g = "g_" + n[2:] + "_lora_"
+                if n in self.lora_names and grads.get(g + "a") is not None:
+                    adapters.append((dyn, params[n + "_lora_a"], params[n + "_lora_b"], grads[g + "a"], grads[g + "b"]))
                 r0 += rows
+            if adapters:
+                ops.lora_wgrad(x, adapters, self.lora.scale * alpha)
         if self.bias_names:
             r0 = 0
             for n, bn in zip(self.names, self.bias_names):
@@ -194,17 +197,6 @@ class LinearGroup:
                 if gb in grads:
                     ops.bias_grad(dy[:, r0:r0 + rows], grads[gb], alpha=alpha)
                 r0 += rows
-
-    def _lora_wgrad(self, n, dy, x, params, grads, alpha):
-        s = self.lora.scale * alpha
-        a, b = params[n + "_lora_a"], params[n + "_lora_b"]
-        ga, gb = grads.get("g_" + n[2:] + "_lora_a"), grads.get("g_" + n[2:] + "_lora_b")
-        if ga is None:
-            return
-        dyb = ops.gemm(dy.contiguous() if dy.stride(-1) != 1 else dy, b.to(dy.dtype))          # (T, r)
-        xa = ops.gemm(x, a.to(x.dtype), trans_b=True)                                            # (T, r)
-        ops.gemm(dyb, x, trans_a=True, alpha=s, beta=1.0, out=ga)                                # (r, in)
-        ops.gemm(dy, xa, trans_a=True, alpha=s, beta=1.0, out=gb)                                # (out, r)
 
 
 def clear_effective_weights(params: Dict[str, torch.Tensor]) -> None:

@@ -272,6 +272,25 @@ def rope_qkv(q, k, v, positions, inv_freq, *, q_out, k_out, v_out, inverse=False
         v_out.copy_(v)
 
 
+def lora_wgrad(x, adapters, scale):
+    """Gradients of the rank-r adapters that share the input ``x (T, K)``: for each ``(dy (T, N), a (r, K), b (N, r), ga, gb)``
+    ``ga += scale * (dy @ b)^T @ x`` and ``gb += scale * dy^T @ (x @ a^T)``; three launches for up to three of them where their
+    shapes allow it, four GEMMs each elsewhere."""
+    adapters = [(dy if dy.stride(-1) == 1 else dy.contiguous(), a.to(x.dtype), b.to(x.dtype), ga, gb) for dy, a, b, ga, gb in adapters]
+    if _GEMM_BACKEND == "tcgen05" and _cuda_bf16(x) and _kernels().lora_wgrad_supported(x, adapters):
+        _count()
+        lora_wgrad_fused(x, adapters, scale)
+        return
+    for dy, a, b, ga, gb in adapters:
+        gemm(gemm(dy, b), x, trans_a=True, alpha=scale, beta=1.0, out=ga)                        # (T, r), then (r, in)
+        gemm(dy, gemm(x, a, trans_b=True), trans_a=True, alpha=scale, beta=1.0, out=gb)          # (T, r), then (out, r)
+
+
+def lora_wgrad_fused(x, adapters, scale):
+    """The kernels themselves (GPU only); ``lora_wgrad`` is the entry that falls back."""
+    _kernels().lora_wgrad(x, adapters, scale)
+
+
 def glu_fwd(gate, up, kind="swiglu"):
     if _cuda_bf16(gate, up):
         _count()
@@ -710,7 +729,7 @@ rope_inv_freq = ref.rope_inv_freq
 # ``FTB_OP_TIMING=1`` brackets every leaf op of this module with CUDA events on the current stream and
 # ``timing_report()`` aggregates them by (op, shape): the per-kernel time table of a training step without a
 # profiler attached.  The events add host work, so a throughput number taken with it on is not a benchmark value.
-_TIMED_OPS = ("gemm", "gemm_glu_fwd", "gemm_glu_bwd", "rmsnorm_fwd", "rmsnorm_bwd", "rope", "rope_qkv_fused", "glu_fwd", "glu_bwd",
+_TIMED_OPS = ("gemm", "gemm_glu_fwd", "gemm_glu_bwd", "rmsnorm_fwd", "rmsnorm_bwd", "rope", "rope_qkv_fused", "lora_wgrad_fused", "glu_fwd", "glu_bwd",
               "glu_bwd_weighted", "attention_fwd", "attention_bwd", "softmax_ce_", "softmax_ce_loss", "embedding_fwd", "embedding_bwd", "adamw_multi", "topk_route",
               "topk_route_bwd", "gather_rows", "moe_combine", "grouped_gemm", "grouped_wgrad", "l2norm_fwd",
               "gated_rmsnorm_fwd", "bias_grad")

@@ -29,7 +29,7 @@ from typing import Dict, List
 ENTRY_POINTS = {
     "gemm_tcgen05": "ftb_gemm_bf16", "elementwise": "ftb_adamw_multi", "attention": "ftb_attn_fwd",
     "comm": "ftb_comm_adamw_push", "moe": "ftb_ep_plan_count", "noalloc": "ftb_rmsnorm_bwd_noalloc",
-    "gdn": "ftb_gdn", "gdn_chunk": "ftb_gdn_chunk_fwd", "seqmix": "ftb_conv1d_fwd", "dp_solver": "ftb_dp_solve",
+    "gdn": "ftb_gdn", "gdn_chunk": "ftb_gdn_chunk_fwd", "lora": "ftb_lora_wgrad", "seqmix": "ftb_conv1d_fwd", "dp_solver": "ftb_dp_solve",
     "copy_engine": "ftb_ce_create",
 }
 OPTIONAL = {"flash_attn": "attention comparison bar", "fla": "Gated DeltaNet comparison bar",
