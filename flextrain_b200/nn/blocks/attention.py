@@ -127,7 +127,7 @@ class GQAAttentionBlock:
             # w_q rows are per-head [query(hd) ‖ gate(hd)] (HF Qwen3-Next layout)
             qg = qkv[:, : 2 * c.q_dim].reshape(T, c.n_heads, 2 * c.head_dim)
             q = qg[:, :, : c.head_dim]
-            gate = qg[:, :, c.head_dim:].reshape(T, c.q_dim)
+            gate = qg[:, :, c.head_dim:]
             off = 2 * c.q_dim
         else:
             q = qkv[:, : c.q_dim].unflatten(1, (c.n_heads, c.head_dim))
@@ -165,7 +165,7 @@ class GQAAttentionBlock:
             slot.put("v_rstd", vr)
         ops.rope_qkv(q if want_q else None, k, v, pos, inv, q_out=xq, k_out=xk, v_out=xv, mrope_sections=sec)
         if want_q and c.gated:
-            slot.put("xgate", gate.contiguous() if slot.buffer is None else gate)
+            ops.copy_heads(gate, slot.out("xgate", h.device))
         return xq, xk, xv
 
     def _kv_for_attention(self, meta: ChunkMeta, xk, xv, ctx: LayerContext, *, write: bool):
@@ -197,7 +197,7 @@ class GQAAttentionBlock:
         if c.gated:
             g = slot.get("xgate")
             raw = slot.put("attn_result", out2)
-            out2 = (raw.to(torch.float32) * torch.sigmoid(g.to(torch.float32))).to(raw.dtype)
+            out2 = ops.attn_gate_fwd(raw, g)
         else:
             out2 = slot.put("attn_result", out2)
         slot.put("softmax_lse", lse)
@@ -230,18 +230,16 @@ class GQAAttentionBlock:
         t = slot._t
         attn_raw = t["attn_result"]
         T = attn_raw.shape[0]
-        if c.gated:
-            sg = torch.sigmoid(t["xgate"].to(torch.float32))
-            attn_in = (attn_raw.to(torch.float32) * sg).to(attn_raw.dtype)
-        else:
-            attn_in = attn_raw
         dattn = self.o.dgrad(dxo, params)                                        # (T, q_dim)
-        self.o.wgrad(dxo, attn_in, params, grads)
-        dgate = None
+        qrows = c.q_dim * (2 if c.gated else 1)
+        new_dqkv = lambda: torch.empty(T, qrows + 2 * c.kv_dim, dtype=dxo.dtype, device=dxo.device)
+        attn_in = attn_raw
         if c.gated:
-            df = dattn.to(torch.float32)
-            dgate = (df * attn_raw.to(torch.float32) * sg * (1 - sg)).to(dattn.dtype)
-            dattn = (df * sg).to(dattn.dtype)
+            dqkv = new_dqkv()
+            qg = dqkv[:, :qrows].view(T, c.n_heads, 2 * c.head_dim)
+            dattn, attn_in = ops.attn_gate_bwd(dattn, attn_raw, t["xgate"], qg[:, :, c.head_dim:])
+        self.o.wgrad(dxo, attn_in, params, grads)
+        del attn_in
         K, V = self._kv_for_attention(meta, t["xk"], t["xv"], ctx, write=False)
         dq, dk, dv = ops.attention_bwd(dattn.view(T, c.n_heads, c.head_dim), t["xq"], K, V,
                                        attn_raw.view(T, c.n_heads, c.head_dim), t["softmax_lse"], meta.cu_seqlens_q,
@@ -252,13 +250,10 @@ class GQAAttentionBlock:
         # inverse RoPE, then QK-norm backward, assembling dqkv in projection-row order
         inv = self._inv_freq(dxo.device)
         pos, sec = meta.positions, c.rope.mrope_sections
-        qrows = c.q_dim * (2 if c.gated else 1)
-        dqkv = torch.empty(T, qrows + 2 * c.kv_dim, dtype=dxo.dtype, device=dxo.device)
         if c.gated:
-            qg = dqkv[:, :qrows].view(T, c.n_heads, 2 * c.head_dim)
             dq_dst = qg[:, :, : c.head_dim]
-            qg[:, :, c.head_dim:].copy_(dgate.view(T, c.n_heads, c.head_dim))
         else:
+            dqkv = new_dqkv()
             dq_dst = dqkv[:, :qrows].unflatten(1, (c.n_heads, c.head_dim))
         dk_dst = dqkv[:, qrows: qrows + c.kv_dim].unflatten(1, (c.n_kv_heads, c.head_dim))
         dv_dst = dqkv[:, qrows + c.kv_dim:].unflatten(1, (c.n_kv_heads, c.head_dim))

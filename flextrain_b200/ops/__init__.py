@@ -272,6 +272,34 @@ def rope_qkv(q, k, v, positions, inv_freq, *, q_out, k_out, v_out, inverse=False
         v_out.copy_(v)
 
 
+def copy_heads(x, out):
+    """``out (T, H * hd) <- x (T, H, hd)``, heads that may lie apart."""
+    if _cuda_bf16(x, out) and _kernels().attn_gate_supported(x, out):
+        _count()
+        _kernels().copy_heads(x, out)
+        return
+    out.view(x.shape).copy_(x)
+
+
+def attn_gate_fwd(x, gate):
+    """Output gate of gated attention: ``x * sigmoid(gate)``, both ``(T, H * hd)``."""
+    if _cuda_bf16(x, gate) and _kernels().attn_gate_supported(x.unsqueeze(1), x, gate):
+        _count()
+        return _kernels().attn_gate_fwd(x, gate)
+    return (x.to(torch.float32) * torch.sigmoid(gate.to(torch.float32))).to(x.dtype)
+
+
+def attn_gate_bwd(d, x, gate, dgate_out):
+    """Backward of :func:`attn_gate_fwd` from ``d``, which may be overwritten; the gate's gradient is written into ``dgate_out
+    (T, H, hd)``, heads that may lie apart.  Returns ``(dx, x * sigmoid(gate))``."""
+    if _cuda_bf16(d, x, gate, dgate_out) and _kernels().attn_gate_supported(dgate_out, d, x, gate):
+        _count()
+        return d, _kernels().attn_gate_bwd(d, x, gate, dgate_out)
+    sg, df, xf = torch.sigmoid(gate.to(torch.float32)), d.to(torch.float32), x.to(torch.float32)
+    dgate_out.copy_((df * xf * sg * (1 - sg)).to(d.dtype).view(dgate_out.shape))
+    return (df * sg).to(d.dtype), (xf * sg).to(x.dtype)
+
+
 def lora_wgrad(x, adapters, scale):
     """Gradients of the rank-r adapters that share the input ``x (T, K)``: for each ``(dy (T, N), a (r, K), b (N, r), ga, gb)``
     ``ga += scale * (dy @ b)^T @ x`` and ``gb += scale * dy^T @ (x @ a^T)``; three launches for up to three of them where their

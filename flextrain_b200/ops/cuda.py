@@ -254,10 +254,9 @@ def grouped_wgrad(dy, x, offsets, gw, *, alpha=1.0, accumulate=True):
 
 # ------------------------------------------------------------------------ elementwise
 def heads_strided(t: torch.Tensor) -> bool:
-    """``(T, H, hd)`` with heads side by side, any token stride that keeps 16-byte pieces aligned, and a head dim the per-head
-    kernels know."""
-    return (t.dim() == 3 and t.shape[2] in (64, 128, 256) and t.stride(2) == 1 and t.stride(1) == t.shape[2]
-            and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 and t.shape[0] * t.shape[1] < 1 << 31)
+    """``(T, H, hd)``, any token and head strides that keep 16-byte pieces aligned, and a head dim the per-head kernels know."""
+    return (t.dim() == 3 and t.shape[2] in (64, 128, 256) and t.stride(2) == 1
+            and t.stride(1) >= t.shape[2] and t.stride(1) % 8 == 0 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 and t.shape[0] * t.shape[1] < 1 << 31)
 
 
 def rows_strided(t: torch.Tensor) -> bool:
@@ -271,8 +270,8 @@ def rmsnorm_heads_fwd(x, w, eps):
     T, H, hd = x.shape
     y = torch.empty(T, H, hd, dtype=x.dtype, device=x.device)
     rstd = torch.empty(T, H, dtype=torch.float32, device=x.device)
-    _check(lib.ftb_rmsnorm_heads_fwd(_ptr(x), c_long(x.stride(0)), _ptr(w), _ptr(y), _ptr(rstd), c_int(T), c_int(H), c_int(hd),
-                                     c_float(eps), _stream()), "ftb_rmsnorm_heads_fwd")
+    _check(lib.ftb_rmsnorm_heads_fwd(_ptr(x), c_long(x.stride(0)), c_long(x.stride(1)), _ptr(w), _ptr(y), _ptr(rstd), c_int(T), c_int(H),
+                                     c_int(hd), c_float(eps), _stream()), "ftb_rmsnorm_heads_fwd")
     return y, rstd
 
 
@@ -280,10 +279,42 @@ def rmsnorm_heads_bwd(dy, x, w, rstd, dx, dw_out):
     """``dx`` (strided as ``x`` may be) is written; the gain's gradient is added to ``dw_out``."""
     lib = load("elementwise")
     T, H, hd = x.shape
-    _check(lib.ftb_rmsnorm_heads_bwd(_ptr(dy), c_long(dy.stride(0)), _ptr(x), c_long(x.stride(0)), _ptr(w), _ptr(rstd), _ptr(dx),
-                                     c_long(dx.stride(0)), _ptr(dw_out), c_int(T), c_int(H), c_int(hd), _stream()),
+    st = lambda t: (_ptr(t), c_long(t.stride(0)), c_long(t.stride(1)))
+    _check(lib.ftb_rmsnorm_heads_bwd(*st(dy), *st(x), _ptr(w), _ptr(rstd), *st(dx), _ptr(dw_out), c_int(T), c_int(H), c_int(hd),
+                                     _stream()),
            "ftb_rmsnorm_heads_bwd")
     return dx
+
+
+def _heads_16(*heads) -> bool:
+    return all(t.dim() == 3 and t.stride(2) == 1 and t.shape[2] % 8 == 0 and t.stride(1) % 8 == 0 and t.stride(0) % 8 == 0
+               and t.stride(1) >= t.shape[2]               and t.data_ptr() % 16 == 0 for t in heads)
+
+
+def attn_gate_supported(heads, *flat) -> bool:
+    """``heads (T, H, hd)`` strided, the others contiguous, all bf16 on 16 bytes."""
+    return (_heads_16(heads) and all(t.dtype == torch.bfloat16 and t.is_cuda for t in (heads,) + flat)
+            and all(t.is_contiguous() and t.data_ptr() % 16 == 0 and t.numel() == heads.numel() for t in flat))
+
+
+def copy_heads(x, out):
+    T, H, hd = x.shape
+    _check(load("elementwise").ftb_copy_heads(_ptr(x), c_long(x.stride(0)), c_long(x.stride(1)), _ptr(out), c_long(T), c_int(H),
+                                              c_int(hd), _stream()), "ftb_copy_heads")
+
+
+def attn_gate_fwd(x, gate):
+    y = torch.empty_like(x)
+    _check(load("elementwise").ftb_attn_gate_fwd(_ptr(x), _ptr(gate), _ptr(y), c_long(x.numel()), _stream()), "ftb_attn_gate_fwd")
+    return y
+
+
+def attn_gate_bwd(d, x, gate, dgate):
+    T, H, hd = dgate.shape
+    y = torch.empty_like(x)
+    _check(load("elementwise").ftb_attn_gate_bwd(_ptr(d), _ptr(x), _ptr(gate), _ptr(y), _ptr(dgate), c_long(dgate.stride(0)),
+                                                 c_long(dgate.stride(1)), c_long(T), c_int(H), c_int(hd), _stream()), "ftb_attn_gate_bwd")
+    return y
 
 
 def rmsnorm_rows_fwd(x, w, eps):
