@@ -27,7 +27,7 @@ import torch
 
 from .. import ops
 from ..core.activation_schema import ON_DEVICE, ActivationSlot, fetch_home, send_home
-from ..core.layer import ChunkMeta, LayerContext
+from ..core.layer import ChunkMeta, LayerContext, ParamSpec
 from ..core.save_level import (HardwareCost, SaveLevelPlan, TransmissionScheduler, build_dp_tables,
                                plan_from_solution)
 from ..core.working_set import WorkingSetConfig
@@ -234,7 +234,7 @@ class ActiveModel:
                         for c, meta in enumerate(metas):
                             ls = self.head.forward_backward(transitions[c], self._token_shard(meta),
                                                             self.buffers.head_params(),
-                                                            {} if forward_only else self.buffers.head_grads(),
+                                                            {} if forward_only else self._head_grads(),
                                                             loss_fn, loss_scale_factor, want_dx=not forward_only)
                             loss_acc += ls.total_loss
                             act_acc += ls.active_tokens
@@ -300,13 +300,34 @@ class ActiveModel:
         before any reduction or update, and the head mirror is refreshed from the embedding after every step
         (:meth:`step`).  Training the mirror separately would untie the model, and an export — which writes the
         embedding only — would lose what the head learnt."""
-        if not getattr(self.head, "tied", False):
+        if not getattr(self.head, "tied", False) or self._tied_in_place():
             return
         ge = self.buffers.embed_grads().get("g_tok_embeddings")
         gh = self.buffers.head_grads().get("g_head_proj")
         if ge is not None and gh is not None:
             ge.add_(gh)
             gh.zero_()
+
+    def _tied_in_place(self) -> bool:
+        """Whether the head's product is added to the embedding's gradient where it lies: without it a tied step reads and
+        writes the whole table three times more (:meth:`_fold_tied_head_grad`).  Parallel runs reduce the two apart."""
+        if not getattr(self.head, "tied", False) or any(p is not None for p in (self.dp, self.tp, self.ep)):
+            return False
+        ge = self.buffers.embed_grads().get("g_tok_embeddings")
+        gh = self.buffers.head_grads().get("g_head_proj")
+        return ge is not None and gh is not None and ge.shape == gh.shape and ge.dtype == gh.dtype and ge.device == gh.device
+
+    def _head_grads(self):
+        grads = self.buffers.head_grads()
+        return {**grads, "g_head_proj": self.buffers.embed_grads()["g_tok_embeddings"]} if self._tied_in_place() else grads
+
+    def _head_update_spec(self):
+        """What the optimizer updates of the head: a tied projection is replaced by the embedding after the step
+        (:meth:`step`), so its own update, of a gradient that is zero, is left out."""
+        spec = self.head.param_spec
+        if not (getattr(self.head, "tied", False) and "g_tok_embeddings" in self.buffers.embed_grads()):
+            return spec
+        return ParamSpec([t for t in spec if t.name != "w_head_proj"])
 
     def grad_norm(self) -> float:
         """Global L2 norm of the accumulated gradients (one host read).  Replicated tensors count once; the parts of
@@ -749,8 +770,9 @@ class ActiveModel:
         opt, rc = self.optimizer, 0
         rc |= opt.step(self.embed.param_spec, bm.embed_params(), bm.embed_grads(), bm.embed_opt(), self.step_num,
                        grad_scale)
-        rc |= opt.step(self.head.param_spec, bm.head_params(), bm.head_grads(), bm.head_opt(), self.step_num,
-                       grad_scale)
+        head_spec = self._head_update_spec()
+        if head_spec is self.head.param_spec or head_spec.trainable():
+            rc |= opt.step(head_spec, bm.head_params(), bm.head_grads(), bm.head_opt(), self.step_num, grad_scale)
         if rc:
             return rc
         nL = len(self.layers)
