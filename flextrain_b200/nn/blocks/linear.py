@@ -88,12 +88,17 @@ class LinearGroup:
         cached = params.get(key)
         if cached is not None:
             return cached
-        eff = torch.cat(ws, 0) if len(ws) > 1 else ws[0].clone()
+        # the product reads the base weight where it lies and writes the sum: no copy of the weight is made first
+        eff = torch.empty(sum(w.shape[0] for w in ws), ws[0].shape[1], dtype=ws[0].dtype, device=ws[0].device)
         r0 = 0
         for n, w in zip(self.names, ws):
+            part = eff[r0:r0 + w.shape[0]]
             if n in self.lora_names:
+                base = w if w.dtype == eff.dtype and w.is_contiguous() and w.data_ptr() % 16 == 0 else part.copy_(w)
                 a, b = params[n + "_lora_a"], params[n + "_lora_b"]
-                ops.gemm(b.to(eff.dtype), a.to(eff.dtype), alpha=self.lora.scale, beta=1.0, out=eff[r0:r0 + w.shape[0]])
+                ops.gemm(b.to(eff.dtype), a.to(eff.dtype), alpha=self.lora.scale, beta=1.0, c=base, out=part)
+            else:
+                part.copy_(w)
             r0 += w.shape[0]
         params[key] = eff
         return eff

@@ -71,3 +71,21 @@ def test_other_forms_keep_the_gemms(case):
         return
     assert not cuda.lora_wgrad_supported(x, ad)
     _check(x, ad, ops.lora_wgrad)
+
+
+@pytest.mark.parametrize("rows", [(64, 32, 32), (1000,), (2048, 256)])
+def test_merged_weight_from_the_base_in_place(rows):
+    """The same bits as the product added to a copy of the weight, the base untouched; a member without an adapter is copied."""
+    from flextrain_b200.nn.blocks.linear import LinearGroup, LoRAConfig
+    torch.manual_seed(0)
+    names = [f"w_{i}" for i in range(len(rows))]
+    lora = LoRAConfig(targets=tuple(names[:2]), rank=16, alpha=8.0)
+    p = {n: torch.randn(r, 256, device="cuda").to(BF) for n, r in zip(names, rows)}
+    for n, r in zip(names[:2], rows):
+        p[n + "_lora_a"], p[n + "_lora_b"] = torch.randn(16, 256, device="cuda").to(BF), torch.randn(r, 16, device="cuda").to(BF)
+    base = {n: p[n].clone() for n in names}
+    want = torch.cat([base[n] for n in names])
+    for n, o in zip(names[:2], (0, rows[0])):
+        ops.gemm(p[n + "_lora_b"], p[n + "_lora_a"], alpha=lora.scale, beta=1.0, out=want[o:o + p[n].shape[0]])
+    assert torch.equal(LinearGroup(names, lora).weight(p), want)
+    assert all(torch.equal(p[n], base[n]) for n in names)
