@@ -891,17 +891,26 @@ __global__ void glu_bwd_weighted_kernel(const bf16* __restrict__ dact, const bf1
 // ----------------------------------------------------------------- softmax cross-entropy
 // One CTA per row. Pass 1: online max / sum over V (bf16 logits). Pass 2: logits <- grad_scale *
 // (softmax - onehot) in place (the second read hits L2). Optional tanh soft-cap chained through.
-constexpr int CE_THREADS = 512;
 // A row is read twice (its second reading is for the gradient, which takes its place), CE_BATCH 16-byte pieces a thread at a
 // time: with one piece in flight the kernel waited for memory.  GRAD = false: held-out loss, the logits are only read, once.
-// 4096 x 262144: 1.10 -> 1.00 ms; 4000 x 151936, loss only: 0.71 ms when the gradient was written too, 0.28 ms so.
-constexpr int CE_BATCH = 4;
-template <bool GRAD>
-__global__ void __launch_bounds__(CE_THREADS) softmax_ce_kernel(bf16* __restrict__ logits,
-                                                                 const long* __restrict__ targets,
-                                                                 const float* __restrict__ loss_mask,
-                                                                 float* __restrict__ loss, int T, int V, long ld,
-                                                                 float grad_scale, float softcap, long ignore_index) {
+// Nothing is used up (two exponentials an element take half of the time, memory two thirds), so what counts is how much is in
+// flight and that the second reading still finds the row in L2.  Rows of 112 KB and more: two blocks of 512 threads an SM, eight
+// pieces a thread; 2048 x 128256 225 -> 210 us (before: four pieces, a test for the target at each element), 4096 x 151936 551 -> 523,
+// 4096 x 262144 977 -> 948, with a soft-cap 1207 -> 1106; 2048 x 65544 117 -> 107.  Shorter rows, two blocks an SM of them and more: four
+// blocks of 256, whose sums over the block weigh less; 8192 x 32000 232 -> 178 (216 as the long rows), 2048 x 50304 98 -> 84 (86);
+// 65536: 113 (107); 128256: 240.  Few short rows as the long ones (16 x 50304 19.1 us, 19.8 with 256 threads).
+constexpr int CE_BATCH = 8, CE_LONG = 57344, CE_ROWS = 2 * 148;
+template <bool CAP>
+__device__ __forceinline__ float ce_cap(float f, float softcap, float inv_cap, float& d) {
+  if (!CAP) return f;
+  const float t = tanhf(f * inv_cap);
+  d = 1.f - t * t;
+  return softcap * t;
+}
+template <bool GRAD, bool CAP, int CE_THREADS>
+__global__ void __launch_bounds__(CE_THREADS, 1024 / CE_THREADS)
+    softmax_ce_kernel(bf16* __restrict__ logits, const long* __restrict__ targets, const float* __restrict__ loss_mask,
+                      float* __restrict__ loss, int T, int V, long ld, float grad_scale, float softcap, long ignore_index) {
   __shared__ float sh[32];
   const int row = blockIdx.x;
   bf16* z = logits + (size_t)row * ld;
@@ -909,7 +918,7 @@ __global__ void __launch_bounds__(CE_THREADS) softmax_ce_kernel(bf16* __restrict
   bool valid = tgt != ignore_index && tgt >= 0 && tgt < V;
   if (loss_mask && loss_mask[row] <= 0.f) valid = false;
   const int nv = V >> 3;
-  const float inv_cap = softcap > 0.f ? 1.f / softcap : 0.f;
+  const float inv_cap = CAP ? 1.f / softcap : 0.f;
   if (!valid) {
     if constexpr (GRAD) {
       const uint4 zero = make_uint4(0, 0, 0, 0);
@@ -919,7 +928,7 @@ __global__ void __launch_bounds__(CE_THREADS) softmax_ce_kernel(bf16* __restrict
     if (threadIdx.x == 0) loss[row] = 0.f;
     return;
   }
-  float m = -INFINITY, s = 0.f;
+  float m = -INFINITY, s = 0.f, unused;
   for (int i0 = threadIdx.x; i0 < nv; i0 += CE_BATCH * CE_THREADS) {
     uint4 v[CE_BATCH];
 #pragma unroll
@@ -933,7 +942,7 @@ __global__ void __launch_bounds__(CE_THREADS) softmax_ce_kernel(bf16* __restrict
       float lm = -INFINITY;
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        if (softcap > 0.f) f[e] = softcap * tanhf(f[e] * inv_cap);
+        f[e] = ce_cap<CAP>(f[e], softcap, inv_cap, unused);
         lm = fmaxf(lm, f[e]);
       }
       const float nm = fmaxf(m, lm);
@@ -945,8 +954,7 @@ __global__ void __launch_bounds__(CE_THREADS) softmax_ce_kernel(bf16* __restrict
     }
   }
   for (int i = (nv << 3) + threadIdx.x; i < V; i += CE_THREADS) {
-    float f = __bfloat162float(z[i]);
-    if (softcap > 0.f) f = softcap * tanhf(f * inv_cap);
+    const float f = ce_cap<CAP>(__bfloat162float(z[i]), softcap, inv_cap, unused);
     const float nm = fmaxf(m, f);
     s = s * __expf(m - nm) + __expf(f - nm);
     m = nm;
@@ -955,14 +963,15 @@ __global__ void __launch_bounds__(CE_THREADS) softmax_ce_kernel(bf16* __restrict
   s = (m == -INFINITY) ? 0.f : s * __expf(m - gm);
   const float gs = block_sum<CE_THREADS / 32>(s, sh);
   const float lse = gm + logf(gs);
+  float target = 0.f;                            // the target's gradient, written once all others are (thread 0)
   if (threadIdx.x == 0) {
-    float zt = __bfloat162float(z[tgt]);
-    if (softcap > 0.f) zt = softcap * tanhf(zt * inv_cap);
+    float d = 1.f;
+    const float zt = ce_cap<CAP>(__bfloat162float(z[tgt]), softcap, inv_cap, d);
     loss[row] = lse - zt;
+    target = (__expf(zt - lse) - 1.f) * grad_scale * d;
   }
   if constexpr (!GRAD) return;
   __syncthreads();  // the target logit is read before anyone overwrites it
-  const int tv = (int)(tgt >> 3), te = (int)(tgt & 7);
   for (int i0 = threadIdx.x; i0 < nv; i0 += CE_BATCH * CE_THREADS) {
     uint4 v[CE_BATCH];
 #pragma unroll
@@ -976,30 +985,31 @@ __global__ void __launch_bounds__(CE_THREADS) softmax_ce_kernel(bf16* __restrict
       unpack8(v[k], f);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        float zc = f[e], dcap = 1.f;
-        if (softcap > 0.f) {
-          const float t = tanhf(f[e] * inv_cap);
-          zc = softcap * t;
-          dcap = 1.f - t * t;
-        }
-        float p = __expf(zc - lse);
-        if (i == tv && e == te) p -= 1.f;
-        f[e] = p * grad_scale * dcap;
+        float d = 1.f;
+        const float zc = ce_cap<CAP>(f[e], softcap, inv_cap, d);
+        f[e] = __expf(zc - lse) * grad_scale * d;
       }
       reinterpret_cast<uint4*>(z)[i] = pack8(f);
     }
   }
   for (int i = (nv << 3) + threadIdx.x; i < V; i += CE_THREADS) {
-    float f = __bfloat162float(z[i]), dcap = 1.f;
-    if (softcap > 0.f) {
-      const float t = tanhf(f * inv_cap);
-      f = softcap * t;
-      dcap = 1.f - t * t;
-    }
-    float p = __expf(f - lse);
-    if (i == tgt) p -= 1.f;
-    z[i] = __float2bfloat16(p * grad_scale * dcap);
+    float d = 1.f;
+    const float f = ce_cap<CAP>(__bfloat162float(z[i]), softcap, inv_cap, d);
+    z[i] = __float2bfloat16(__expf(f - lse) * grad_scale * d);
   }
+  __syncthreads();
+  if (threadIdx.x == 0) z[tgt] = __float2bfloat16(target);
+}
+
+template <bool GRAD>
+void run_softmax_ce(bf16* logits, const long* targets, const float* loss_mask, float* loss, int T, int V, long ld, float grad_scale,
+                    float softcap, long ignore_index, cudaStream_t s) {
+  const bool cap = softcap > 0.f;
+  auto wide = cap ? softmax_ce_kernel<GRAD, true, 512> : softmax_ce_kernel<GRAD, false, 512>;
+  auto narrow = cap ? softmax_ce_kernel<GRAD, true, 256> : softmax_ce_kernel<GRAD, false, 256>;
+  const bool is_long = V > CE_LONG || T < CE_ROWS;
+  (is_long ? wide : narrow)<<<T, is_long ? 512 : 256, 0, s>>>(logits, targets, loss_mask, loss, T, V, ld, grad_scale, softcap,
+                                                              ignore_index);
 }
 
 // ----------------------------------------------------------------------------- embedding
@@ -1693,8 +1703,7 @@ int ftb_softmax_ce(void* logits, const long* targets, const float* loss_mask, fl
                    float grad_scale, float softcap, long ignore_index, cudaStream_t s) {
   if (T == 0) return 0;
   if (ld % 8) return -2;
-  softmax_ce_kernel<true><<<T, CE_THREADS, 0, s>>>((bf16*)logits, targets, loss_mask, loss, T, V, ld, grad_scale, softcap,
-                                                   ignore_index);
+  run_softmax_ce<true>((bf16*)logits, targets, loss_mask, loss, T, V, ld, grad_scale, softcap, ignore_index, s);
   CHECK_LAUNCH();
 }
 // The losses alone; the logits stay as they are.
@@ -1702,8 +1711,7 @@ int ftb_softmax_ce_loss(const void* logits, const long* targets, const float* lo
                         float softcap, long ignore_index, cudaStream_t s) {
   if (T == 0) return 0;
   if (ld % 8) return -2;
-  softmax_ce_kernel<false><<<T, CE_THREADS, 0, s>>>((bf16*)logits, targets, loss_mask, loss, T, V, ld, 0.f, softcap,
-                                                    ignore_index);
+  run_softmax_ce<false>((bf16*)logits, targets, loss_mask, loss, T, V, ld, 0.f, softcap, ignore_index, s);
   CHECK_LAUNCH();
 }
 // bytes of zeros at p (a memory node under capture)
