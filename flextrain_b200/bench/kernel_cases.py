@@ -93,13 +93,14 @@ def main(case: str) -> None:
         fl = 2.0 * T * HV * dk * dv * 3          # decay+predict, update, read-out: 3 multiply-adds per state element
         if case != "gdn_bwd":
             ms = _time(lambda: la.gdn_fwd(q, kk, v, g, beta, cu, None, want_r=True))
-            print(f"{case}: {S} x {L} tokens, HV={HV} dk={dk} dv={dv}  {ms:.3f} ms  {fl / ms / 1e9:.1f} TFLOP/s fp32 "
-                  f"(state recurrence on CUDA cores)")
+            print(f"{case}: {S} x {L} tokens, HV={HV} dk={dk} dv={dv}  {ms:.3f} ms  {fl / ms / 1e9:.1f} TFLOP/s "
+                  f"of the recurrence's multiply-adds")
         else:
             o, fin, r = la.gdn_fwd(q, kk, v, g, beta, cu, None, want_r=True)
             d_o = torch.randn_like(o)
             ms = _time(lambda: la.gdn_bwd(q, kk, v, g, beta, cu, None, fin, r, d_o))
-            print(f"{case}: {S} x {L} tokens, HV={HV} dk={dk} dv={dv}  {ms:.3f} ms  {2.2 * fl / ms / 1e9:.1f} TFLOP/s fp32")
+            print(f"{case}: {S} x {L} tokens, HV={HV} dk={dk} dv={dv}  {ms:.3f} ms  {2.2 * fl / ms / 1e9:.1f} TFLOP/s "
+                  f"of the recurrence's multiply-adds")
     elif case in ("attn_fwd", "attn_bwd", "attn_bwd_unordered", "attn_fwd_one_tile", "attn_fwd_32k", "attn_bwd_32k",
                   "attn_bwd_thread_reds", "attn_bwd_32k_thread_reds"):
         if case.endswith("_thread_reds"):      # dQ by per-thread 16-byte reductions (the earlier drain), same GPU
