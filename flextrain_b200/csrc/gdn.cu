@@ -62,6 +62,9 @@ struct GdnArgs {
   int HK, HV, DV;
   float scale;
   int vec;             // every tensor of rows starts on 16 bytes
+  // what is done again for the chunk kernels (REDO)
+  long v_gap, dv_gap;  // elements of v / dv between a token's last head and the next token
+  const int* only;     // (nseq, HV): run the (sequence, head) pairs marked there, leave the others alone
 };
 
 __device__ __forceinline__ float half_warp_sum(float x) {   // over the 16 lanes that share tj
@@ -184,7 +187,7 @@ __device__ __forceinline__ void put_bf16(float* dst, const uint4& u, float scale
   reinterpret_cast<float4*>(dst)[0] = make_float4(f[0], f[1], f[2], f[3]);
   reinterpret_cast<float4*>(dst)[1] = make_float4(f[4], f[5], f[6], f[7]);
 }
-template <int DK, int NC, bool GRAD>
+template <int DK, int NC, bool GRAD, bool REDO>
 struct Incoming {
   uint4 k, q, x;
   float g, b;
@@ -199,7 +202,7 @@ struct Incoming {
     const int t = e / NC, c = e % NC;
     if (t < nt) {
       const size_t off = ((size_t)(tb + t) * a.HV + hv) * a.DV + col0 + c;
-      if (tid < 32) x = load_piece(a.v + off, a.vec);
+      if (tid < 32) x = load_piece(a.v + off + (REDO ? (tb + t) * a.v_gap : 0), a.vec);
       else if (GRAD && tid < 64) x = load_piece(a.d_o + off, a.vec);
       else if (GRAD) x = load_piece(rows + off, a.vec);
     }
@@ -229,7 +232,7 @@ struct Incoming {
 };
 
 // MODE 0: forward (o, r, final state).  MODE 1: pass F of the backward (dq, dk += S^ dr).
-template <int RPT, int CPT, int MODE>
+template <int RPT, int CPT, int MODE, bool REDO>
 __global__ void __launch_bounds__(NT) gdn_forward_kernel(const GdnArgs a) {
   constexpr int DK = 16 * RPT, NC = 8 * CPT, NP = RPT == 1 ? 1 : RPT / 2;
   __shared__ __align__(16) float k_s[TB][DK], q_s[TB][DK];
@@ -239,6 +242,7 @@ __global__ void __launch_bounds__(NT) gdn_forward_kernel(const GdnArgs a) {
   __shared__ __align__(16) float acc_k[MODE == 1 ? 4 : 1][TB][MODE == 1 ? DK : 1];
   const int tid = threadIdx.x, ti = tid & 15, tj = tid >> 4, warp = tid >> 5;
   const int col0 = blockIdx.x * NC, hv = blockIdx.y, seq = blockIdx.z;
+  if (REDO && a.only[seq * a.HV + hv] == 0) return;
   const int hk = hv / (a.HV / a.HK);
   const int t0 = a.cu[seq], t1 = a.cu[seq + 1];
   f32x2 S[NP][CPT];
@@ -248,7 +252,7 @@ __global__ void __launch_bounds__(NT) gdn_forward_kernel(const GdnArgs a) {
     for (int cc = 0; cc < CPT; ++cc)
       S[j][cc] = a.state_in ? load_state<RPT>(a.state_in + ((size_t)seq * a.HV + hv) * DK * a.DV + col0 + tj * CPT + cc,
                                               a.DV, ti, j) : 0ull;
-  Incoming<DK, NC, MODE == 1> in;
+  Incoming<DK, NC, MODE == 1, REDO> in;
   if (t0 < t1) in.fetch(a, a.de, t0, min(TB, t1 - t0), hk, hv, col0);
   for (int tb = t0; tb < t1; tb += TB) {
     const int nt = min(TB, t1 - tb);
@@ -387,7 +391,7 @@ __global__ void __launch_bounds__(NT) gdn_forward_kernel(const GdnArgs a) {
 }
 
 // Pass R: reverse in time.  state_in = gradient of the final state (or null), state_out = gradient of the initial one.
-template <int RPT, int CPT>
+template <int RPT, int CPT, bool REDO>
 __global__ void __launch_bounds__(NT) gdn_reverse_kernel(const GdnArgs a) {
   constexpr int DK = 16 * RPT, NC = 8 * CPT, NP = RPT == 1 ? 1 : RPT / 2;
   __shared__ __align__(16) float k_s[TB][DK], q_s[TB][DK];
@@ -397,6 +401,7 @@ __global__ void __launch_bounds__(NT) gdn_reverse_kernel(const GdnArgs a) {
   __shared__ float acc_b[4][TB];
   const int tid = threadIdx.x, ti = tid & 15, tj = tid >> 4, warp = tid >> 5;
   const int col0 = blockIdx.x * NC, hv = blockIdx.y, seq = blockIdx.z;
+  if (REDO && a.only[seq * a.HV + hv] == 0) return;
   const int hk = hv / (a.HV / a.HK);
   const int t0 = a.cu[seq], t1 = a.cu[seq + 1];
   f32x2 dS[NP][CPT];
@@ -407,7 +412,7 @@ __global__ void __launch_bounds__(NT) gdn_reverse_kernel(const GdnArgs a) {
       dS[j][cc] = a.state_in ? load_state<RPT>(a.state_in + ((size_t)seq * a.HV + hv) * DK * a.DV + col0 + tj * CPT + cc,
                                                a.DV, ti, j) : 0ull;
   const int nblk = (t1 - t0 + TB - 1) / TB;
-  Incoming<DK, NC, true> in;
+  Incoming<DK, NC, true, REDO> in;
   if (nblk > 0) in.fetch(a, a.r, t0 + (nblk - 1) * TB, t1 - t0 - (nblk - 1) * TB, hk, hv, col0);
   for (int blk = nblk - 1; blk >= 0; --blk) {
     const int tb = t0 + blk * TB;
@@ -449,7 +454,7 @@ __global__ void __launch_bounds__(NT) gdn_reverse_kernel(const GdnArgs a) {
         if (ti == 0) {
           const size_t off = ((size_t)(tb + t) * a.HV + hv) * a.DV + col0 + tj * CPT + cc;
           a.de[off] = de[cc];
-          a.dv[off] = __float2bfloat16(bt * de[cc]);
+          a.dv[off + (REDO ? (tb + t) * a.dv_gap : 0)] = __float2bfloat16(bt * de[cc]);
         }
       }
       db += __shfl_xor_sync(0xffffffffu, db, 16);       // every lane of a half warp holds the same db
@@ -536,12 +541,24 @@ __global__ void __launch_bounds__(1024) suffix_sum_kernel(const float* __restric
   }
 }
 
-template <int RPT, int CPT>
+// Zeros where the two backward passes add up, for the pairs marked in `only`.
+__global__ void __launch_bounds__(NT) gdn_clear_kernel(const GdnArgs a, int DK) {
+  const int hv = blockIdx.x, seq = blockIdx.y;
+  if (a.only[seq * a.HV + hv] == 0) return;
+  const int t0 = a.cu[seq], t1 = a.cu[seq + 1];
+  for (int t = t0; t < t1; ++t) {
+    const size_t th = (size_t)t * a.HV + hv;
+    for (int i = threadIdx.x; i < DK; i += NT) a.dq[th * DK + i] = a.dk[th * DK + i] = 0.f;
+    if (threadIdx.x == 0) a.dbeta[th] = a.sacc[th] = 0.f;
+  }
+}
+
+template <int RPT, int CPT, bool REDO>
 int launch_all(int pass, const GdnArgs& a, int nseq, cudaStream_t s) {
   dim3 grid(a.DV / (8 * CPT), a.HV, nseq);
-  if (pass == 0) gdn_forward_kernel<RPT, CPT, 0><<<grid, NT, 0, s>>>(a);
-  else if (pass == 1) gdn_reverse_kernel<RPT, CPT><<<grid, NT, 0, s>>>(a);
-  else gdn_forward_kernel<RPT, CPT, 1><<<grid, NT, 0, s>>>(a);
+  if (pass == 0) gdn_forward_kernel<RPT, CPT, 0, REDO><<<grid, NT, 0, s>>>(a);
+  else if (pass == 1) gdn_reverse_kernel<RPT, CPT, REDO><<<grid, NT, 0, s>>>(a);
+  else gdn_forward_kernel<RPT, CPT, 1, REDO><<<grid, NT, 0, s>>>(a);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -400 - (int)e;
 }
@@ -556,12 +573,12 @@ int cols_per_thread(int nseq, int HV, int DV) {
   return 0;
 }
 
-template <int RPT>
+template <int RPT, bool REDO = false>
 int launch_cols(int pass, const GdnArgs& a, int nseq, cudaStream_t s) {
   switch (cols_per_thread(nseq, a.HV, a.DV)) {
-    case 4: return launch_all<RPT, 4>(pass, a, nseq, s);
-    case 2: return launch_all<RPT, 2>(pass, a, nseq, s);
-    case 1: return launch_all<RPT, 1>(pass, a, nseq, s);
+    case 4: return launch_all<RPT, 4, REDO>(pass, a, nseq, s);
+    case 2: return launch_all<RPT, 2, REDO>(pass, a, nseq, s);
+    case 1: return launch_all<RPT, 1, REDO>(pass, a, nseq, s);
     default: return -2;
   }
 }
@@ -608,7 +625,7 @@ int ftb_gdn(int pass, const void* q, const void* k, const void* v, const float* 
             cudaStream_t s) {
   if (nseq <= 0) return 0;
   if (HV % HK) return -2;
-  GdnArgs a;
+  GdnArgs a = {};
   a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.g = g; a.beta = beta; a.cu = cu;
   a.state_in = state_in; a.state_out = state_out; a.o = (bf16*)o; a.r = r; a.d_o = (const bf16*)d_o; a.de = de;
   a.dv = (bf16*)dv; a.dbeta = dbeta; a.dq = dq; a.dk = dk; a.sacc = sacc; a.HK = HK; a.HV = HV; a.DV = DV; a.scale = scale;
@@ -620,6 +637,39 @@ int ftb_gdn(int pass, const void* q, const void* k, const void* v, const float* 
     case 128: return launch_cols<8>(pass, a, nseq, s);
     default: return -2;
   }
+}
+
+// What the chunk kernels (gdn_chunk.cu, heads of 128 x 128) marked in `only` (nseq, HV), because infinities or NaN came up in it,
+// done again token by token, in place of what they wrote; v and dv with the token strides they may have there.  Blocks of
+// pairs that are not marked return at once: 2 to 3 us a launch.
+int ftb_gdn_redo_fwd(const int* only, const void* q, const void* k, const void* v, long v_ts, const float* g, const float* beta,
+                     const int* cu, int nseq, const float* state_in, float* state_out, void* o, float* r, int HK, int HV, float scale,
+                     cudaStream_t s) {
+  if (nseq <= 0) return 0;
+  GdnArgs a = {};
+  a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.g = g; a.beta = beta; a.cu = cu; a.state_in = state_in;
+  a.state_out = state_out; a.o = (bf16*)o; a.r = r; a.HK = HK; a.HV = HV; a.DV = 128; a.scale = scale;
+  a.vec = 1; a.v_gap = v_ts - (long)HV * 128; a.only = only;
+  return launch_cols<8, true>(0, a, nseq, s);
+}
+int ftb_gdn_redo_bwd(const int* only, const void* q, const void* k, const void* v, long v_ts, const float* g, const float* beta,
+                     const int* cu, int nseq, const float* state_in, const float* dstate_in, float* dstate_out, const float* r,
+                     const void* d_o, float* de, void* dv, long dv_ts, float* dbeta, float* dq, float* dk, float* sacc, int HK, int HV,
+                     float scale, cudaStream_t s) {
+  if (nseq <= 0) return 0;
+  GdnArgs a = {};
+  a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.g = g; a.beta = beta; a.cu = cu; a.state_in = dstate_in;
+  a.state_out = dstate_out; a.r = const_cast<float*>(r); a.d_o = (const bf16*)d_o; a.de = de; a.dv = (bf16*)dv; a.dbeta = dbeta;
+  a.dq = dq; a.dk = dk; a.sacc = sacc; a.HK = HK; a.HV = HV; a.DV = 128; a.scale = scale;
+  a.vec = 1; a.v_gap = v_ts - (long)HV * 128; a.dv_gap = dv_ts - (long)HV * 128; a.only = only;
+  gdn_clear_kernel<<<dim3(HV, nseq), NT, 0, s>>>(a, 128);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return -400 - (int)e;
+  const int rc = launch_cols<8, true>(1, a, nseq, s);
+  if (rc) return rc;
+  a.state_in = state_in;
+  a.state_out = nullptr;
+  return launch_cols<8, true>(2, a, nseq, s);
 }
 
 }  // extern "C"

@@ -27,8 +27,8 @@
 // what the warps share (K, Q, the inverse).  The backward products that sum over value columns (dQ, dK) are the exception: there
 // the state goes through shared memory once a chunk, and a warp owns tokens.
 //
-// Measured, ms, token by token (gdn.cu) / so, 32 heads: 16 x 1024 tokens forward 2.19 / 1.00, backward 7.98 / 4.12; one sequence
-// of 16384 7.5 / 3.2 and 25.4 / 14.8; two of 8192 4.6 / 1.7 and 15.1 / 7.7; 512 tokens 0.22 / 0.12 and 0.81 / 0.49; 300 sequences of
+// Measured, ms, token by token (gdn.cu) / so, 32 heads: 16 x 1024 tokens forward 2.19 / 1.02, backward 7.98 / 4.19; one sequence
+// of 16384 7.5 / 3.3 and 25.4 / 15.0; two of 8192 4.6 / 1.8 and 15.1 / 7.8; 512 tokens 0.22 / 0.13 and 0.81 / 0.51; 300 sequences of
 // 33, mostly half-empty chunks, 1.60 / 1.29 and 5.16 / 5.33.  Errors against fp64 (2-norm, gates as a model's): final state 4.8e-8
 // / 6.9e-8, dq 1.16e-7 / 1.13e-7, dk 1.54e-7 / 1.14e-7, dg 1.0e-5 / 4.4e-6; with slow decay (0.01 a token) 2.0e-6 / 1.4e-7, 1.6e-6
 // / 1.8e-7, 2.0e-6 / 2.3e-7.  What bounds it now: the chain of a sequence, product after product; mma.sync (537 TFLOP/s) is in
@@ -66,6 +66,7 @@ struct Args {
   float* tri_p;            // (slots, HV, 10, 16, 16)  P
   double* gsum;            // (slots, HV, 64)          G in powers of two
   int* order;              // (nseq)  sequences, longest first
+  int* redo;               // (nseq, HV)  1: infinities or NaN came up, the results do not count
   int HK, HV, nseq;
   long T, v_ts, dv_ts;
   float scale;
@@ -388,6 +389,7 @@ struct alignas(16) Gates {     // of the chunk at work
   float dec[C];                // exp(G_C - G_i)
   float bet[C];
   float end;                   // exp(G_C)
+  int bad;                     // 1: something was not finite so far
 };
 
 __device__ __forceinline__ void make_gates(Gates* s, const Args& a, long slot, int t0, int n, int hv, int tid) {
@@ -456,6 +458,34 @@ __device__ __forceinline__ void tri_times(float (&acc)[8][4], const float (&x)[8
     }
   }
 }
+// Infinities and NaN.  A triangular product multiplies the zeros above the diagonal of its 16 x 16 blocks too, and an infinity has no
+// three terms, so a value that is not finite would reach tokens that it does not concern.  Each of the chain kernels marks
+// the pairs of sequence and head where one came up, and these are done again token by token (ftb_gdn_redo_fwd and _bwd of
+// gdn.cu).  What a token writes into the state stays in it: 0 * x, added up, is 0 for finite x alone, also of the state at the end.
+// (The mark is in shared memory: a register for it would be one more to spill.)  16 x 1024 tokens, 32 heads: forward 1.00 -> 1.02 ms,
+// backward 4.12 -> 4.19, for the look and the launches that follow.
+__device__ __forceinline__ void add_zero_times(float& nan, float x) {
+  asm volatile("fma.rn.f32 %0, %1, 0f00000000, %0;" : "+f"(nan) : "f"(x));
+}
+__device__ __forceinline__ void mark(Gates* gt, float nan) {
+  if (__float_as_uint(nan) & 0x7fffffffu) gt->bad = 1;
+}
+template <int N>
+__device__ __forceinline__ void look_at(Gates* gt, const float (&x)[N][4]) {
+  float n[4] = {};
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) add_zero_times(n[e], x[i][e]);
+  mark(gt, (n[0] + n[1]) + (n[2] + n[3]));
+}
+__device__ __forceinline__ void look_at(Gates* gt, float x, float y) {
+  float n = 0.f;
+  add_zero_times(n, x);
+  add_zero_times(n, y);
+  mark(gt, n);
+}
+
 // The value columns of a chunk's rows in shared memory (the warp's own 16 columns) out to global memory, 16 bytes a lane.
 __device__ __forceinline__ void store_rows(bf16* dst, long row_stride, uint32_t tile, int warp, int n, int lane) {
 #pragma unroll
@@ -501,6 +531,7 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_forward_kernel(const Args a) 
   float S[16][4];
   load_state(S, a.state_in ? a.state_in + ((size_t)seq * a.HV + hv) * DK * DV : nullptr, warp * 16, lane);
   if (nc > 0) fetch(0);
+  if (tid == 0) gt->bad = 0;
   for (int c = 0; c < nc; ++c) {
     cp_wait_all();
     __syncthreads();                               // this chunk is there, and the one before is done with everything
@@ -564,6 +595,7 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_forward_kernel(const Args a) 
       Y[nb][3] *= b.y;
     }
     tri_times(O, Y, smem_addr(planes_p), lane);
+    look_at(gt, O);
     __syncwarp();                                  // the output takes the place of v in the warp's own columns
 #pragma unroll
     for (int np = 0; np < 4; ++np)
@@ -593,6 +625,10 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_forward_kernel(const Args a) 
     }
   }
   if (a.state_out) store_state(a.state_out + ((size_t)seq * a.HV + hv) * DK * DV, S, warp * 16, lane);
+  __syncthreads();
+  look_at(gt, S);
+  __syncthreads();
+  if (tid == 0) a.redo[seq * a.HV + hv] = gt->bad;
 }
 
 // ================================================================================================ backward, reverse in time
@@ -710,6 +746,7 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_reverse_kernel(const Args a) 
   float X[16][4];
   load_state(X, a.state_in ? a.state_in + ((size_t)seq * a.HV + hv) * DK * DV : nullptr, warp * 16, lane);
   if (nc > 0) fetch(nc - 1);
+  if (tid == 0) gt->bad = 0;
   for (int c = nc - 1; c >= 0; --c) {
     cp_wait_all();
     __syncthreads();
@@ -853,11 +890,13 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_reverse_kernel(const Args a) 
       }
       kd += __shfl_xor_sync(0xffffffffu, kd, 1);
       kd += __shfl_xor_sync(0xffffffffu, kd, 2);
+      look_at(gt, kd, 0.f);
       if ((tid & 3) == 0 && row < n) a.sacc[(long)(t + row) * a.HV + hv] = -kd;
       if (tid < n) {
         float s8 = 0.f;
 #pragma unroll
         for (int w = 0; w < 8; ++w) s8 += dot[w * C + tid];
+        look_at(gt, s8, 0.f);
         a.dbeta[(long)(t + tid) * a.HV + hv] = s8;
       }
     }
@@ -899,6 +938,10 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_reverse_kernel(const Args a) 
     store_rows(a.dv + (long)t * a.dv_ts + hv * DV, a.dv_ts, d_s, warp, n, lane);
   }
   if (a.state_out) store_state(a.state_out + ((size_t)seq * a.HV + hv) * DK * DV, X, warp * 16, lane);
+  __syncthreads();
+  look_at(gt, X);
+  __syncthreads();
+  if (tid == 0) a.redo[seq * a.HV + hv] = gt->bad;
 }
 
 // ================================================================================================ backward, forward in time
@@ -945,6 +988,7 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
   float S[16][4];
   load_state(S, a.state_in ? a.state_in + ((size_t)seq * a.HV + hv) * DK * DV : nullptr, warp * 16, lane);
   if (nc > 0) fetch(0);
+  if (tid == 0) gt->bad = 0;
   for (int c = 0; c < nc; ++c) {
     const int t = t0 + c * C, n = min(C, t1 - t);
     make_gates(gt, a, slot0 + c, t, n, hv, tid);
@@ -1166,6 +1210,7 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
         }
         sc += __shfl_xor_sync(0xffffffffu, sc, 1);
         sc += __shfl_xor_sync(0xffffffffu, sc, 2);
+        look_at(gt, sc, w_ii);
         if ((lane & 3) == 0) sums[half * C + r] = sc;
       }
     }
@@ -1202,11 +1247,17 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
       const float c1 = col1[tid] + col1[C + tid] + col1[2 * C + tid] + col1[3 * C + tid];
       const float c2 = col2[tid] + col2[C + tid] + col2[2 * C + tid] + col2[3 * C + tid];
       const long at = (long)(t + tid) * a.HV + hv;
+      const float sc = (sums[tid] + sums[C + tid]) - 2.f * (c1 + gt->bet[tid] * c2);
       a.dbeta[at] += c2;
-      a.sacc[at] += (sums[tid] + sums[C + tid]) - 2.f * (c1 + gt->bet[tid] * c2);
+      a.sacc[at] += sc;
+      look_at(gt, c2, sc);
     }
     __syncthreads();
   }
+  __syncthreads();
+  look_at(gt, S);
+  __syncthreads();
+  if (gt->bad && tid == 0) a.redo[seq * a.HV + hv] = 1;   // (or the reverse pass has seen one)
 }
 
 template <typename F>
@@ -1228,9 +1279,10 @@ long ftb_gdn_chunk_bytes(long T, int nseq, int HV) {
   return slots * HV * (2L * kTri * 4 + C * 8) + (nseq + 15L) / 16 * 64;
 }
 
-// What gdn.cu's pass 0 does (o, r, final state), for DK = DV = 128 and tensors on 16 bytes.  Returns -2 for anything else.
+// What gdn.cu's pass 0 does (o, r, final state), for DK = DV = 128 and tensors on 16 bytes.  Returns -2 for anything else.  redo
+// (nseq, HV): where ftb_gdn_redo_fwd has to follow (ftb_gdn_redo_bwd for the one below).
 int ftb_gdn_chunk_fwd(const void* q, const void* k, const void* v, long v_ts, const float* g, const float* beta, const int* cu,
-                      int nseq, long T, const float* state_in, float* state_out, void* o, float* r, void* work, int HK, int HV,
+                      int nseq, long T, const float* state_in, float* state_out, void* o, float* r, void* work, int* redo, int HK, int HV,
                       float scale, cudaStream_t s) {
   if (nseq <= 0) return 0;
   if (HK <= 0 || HV % HK || nseq > 65535 || HK > 65535 || v_ts % 8) return -2;
@@ -1243,6 +1295,7 @@ int ftb_gdn_chunk_fwd(const void* q, const void* k, const void* v, long v_ts, co
   a.tri_t = (float*)(a.gsum + slots * HV * C);
   a.tri_p = a.tri_t + slots * HV * kTri;
   a.order = (int*)(a.tri_p + slots * HV * kTri);
+  a.redo = redo;
   const int rc = launch(gdn_prep_kernel, dim3((unsigned)slots, HK), 128, kPrepSmem, a, s);
   if (rc) return rc;
   return launch(gdn_chunk_forward_kernel, dim3(HV, nseq), NT, kFwdSmem, a, s);
@@ -1252,7 +1305,7 @@ int ftb_gdn_chunk_fwd(const void* q, const void* k, const void* v, long v_ts, co
 int ftb_gdn_chunk_bwd(const void* q, const void* k, const void* v, long v_ts, const float* g, const float* beta, const int* cu,
                       int nseq, long T, const float* state_in, const float* dstate_in, float* dstate_out, const float* r,
                       const void* d_o, float* dr, void* dv, long dv_ts, float* dbeta, float* dq, float* dk, float* sacc, void* work,
-                      int HK, int HV, float scale, cudaStream_t s) {
+                      int* redo, int HK, int HV, float scale, cudaStream_t s) {
   if (nseq <= 0) return 0;
   if (HK <= 0 || HV % HK || nseq > 65535 || HK > 65535 || v_ts % 8 || dv_ts % 8) return -2;
   if ((((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)r | (uintptr_t)d_o | (uintptr_t)dr | (uintptr_t)dv | (uintptr_t)dq |
@@ -1266,6 +1319,7 @@ int ftb_gdn_chunk_bwd(const void* q, const void* k, const void* v, long v_ts, co
   a.tri_t = (float*)(a.gsum + slots * HV * C);
   a.tri_p = a.tri_t + slots * HV * kTri;
   a.order = (int*)(a.tri_p + slots * HV * kTri);
+  a.redo = redo;
   int rc = launch(gdn_prep_kernel, dim3((unsigned)slots, HK), 128, kPrepSmem, a, s);
   if (rc) return rc;
   a.state_in = dstate_in;

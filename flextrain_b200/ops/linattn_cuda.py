@@ -195,11 +195,11 @@ def gdn_fwd(q, k, v, g, beta, cu, state_in=None, scale=None, want_r=False):
     r = torch.empty(T, HV, DV, dtype=F32, device=q.device) if want_r else None
     sin = state_in.to(F32).contiguous() if state_in is not None else None
     if _chunked(S, q, v, k) and _head_rows(v):
-        work = _chunk_work(T, S, HV, q.device)
-        rc = load("gdn_chunk").ftb_gdn_chunk_fwd(
-            _ptr(q), _ptr(k), _ptr(v), c_long(v.stride(0)), _ptr(g), _ptr(beta), _ptr(cu), c_int(S), c_long(T), _ptr(sin), _ptr(fin),
-            _ptr(o), _ptr(r), _ptr(work), c_int(HK), c_int(HV), c_float(scale), _stream())
-        _check(rc, "ftb_gdn_chunk_fwd")
+        work, redo = _chunk_work(T, S, HV, q.device), torch.empty(S, HV, dtype=torch.int32, device=q.device)
+        ins = (_ptr(q), _ptr(k), _ptr(v), c_long(v.stride(0)), _ptr(g), _ptr(beta), _ptr(cu), c_int(S))
+        outs, end = (_ptr(sin), _ptr(fin), _ptr(o), _ptr(r)), (c_int(HK), c_int(HV), c_float(scale), _stream())
+        _check(load("gdn_chunk").ftb_gdn_chunk_fwd(*ins, c_long(T), *outs, _ptr(work), _ptr(redo), *end), "ftb_gdn_chunk_fwd")
+        _check(load("gdn").ftb_gdn_redo_fwd(_ptr(redo), *ins, *outs, *end), "ftb_gdn_redo_fwd")
         return o, fin, r
     _gdn(0, q, k, v.contiguous(), g, beta, cu, sin, fin, o, r, None, None, None, None, None, None, None, scale)
     return o, fin, r
@@ -231,12 +231,13 @@ def gdn_bwd(q, k, v, g, beta, cu, state_in, final_state, r, d_o, dstate_final=No
     dq_hv, dk_hv = (new(T, HV, DK, dtype=F32, device=dev) for _ in range(2))
     dstate_in = torch.empty(S, HV, DK, DV, dtype=F32, device=dev)
     if chunked:
-        work = _chunk_work(T, S, HV, dev)
-        rc = load("gdn_chunk").ftb_gdn_chunk_bwd(
-            _ptr(q), _ptr(k), _ptr(v), c_long(v.stride(0)), _ptr(g), _ptr(beta), _ptr(cu), c_int(S), c_long(T), _ptr(sin), _ptr(dsf),
-            _ptr(dstate_in), _ptr(r), _ptr(d_o), _ptr(de), _ptr(dv), c_long(dv.stride(0)), _ptr(dbeta), _ptr(dq_hv), _ptr(dk_hv),
-            _ptr(s), _ptr(work), c_int(HK), c_int(HV), c_float(scale), _stream())
-        _check(rc, "ftb_gdn_chunk_bwd")
+        work, redo = _chunk_work(T, S, HV, dev), torch.empty(S, HV, dtype=torch.int32, device=dev)
+        ins = (_ptr(q), _ptr(k), _ptr(v), c_long(v.stride(0)), _ptr(g), _ptr(beta), _ptr(cu), c_int(S))
+        outs = (_ptr(sin), _ptr(dsf), _ptr(dstate_in), _ptr(r), _ptr(d_o), _ptr(de), _ptr(dv), c_long(dv.stride(0)), _ptr(dbeta),
+                _ptr(dq_hv), _ptr(dk_hv), _ptr(s))
+        end = (c_int(HK), c_int(HV), c_float(scale), _stream())
+        _check(load("gdn_chunk").ftb_gdn_chunk_bwd(*ins, c_long(T), *outs, _ptr(work), _ptr(redo), *end), "ftb_gdn_chunk_bwd")
+        _check(load("gdn").ftb_gdn_redo_bwd(_ptr(redo), *ins, *outs, *end), "ftb_gdn_redo_bwd")
     else:
         v = v.contiguous()
         _gdn(1, q, k, v, g, beta, cu, dsf, dstate_in, None, r, d_o, de, dv, dbeta, None, dk_hv, s, scale)
