@@ -201,6 +201,7 @@ class ActiveModel:
         loss_acc = torch.zeros((), dtype=torch.float32, device=self.device)
         act_acc = torch.zeros((), dtype=torch.int64, device=self.device)
         pending_losses = []
+        in_place = False                                   # a tied head's gradient, see _tied_in_place
         with _nvtx("Fwd+Bwd"):
             for r, rseqs in enumerate(rounds):
                 with _nvtx(f"Round {r}"):
@@ -221,6 +222,7 @@ class ActiveModel:
                     if self._zero_grad and not forward_only:
                         self._zero_all_grads()
                         self._zero_grad = False
+                        in_place = len(rounds) == len(metas) == 1 and self._tied_in_place()
                     ctx_base = dict(kv_window=self.buffers.kv_window, total_tokens_per_step=total_tokens_per_step,
                                     tp=self.tp, ep=self.ep,
                                     param_gather=(self.dp.first_gemm if getattr(self.dp, "defer", False) else None))
@@ -234,7 +236,7 @@ class ActiveModel:
                         for c, meta in enumerate(metas):
                             ls = self.head.forward_backward(transitions[c], self._token_shard(meta),
                                                             self.buffers.head_params(),
-                                                            {} if forward_only else self._head_grads(),
+                                                            {} if forward_only else self._head_grads(in_place),
                                                             loss_fn, loss_scale_factor, want_dx=not forward_only)
                             loss_acc += ls.total_loss
                             act_acc += ls.active_tokens
@@ -252,7 +254,8 @@ class ActiveModel:
                         self.embed.finalize_round()
                     self.events.clear_per_round()
         if not forward_only:
-            self._fold_tied_head_grad()
+            if not in_place:
+                self._fold_tied_head_grad()
             if self.dp is not None:
                 self.dp.on_embed_head_grads_ready()
         # one host read for the whole call
@@ -300,7 +303,7 @@ class ActiveModel:
         before any reduction or update, and the head mirror is refreshed from the embedding after every step
         (:meth:`step`).  Training the mirror separately would untie the model, and an export — which writes the
         embedding only — would lose what the head learnt."""
-        if not getattr(self.head, "tied", False) or self._tied_in_place():
+        if not getattr(self.head, "tied", False):
             return
         ge = self.buffers.embed_grads().get("g_tok_embeddings")
         gh = self.buffers.head_grads().get("g_head_proj")
@@ -309,17 +312,20 @@ class ActiveModel:
             gh.zero_()
 
     def _tied_in_place(self) -> bool:
-        """Whether the head's product is added to the embedding's gradient where it lies: without it a tied step reads and
-        writes the whole table three times more (:meth:`_fold_tied_head_grad`).  Parallel runs reduce the two apart."""
+        """Whether the head's product may be added to the embedding's gradient where it lies: without it a tied step reads and
+        writes the whole table three times more (:meth:`_fold_tied_head_grad`).  Parallel runs reduce the two apart.  It is
+        done for the only chunk of a step's first call: the head's sum starts from zero there as it would in a table of its own,
+        and the embedding's share, added up in fp32, meets it in one rounding.  Further chunks and calls would have every sum
+        rounded at the size of all that there is so far, so the two shares of a call are summed apart and then folded."""
         if not getattr(self.head, "tied", False) or any(p is not None for p in (self.dp, self.tp, self.ep)):
             return False
         ge = self.buffers.embed_grads().get("g_tok_embeddings")
         gh = self.buffers.head_grads().get("g_head_proj")
         return ge is not None and gh is not None and ge.shape == gh.shape and ge.dtype == gh.dtype and ge.device == gh.device
 
-    def _head_grads(self):
+    def _head_grads(self, in_place: bool):
         grads = self.buffers.head_grads()
-        return {**grads, "g_head_proj": self.buffers.embed_grads()["g_tok_embeddings"]} if self._tied_in_place() else grads
+        return {**grads, "g_head_proj": self.buffers.embed_grads()["g_tok_embeddings"]} if in_place else grads
 
     def _head_update_spec(self):
         """What the optimizer updates of the head: a tied projection is replaced by the embedding after the step

@@ -40,3 +40,33 @@ def test_tied_gradient_in_place(optimizer):
     assert o.keys() == o1.keys()
     for k in o:                                    # the head's own state: zero for the projection, updated for the norm
         torch.testing.assert_close(o[k], o1[k], rtol=1e-3, atol=1e-6)
+
+
+def _table_gradient(calls, seqs, chunk, *, grad_dtype=torch.bfloat16, in_place=True):
+    from flextrain_b200.engine.host_memory import UnpinnedHostBackend
+    torch.manual_seed(0)
+    am = ft.from_dims(DIMS, arch="gemma3", optimizer=ft.AdamW(lr=1e-3), max_seq_len=48, max_global_batch_tokens=96,
+                      max_gpu_mem_bytes=8 << 30, max_host_mem_bytes=8 << 30, hyperparams={"sliding_window": 16, "layer_pattern": "SF"},
+                      device="cpu", compute_dtype=torch.bfloat16, master_dtype=torch.bfloat16, grad_dtype=grad_dtype,
+                      working_set=ft.WorkingSetConfig.simple(max_seq_len=48, max_global_batch_tokens=96, chunk=chunk),
+                      host_backend=UnpinnedHostBackend())
+    if not in_place:
+        am._tied_in_place = lambda: False
+    g = torch.Generator().manual_seed(1)
+    chunks = 0
+    for _ in range(calls):
+        ids = [torch.randint(0, 32, (n,), generator=g) for n in seqs]             # few token ids: rows that many tokens add to
+        chunks += am.fwd_bwd([ft.Sequence(i, targets=torch.roll(i, -1)) for i in ids], loss_scale_factor=1.0).n_chunks
+    return am.buffers.embed_grads()["g_tok_embeddings"].double(), chunks
+
+
+@pytest.mark.parametrize("calls,seqs,chunk", [(1, (48,), 48), (1, (40, 40), 48), (8, (48,), 48), (8, (40, 40), 48)])
+def test_bf16_table_gradient_over_several_calls(calls, seqs, chunk):
+    """bf16 gradients against the same sums in fp32: adding the head's share where the embedding's lies costs no precision over
+    adding up each by itself, however many calls and chunks a step has."""
+    want, n = _table_gradient(calls, seqs, chunk, grad_dtype=torch.float32)
+    assert n == calls * len(seqs)
+    err = [float((_table_gradient(calls, seqs, chunk, in_place=p)[0] - want).norm() / want.norm()) for p in (True, False)]
+    # each sum of a call is rounded once and each call's total once: 2^-9 of an element's size at the most, added up over the calls
+    assert err[1] <= 2.0 ** -9 * (1 + calls * len(seqs))
+    assert err[0] <= 1.02 * err[1]
