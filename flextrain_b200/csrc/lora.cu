@@ -404,7 +404,9 @@ int run_all(const DownArgs& d, int nd, const UpArgs& u, int nu, int runs, const 
   auto up = lora_up_kernel<R>;
   const bool many = d.T >= MANY_TOKENS;
   const int down_smem = many ? down_stages(R) * down_stage_bytes(R) : 8 * 32 * nw * R * 4;
-  e = cudaFuncSetAttribute(many ? rows : direct, cudaFuncAttributeMaxDynamicSharedMemorySize, down_smem);
+  // (the most that a kernel may ever ask for, whatever this call needs: another thread's call may be between this and its launch)
+  e = many ? cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, down_stages(R) * down_stage_bytes(R))
+           : cudaFuncSetAttribute(direct, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 32 * MAXW * R * 4);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(up, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGES * up_stage_bytes(R));
   if (e != cudaSuccess) return -300 - (int)e;
   if (many) rows<<<dim3((d.T + DROWS - 1) / DROWS, nd), 256, down_smem, s>>>(d);

@@ -89,3 +89,31 @@ def test_merged_weight_from_the_base_in_place(rows):
         ops.gemm(p[n + "_lora_b"], p[n + "_lora_a"], alpha=lora.scale, beta=1.0, out=want[o:o + p[n].shape[0]])
     assert torch.equal(LinearGroup(names, lora).weight(p), want)
     assert all(torch.equal(p[n], base[n]) for n in names)
+
+
+def test_two_threads():
+    """One adapter in one thread and three in another, whose launches take different amounts of shared memory."""
+    import threading
+    errors = []
+
+    def work(N):
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                x, ad = _inputs(64, 64, N, 32, torch.float32)
+                want = [t.clone() for a in ad for t in a[3:]]
+                ops.lora_wgrad(x, ad, 1.0)
+                step = [t - w for t, w in zip((t for a in ad for t in a[3:]), want)]
+                for _ in range(1500):
+                    ops.lora_wgrad(x, ad, 1.0)
+                for t, w, s in zip((t for a in ad for t in a[3:]), want, step):       # 1501 additions, each rounded in fp32
+                    assert (t - w - 1501 * s).abs().max() <= 1501 * 2.0 ** -22 * (w.abs() + 1501 * s.abs()).max()
+        except Exception as e:                     # noqa: BLE001 (reported in the main thread)
+            errors.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(n,)) for n in ((32,), (32, 32, 32), (32,))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
