@@ -251,7 +251,13 @@ def rope_qkv_fused(_heads, *args):
 
 def rope_qkv(q, k, v, positions, inv_freq, *, q_out, k_out, v_out, inverse=False, mrope_sections=None):
     """``q`` and ``k`` rotated into ``q_out`` and ``k_out``, ``v`` copied into ``v_out`` (pairs may be None); one launch where the
-    heads allow it.  ``q`` may be fp32 (the attention backward's accumulators)."""
+    heads allow it.  ``q`` may be fp32 (the attention backward's accumulators).  All have the tokens of ``positions``, and a
+    source and its output the same shape."""
+    pairs = ((q, q_out), (k, k_out), (v, v_out))
+    tokens = positions.shape[0]
+    if any((x is None) != (o is None) or x is not None and (x.shape != o.shape or x.dim() != 3 or x.shape[0] != tokens) for x, o in pairs):
+        raise ValueError(f"rope_qkv: {tokens} positions, " + ", ".join(
+            f"{n} {None if x is None else tuple(x.shape)} -> {None if o is None else tuple(o.shape)}" for n, (x, o) in zip("qkv", pairs)))
     if (k is not None and _cuda_bf16(k)) or (k is None and q is not None and q.is_cuda):
         kn = _kernels()
         pos = positions.to(torch.int32).contiguous()
@@ -259,7 +265,7 @@ def rope_qkv(q, k, v, positions, inv_freq, *, q_out, k_out, v_out, inverse=False
             _count()
             rope_qkv_fused(k if k is not None else q, q, k, v, pos, inv_freq, q_out, k_out, v_out, inverse)
             return
-    for x, o in ((q, q_out), (k, k_out)):
+    for x, o in pairs[:2]:
         if x is None:
             continue
         if x.dtype != o.dtype:

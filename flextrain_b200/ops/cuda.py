@@ -419,9 +419,10 @@ def rope_qkv_supported(q, k, v, q_out, k_out, v_out, positions, inv_freq, mrope_
         if t is None:
             continue
         if not (t.is_cuda and (t.dtype == torch.bfloat16 or (t is q and t.dtype == torch.float32)) and t.shape[2] == hd
-                and t.stride(2) == 1 and t.stride(1) == hd and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0):
+                and t.shape[0] == positions.numel() and t.stride(2) == 1 and t.stride(1) == hd and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0):
             return False
-    return True
+    # (the kernel takes the number of tokens and of heads from one tensor for all)
+    return all((x is None) == (o is None) and (x is None or x.shape == o.shape) for x, o in ((q, q_out), (k, k_out), (v, v_out)))
 
 
 def rope_qkv(q, k, v, positions, inv_freq, q_out, k_out, v_out, inverse=False):
