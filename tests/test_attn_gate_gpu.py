@@ -54,3 +54,32 @@ def test_norm_of_heads_apart(T, H, hd):
     n = T * H                                                      # n fp32 additions of |dy xh|, in any order
     assert ((dw.double() - (dy.double() * xh).sum((0, 1))).abs() <= n * 2.0 ** -23 * (dy.double() * xh).abs().sum((0, 1)) + 1e-6).all()
     assert ((dw - dw1).abs() <= n * 2.0 ** -22 * (dy.double() * xh).abs().sum((0, 1)) + 1e-6).all()
+
+
+@pytest.mark.parametrize("span", [1, 10, 40, 80])
+def test_gate_is_rounded_as_the_fp32_chain_is(span):
+    """Results that are not the correctly rounded ones: fp32 is off by some 2^-24, a bf16 boundary lies every 2^-8, so there are
+    some 1e-5 of them; not more than 1.5 times as many as in the tensor library's chain of fp32 operations (and 40, by chance)."""
+    torch.manual_seed(span)
+    T, H, hd = 2048, 16, 128
+    x, d = (torch.randn(T, H * hd, device="cuda").to(BF) for _ in range(2))
+    gate = ((torch.rand(T, H * hd, device="cuda") * 2 - 1) * span).to(BF)
+    s, s32 = torch.sigmoid(gate.double()), torch.sigmoid(gate.float())
+    dst = torch.empty(T, H, hd, device="cuda", dtype=BF)
+    fwd = ops.attn_gate_fwd(x, gate)
+    dx, y = ops.attn_gate_bwd(d.clone(), x, gate, dst)
+    for got, t in ((fwd, x), (y, x), (dx, d)):
+        want = (t.double() * s).float().to(BF)
+        off, chain = (int((r != want).sum()) for r in (got, (t.float() * s32).to(BF)))
+        assert off <= 1.5 * chain + 40
+    want = (d.double() * x.double() * s * (1 - s32.double())).float().to(BF).view_as(dst)      # (1 - s in fp32 on both sides)
+    off, chain = (int((r != want).sum()) for r in (dst, (d.float() * x.float() * s32 * (1 - s32)).to(BF).view_as(dst)))
+    assert off <= 1.5 * chain + 0.02 * dst.numel()     # (a fp32 sigmoid next to 1 that is one unit off changes 1 - s by far more)
+
+
+def test_gate_that_is_not_finite():
+    gate = torch.tensor([float("nan"), float("inf"), float("-inf"), 3e38, -3e38, 89.0, -89.0, 0.0], device="cuda").to(BF)[None]
+    x = torch.full_like(gate, 2.0)
+    want = (x.float() * torch.sigmoid(gate.float())).to(BF)
+    for got in (ops.attn_gate_fwd(x, gate), ops.attn_gate_bwd(x.clone(), x, gate, torch.empty(1, 1, 8, device="cuda", dtype=BF))[0]):
+        assert got[0, 0].isnan() and torch.allclose(got[0, 1:], want[0, 1:], rtol=0, atol=1e-37)
