@@ -27,12 +27,21 @@
 // what the warps share (K, Q, the inverse).  The backward products that sum over value columns (dQ, dK) are the exception: there
 // the state goes through shared memory once a chunk, and a warp owns tokens.
 //
-// Measured, ms, token by token (gdn.cu) / so, 32 heads: 16 x 1024 tokens forward 2.19 / 1.02, backward 7.98 / 4.19; one sequence
-// of 16384 7.5 / 3.3 and 25.4 / 15.0; two of 8192 4.6 / 1.8 and 15.1 / 7.8; 512 tokens 0.22 / 0.13 and 0.81 / 0.51; 300 sequences of
-// 33, mostly half-empty chunks, 1.60 / 1.29 and 5.16 / 5.33.  Errors against fp64 (2-norm, gates as a model's): final state 4.8e-8
-// / 6.9e-8, dq 1.16e-7 / 1.13e-7, dk 1.54e-7 / 1.14e-7, dg 1.0e-5 / 4.4e-6; with slow decay (0.01 a token) 2.0e-6 / 1.4e-7, 1.6e-6
-// / 1.8e-7, 2.0e-6 / 2.3e-7.  What bounds it now: the chain of a sequence, product after product; mma.sync (537 TFLOP/s) is in
-// use for about half of the time.
+// Measured, ms, token by token (gdn.cu) / so, 32 heads: 16 x 1024 tokens forward 2.19 / 1.05, backward 7.98 / 4.22; one sequence
+// of 16384 7.5 / 3.3 and 25.4 / 15.1; two of 8192 4.6 / 1.8 and 15.1 / 7.8; 512 tokens 0.22 / 0.13 and 0.81 / 0.51; 300 sequences of
+// 33, mostly half-empty chunks, 1.60 / 1.29 and 5.16 / 5.33.  What bounds it now: the chain of a sequence, product after
+// product; mma.sync (537 TFLOP/s) is in use for about half of the time.
+//
+// Errors against fp64 in 1e-8 (2-norm, four sequences of 512, token by token / so):
+//                                final state   dq          dk          dbeta       dg
+//   decay 0.25 a token           4.9 / 6.6     11.5 / 11   15 / 11     13 / 14     820 / 310
+//   gates as a model starts      16 / 8.7      17 / 14     20 / 15     18 / 15     190 / 160
+//   decay 0.99 a token           132 / 11      123 / 16    141 / 20    132 / 19    240 / 67
+//   keys that resemble each      15 / 11       16 / 16     19 / 18     13 / 20     270 / 380
+//     other (cosine 0.5)
+// Larger in four places, all in the last bits of fp32: what the tensor cores cut off within a product over 16, which weighs where
+// one token makes up most of the state, or where the parts of a sum cancel.  (K K^T and Q K^T in one accumulator over all of
+// 128, and the exponentials in fp32: dbeta 20, 21, 23 and 27, dg of the last row 480.)
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -153,6 +162,12 @@ __device__ __forceinline__ void prod3(float (&c)[4], const uint32_t (&a)[3][4], 
   mma(d, a[0], b0, b1);
   add4(c, d);
 }
+// both as they are
+__device__ __forceinline__ void prod1(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  float d[4];
+  mma_zero(d, a, b0, b1);
+  add4(c, d);
+}
 // a as it is, b in three terms
 __device__ __forceinline__ void prod3(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[3][2]) {
   float d[4];
@@ -188,21 +203,22 @@ __device__ __forceinline__ uint32_t pack_bf(float x, float y) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// 2^x for a difference of sums: the whole part goes into the exponent, 2^f, |f| <= 1/2, by its series (the term of f^8 is below
-// 6e-9).  The hardware's approximation is off by 2^-22, and rounding x to fp32 first would cost another |x| 2^-25.
+// 2^x for a difference of sums, rounded once: the whole part goes into the exponent, 2^f, |f| <= 1/2, is its series in fp64 (the term
+// of f^9 is below 2e-10).  The hardware's approximation is off by 2^-22, and rounding x to fp32 first would cost another |x| 2^-25.
 __device__ __forceinline__ float exp2_of(double x) {
   if (x < -126.0) return 0.f;
   if (x > 127.0) return x > 128.0 ? __int_as_float(0x7f800000) : exp2f((float)x);
-  const float n = rintf((float)x), f = (float)(x - (double)n);
-  float p = 1.52527338e-5f;                        // ln(2)^k / k!, k = 7 .. 0
-  p = p * f + 1.54035304e-4f;
-  p = p * f + 1.33335581e-3f;
-  p = p * f + 9.61812911e-3f;
-  p = p * f + 5.55041087e-2f;
-  p = p * f + 2.40226507e-1f;
-  p = p * f + 6.93147181e-1f;
-  p = p * f + 1.f;
-  return p * __int_as_float(((int)n + 127) << 23);
+  const double n = rint(x), f = (x - n) * 0.69314718055994531;
+  double p = 1.0 / 40320;                          // 1 / k!, k = 8 .. 0
+  p = p * f + 1.0 / 5040;
+  p = p * f + 1.0 / 720;
+  p = p * f + 1.0 / 120;
+  p = p * f + 1.0 / 24;
+  p = p * f + 1.0 / 6;
+  p = p * f + 0.5;
+  p = p * f + 1.0;
+  p = p * f + 1.0;
+  return (float)p * __int_as_float(((int)n + 127) << 23);
 }
 
 // ---- shared-memory tiles.  (64, 128) bf16 with 256-byte rows: the 16-byte piece c of row r lies at piece c ^ (r & 7).
@@ -305,10 +321,10 @@ __global__ void __launch_bounds__(128, 3) gdn_prep_kernel(const Args a) {
     for (int jb = 0; jb < 4; ++jb)
       if (jb <= warp) {
         ldsm(b, smem_addr(k_s) + tile_rc(jb * 16, kb * 2, lane));
-        mma(kk[2 * jb], ka, b[0], b[1]);
-        mma(kk[2 * jb + 1], ka, b[2], b[3]);
-        mma(qk[2 * jb], qa, b[0], b[1]);
-        mma(qk[2 * jb + 1], qa, b[2], b[3]);
+        prod1(kk[2 * jb], ka, b[0], b[1]);
+        prod1(kk[2 * jb + 1], ka, b[2], b[3]);
+        prod1(qk[2 * jb], qa, b[0], b[1]);
+        prod1(qk[2 * jb + 1], qa, b[2], b[3]);
       }
   }
   const int rep = a.HV / a.HK;
@@ -1062,8 +1078,8 @@ __global__ void __launch_bounds__(NT, 1) gdn_chunk_grad_kernel(const Args a) {
         }
         ldsm(f, (second ? k_s : q_s) + tile_cr(ib * 16, kb * 2, lane));
         ldsm(b, k_s + tile_rc(jb * 16, kb * 2, lane));
-        mma(x[0], f, b[0], b[1]);
-        mma(x[1], f, b[2], b[3]);
+        prod1(x[0], f, b[0], b[1]);
+        prod1(x[1], f, b[2], b[3]);
       }
       char* w = (second ? w2_s : w1_s) + bl * 512;
       float* col = (second ? col2 : col1) + ib * C + jb * 16;

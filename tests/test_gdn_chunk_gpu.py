@@ -144,3 +144,27 @@ def test_rows_off_the_16_byte_grid_take_the_recurrent_kernels():
     odd = buf[1:].view_as(v).copy_(v)
     a, b = la.gdn_fwd(q, k, v, g, beta, _cu(lens))[:2], la.gdn_fwd(q, k, odd, g, beta, _cu(lens))[:2]
     assert _rel(a[0], b[0]) < 2.0 ** -8 and _rel(a[1], b[1]) < 2e-5
+
+
+@pytest.mark.parametrize("gates", ["strong", "model", "slow", "none"])
+def test_precision_is_that_of_fp32(gates):
+    """Errors in units of 2^-24, the rounding of fp32, over sequences of several chunks.  A result goes through some ten roundings
+    (16 allowed; measured 1 to 5); a product that kept two bf16 terms of an fp32 operand, 2^-16 of it cut off, would be off by a
+    hundred.  dg adds up, over all later tokens, differences that cancel to a tenth and less (256 allowed; measured 7 to 60)."""
+    from flextrain_b200.ops import linattn_cuda as la
+    lens, HK, HV = [256, 200, 300], 2, 4
+    T = sum(lens)
+    q, k, v, _, beta, do = _inputs(lens, HK, HV, 1.0)
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    n = torch.randn(T, HV, device=DEV, generator=gen)
+    g = {"strong": -F.softplus(n + 1), "model": -F.softplus(n - 4) * torch.tensor([1.0, 4, 9, 16], device=DEV),
+         "slow": -0.01 * n.abs(), "none": torch.zeros_like(n)}[gates]
+    cu = _cu(lens)
+    o, fin, r = la.gdn_fwd(q, k, v, g, beta, cu, want_r=True)
+    got = la.gdn_bwd(q, k, v, g, beta, cu, None, fin, r, do)
+    leaves = [t.double().requires_grad_(True) for t in (q, k, v, g, beta)]
+    zero = torch.zeros(len(lens), HV, 128, 128, device=DEV, dtype=F64)
+    ow, fw = _recurrence(*leaves, zero, lens, 128 ** -0.5)
+    wq, wk, _, wg, wb = torch.autograd.grad(ow, leaves, do.double())
+    for a, w, units in ((fin, fw, 16), (got[0], wq, 16), (got[1], wk, 16), (got[4], wb, 16), (got[3], wg, 256)):
+        assert _rel(a, w) <= units * 2.0 ** -24
