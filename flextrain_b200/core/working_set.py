@@ -148,15 +148,16 @@ def baseline_model_memory(layers, embed, head, optimizer, probe_tokens: int = 40
     return ModelMemory(lp, lm, lg, lo, eh, af, at, flops, head_flops, [r / max(flops, 1e-9) for r in redo])
 
 
-# Temporaries that no shape below stands for: the fp32 slabs of a GEMM with a cut reduction while a chunk is in flight, and a
-# batch of the Muon iteration during the update, when the chunk's own temporaries are free.
+# Temporaries that no shape below stands for: the fp32 slabs of a GEMM with a cut reduction or the parts of adapters' gradients
+# while a chunk is in flight, and a batch of the Muon iteration during the update, when the chunk's own temporaries are free.
 WORKSPACE_ALLOWANCE = 256 << 20
 
 
 def _workspace_bytes(layers, head, chunk: int, act_bytes: int = 2, head_rows: Optional[int] = None) -> int:
     """Transient GPU memory while one chunk is in flight: residual stream in/out, the widest projection output
-    and its gradient, attention workspace, and one head micro-chunk of logits."""
-    widest = 0
+    and its gradient, attention workspace, what Gated DeltaNet keeps of its chunks, and one head micro-chunk of logits."""
+    from ..ops.linattn_cuda import chunk_work_most
+    widest = lin = 0
     d = 0
     for l in layers:
         c = l.cfg
@@ -168,10 +169,12 @@ def _workspace_bytes(layers, head, chunk: int, act_bytes: int = 2, head_rows: Op
             w = max(w, 3 * c.ffn.ffn_dim)
         if c.moe is not None:
             w = max(w, 3 * c.moe.expert_dim * c.moe.top_k + 3 * c.moe.shared_dim)
+        if getattr(c, "gdn", None) is not None:
+            lin = max(lin, chunk_work_most(chunk, c.gdn.n_v_heads, c.gdn.head_k_dim, c.gdn.head_v_dim))
         widest = max(widest, w)
     per_tok = (4 * d + 2 * widest) * act_bytes
     head_ws = min(chunk, head_rows or head.head_chunk_size) * head.vocab_size * act_bytes * 2
-    return chunk * per_tok + head_ws + WORKSPACE_ALLOWANCE
+    return chunk * per_tok + head_ws + lin + WORKSPACE_ALLOWANCE
 
 
 def determine_working_set_config(*, layers, embed, head, optimizer, max_seq_len: int, max_global_batch_tokens: int,

@@ -417,12 +417,14 @@ int run_all(const DownArgs& d, int nd, const UpArgs& u, int nu, int runs, const 
   return e == cudaSuccess ? 0 : -400 - (int)e;
 }
 
-// Runs of tokens: as many as make (waves of 2 blocks an SM) x (steps of a run, and 4 for its start and its end) least.
-int runs_of(int T, int blocks, int* run) {
+// Runs of tokens: as many as make (waves of 2 blocks an SM) x (steps of a run, and 4 for its start and its end) least, and as keep
+// the parts (one_run bytes each) within the workspace that a plan sets aside.
+constexpr long PART_BYTES = 64L << 20;
+int runs_of(int T, int blocks, long one_run, int* run) {
   long best = 0;
   int runs = 1;
   *run = STEP;
-  for (int n = 1; n <= 32 && (n - 1) * 256 < T; ++n) {
+  for (int n = 1; n <= 32 && (n - 1) * 256 < T && (n == 1 || n * one_run <= PART_BYTES); ++n) {
     const int steps = ((T + n - 1) / n + STEP - 1) / STEP;
     const long cost = (long)((blocks * n + 2 * 148 - 1) / (2 * 148)) * (steps + 4);
     if (n == 1 || cost < best) { best = cost; runs = n; *run = steps * STEP; }
@@ -440,7 +442,7 @@ long ftb_lora_wgrad_bytes(int n, int T, int K, const int* N, int R) {
   int blocks = blocks_of(K), run;
   long columns = (long)n * K;
   for (int i = 0; i < n; ++i) { blocks += blocks_of(N[i]); columns += N[i]; }
-  return 2L * n * ((long)T * R * 2 + 256) + columns * R * 4 * runs_of(T, blocks, &run) + 256;
+  return 2L * n * ((long)T * R * 2 + 256) + columns * R * 4 * runs_of(T, blocks, columns * R * 4, &run) + 256;
 }
 
 // ga_i (R, K) += scale * (dy_i b_i)^T x,  gb_i (N_i, R) += scale * dy_i^T (x a_i^T)  for n <= 3 adapters of one input x (T, K).
@@ -467,8 +469,9 @@ int ftb_lora_wgrad(int n, const void* x, long ldx, int T, int K, const void* con
   FinArgs f = {};
   d.T = u.T = T;
   int blocks = blocks_of(K);
-  for (int i = 0; i < n; ++i) blocks += blocks_of(N[i]);
-  const int runs = runs_of(T, blocks, &u.run);
+  long columns = (long)n * K;
+  for (int i = 0; i < n; ++i) { blocks += blocks_of(N[i]); columns += N[i]; }
+  const int runs = runs_of(T, blocks, columns * R * 4, &u.run);
   bf16 *xa[MAXW], *dyb[MAXW];
   for (int i = 0; i < n; ++i) {
     xa[i] = (bf16*)take((long)T * R * 2);

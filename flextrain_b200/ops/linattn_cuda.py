@@ -165,16 +165,28 @@ def _gdn(pass_, q, k, v, g, beta, cu, state_in, state_out, o, r, d_o, de, dv, db
     _check(rc, f"ftb_gdn(pass {pass_})")
 
 
+CHUNK, CHUNK_SHORTEST = 64, 40
+
+
 def _chunked(S: int, q: torch.Tensor, v: torch.Tensor, *rest: torch.Tensor) -> bool:
     """Heads of 128 x 128 on 16 bytes run in chunks of 64 tokens on the tensor cores (``csrc/gdn_chunk.cu``, with the figures);
     sequences of fewer than 40 tokens on average leave their chunks too empty for that and go token by token."""
-    return (q.shape[2] == 128 and v.shape[2] == 128 and q.shape[0] >= 40 * S
+    return (q.shape[2] == 128 and v.shape[2] == 128 and q.shape[0] >= CHUNK_SHORTEST * S
             and all(t.data_ptr() % 16 == 0 for t in (q, v, *rest)))
 
 
 def _head_rows(x: torch.Tensor) -> bool:
     """``(T, H, D)`` with the heads of a token side by side: a view of a wider projection, or contiguous."""
     return x.stride(2) == 1 and x.stride(1) == x.shape[2] and x.stride(0) % 8 == 0
+
+
+def chunk_work_most(T: int, HV: int, dk: int, dv: int) -> int:
+    """The most that :func:`_chunk_work` and the marks beside it take for T tokens, however they fall into sequences: two
+    triangles of 10 blocks of 16 x 16 and a sum of gates for each chunk and value head (0 for other head sizes)."""
+    if (dk, dv) != (128, 128):
+        return 0
+    S = T // CHUNK_SHORTEST
+    return (T // CHUNK + S) * HV * (2 * 10 * 256 * 4 + CHUNK * 8) + (S + 15) // 16 * 64 + S * HV * 4
 
 
 def _chunk_work(T: int, S: int, HV: int, device) -> torch.Tensor:

@@ -1,5 +1,8 @@
 """The temporaries that the kernels' bindings allocate by themselves stay inside what a plan sets aside for them."""
+import ctypes
+import math
 import random
+import types
 
 import pytest
 
@@ -34,3 +37,41 @@ def test_batches_of_the_muon_iteration(seed):
         nbytes = 2 * nb * (2 * rows * n + 2 * side * side)
         assert nbytes <= (WORKSPACE_ALLOWANCE if nb > 1 else max(WORKSPACE_ALLOWANCE, 8 * rows * n))
         assert nb >= 1
+
+
+@pytest.mark.parametrize("seed", range(3))
+def test_parts_of_adapter_gradients(seed):
+    """Not at once with a GEMM whose reduction is cut: at most half of the allowance, too."""
+    lib = k.load("lora")
+    lib.ftb_lora_wgrad_bytes.restype = ctypes.c_long
+    rng = random.Random(seed)
+    log = lambda lo, hi: int(math.exp(rng.uniform(math.log(lo), math.log(hi + 1))))
+    shapes = [(rng.randint(1, 3), log(1, 131072), 32 * log(1, 1024), rng.choice((8, 16, 32))) for _ in range(3000)]
+    for n, T, K, R in shapes + [(3, 59205, 23360, 32), (3, 131072, 32768, 32)]:
+        N = (ctypes.c_int * n)(*(32 * log(1, 2048) for _ in range(n)))
+        assert 0 < lib.ftb_lora_wgrad_bytes(n, T, K, N, R) <= WORKSPACE_ALLOWANCE // 2
+
+
+@pytest.mark.parametrize("seed", range(3))
+def test_chunks_of_gated_deltanet(seed):
+    """A plan counts them, for as many sequences as the chunked kernels take."""
+    from flextrain_b200.core.working_set import _workspace_bytes
+    from flextrain_b200.ops import linattn_cuda as la
+    lib = k.load("gdn_chunk")
+    lib.ftb_gdn_chunk_bytes.restype = ctypes.c_long
+    rng = random.Random(seed)
+    for _ in range(1000):
+        T, HV = rng.randint(1, 65536), rng.choice((1, 4, 16, 32, 64))
+        S = rng.randint(0, T // 40)
+        took = lib.ftb_gdn_chunk_bytes(ctypes.c_long(T), S, HV) + S * HV * 4
+        assert took <= la.chunk_work_most(T, HV, 128, 128)
+    assert la.chunk_work_most(4096, 8, 64, 128) == 0                              # other heads go token by token
+    with_, without = (_plan_workspace(_workspace_bytes, dim) for dim in (128, 64))
+    assert with_ - without >= lib.ftb_gdn_chunk_bytes(ctypes.c_long(8192), 8192 // 40, 32)
+
+
+def _plan_workspace(workspace_bytes, head_dim):
+    layer = types.SimpleNamespace(cfg=types.SimpleNamespace(
+        d_model=2048, attn=None, moe=None, ffn=types.SimpleNamespace(ffn_dim=6144),
+        gdn=types.SimpleNamespace(n_v_heads=32, head_k_dim=head_dim, head_v_dim=head_dim)))
+    return workspace_bytes([layer], types.SimpleNamespace(head_chunk_size=1024, vocab_size=32000), 8192)
