@@ -1415,13 +1415,20 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParam
   return e == cudaSuccess ? 0 : -400 - static_cast<int>(e);
 }
 
+// Whether a product (in slices of k) takes tiles of 512 x 256: long sums (Ring2), and not a wave more of twice the work.
+static bool wide_tiles(int M, int N, int k, int slices, int pairs) {
+  const int columns = (N + BN2 - 1) / BN2 * slices;
+  const int tiles = (M + 2 * BM - 1) / (2 * BM) * columns, wide = (M + 4 * BM - 1) / (4 * BM) * columns;
+  return k >= WIDE_K && 2 * ((wide + pairs - 1) / pairs) <= (tiles + pairs - 1) / pairs;
+}
+
 // Plain products (and slices of one) on 256 x 256 tiles, or on 512 x 256.
 static int launch2_major(int a_mn, int b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int most, cudaStream_t s) {
   const int slices = p.split_k > 1 ? p.split_k : 1, k = p.split_k > 1 ? p.k_per_split : p.K;
   const int columns = (p.N + BN2 - 1) / BN2 * slices;
   const int tiles = (p.M + 2 * BM - 1) / (2 * BM) * columns, wide = (p.M + 4 * BM - 1) / (4 * BM) * columns;
   const int pairs = most / 2 > 0 ? most / 2 : 1;
-  if (k >= WIDE_K && 2 * ((wide + pairs - 1) / pairs) <= (tiles + pairs - 1) / pairs) {
+  if (wide_tiles(p.M, p.N, k, slices, pairs)) {
     const int grid = 2 * (wide < pairs ? wide : pairs);
     if (!a_mn && !b_mn) return launch2<false, false, 0, 0, 2>(ta, tb, p, grid, s);
     if (!a_mn && b_mn) return launch2<false, true, 0, 0, 2>(ta, tb, p, grid, s);
@@ -1506,6 +1513,8 @@ int ftb_gemm_dies_from_latencies(const float* cycles, int pairs, unsigned char* 
   for (int i = 0; i < pairs; ++i) pair_of[i] = m.pair_of[i];
   return m.first_die;
 }
+// Whether a product cut into `splits` slices of k takes tiles of 512 x 256 on `ctas` SMs.
+int ftb_gemm_wide_tiles(int M, int N, int k, int splits, int ctas) { return wide_tiles(M, N, k, splits, ctas / 2 > 0 ? ctas / 2 : 1); }
 // What was measured of the current device: the numbers of its pairs and how many are on the first die (0: not known yet).
 int ftb_gemm_dies(unsigned char* pair_of, int* pairs, cudaStream_t stream) {
   const DieMap m = measure_dies(stream);
