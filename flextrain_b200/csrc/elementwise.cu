@@ -754,14 +754,14 @@ __device__ __forceinline__ void act_and_grad(float g, int kind, float& a, float&
 
 // Output gate of gated attention.  Bound by memory: one pass each way, 16 bytes a thread.  The heads of a projection lie
 // [query | gate], so the gate is read (copy) and its gradient written (bwd) a head at a time, `ld` and `hs` elements apart.
-// 16384 tokens, 16 heads of 256, us: copy 162 -> 53, out = x * sigmoid(gate) 620 -> 72, all of the backward 1810 -> 135 (chains of fp32
+// 16384 tokens, 16 heads of 256, us: copy 162 -> 53, out = x * sigmoid(gate) 620 -> 83, all of the backward 1810 -> 140 (chains of fp32
 // element-wise passes before).
 // The sigmoid is rounded as a chain of fp32 operations rounds it: e^-x by Cody and Waite's reduction, -x = n ln 2 + r with ln 2 in two
-// parts, and the series of e^r, |r| < 0.35 (the term of r^8 is below 6e-9), then a reciprocal with a step of Newton's; the
+// parts, and the series of e^r, |r| < 0.35 (the term of r^8 is below 6e-9), then a reciprocal rounded to nearest; the
 // hardware's exponential alone is off by |x| 2^-24 and more (9e-5 of the bf16 results for gates up to 80 were not the nearest, 5e-6 so,
-// 2e-5 from the tensor library) and took 59 us where this takes 72, backward 123 and 135.  Past 88 the sigmoid is 0 or 1 in any case.
+// 2e-5 from the tensor library) and took 59 us where this takes 83, backward 123 and 140.  Past 88 the sigmoid is 0 or 1 in any case.
 __device__ __forceinline__ float sigmoid_of(float x) {
-  float y = -x, q;
+  float y = -x;
   asm("min.NaN.f32 %0, %0, %1;" : "+f"(y) : "f"(88.f));
   asm("max.NaN.f32 %0, %0, %1;" : "+f"(y) : "f"(-87.f));
   const float shifted = fmaf(y, 1.44269504f, 12582912.f), n = shifted - 12582912.f;      // 1.5 * 2^23: n in the lowest bits
@@ -775,9 +775,7 @@ __device__ __forceinline__ float sigmoid_of(float x) {
   p = fmaf(p, r, 0.5f);
   p = fmaf(p, r, 1.f);
   p = fmaf(p, r, 1.f);
-  const float d = fmaf(p, __uint_as_float((__float_as_uint(shifted) << 23) + 0x3f800000u), 1.f);
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(d));
-  return fmaf(q, fmaf(-d, q, 1.f), q);
+  return __frcp_rn(fmaf(p, __uint_as_float((__float_as_uint(shifted) << 23) + 0x3f800000u), 1.f));
 }
 
 __global__ void __launch_bounds__(256) copy_heads_kernel(const bf16* __restrict__ x, long ld, long hs, bf16* __restrict__ y, long nvec,
