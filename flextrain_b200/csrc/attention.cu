@@ -1491,14 +1491,14 @@ extern "C" {
 
 // dout / q / out (Tq, H, hd), k / v (Tk, KV, hd) bf16 with token strides; lse (H, Tq) from the forward.
 // Workspaces supplied by the caller: delta (H, Tq) fp32, dq_acc (Tq, H, hd) fp32 ZEROED.
-// Outputs: dq (bf16, converted from dq_acc), dk, dv (Tk, KV, hd) bf16 contiguous, every row written.
+// Outputs: dQ, in fp32 in dq_acc; dk, dv (Tk, KV, hd) bf16 contiguous, every row written.
 // dq_sem: NULL, or 1 + (sum over sequences of ceil(len_q / 128)) x H x 4 int32 words, ZEROED (word 0 is the kernel's
 //   give-up flag, the rest one counter per (query tile, head, 32 rows)): makes the dQ summation order
 // fixed (bit-reproducible gradients) at the price of ordering the CTAs that share a query tile.
 // max_k: the longest sequence's keys (it chooses the order of the work only).
 int ftb_attn_bwd(const void* dout, const void* q, const void* k, const void* v, const void* out, const float* lse,
-                 float* delta, float* dq_acc, int* dq_sem, void* dq, void* dk, void* dv, const int* cu_q, const int* cu_k,
-                 int num_seqs, int total_q, int total_k, int H, int KV, int hd, long q_stride, long k_stride,
+                 float* delta, float* dq_acc, int* dq_sem, void* dk, void* dv, const int* cu_q, const int* cu_k, int num_seqs,
+                 int total_q, int total_k, int H, int KV, int hd, long q_stride, long k_stride,
                  long v_stride, long do_stride, long o_stride, float scale, float softcap, int causal, int window,
                  int max_tiles, int max_k, cudaStream_t stream) {
   if (total_q <= 0 || num_seqs <= 0) return 0;

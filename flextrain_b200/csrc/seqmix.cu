@@ -877,10 +877,6 @@ int ftb_l2norm_rep_bwd(const float* dy, int rep, const void* x, long ldx, const 
                                                                        rows, H, D);
   CHECK_LAUNCH();
 }
-int ftb_l2norm_strided_bwd(const float* dy, const void* x, long ldx, const float* rnorm, void* dx, long lddx, long T,
-                           int H, int D, cudaStream_t s) {
-  return ftb_l2norm_rep_bwd(dy, 1, x, ldx, rnorm, dx, lddx, T, H, D, s);
-}
 
 // z: rows of the heads of a token side by side, tokens ldz elements apart; o, y contiguous.  -2: not rows of these kernels.
 int ftb_gated_rmsnorm_strided_fwd(const void* o, const void* z, long ldz, int H, const float* w, void* y, long T, int D, float eps,

@@ -67,7 +67,7 @@ def bwd(dout, q, k, v, out, lse, cu_q, cu_k, max_q, max_k, *, scale, causal=True
     det = deterministic_default() if deterministic is None else bool(deterministic)
     sem = torch.zeros(1 + (Tq // 128 + nseq) * H * 4, dtype=torch.int32, device=q.device) if det else None
     rc = lib.ftb_attn_bwd(_ptr(dout), _ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(lse), _ptr(delta), _ptr(dq_acc),
-                          _ptr(sem), None, _ptr(dk), _ptr(dv), _ptr(cu_q), _ptr(cu_k), c_int(nseq), c_int(Tq), c_int(Tk),
+                          _ptr(sem), _ptr(dk), _ptr(dv), _ptr(cu_q), _ptr(cu_k), c_int(nseq), c_int(Tq), c_int(Tk),
                           c_int(H), c_int(KV), c_int(hd), c_long(q.stride(0)), c_long(k.stride(0)),
                           c_long(v.stride(0)), c_long(dout.stride(0)), c_long(out.stride(0)), c_float(scale),
                           c_float(float(softcap or 0.0)), c_int(1 if causal else 0), c_int(int(window or 0)),

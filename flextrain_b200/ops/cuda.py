@@ -288,7 +288,7 @@ def rmsnorm_heads_bwd(dy, x, w, rstd, dx, dw_out):
 
 def _heads_16(*heads) -> bool:
     return all(t.dim() == 3 and t.stride(2) == 1 and t.shape[2] % 8 == 0 and t.stride(1) % 8 == 0 and t.stride(0) % 8 == 0
-               and t.stride(1) >= t.shape[2]               and t.data_ptr() % 16 == 0 for t in heads)
+               and t.stride(1) >= t.shape[2] and t.data_ptr() % 16 == 0 for t in heads)
 
 
 def attn_gate_supported(heads, *flat) -> bool:
