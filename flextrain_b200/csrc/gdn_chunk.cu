@@ -28,20 +28,20 @@
 // the state goes through shared memory once a chunk, and a warp owns tokens.
 //
 // Measured, ms, token by token (gdn.cu) / so, 32 heads: 16 x 1024 tokens forward 2.19 / 1.05, backward 7.98 / 4.22; one sequence
-// of 16384 7.5 / 3.3 and 25.4 / 15.1; two of 8192 4.6 / 1.8 and 15.1 / 7.8; 512 tokens 0.22 / 0.13 and 0.81 / 0.51; 300 sequences of
+// of 16384 7.5 / 3.3 and 25.4 / 15.0; two of 8192 4.6 / 1.8 and 15.1 / 7.8; 512 tokens 0.22 / 0.13 and 0.81 / 0.51; 300 sequences of
 // 33, mostly half-empty chunks, 1.60 / 1.29 and 5.16 / 5.33.  What bounds it now: the chain of a sequence, product after
 // product; mma.sync (537 TFLOP/s) is in use for about half of the time.
 //
-// Errors against fp64 in 1e-8 (2-norm, four sequences of 512, token by token / so):
+// Errors against fp64 in 1e-8 (2-norm, four sequences of 512, mean of three seeds, token by token / so):
 //                                final state   dq          dk          dbeta       dg
-//   decay 0.25 a token           4.9 / 6.6     11.5 / 11   15 / 11     13 / 14     820 / 310
-//   gates as a model starts      16 / 8.7      17 / 14     20 / 15     18 / 15     190 / 160
-//   decay 0.99 a token           132 / 11      123 / 16    141 / 20    132 / 19    240 / 67
-//   keys that resemble each      15 / 11       16 / 16     19 / 18     13 / 20     270 / 380
+//   decay 0.25 a token           4.4 / 6.6     11.2 / 10.7 15.1 / 10.8 12.5 / 13.6 1003 / 400
+//   gates as a model starts      37.7 / 9.6    44 / 14.9   49 / 16.9   45 / 16.0   156 / 118
+//   decay 0.99 a token           336 / 10.9    305 / 16.3  349 / 20.2  321 / 18.7  513 / 75
+//   keys that resemble each      36.5 / 15.7   42.5 / 19.1 49 / 19.3   45.5 / 28.1 154 / 153
 //     other (cosine 0.5)
-// Larger in four places, all in the last bits of fp32: what the tensor cores cut off within a product over 16, which weighs where
-// one token makes up most of the state, or where the parts of a sum cancel.  (K K^T and Q K^T in one accumulator over all of
-// 128, and the exponentials in fp32: dbeta 20, 21, 23 and 27, dg of the last row 480.)
+// Larger in two places, by a unit in the last place of fp32, where a state forgets three quarters of itself at each token.  (K K^T and
+// Q K^T in one accumulator over all of 128, and the exponentials in fp32: a quarter more in dbeta.  The largest terms of every product
+// in an accumulator of their own: those two figures 6.6 and 13.0, the others a tenth less, for 1.29 and 4.80 ms in place of 1.10 and 4.23.)
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
