@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_bwd_kernel(const bf16* __r
 // us, block per row / so, forward: 16384 x 768 22.7 / 9.9, 9377 x 1024 14.6 / 8.2, 16384 x 2048 28.7 / 25.4; backward with its sum
 // of dw: 58.6 / 28.6, 37.9 / 22.6, 79.3 / 66.5, 8192 x 1152 36.6 / 24.7, 16384 x 3072 98.2 / 89.3.
 template <int NV>
-__global__ void __launch_bounds__(RN_THREADS, 3) rmsnorm_warp_fwd_kernel(const bf16* __restrict__ x, const float* __restrict__ w,
+__global__ void __launch_bounds__(RN_THREADS) rmsnorm_warp_fwd_kernel(const bf16* __restrict__ x, const float* __restrict__ w,
                                                                       bf16* __restrict__ y, float* __restrict__ rstd_out, int T,
                                                                       int D, float eps, long ldx) {
   const int lane = threadIdx.x & 31, nv = D >> 3, step = gridDim.x * (RN_THREADS / 32);
@@ -250,14 +250,13 @@ __global__ void __launch_bounds__(RN_THREADS, 3) rmsnorm_warp_fwd_kernel(const b
       const int i = lane + j * 32;
       v[j] = i < nv ? xr[i] : make_uint4(0, 0, 0, 0);
     }
-    float ss = 0.f;                              // (a piece by itself first: beside an element that outweighs its row, a sum
-#pragma unroll                                   // over all of a lane's elements would lose the others one by one)
+    float ss = 0.f;
+#pragma unroll
     for (int j = 0; j < NV; ++j) {
-      float f[8], s8 = 0.f;
+      float f[8];
       unpack8(v[j], f);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) s8 += f[e] * f[e];
-      ss += s8;
+      for (int e = 0; e < 8; ++e) ss += f[e] * f[e];
     }
     const float r = rsqrtf(warp_sum(ss) / (float)D + eps);
     if (lane == 0 && rstd_out) rstd_out[row] = r;
@@ -332,7 +331,7 @@ __global__ void __launch_bounds__(RN_THREADS, 2) rmsnorm_warp_bwd_kernel(const b
     for (int j = 0; j < NV; ++j) {
       const int i = lane + j * LANES;
       if (i < nv) {
-        float xf[8], gf[8], wf[8], d8 = 0.f;
+        float xf[8], gf[8], wf[8];
         unpack8(xv[j], xf);
         unpack8(gv[j], gf);
         gain(i, wf);
@@ -340,9 +339,8 @@ __global__ void __launch_bounds__(RN_THREADS, 2) rmsnorm_warp_bwd_kernel(const b
         for (int e = 0; e < 8; ++e) {
           const float xh = xf[e] * r;
           dwacc[j][e] += gf[e] * xh;
-          d8 += gf[e] * wf[e] * xh;
+          dot += gf[e] * wf[e] * xh;
         }
-        dot += d8;
       }
     }
     dot = warp_sum(dot);
